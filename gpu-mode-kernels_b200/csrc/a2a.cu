@@ -11,6 +11,7 @@
 #include "a2a.h"
 #include "a2a_kernels.cuh"
 #include "a2a_pipe.cuh"
+#include "a2a_solo.cuh"
 
 using namespace a2a;
 
@@ -18,7 +19,7 @@ namespace {
 
 constexpr int kTraceBlocks = 2048;  // blocks the in-kernel trace buffer has room for
 constexpr size_t kMaxSmemBytes = 200 * 1024;  // routing bitmap budget per block (227 KB is the sm_100 limit)
-constexpr size_t kMaxPipeSmemBytes = 100 * 1024;  // pipelined kernels: two blocks per SM must fit
+constexpr size_t kMaxPipeSmemBytes = 100 * 1024;  // pipelined kernel of several ranks: two blocks per SM must fit
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -202,10 +203,12 @@ int validate(const a2a_config& c) {
         // FP8: a warp assembles a whole wire row in its own stage of the sender ring
         if (c.payload == A2A_PAYLOAD_FP8 && make_layout(c).stage_row_bytes > kWarpStageBytes) return A2A_ERR_CONFIG;
         if (c.chunks > 1) return A2A_ERR_CONFIG;
+        // one rank has no senders and routes inside its one kernel; only its stepped roles need the tables
+        const size_t room = c.world_size == 1 ? kMaxSmemBytes : kMaxPipeSmemBytes;
         const int senders = pipe_senders(c);
         if (c.world_size > 1 && senders < 2) return A2A_ERR_CONFIG;  // blocks 0 and 1 carry the watchers
-        if (pipe_sender_smem(c.max_num_tokens, c.world_size, senders) > kMaxPipeSmemBytes ||
-            pipe_router_smem(c.max_num_tokens, c.num_experts / c.world_size) > kMaxPipeSmemBytes)
+        if ((c.world_size > 1 && pipe_sender_smem(c.max_num_tokens, c.world_size, senders) > room) ||
+            pipe_router_smem(c.max_num_tokens, c.num_experts / c.world_size) > room)
             return A2A_ERR_CONFIG;
     }
     return A2A_OK;
@@ -276,6 +279,15 @@ KernelFn pipe_fn(const a2a_ctx* c, int role) {
     return c->cfg.dtype == A2A_DTYPE_BF16 ? pipe_fn_t<__nv_bfloat16>(c, role) : pipe_fn_t<__half>(c, role);
 }
 
+// the one launch of a pipelined context of world size 1
+template <int U>
+KernelFn solo_fn(const a2a_ctx* c) {
+    const bool bf = c->cfg.dtype == A2A_DTYPE_BF16;
+    if (c->cfg.payload == A2A_PAYLOAD_FP8)
+        return bf ? solo_kernel<__nv_bfloat16, A2A_PAYLOAD_FP8, U> : solo_kernel<__half, A2A_PAYLOAD_FP8, U>;
+    return bf ? solo_kernel<__nv_bfloat16, A2A_PAYLOAD_DEDUP, U> : solo_kernel<__half, A2A_PAYLOAD_DEDUP, U>;
+}
+
 KernelFn combine_fn(const a2a_ctx* c) {
     return c->cfg.dtype == A2A_DTYPE_BF16 ? (KernelFn)combine_kernel<__nv_bfloat16> : (KernelFn)combine_kernel<__half>;
 }
@@ -291,6 +303,22 @@ int launch(a2a_ctx* c, KernelFn fn, int grid, int smem, cudaStream_t st, bool co
     c->launches++;
     if (e != cudaSuccess) return -(int)e;
     return A2A_OK;
+}
+
+// The forward of one rank.  A warp's item is one or two 16-byte vectors per lane of a token's row: two
+// where that still gives every warp of two blocks per SM an item (headline workload, 256 tokens of 7168:
+// 9.4 us against 9.7 with one and 10.2 with four; 2048 tokens 61.0 / 62.1 / 61.5), one below that, where
+// more warps with less to do each finish sooner (one token of 2048: 4.1 against 4.2 and 4.6 us).  Two
+// blocks per SM: with a third or fourth that does not fit beside them a second, nearly empty wave of
+// blocks starts after the first (headline 13.2 us).
+int launch_solo(a2a_ctx* c, cudaStream_t st) {
+    const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = 2LL * c->num_sms;
+    const long long two = c->cur_tokens * ((nvec + 63) / 64), one = c->cur_tokens * ((nvec + 31) / 32);
+    const bool wide = two >= cap * warps;
+    long long blocks = ((wide ? two : one) + warps - 1) / warps;
+    if (blocks > cap) blocks = cap;
+    if (blocks < 1) blocks = 1;
+    return launch(c, wide ? solo_fn<2>(c) : solo_fn<1>(c), (int)blocks, 0, st);
 }
 
 int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
@@ -492,21 +520,22 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, cfg->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, cfg->device);
     if (pipelined) {
-        const size_t a = pipe_sender_smem(T, cfg->world_size, p.senders), b = pipe_router_smem(T, L);
+        const size_t a = cfg->world_size > 1 ? pipe_sender_smem(T, cfg->world_size, p.senders) : 0, b = pipe_router_smem(T, L);
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
         for (int role = -1; role <= 2 && e == cudaSuccess; ++role)
-            e = cudaFuncSetAttribute((const void*)pipe_fn(c, role), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kMaxPipeSmemBytes);
-        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute((const void*)pipe_fn(c, role), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
+        if (e == cudaSuccess && cfg->world_size == 1) {
+            c->forward_grid = c->num_sms;
+            c->fused = true;  // the solo kernel: no block waits for another
+        } else if (e == cudaSuccess) {
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)pipe_fn(c, -1), kThreads, c->pipe_smem);
-        if (e == cudaSuccess) {
             if (occ > 2) occ = 2;
             c->forward_grid = c->num_sms * occ;
             c->fused = true;
             // the one launch needs every block resident and room for the roles: senders, one router per
             // destination, and at least as many expert blocks again
-            const int watchers = (cfg->payload == A2A_PAYLOAD_FP8 && cfg->world_size > 1) ? 2 : 0;
-            if (coop == 0 || c->forward_grid < watchers + p.senders + 2 * cfg->world_size * p.routers) {
+            const int watchers = cfg->payload == A2A_PAYLOAD_FP8 ? 2 : 0;
+            if (e == cudaSuccess && (coop == 0 || c->forward_grid < watchers + p.senders + 2 * cfg->world_size * p.routers)) {
                 a2a_destroy(c);
                 return A2A_ERR_CONFIG;
             }
@@ -668,7 +697,9 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
         c->p.x = x;
         c->p.w = w;
         c->p.y = y;
-        r = launch(c, pipe_fn(c, -1), c->forward_grid, c->pipe_smem, st, /*cooperative=*/true);
+        r = c->cfg.world_size == 1
+            ? launch_solo(c, st)
+            : launch(c, pipe_fn(c, -1), c->forward_grid, c->pipe_smem, st, /*cooperative=*/true);
         if (r == A2A_OK) c->sent = true;
         return r;
     }

@@ -541,6 +541,30 @@ __device__ __forceinline__ void router_role(const DevParams& p, uint8_t* smem, i
     if (tid == 0) arrive_dest(p, d, expected);
 }
 
+// A vector of a row of this rank as it would look after crossing the wire in e4m3: the 16 lanes of a
+// 128-value block quantise it with its scale and dequantise it again.  All 32 lanes call it; a lane
+// without a vector (`valid` false) only takes part in the shuffles.
+template <typename T>
+__device__ __forceinline__ uint4 fp8_round_trip(const uint4& q, bool valid) {
+    float f[8];
+    float amax = 0.f;
+    if (valid) {
+        unpack8<T>(q, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
+    }
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (!valid) return q;
+    const float sc = amax > 0.f ? amax / 448.f : 1.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = f[i] / sc;
+    unpack8_e4m3(pack8_e4m3(f), f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] *= sc;
+    return pack8<T>(f);
+}
+
 // One 128-vector (2 KB) chunk of a wire row as four 16-byte vectors of T per lane.
 // Own rows are read from x (FP8: through the same quantise / dequantise arithmetic the wire applies).
 template <typename T, int PAYLOAD>
@@ -558,23 +582,9 @@ __device__ __forceinline__ void load_wire_chunk(const DevParams& p, bool own, co
             const int v = v0 + u * 32 + lane;
             float f[8];
             if (own) {  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
-                float amax = 0.f;
-                if (v < nvec) {
-                    unpack8<T>(ld_input(reinterpret_cast<const uint4*>(src) + v), f);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-                }
-#pragma unroll
-                for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                if (v < nvec) {
-                    const float sc = amax > 0.f ? amax / 448.f : 1.f;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) f[i] = f[i] / sc;
-                    unpack8_e4m3(pack8_e4m3(f), f);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) f[i] *= sc;
-                    q[u] = pack8<T>(f);
-                }
+                uint4 own_q = make_uint4(0u, 0u, 0u, 0u);
+                if (v < nvec) own_q = ld_input(reinterpret_cast<const uint4*>(src) + v);
+                q[u] = fp8_round_trip<T>(own_q, v < nvec);
             } else if (v < nvec) {
                 unpack8_e4m3(ld_stream(reinterpret_cast<const uint2*>(src) + v), f);
                 const float sc = ld_stream(reinterpret_cast<const float*>(src + p.H) + (v >> 4));

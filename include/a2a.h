@@ -53,7 +53,8 @@ enum {
     A2A_SCHEDULE_PHASED = 0,    /* routing, sending, expert pass and combine one after the other      */
     A2A_SCHEDULE_PIPELINED = 1  /* blocks with fixed roles (senders driving the copy engine, routers,
                                    experts, watchers) run the phases concurrently, per peer; needs the
-                                   DEDUP or FP8 payload and a device with cooperative launch         */
+                                   DEDUP or FP8 payload and a device with cooperative launch.  With one
+                                   rank: blocks that each take a share of the tokens all the way       */
 };
 
 /* How expert outputs get back to the token's rank. */

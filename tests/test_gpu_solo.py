@@ -1,0 +1,106 @@
+"""The one-launch kernel of world size 1 where its split can go wrong: rows that end inside a warp's
+item, one token, more tokens per block than it resolves at a time, K beyond one vector of indices,
+token counts whose stepped roles need more than half an SM's shared memory.
+
+Dispatch is held bit for bit against the CPU checker; outputs against the same sums in 64 bits within
+the roundings the kernel makes, and bit for bit against the stepped roles, which are other kernels.
+"""
+import pytest
+import torch
+
+import gpu_mode_kernels_b200 as pkg
+from gpu_mode_kernels_b200 import _lib
+from gpu_mode_kernels_b200.all2all import A2AContext
+from gpu_mode_kernels_b200.local_world import LocalWorld
+from oracle import a2a_oracle as O
+from parity import fp8_roundtrip
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def bits(t):
+    return t.contiguous().view(torch.int16)
+
+
+@pytest.mark.parametrize("E,K,H,T,n,dtype,payload", [
+    (8, 1, 8, 1, 1, torch.bfloat16, "dedup"),         # a row of one vector
+    (6, 3, 520, 33, 20, torch.float16, "dedup"),      # 65 vectors: one past two lanes' worth
+    (64, 6, 2048, 4, 0, torch.float16, "dedup"),      # no tokens
+    (1024, 32, 128, 40, 40, torch.bfloat16, "dedup"), # limits of E and K
+    (8, 2, 72, 6000, 5003, torch.bfloat16, "dedup"),  # 17 tokens per block: a second round for some blocks
+    (256, 8, 7168, 256, 255, torch.bfloat16, "dedup"),
+    (256, 8, 64, 2048, 2048, torch.float16, "dedup"), # stepped roles: 133 KB of routing tables
+    (6, 3, 640, 33, 33, torch.float16, "fp8"),
+    (32, 4, 7168, 200, 199, torch.bfloat16, "fp8"),
+])
+def test_forward_against_the_checker_and_the_stepped_roles(E, K, H, T, n, dtype, payload):
+    cfg, rd, _, _ = pkg.generate_input(E, K, H, T, seed=11, rank=0, world_size=1, dtype=dtype, weights="rand")
+    rd.num_tokens = n
+    rd.x, rd.indices, rd.weights = rd.x[:n], rd.indices[:n], rd.weights[:n]
+    disp, _ = O.simulate(cfg, 1, [rd])
+    ctx = A2AContext(cfg, 0, 1, device=0, payload=payload, schedule="pipelined", combine="push")
+    world = LocalWorld(cfg, 1, payload=payload, schedule="pipelined", combine="push")
+    try:
+        d = rd.to(DEV)
+        before = ctx.launches
+        y = ctx.forward(d.x, d.indices, d.weights)
+        assert ctx.launches == before + 1
+        slots, sent = ctx.route_tables()
+        counts, rows, meta = ctx.export_dispatch()
+        torch.cuda.synchronize()
+        ctx.check()
+        want_slots, want_sent = O.route_tables(rd.indices, E)
+        assert torch.equal(slots.cpu(), want_slots) and torch.equal(sent.cpu(), want_sent)
+        assert torch.equal(counts.cpu(), disp[0].expert_num_tokens)
+        held = counts.cpu().tolist()
+        got = torch.cat([rows[e, :h] for e, h in enumerate(held)], 0).cpu()
+        assert torch.equal(torch.cat([meta[e, :h] for e, h in enumerate(held)], 0).cpu(), disp[0].meta)
+        want = disp[0].rows
+        if payload == "fp8":
+            want = fp8_roundtrip(want, dtype)
+        assert torch.equal(bits(got), bits(want))  # rank 0: the placeholder op multiplies by one
+        # K fp32 multiply-adds (each within 2^-24 of the terms' magnitudes), then one rounding to the element
+        # type (half an ulp: a bf16 significand has 8 bits, so 2^-8 of the result; fp16 11 bits, 2^-11; 2^-25 where fp16 is subnormal)
+        x = (fp8_roundtrip(rd.x, dtype) if payload == "fp8" and n else rd.x).double()
+        w = rd.weights.double()
+        exact, terms = x * w.sum(1, keepdim=True), x.abs() * w.sum(1, keepdim=True)
+        bound = exact.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) + 2.0 ** -25 + (K + 1) * 2.0 ** -24 * terms
+        assert bool(((y.cpu().double() - exact).abs() <= bound).all())
+        ref = world.forward_pipelined([d])[0]
+        torch.cuda.synchronize()
+        world.check()
+        assert torch.equal(bits(ref), bits(y))
+    finally:
+        ctx.close()
+        world.close()
+
+
+def test_dropped_pairs_match_the_stepped_roles_and_phases_can_follow():
+    """Indices out of range and repeated, the repeats also across the eight indices the kernel loads
+    together and in tokens before the reading block's own; then a combine called on its own, which
+    must find the flags of the forward up."""
+    E, K, H, T = 16, 11, 2048, 300
+    cfg, rd, _, _ = pkg.generate_input(E, K, H, T, seed=12, rank=0, world_size=1, weights="rand")
+    rd.indices[3, 9] = rd.indices[3, 1]
+    rd.indices[3, 2] = rd.indices[3, 1]
+    rd.indices[150, 10] = rd.indices[150, 8]
+    rd.indices[299] = -1
+    rd.indices[20, 0] = E
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push", timeout_ms=500)
+    world = LocalWorld(cfg, 1, payload="dedup", schedule="pipelined", combine="push")
+    try:
+        d = rd.to(DEV)
+        y = ctx.forward(d.x, d.indices, d.weights)
+        ref = world.forward_pipelined([d])[0]
+        tables, want = ctx.route_tables(), world.ctxs[0].route_tables()
+        again = torch.empty_like(y)
+        _lib.check(ctx.lib.a2a_combine(ctx._h, d.weights.data_ptr(), again.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert ctx.peek() == _lib.A2A_ERR_ROUTING and world.ctxs[0].peek() == _lib.A2A_ERR_ROUTING
+        assert all(torch.equal(a, b) for a, b in zip(tables, want))
+        assert torch.equal(bits(ref), bits(y)) and torch.equal(bits(again), bits(y))
+        assert not y[299].any()
+    finally:
+        ctx.close()
+        world.close()
