@@ -83,6 +83,23 @@ def test_ragged_sizes_and_unaligned_starts(size, offset):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("size", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1, 148 * 512 * 16 + 5, (1 << 25) - 1, 1 << 25, (1 << 25) + 31])
+@pytest.mark.parametrize("offset,frequent", [(0, 0.0), (9, 0.9)])
+def test_either_side_of_the_launch_rules(size, offset, frequent):
+    """One cluster / two launches, one block / three blocks per SM, one vector more than a grid holds; twice
+    into the same output, the second time on other data."""
+    g = torch.Generator().manual_seed(size + offset)
+    out = torch.full((256,), 3, dtype=torch.int64, device="cuda:0")
+    from gpu_mode_kernels_b200.histogram import histogram256
+
+    for value in (0, 255):
+        base = torch.randint(0, 256, (size + offset,), dtype=torch.uint8, generator=g)
+        base[torch.rand(base.numel(), generator=g) < frequent] = value
+        histogram256(base.to("cuda:0")[offset:], out)
+        assert torch.equal(out.cpu(), HO.ref_histogram(base[offset:]))
+
+
+@pytest.mark.gpu
 def test_degenerate_inputs_and_two_calls_in_a_row():
     same = torch.full((1 << 22,), 200, dtype=torch.uint8)
     h = _run(same.to("cuda:0"))
