@@ -17,6 +17,8 @@ DTYPE_BF16, DTYPE_FP16 = 0, 1
 PAYLOAD = {"direct": 0, "dedup": 1, "fp8": 2}
 SCHEDULE = {"phased": 0, "pipelined": 1}
 COMBINE = {"pull": 0, "push": 1}
+GROUP_PHASE = {"pipe_send": 0, "pipe_expert": 1, "pipe_combine": 2, "send": 3, "recv": 4, "expert": 5, "recv_expert": 6,
+               "combine": 7}
 MAX_WORLD, MAX_EXPERTS, MAX_TOPK = 8, 1024, 32
 
 
@@ -29,6 +31,12 @@ class Config(C.Structure):
 class Status(C.Structure):
     _fields_ = [("code", C.c_int32), ("rank", C.c_int32), ("peer", C.c_int32), ("phase", C.c_int32),
                 ("epoch", C.c_uint32), ("detail", C.c_int32)]
+
+
+class Call(C.Structure):
+    """One rank's tensors in a call on a whole group."""
+    _fields_ = [("x", C.c_void_p), ("topk_idx", C.c_void_p), ("topk_weights", C.c_void_p), ("y", C.c_void_p),
+                ("num_tokens", C.c_int32)]
 
 
 class A2AError(RuntimeError):
@@ -50,6 +58,7 @@ SIGNATURES = {
     "a2a_fingerprint": (_I, [C.POINTER(Config), _VP]),
     "a2a_check_handles": (_I, [C.POINTER(Config), _VP, C.c_size_t, C.c_char_p, C.c_size_t]),
     "a2a_pipe_step": (_I, [_VP, _I, _VP, _VP, _VP, _VP, _I, _VP]),
+    "a2a_group_step": (_I, [C.POINTER(_VP), _I, C.POINTER(Call), _VP]),
     "a2a_attach_local_peers": (_I, [_VP, C.POINTER(_VP)]),
     "a2a_route": (_I, [_VP, _VP, _I, _VP]),
     "a2a_dispatch_send": (_I, [_VP, _VP, _VP]),

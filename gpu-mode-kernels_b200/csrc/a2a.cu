@@ -247,36 +247,35 @@ auto select_tp(const a2a_ctx* c, A... a) {
 }
 
 using KernelFn = void (*)(DevParams);
-template <typename T, int P> struct SendSel { static KernelFn get() { return send_kernel<T, P>; } };
+using GroupFn = void (*)(GroupParams);
+template <typename T, int P> struct SendSel { static GroupFn get() { return send_kernel<T, P>; } };
 template <typename T, int P> struct ForwardSel { static KernelFn get() { return forward_kernel<T, P>; } };
 template <typename T, int P> struct ExpertSel {
     // the receive-side launches of the public phases
-    static KernelFn get(bool wait, bool fanout, bool scale, bool publish) {
+    static GroupFn get(bool wait, bool fanout, bool scale, bool publish) {
         if (wait && fanout && scale && publish) return expert_kernel<T, P, true, true, true, true>;      // recv + expert fused
         if (wait && fanout && !scale && !publish) return expert_kernel<T, P, true, true, false, false>;  // dispatch_recv
         if (!wait && !fanout && scale && publish) return expert_kernel<T, P, false, false, true, true>;  // expert_placeholder
         return expert_kernel<T, P, false, false, false, true>;                                           // expert_done
     }
 };
-// pipelined schedule: (element type, payload, push/pull) -> kernel; role -1 = the one-launch kernel
-template <typename T, int P, bool PUSH>
-KernelFn pipe_fn_tp(int role) {
-    switch (role) {
-        case 0: return pipe_role_kernel<T, P, PUSH, 0>;
-        case 1: return pipe_role_kernel<T, P, PUSH, 1>;
-        case 2: return pipe_role_kernel<T, P, PUSH, 2>;
-        default: return pipe_forward_kernel<T, P, PUSH>;
+// pipelined schedule: (element type, payload, push/pull) -> kernel
+template <typename T, int P, bool PUSH> struct PipeForward { static KernelFn get() { return pipe_forward_kernel<T, P, PUSH>; } };
+template <typename T, int P, bool PUSH> struct PipeRole {
+    static GroupFn get(int role) {
+        return role == 0 ? pipe_role_kernel<T, P, PUSH, 0> : role == 1 ? pipe_role_kernel<T, P, PUSH, 1> : pipe_role_kernel<T, P, PUSH, 2>;
     }
-}
-template <typename T>
-KernelFn pipe_fn_t(const a2a_ctx* c, int role) {
+};
+template <template <typename, int, bool> class F, typename T, typename... A>
+auto select_pipe_t(const a2a_ctx* c, A... a) {
     const bool push = c->cfg.combine == A2A_COMBINE_PUSH;
     if (c->cfg.payload == A2A_PAYLOAD_FP8)
-        return push ? pipe_fn_tp<T, A2A_PAYLOAD_FP8, true>(role) : pipe_fn_tp<T, A2A_PAYLOAD_FP8, false>(role);
-    return push ? pipe_fn_tp<T, A2A_PAYLOAD_DEDUP, true>(role) : pipe_fn_tp<T, A2A_PAYLOAD_DEDUP, false>(role);
+        return push ? F<T, A2A_PAYLOAD_FP8, true>::get(a...) : F<T, A2A_PAYLOAD_FP8, false>::get(a...);
+    return push ? F<T, A2A_PAYLOAD_DEDUP, true>::get(a...) : F<T, A2A_PAYLOAD_DEDUP, false>::get(a...);
 }
-KernelFn pipe_fn(const a2a_ctx* c, int role) {
-    return c->cfg.dtype == A2A_DTYPE_BF16 ? pipe_fn_t<__nv_bfloat16>(c, role) : pipe_fn_t<__half>(c, role);
+template <template <typename, int, bool> class F, typename... A>
+auto select_pipe(const a2a_ctx* c, A... a) {
+    return c->cfg.dtype == A2A_DTYPE_BF16 ? select_pipe_t<F, __nv_bfloat16>(c, a...) : select_pipe_t<F, __half>(c, a...);
 }
 
 // the one launch of a pipelined context of world size 1
@@ -288,8 +287,8 @@ KernelFn solo_fn(const a2a_ctx* c) {
     return bf ? solo_kernel<__nv_bfloat16, A2A_PAYLOAD_DEDUP, U> : solo_kernel<__half, A2A_PAYLOAD_DEDUP, U>;
 }
 
-KernelFn combine_fn(const a2a_ctx* c) {
-    return c->cfg.dtype == A2A_DTYPE_BF16 ? (KernelFn)combine_kernel<__nv_bfloat16> : (KernelFn)combine_kernel<__half>;
+GroupFn combine_fn(const a2a_ctx* c) {
+    return c->cfg.dtype == A2A_DTYPE_BF16 ? (GroupFn)combine_kernel<__nv_bfloat16> : (GroupFn)combine_kernel<__half>;
 }
 
 int launch(a2a_ctx* c, KernelFn fn, int grid, int smem, cudaStream_t st, bool cooperative = false) {
@@ -303,6 +302,40 @@ int launch(a2a_ctx* c, KernelFn fn, int grid, int smem, cudaStream_t st, bool co
     c->launches++;
     if (e != cudaSuccess) return -(int)e;
     return A2A_OK;
+}
+
+// One phase of the `n` contexts in cs[] as one launch of `blocks` blocks for each; `adjust` may set what
+// this launch's blocks agree on (senders, routers).  A trace has a slot per block of the grid, so contexts
+// that are being traced are launched one by one.
+template <typename Adjust>
+int launch_ranks(a2a_ctx* const* cs, int n, GroupFn fn, int blocks, int smem, cudaStream_t st, Adjust adjust) {
+    bool traced = false;
+    for (int r = 0; r < n; ++r) traced |= cs[r]->p.trace != nullptr;
+    if (traced && n > 1) {
+        for (int r = 0; r < n; ++r) {
+            const int rc = launch_ranks(cs + r, 1, fn, blocks, smem, st, adjust);
+            if (rc != A2A_OK) return rc;
+        }
+        return A2A_OK;
+    }
+    GroupParams g;
+    for (int r = 0; r < n; ++r) {
+        g.p[r] = call_params(cs[r]);
+        adjust(g.p[r]);
+        cs[r]->launches++;
+    }
+    g.n = n;
+    if (traced) {
+        if (blocks > kTraceBlocks) g.p[0].trace = nullptr;
+        else cs[0]->last_grid = blocks;
+    }
+    void* args[] = {&g};
+    const cudaError_t e = cudaLaunchKernel((const void*)fn, dim3(n * blocks), dim3(kThreads), args, smem, st);
+    return e == cudaSuccess ? A2A_OK : -(int)e;
+}
+
+int launch_ranks(a2a_ctx* const* cs, int n, GroupFn fn, int blocks, int smem, cudaStream_t st) {
+    return launch_ranks(cs, n, fn, blocks, smem, st, [](DevParams&) {});
 }
 
 // The forward of one rank.  A warp's item is one or two 16-byte vectors per lane of a token's row: two
@@ -321,10 +354,16 @@ int launch_solo(a2a_ctx* c, cudaStream_t st) {
     return launch(c, wide ? solo_fn<2>(c) : solo_fn<1>(c), (int)blocks, 0, st);
 }
 
-int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
+int check_call(const a2a_ctx* c, const int32_t* idx, int T) {
     if (!c->peers_ready) return A2A_ERR_STATE;
     if (T < 0 || T > c->cfg.max_num_tokens || (T > 0 && idx == nullptr)) return A2A_ERR_CONFIG;
     if (reinterpret_cast<uintptr_t>(idx) % 4 != 0) return A2A_ERR_CONFIG;
+    return A2A_OK;
+}
+
+int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
+    const int rc = check_call(c, idx, T);
+    if (rc != A2A_OK) return rc;
     c->epoch++;
     c->cur_tokens = T;
     c->p.idx = idx;
@@ -339,40 +378,137 @@ int do_route(a2a_ctx* c, const int32_t* idx, int T, cudaStream_t st) {
     return launch(c, route_kernel, 1, c->smem_bytes, st);
 }
 
-int do_send(a2a_ctx* c, const void* x, cudaStream_t st) {
-    if (!c->routed || c->sent) return A2A_ERR_STATE;
-    if (c->cur_tokens > 0 && x == nullptr) return A2A_ERR_CONFIG;
-    if (!rows_aligned(x)) return A2A_ERR_CONFIG;
-    c->p.x = x;
-    const long long items = (long long)c->cur_tokens *
+// Sender and router blocks per rank where `n` ranks share one launch on one GPU: two blocks per SM run at
+// a time, and the launch should have no more.  One router per destination leaves the most senders: eight
+// ranks of 256 tokens of 7168, top-8 of 256 experts: 59 us with 29 senders and 8 routers each, 70 with 21
+// and 16; of 2048, top-6 of 64, skewed: 46 against 52.  No more senders than a rank has wire rows.
+void share_send_blocks(const a2a_ctx* c, int n, int tokens, int* senders, int* routers, int* smem) {
+    const int ws = c->cfg.world_size, K = c->cfg.experts_per_token, T = c->cfg.max_num_tokens;
+    const long long rows = (long long)tokens * (K < ws - 1 ? K : ws - 1);
+    int ns = 2 * c->num_sms / n - ws;
+    if (ns > rows) ns = (int)rows;
+    if (ns < 2) ns = 2;
+    if (pipe_sender_smem(T, ws, ns) > kMaxPipeSmemBytes) ns = c->p.senders;  // fewer blocks have longer token lists
+    const size_t a = pipe_sender_smem(T, ws, ns), b = pipe_router_smem(T, c->p.L);
+    *senders = ns;
+    *routers = 1;
+    *smem = (int)align_up(a > b ? a : b, 128);
+}
+
+// The phases below take the contexts of all ranks that share this launch: one, or a whole group on one GPU.
+// Arguments are checked for every rank before anything is launched.
+
+int most_tokens(a2a_ctx* const* cs, int n) {
+    int t = 0;
+    for (int r = 0; r < n; ++r) t = cs[r]->cur_tokens > t ? cs[r]->cur_tokens : t;
+    return t;
+}
+
+// Blocks per rank: the grid that serves `items` of one rank, or this rank's share of the chip.
+int grid_for_ranks(const a2a_ctx* c, int n, long long items, int per_sm) {
+    const int share = c->num_sms * per_sm / n;
+    const int g = grid_for(c, items, per_sm);
+    return g < share ? g : (share < 1 ? 1 : share);
+}
+
+int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st) {
+    for (int r = 0; r < n; ++r) {
+        if (!cs[r]->routed || cs[r]->sent) return A2A_ERR_STATE;
+        if (cs[r]->cur_tokens > 0 && x[r] == nullptr) return A2A_ERR_CONFIG;
+        if (!rows_aligned(x[r])) return A2A_ERR_CONFIG;
+    }
+    for (int r = 0; r < n; ++r) cs[r]->p.x = x[r];
+    const a2a_ctx* c = cs[0];
+    const long long items = (long long)most_tokens(cs, n) *
         (c->cfg.payload == A2A_PAYLOAD_DIRECT ? c->cfg.experts_per_token : c->cfg.world_size);
-    int r = launch(c, select_tp<SendSel>(c), grid_for(c, items, 8), c->smem_bytes, st);
-    if (r == A2A_OK) c->sent = true;
-    return r;
+    const int rc = launch_ranks(cs, n, select_tp<SendSel>(c), grid_for_ranks(c, n, items, 8), c->smem_bytes, st);
+    if (rc == A2A_OK)
+        for (int r = 0; r < n; ++r) cs[r]->sent = true;
+    return rc;
 }
 
 // grid of the receive-side kernels: a multiple of the world size so every source gets the same share
-int expert_grid(const a2a_ctx* c, int per_sm) {
+int expert_grid(const a2a_ctx* c, int n, int per_sm) {
     const int ws = c->cfg.world_size;
-    int g = c->num_sms * per_sm;
+    int g = c->num_sms * per_sm / n;
     g = (g / ws) * ws;
     return g < ws ? ws : g;
 }
 
-int do_expert(a2a_ctx* c, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st) {
-    if (!c->sent) return A2A_ERR_STATE;
-    return launch(c, select_tp<ExpertSel>(c, wait, fanout, scale, publish), grid, c->smem_bytes, st);
+int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st) {
+    for (int r = 0; r < n; ++r)
+        if (!cs[r]->sent) return A2A_ERR_STATE;
+    return launch_ranks(cs, n, select_tp<ExpertSel>(cs[0], wait, fanout, scale, publish), grid, cs[0]->smem_bytes, st);
 }
 
-int do_combine(a2a_ctx* c, const float* w, void* y, cudaStream_t st) {
-    if (!c->sent) return A2A_ERR_STATE;
-    if (c->cur_tokens > 0 && (w == nullptr || y == nullptr)) return A2A_ERR_CONFIG;
-    if (!rows_aligned(y) || reinterpret_cast<uintptr_t>(w) % 4 != 0) return A2A_ERR_CONFIG;
-    c->p.w = w;
-    c->p.y = y;
+int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st) {
+    for (int r = 0; r < n; ++r) {
+        if (!cs[r]->sent) return A2A_ERR_STATE;
+        if (cs[r]->cur_tokens > 0 && (w[r] == nullptr || y[r] == nullptr)) return A2A_ERR_CONFIG;
+        if (!rows_aligned(y[r]) || reinterpret_cast<uintptr_t>(w[r]) % 4 != 0) return A2A_ERR_CONFIG;
+    }
+    for (int r = 0; r < n; ++r) {
+        cs[r]->p.w = w[r];
+        cs[r]->p.y = y[r];
+    }
+    const a2a_ctx* c = cs[0];
     const int nseg = (c->cfg.hidden_dim / 8 + 63) / 64;  // a warp per (token, 1 KB segment)
-    const long long warps = (long long)c->cur_tokens * nseg;
-    return launch(c, combine_fn(c), grid_for(c, (warps + kThreads / 32 - 1) / (kThreads / 32), 8), 0, st);
+    const long long warps = (long long)most_tokens(cs, n) * nseg;
+    return launch_ranks(cs, n, combine_fn(c), grid_for_ranks(c, n, (warps + kThreads / 32 - 1) / (kThreads / 32), 8), 0, st);
+}
+
+// Role 0 of the pipelined kernel: its tensors are checked and the call begun on every rank.
+int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st) {
+    for (int r = 0; r < n; ++r) {
+        const a2a_call& k = calls[r];
+        const int rc = check_call(cs[r], k.topk_idx, k.num_tokens);
+        if (rc != A2A_OK) return rc;
+        if (k.num_tokens > 0 && (k.x == nullptr || k.topk_weights == nullptr || k.y == nullptr)) return A2A_ERR_CONFIG;
+        if (!rows_aligned(k.x) || !rows_aligned(k.y) || reinterpret_cast<uintptr_t>(k.topk_weights) % 4 != 0) return A2A_ERR_CONFIG;
+    }
+    for (int r = 0; r < n; ++r) {
+        const a2a_call& k = calls[r];
+        begin_call(cs[r], k.topk_idx, k.num_tokens);
+        cs[r]->p.x = k.x;
+        cs[r]->p.w = k.topk_weights;
+        cs[r]->p.y = k.y;  // with one rank and the PUSH combine the expert blocks already write the output
+    }
+    const a2a_ctx* c = cs[0];
+    const int ws = c->cfg.world_size;
+    int ns = c->p.senders, nr = c->p.routers, smem = c->pipe_smem;
+    if (n > 1) share_send_blocks(c, n, most_tokens(cs, n), &ns, &nr, &smem);
+    const int rc = launch_ranks(cs, n, select_pipe<PipeRole>(c, 0), ns + ws * nr, smem, st, [=](DevParams& p) {
+        p.senders = ns;
+        p.routers = nr;
+    });
+    if (rc == A2A_OK)
+        for (int r = 0; r < n; ++r) cs[r]->sent = true;
+    return rc;
+}
+
+// Roles 1 and 2: a watcher block and this rank's share of two blocks per SM (of four or eight, where a
+// group shares the launch: 134 us against 145 and 159 for role 1 of the workload named above).
+int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
+    for (int r = 0; r < n; ++r)
+        if (!cs[r]->sent) return A2A_ERR_STATE;
+    const a2a_ctx* c = cs[0];
+    const int blocks = c->num_sms * 2 / n;
+    const int smem = role == 1 && c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
+    return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), 1 + (blocks < 1 ? 1 : blocks), smem, st);
+}
+
+// The contexts of every rank of one group, all on one GPU?
+int check_group(a2a_ctx* const* group) {
+    if (group == nullptr || group[0] == nullptr) return A2A_ERR_CONFIG;
+    const Fingerprint mine = fingerprint_of(group[0]->cfg);
+    for (int r = 0; r < group[0]->cfg.world_size; ++r) {
+        const a2a_ctx* c = group[r];
+        if (c == nullptr || c->cfg.rank != r || c->cfg.device != group[0]->cfg.device) return A2A_ERR_CONFIG;
+        const Fingerprint f = fingerprint_of(c->cfg);
+        if (memcmp(&f, &mine, sizeof(f)) != 0) return A2A_ERR_CONFIG;
+        if (!c->peers_ready) return A2A_ERR_STATE;
+    }
+    return A2A_OK;
 }
 
 }  // namespace
@@ -508,11 +644,13 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     // Kernel attributes are per function and device, not per context: opt every routing-carrying
     // kernel in for the whole shared-memory budget, then size this context's own launches.
     c->smem_bytes = (int)(block_smem_ints(E, T, K) * sizeof(int));
-    KernelFn fns[] = {route_kernel, select_tp<SendSel>(c), select_tp<ForwardSel>(c),
-                      select_tp<ExpertSel>(c, true, true, true, true), select_tp<ExpertSel>(c, true, true, false, false),
-                      select_tp<ExpertSel>(c, false, false, true, true), select_tp<ExpertSel>(c, false, false, false, true)};
-    for (KernelFn fn : fns) {
-        e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
+    const void* fns[] = {(const void*)route_kernel, (const void*)select_tp<SendSel>(c), (const void*)select_tp<ForwardSel>(c),
+                         (const void*)select_tp<ExpertSel>(c, true, true, true, true),
+                         (const void*)select_tp<ExpertSel>(c, true, true, false, false),
+                         (const void*)select_tp<ExpertSel>(c, false, false, true, true),
+                         (const void*)select_tp<ExpertSel>(c, false, false, false, true)};
+    for (const void* fn : fns) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
         if (e != cudaSuccess) break;
     }
     int coop = 0, occ = 0;
@@ -522,13 +660,14 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     if (pipelined) {
         const size_t a = cfg->world_size > 1 ? pipe_sender_smem(T, cfg->world_size, p.senders) : 0, b = pipe_router_smem(T, L);
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
-        for (int role = -1; role <= 2 && e == cudaSuccess; ++role)
-            e = cudaFuncSetAttribute((const void*)pipe_fn(c, role), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
+        const void* roles[] = {(const void*)select_pipe<PipeForward>(c), (const void*)select_pipe<PipeRole>(c, 0)};
+        for (const void* fn : roles)
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
         if (e == cudaSuccess && cfg->world_size == 1) {
             c->forward_grid = c->num_sms;
             c->fused = true;  // the solo kernel: no block waits for another
         } else if (e == cudaSuccess) {
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)pipe_fn(c, -1), kThreads, c->pipe_smem);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)select_pipe<PipeForward>(c), kThreads, c->pipe_smem);
             if (occ > 2) occ = 2;
             c->forward_grid = c->num_sms * occ;
             c->fused = true;
@@ -643,39 +782,39 @@ int a2a_route(a2a_ctx* c, const int32_t* idx, int T, void* stream) {
 int a2a_dispatch_send(a2a_ctx* c, const void* x, void* stream) {
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
-    return do_send(c, x, as_stream(stream));
+    return do_send(&c, 1, &x, as_stream(stream));
 }
 
 int a2a_dispatch_recv(a2a_ctx* c, void* stream) {
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
     // DIRECT: the rows are already in place; a minimal grid just waits for every source
-    const int grid = c->cfg.payload == A2A_PAYLOAD_DIRECT ? c->cfg.world_size : expert_grid(c, 4);
-    return do_expert(c, true, true, false, false, grid, as_stream(stream));
+    const int grid = c->cfg.payload == A2A_PAYLOAD_DIRECT ? c->cfg.world_size : expert_grid(c, 1, 4);
+    return do_expert(&c, 1, true, true, false, false, grid, as_stream(stream));
 }
 
 int a2a_expert_placeholder(a2a_ctx* c, void* stream) {
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
-    return do_expert(c, false, false, true, true, expert_grid(c, 4), as_stream(stream));
+    return do_expert(&c, 1, false, false, true, true, expert_grid(c, 1, 4), as_stream(stream));
 }
 
 int a2a_dispatch_recv_expert(a2a_ctx* c, void* stream) {
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
-    return do_expert(c, true, true, true, true, expert_grid(c, 4), as_stream(stream));
+    return do_expert(&c, 1, true, true, true, true, expert_grid(c, 1, 4), as_stream(stream));
 }
 
 int a2a_expert_done(a2a_ctx* c, void* stream) {
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
-    return do_expert(c, false, false, false, true, expert_grid(c, 1), as_stream(stream));
+    return do_expert(&c, 1, false, false, false, true, expert_grid(c, 1, 1), as_stream(stream));
 }
 
 int a2a_combine(a2a_ctx* c, const float* w, void* y, void* stream) {
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
-    return do_combine(c, w, y, as_stream(stream));
+    return do_combine(&c, 1, &w, &y, as_stream(stream));
 }
 
 int a2a_set_fused(a2a_ctx* c, int on) {
@@ -699,7 +838,7 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
         c->p.y = y;
         r = c->cfg.world_size == 1
             ? launch_solo(c, st)
-            : launch(c, pipe_fn(c, -1), c->forward_grid, c->pipe_smem, st, /*cooperative=*/true);
+            : launch(c, select_pipe<PipeForward>(c), c->forward_grid, c->pipe_smem, st, /*cooperative=*/true);
         if (r == A2A_OK) c->sent = true;
         return r;
     }
@@ -711,11 +850,11 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
         if (r == A2A_OK) c->sent = true;
         return r;
     }
-    r = do_send(c, x, st);
+    r = do_send(&c, 1, &x, st);
     if (r != A2A_OK) return r;
-    r = do_expert(c, true, true, true, true, expert_grid(c, 4), st);
+    r = do_expert(&c, 1, true, true, true, true, expert_grid(c, 1, 4), st);
     if (r != A2A_OK) return r;
-    return do_combine(c, w, y, st);
+    return do_combine(&c, 1, &w, &y, st);
 }
 
 int a2a_forward_host(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, void* y, int T, void* stream) {
@@ -740,22 +879,51 @@ int a2a_pipe_step(a2a_ctx* c, int role, const void* x, const int32_t* idx, const
     if (c == nullptr || role < 0 || role > 2) return A2A_ERR_CONFIG;
     if (c->cfg.schedule != A2A_SCHEDULE_PIPELINED) return A2A_ERR_STATE;
     DeviceGuard guard(c->cfg.device);
+    if (role != 0) return do_pipe_rest(&c, 1, role, as_stream(stream));
+    const a2a_call call = {x, idx, w, y, T};
+    return do_pipe_send(&c, 1, &call, as_stream(stream));
+}
+
+int a2a_group_step(a2a_ctx* const* group, int phase, const a2a_call* calls, void* stream) {
+    int rc = check_group(group);
+    if (rc != A2A_OK) return rc;
+    const a2a_ctx* c = group[0];
+    const int n = c->cfg.world_size;
+    const bool pipe_phase = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_PIPE_EXPERT || phase == A2A_GROUP_PIPE_COMBINE;
+    if (pipe_phase && c->cfg.schedule != A2A_SCHEDULE_PIPELINED) return A2A_ERR_STATE;
+    const bool takes_tensors = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_SEND || phase == A2A_GROUP_COMBINE;
+    if (takes_tensors && calls == nullptr) return A2A_ERR_CONFIG;
+    DeviceGuard guard(c->cfg.device);
     cudaStream_t st = as_stream(stream);
-    const int ws = c->cfg.world_size;
-    if (role == 0) {
-        int r = begin_call(c, idx, T);
-        if (r != A2A_OK) return r;
-        if (T > 0 && (x == nullptr || w == nullptr || y == nullptr)) return A2A_ERR_CONFIG;
-        if (!rows_aligned(x) || !rows_aligned(y) || reinterpret_cast<uintptr_t>(w) % 4 != 0) return A2A_ERR_CONFIG;
-        c->p.x = x;
-        c->p.w = w;
-        c->p.y = y;  // with one rank and the PUSH combine the expert blocks already write the output
-        r = launch(c, pipe_fn(c, 0), c->p.senders + ws * c->p.routers, c->pipe_smem, st);
-        if (r == A2A_OK) c->sent = true;
-        return r;
+    const void* x[A2A_MAX_WORLD];
+    const float* w[A2A_MAX_WORLD];
+    void* y[A2A_MAX_WORLD];
+    for (int r = 0; takes_tensors && r < n; ++r) {
+        x[r] = calls[r].x;
+        w[r] = calls[r].topk_weights;
+        y[r] = calls[r].y;
     }
-    if (!c->sent) return A2A_ERR_STATE;
-    return launch(c, pipe_fn(c, role), 1 + c->num_sms * 2, c->pipe_smem, st);
+    switch (phase) {
+        case A2A_GROUP_PIPE_SEND: return do_pipe_send(group, n, calls, st);
+        case A2A_GROUP_PIPE_EXPERT: return do_pipe_rest(group, n, 1, st);
+        case A2A_GROUP_PIPE_COMBINE: return do_pipe_rest(group, n, 2, st);
+        case A2A_GROUP_SEND:
+            for (int r = 0; r < n; ++r) {
+                rc = check_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
+                if (rc != A2A_OK) return rc;
+                if (calls[r].num_tokens > 0 && x[r] == nullptr) return A2A_ERR_CONFIG;
+                if (!rows_aligned(x[r])) return A2A_ERR_CONFIG;
+            }
+            for (int r = 0; r < n; ++r) begin_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
+            return do_send(group, n, x, st);
+        case A2A_GROUP_RECV:
+            return do_expert(group, n, true, true, false, false,
+                             c->cfg.payload == A2A_PAYLOAD_DIRECT ? n : expert_grid(c, n, 4), st);
+        case A2A_GROUP_EXPERT: return do_expert(group, n, false, false, true, true, expert_grid(c, n, 4), st);
+        case A2A_GROUP_RECV_EXPERT: return do_expert(group, n, true, true, true, true, expert_grid(c, n, 4), st);
+        case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st);
+        default: return A2A_ERR_CONFIG;
+    }
 }
 
 int a2a_barrier(a2a_ctx* c, void* stream) {

@@ -108,6 +108,13 @@ struct DevParams {
     void* y;
 };
 
+// The ranks one launch serves: a rank's own (n = 1) or, where a whole group lives on this GPU, all of them.
+// Block i works for rank position i % n as that rank's block i / n.
+struct GroupParams {
+    DevParams p[A2A_MAX_WORLD];
+    int n;
+};
+
 __device__ __forceinline__ long long global_ns() {
     long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -296,16 +303,16 @@ __device__ __forceinline__ bool watch_and_republish(const DevParams& p, int kind
 }
 
 // All threads of the block call this after their last store of a phase.  Returns true in
-// exactly one block of the grid: the one that arrived last.  The caller of that block
+// exactly one of the `blocks` blocks that share the ticket: the one that arrived last.  The caller of that block
 // must fence (system scope) before it publishes; every store of every block is then
 // ordered before the publication.
-__device__ __forceinline__ bool grid_arrive_last(uint32_t* ticket) {
+__device__ __forceinline__ bool grid_arrive_last(uint32_t* ticket, int blocks) {
     __shared__ int s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();  // gpu scope: cheap, and enough between blocks of one GPU
         const uint32_t t = atomicAdd(ticket, 1u);
-        const int last = (t == gridDim.x - 1);
+        const int last = (t == (uint32_t)blocks - 1u);
         if (last) *ticket = 0;  // everyone has arrived: re-arm for the next launch
         s_last = last;
     }

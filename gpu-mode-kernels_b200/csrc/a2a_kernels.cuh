@@ -174,12 +174,12 @@ __device__ __forceinline__ void copy_row(const uint4* __restrict__ src, uint4* _
 // Work is done chunk of tokens by chunk; the block that finishes a chunk last publishes it.
 // ---------------------------------------------------------------------------
 template <typename T, int PAYLOAD>
-__device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& s, int c) {
+__device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& s, int c, int b, int G) {
     const int tid = threadIdx.x;
     const int K = p.K, nvec = p.H >> 3;
     const int ta = chunk_begin(p, c), tb = chunk_end(p, c);  // this chunk's tokens
     if (PAYLOAD == A2A_PAYLOAD_DIRECT) {
-        for (int pair = ta * K + (int)blockIdx.x; pair < tb * K; pair += gridDim.x) {
+        for (int pair = ta * K + b; pair < tb * K; pair += G) {
             const int t = pair / K, k = pair - t * K;
             const int e = s.idx[pair];
             const int j = pair_slot(p, s, t, k, e);
@@ -192,7 +192,7 @@ __device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& 
             if (tid == 0) reinterpret_cast<int*>(p.peer[d] + p.off_meta)[row] = (t << 8) | k;
         }
     } else {
-        for (int it = ta * p.ws + (int)blockIdx.x; it < tb * p.ws; it += gridDim.x) {
+        for (int it = ta * p.ws + b; it < tb * p.ws; it += G) {
             const int t = it / p.ws, d = it - t * p.ws;
             // which of the token's experts live on d: each of them gets its slab row's (token, k)
             // word there; the row itself crosses the wire once
@@ -240,16 +240,16 @@ __device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& 
             }
         }
     }
-    if (grid_arrive_last(p.tickets + kTicketSend * kMaxChunks + c)) publish_dispatch(p, s, c);
+    if (grid_arrive_last(p.tickets + kTicketSend * kMaxChunks + c, G)) publish_dispatch(p, s, c);
 }
 
 // The sending half as its own kernel: routing, then every chunk in order.
 template <typename T, int PAYLOAD>
-__device__ __forceinline__ void send_phase(const DevParams& p, const BlockSmem& s) {
+__device__ __forceinline__ void send_phase(const DevParams& p, const BlockSmem& s, int b, int G) {
     stamp(p, kStampStart);
     route_build(p, s);
     stamp(p, kStampRouted);
-    for (int c = 0; c < p.chunks; ++c) send_chunk<T, PAYLOAD>(p, s, c);
+    for (int c = 0; c < p.chunks; ++c) send_chunk<T, PAYLOAD>(p, s, c, b, G);
     stamp(p, kStampSent);
 }
 
@@ -340,18 +340,18 @@ __device__ __forceinline__ void rows_of_source(const DevParams& p, int* pre, int
 }
 
 template <typename T, int PAYLOAD, bool WAIT, bool FANOUT, bool SCALE, bool PUBLISH>
-__device__ __forceinline__ void expert_chunk(const DevParams& p, const BlockSmem& sm, int c) {
+__device__ __forceinline__ void expert_chunk(const DevParams& p, const BlockSmem& sm, int c, int b, int G) {
     __shared__ int s_seen;
     const int tid = threadIdx.x;
     const uint32_t want = flag_value(p, c);
     // block b serves source b % ws together with the other blocks of that residue;
     // a grid smaller than the world size lets each block walk several sources alone
-    const bool many = (int)gridDim.x >= p.ws;
-    const int s_first = many ? (int)blockIdx.x % p.ws : (int)blockIdx.x;
-    const int s_step = many ? p.ws * A2A_MAX_WORLD : (int)gridDim.x;  // many: exactly one source
+    const bool many = G >= p.ws;
+    const int s_first = many ? b % p.ws : b;
+    const int s_step = many ? p.ws * A2A_MAX_WORLD : G;  // many: exactly one source
     for (int s = s_first; s < p.ws; s += s_step) {
-        const int part = many ? (int)blockIdx.x / p.ws : 0;
-        const int nparts = many ? ((int)gridDim.x - s + p.ws - 1) / p.ws : 1;
+        const int part = many ? b / p.ws : 0;
+        const int nparts = many ? (G - s + p.ws - 1) / p.ws : 1;
         if (WAIT) {
             // part 0 watches a peer's flag at system scope and hands it on; the rest, and everybody
             // for our own rank (whose publisher writes the local word itself), wait locally
@@ -371,7 +371,7 @@ __device__ __forceinline__ void expert_chunk(const DevParams& p, const BlockSmem
         __syncthreads();  // sm.pre / sm.base are reused by the next source
     }
     if (PUBLISH) {
-        if (grid_arrive_last(p.tickets + kTicketExpert * kMaxChunks + c)) {
+        if (grid_arrive_last(p.tickets + kTicketExpert * kMaxChunks + c, G)) {
             // after a timeout the outputs are incomplete: say nothing, the home ranks run into their own budget
             if (tid == 0) s_seen = (ld_volatile_i32(&p.status->code) != A2A_ERR_TIMEOUT) ? 1 : 0;
             __syncthreads();
@@ -382,8 +382,8 @@ __device__ __forceinline__ void expert_chunk(const DevParams& p, const BlockSmem
 
 // The receive side as its own kernel: every chunk in order.
 template <typename T, int PAYLOAD, bool WAIT, bool FANOUT, bool SCALE, bool PUBLISH>
-__device__ __forceinline__ void expert_phase(const DevParams& p, const BlockSmem& sm) {
-    for (int c = 0; c < p.chunks; ++c) expert_chunk<T, PAYLOAD, WAIT, FANOUT, SCALE, PUBLISH>(p, sm, c);
+__device__ __forceinline__ void expert_phase(const DevParams& p, const BlockSmem& sm, int b, int G) {
+    for (int c = 0; c < p.chunks; ++c) expert_chunk<T, PAYLOAD, WAIT, FANOUT, SCALE, PUBLISH>(p, sm, c, b, G);
     stamp(p, kStampExpertDone);
 }
 
@@ -503,18 +503,21 @@ __global__ void __launch_bounds__(kThreads) route_kernel(const __grid_constant__
 }
 
 template <typename T, int PAYLOAD>
-__global__ void __launch_bounds__(kThreads) send_kernel(const __grid_constant__ DevParams p) {
-    send_phase<T, PAYLOAD>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max));
+__global__ void __launch_bounds__(kThreads) send_kernel(const __grid_constant__ GroupParams g) {
+    const DevParams& p = g.p[blockIdx.x % g.n];
+    send_phase<T, PAYLOAD>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), (int)blockIdx.x / g.n, (int)gridDim.x / g.n);
 }
 
 template <typename T, int PAYLOAD, bool WAIT, bool FANOUT, bool SCALE, bool PUBLISH>
-__global__ void __launch_bounds__(kThreads) expert_kernel(const __grid_constant__ DevParams p) {
-    expert_phase<T, PAYLOAD, WAIT, FANOUT, SCALE, PUBLISH>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max));
+__global__ void __launch_bounds__(kThreads) expert_kernel(const __grid_constant__ GroupParams g) {
+    const DevParams& p = g.p[blockIdx.x % g.n];
+    expert_phase<T, PAYLOAD, WAIT, FANOUT, SCALE, PUBLISH>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), (int)blockIdx.x / g.n,
+                                                           (int)gridDim.x / g.n);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) combine_kernel(const __grid_constant__ DevParams p) {
-    combine_phase<T>(p, (int)blockIdx.x, (int)gridDim.x, true);
+__global__ void __launch_bounds__(kThreads) combine_kernel(const __grid_constant__ GroupParams g) {
+    combine_phase<T>(g.p[blockIdx.x % g.n], (int)blockIdx.x / g.n, (int)gridDim.x / g.n, true);
 }
 
 // The whole path in one launch.  Launched cooperatively so that every block is
@@ -531,11 +534,11 @@ __global__ void __launch_bounds__(kThreads) forward_kernel(const __grid_constant
     route_build(p, s);
     stamp(p, kStampRouted);
     for (int c = 0; c < p.chunks; ++c) {
-        send_chunk<T, PAYLOAD>(p, s, c);
-        if (c >= 1) expert_chunk<T, PAYLOAD, true, true, true, true>(p, s, c - 1);
+        send_chunk<T, PAYLOAD>(p, s, c, (int)blockIdx.x, (int)gridDim.x);
+        if (c >= 1) expert_chunk<T, PAYLOAD, true, true, true, true>(p, s, c - 1, (int)blockIdx.x, (int)gridDim.x);
     }
     stamp(p, kStampSent);
-    expert_chunk<T, PAYLOAD, true, true, true, true>(p, s, p.chunks - 1);
+    expert_chunk<T, PAYLOAD, true, true, true, true>(p, s, p.chunks - 1, (int)blockIdx.x, (int)gridDim.x);
     stamp(p, kStampExpertDone);
     combine_phase<T>(p, (int)blockIdx.x, (int)gridDim.x, true);
 }

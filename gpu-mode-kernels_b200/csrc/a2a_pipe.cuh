@@ -618,6 +618,7 @@ __device__ __forceinline__ void load_wire_chunk(const DevParams& p, bool own, co
 constexpr int kExpertWorkers = kThreads / 32 - 2;
 
 constexpr int kReturnSlotBytes = 2048;  // one 2 KB chunk of a partial row, two slots per worker warp
+constexpr int kReturnSmemBytes = kExpertWorkers * 2 * kReturnSlotBytes;
 
 template <typename T, int PAYLOAD, bool PUSH>
 __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, int xb, int nxb) {
@@ -913,8 +914,8 @@ __device__ __forceinline__ void combine_home_role(const DevParams& p, int cb, in
 
 // PULL combine never reads a rank it has no pair on, but a rank may only start its next call
 // once EVERY peer is through with this one's records; one thread sees to that.
-__device__ __forceinline__ void wait_all_experts(const DevParams& p) {
-    if (blockIdx.x == 0 && threadIdx.x == 0)
+__device__ __forceinline__ void wait_all_experts(const DevParams& p, int b) {
+    if (b == 0 && threadIdx.x == 0)
         for (int d = 0; d < p.ws; ++d)
             if (!wait_flag_gpu(seen_ptr(p, kFlagExpert, d), flag_value(p, 0), p, kPhaseCombine, d)) break;
 }
@@ -967,17 +968,18 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
         combine_home_role<T>(p, b, G);
     } else {
         combine_phase<T>(p, b, G, /*own_watchers=*/false);
-        wait_all_experts(p);
+        wait_all_experts(p, b);
     }
 }
 
-// The same roles as separate launches, for stepping several ranks on ONE GPU (a kernel that
-// waits never shares the GPU with the kernel it waits for) and for callers that want the
-// phases apart.  ROLE 0: senders + routers.  1: one watcher block + experts.  2: one
-// watcher block + combine.
+// The same roles as separate launches: for callers that want the phases apart, and for stepping a group
+// that lives on ONE GPU -- a kernel that waits never shares the GPU with the kernel it waits for, so what
+// runs together is one role of every rank.  ROLE 0: senders + routers.  1: one watcher block + experts.
+// 2: one watcher block + combine.
 template <typename T, int PAYLOAD, bool PUSH, int ROLE>
-__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ DevParams p) {
-    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ GroupParams g) {
+    const DevParams& p = g.p[blockIdx.x % g.n];
+    const int G = (int)gridDim.x / g.n, b = (int)blockIdx.x / g.n;
     const int ns = p.ws > 1 ? p.senders : 0;
     stamp(p, kStampStart);
     if (ROLE == 0) {
@@ -1001,7 +1003,7 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_con
         } else {
             combine_phase<T>(p, b - 1, G - 1, /*own_watchers=*/false);
         }
-        if (!PUSH) wait_all_experts(p);
+        if (!PUSH) wait_all_experts(p, b);
     }
 }
 

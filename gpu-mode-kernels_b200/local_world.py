@@ -1,8 +1,8 @@
 """Several ranks on ONE GPU, run phase by phase in one process.
 
 Kernels that wait on a peer must never share a GPU with the kernel they wait
-for, so the ranks here are stepped in lock-step: every rank's sending kernel is
-enqueued before any rank's waiting kernel, on one stream, and each wait finds its
+for, so the ranks here are stepped in lock-step: one launch runs a phase of every
+rank, the sending phase before any waiting one, on one stream, and each wait finds its
 flag already set.  The kernels, addresses, flags and epochs are exactly those of
 a real multi-GPU run; only CUDA IPC and true concurrency are not exercised.
 Validation tool: parity tests and the smoke check use it to cover world sizes
@@ -10,10 +10,12 @@ Validation tool: parity tests and the smoke check use it to cover world sizes
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import List, Sequence
 
 import torch
 
+from . import _lib
 from .all2all import A2AContext
 from .task import MoEConfig
 
@@ -29,40 +31,63 @@ class LocalWorld:
         ]
         A2AContext.attach_local(self.ctxs)
 
+    def _step(self, phase: str, calls=None) -> None:
+        handles = (C.c_void_p * self.world_size)(*[c._h for c in self.ctxs])
+        _lib.check(self.ctxs[0].lib.a2a_group_step(handles, _lib.GROUP_PHASE[phase], calls, A2AContext._stream()))
+
+    def _send(self, rank_datas: Sequence) -> None:
+        """route + dispatch_send on every rank, in one launch."""
+        calls = (_lib.Call * self.world_size)()
+        for call, c, rd in zip(calls, self.ctxs, rank_datas):
+            assert rd.indices.dtype == torch.int32 and rd.indices.is_contiguous() and rd.indices.is_cuda
+            assert rd.x.dtype == self.cfg.in_dtype and rd.x.is_contiguous() and rd.x.is_cuda
+            call.x, call.topk_idx, call.num_tokens = rd.x.data_ptr(), rd.indices.data_ptr(), rd.indices.shape[0]
+        self._step("send", calls)
+        for c, rd in zip(self.ctxs, rank_datas):
+            c._num_tokens, c._keep = rd.indices.shape[0], [rd.indices, rd.x]
+
+    def _combine(self, rank_datas: Sequence) -> List[torch.Tensor]:
+        calls, ys = (_lib.Call * self.world_size)(), []
+        for call, c, rd in zip(calls, self.ctxs, rank_datas):
+            assert rd.weights.dtype == torch.float32 and rd.weights.is_contiguous() and rd.weights.is_cuda
+            ys.append(torch.empty(c._num_tokens, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=c.device))
+            call.topk_weights, call.y = rd.weights.data_ptr(), ys[-1].data_ptr()
+            c._keep.append(rd.weights)
+        self._step("combine", calls)
+        return ys
+
     def dispatch(self, rank_datas: Sequence) -> None:
         """route + dispatch on every rank (rank_datas hold device tensors)."""
-        for c, rd in zip(self.ctxs, rank_datas):
-            c.route(rd.indices)
-        for c, rd in zip(self.ctxs, rank_datas):
-            c.dispatch_send(rd.x)
-        for c in self.ctxs:
-            c.dispatch_recv()
+        self._send(rank_datas)
+        self._step("recv")
 
     def forward_phases(self, rank_datas: Sequence) -> List[torch.Tensor]:
         """The four public phases, one after the other."""
         self.dispatch(rank_datas)
-        for c in self.ctxs:
-            c.expert_placeholder()
-        return [c.combine(rd.weights) for c, rd in zip(self.ctxs, rank_datas)]
+        self._step("expert")
+        return self._combine(rank_datas)
 
     def forward(self, rank_datas: Sequence) -> List[torch.Tensor]:
-        """The kernels a2a_forward launches (route, send, recv+expert fused, combine), in lock-step."""
-        for c, rd in zip(self.ctxs, rank_datas):
-            c.route(rd.indices)
-        for c, rd in zip(self.ctxs, rank_datas):
-            c.dispatch_send(rd.x)
-        for c in self.ctxs:
-            c.dispatch_recv_expert()
-        return [c.combine(rd.weights) for c, rd in zip(self.ctxs, rank_datas)]
+        """The kernels a2a_forward launches (send, recv+expert fused, combine), in lock-step."""
+        self._send(rank_datas)
+        self._step("recv_expert")
+        return self._combine(rank_datas)
 
     def forward_pipelined(self, rank_datas: Sequence) -> List[torch.Tensor]:
-        """The roles of the pipelined one-launch kernel as three launches per rank, in lock-step:
+        """The roles of the pipelined one-launch kernel as three launches, in lock-step:
         every rank's senders and routers, then every rank's expert blocks, then every rank's combine."""
-        for c, rd in zip(self.ctxs, rank_datas):
-            c.pipe_step(0, rd.x, rd.indices, rd.weights)
-        for c in self.ctxs:
-            c.pipe_step(1)
-        return [c.pipe_step(2) for c in self.ctxs]
+        calls, ys = (_lib.Call * self.world_size)(), []
+        for call, c, rd in zip(calls, self.ctxs, rank_datas):
+            n = c._check_inputs(rd.x, rd.indices, rd.weights, None, on_device=True)
+            ys.append(torch.empty(n, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=c.device))
+            call.x, call.topk_idx, call.topk_weights = rd.x.data_ptr(), rd.indices.data_ptr(), rd.weights.data_ptr()
+            call.y, call.num_tokens = ys[-1].data_ptr(), n
+        self._step("pipe_send", calls)
+        for c, rd, y in zip(self.ctxs, rank_datas, ys):
+            c._num_tokens, c._y, c._keep = y.shape[0], y, [rd.x, rd.indices, rd.weights, y]
+        self._step("pipe_expert")
+        self._step("pipe_combine")
+        return ys
 
     def check(self) -> None:
         for c in self.ctxs:

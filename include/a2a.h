@@ -219,6 +219,24 @@ int a2a_forward_host(a2a_ctx* ctx, const void* x_host, const int32_t* topk_idx_h
 int a2a_pipe_step(a2a_ctx* ctx, int role, const void* x, const int32_t* topk_idx, const float* topk_weights,
                   void* y, int num_tokens, void* stream);
 
+/* One phase of EVERY rank of a group that lives on one GPU, as one launch: `group` holds the contexts of
+ * all ranks in rank order (same configuration, same device, attached).  What runs together never waits for
+ * itself, so the phases are called in order -- PIPE_SEND, PIPE_EXPERT, PIPE_COMBINE are the roles of
+ * a2a_pipe_step (pipelined contexts); SEND is a2a_route + a2a_dispatch_send, RECV, EXPERT, RECV_EXPERT and
+ * COMBINE the entry points of those names.  `calls` (one per rank, rank order) is read by PIPE_SEND (all
+ * fields), SEND (x, topk_idx, num_tokens) and COMBINE (topk_weights, y), and may be NULL otherwise.
+ * Nothing is launched, and no call begun, unless the arguments of every rank are valid. */
+enum { A2A_GROUP_PIPE_SEND = 0, A2A_GROUP_PIPE_EXPERT = 1, A2A_GROUP_PIPE_COMBINE = 2, A2A_GROUP_SEND = 3,
+       A2A_GROUP_RECV = 4, A2A_GROUP_EXPERT = 5, A2A_GROUP_RECV_EXPERT = 6, A2A_GROUP_COMBINE = 7 };
+typedef struct a2a_call {
+    const void* x;
+    const int32_t* topk_idx;
+    const float* topk_weights;
+    void* y;
+    int32_t num_tokens;
+} a2a_call;
+int a2a_group_step(a2a_ctx* const* group, int phase, const a2a_call* calls, void* stream);
+
 /* Cross-GPU rendezvous on the device: returns (on the stream) once every rank's
  * stream has reached it.  Bounded wait.  Used to align ranks before timing.
  * Plays the role of dist.barrier() around the timed call (my_eval.py:160-172). */

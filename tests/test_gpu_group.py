@@ -1,0 +1,102 @@
+"""One launch per phase for a whole group on one GPU: the same bits as the phases called rank by rank, and
+nothing begun when one rank's arguments are refused."""
+import ctypes as C
+
+import pytest
+import torch
+
+import gpu_mode_kernels_b200 as pkg
+from gpu_mode_kernels_b200 import _lib
+from gpu_mode_kernels_b200.all2all import A2AError
+from gpu_mode_kernels_b200.local_world import LocalWorld
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def bits(t):
+    return t.contiguous().view(torch.int16)
+
+
+def rank_by_rank(world, rds):
+    if world.ctxs[0].schedule == "pipelined":
+        for c, rd in zip(world.ctxs, rds):
+            c.pipe_step(0, rd.x, rd.indices, rd.weights)
+        for c in world.ctxs:
+            c.pipe_step(1)
+        return [c.pipe_step(2) for c in world.ctxs]
+    for c, rd in zip(world.ctxs, rds):
+        c.route(rd.indices)
+    for c, rd in zip(world.ctxs, rds):
+        c.dispatch_send(rd.x)
+    for c in world.ctxs:
+        c.dispatch_recv()
+    for c in world.ctxs:
+        c.expert_placeholder()
+    return [c.combine(rd.weights) for c, rd in zip(world.ctxs, rds)]
+
+
+def state(world):
+    return [t for c in world.ctxs for t in c.route_tables() + c.export_dispatch()]
+
+
+@pytest.mark.parametrize("schedule,payload,combine", [
+    ("pipelined", "dedup", "push"), ("pipelined", "dedup", "pull"), ("pipelined", "fp8", "push"),
+    ("phased", "direct", "pull"), ("phased", "dedup", "pull"), ("phased", "fp8", "pull"),
+])
+@pytest.mark.parametrize("E,K,H,T,ws", [
+    (8, 2, 128, 1, 2),       # one token: fewer wire rows than sender blocks
+    (12, 3, 2944, 70, 3),    # ranks that do not divide the grid, rows that end inside a warp's piece
+    (64, 6, 2048, 300, 8),   # more than one round of 256 tokens
+])
+def test_group_launches_equal_the_phases_rank_by_rank(schedule, payload, combine, E, K, H, T, ws):
+    sets = [[pkg.generate_input(E, K, H, T, seed=s, rank=r, world_size=ws, ragged=T > 1) for r in range(ws)] for s in (3, 4)]
+    world = LocalWorld(sets[0][0][0], ws, payload=payload, schedule=schedule, combine=combine)
+    grouped = world.forward_pipelined if schedule == "pipelined" else world.forward_phases
+    try:
+        for datas in sets:  # ranks of different token counts, then others on the same contexts
+            rds = [d[1].to(DEV) for d in datas]
+            want = [bits(y) for y in rank_by_rank(world, rds)]
+            tables = state(world)
+            before = [c.launches for c in world.ctxs]
+            got = grouped(rds)
+            assert all(c.launches - b == (3 if schedule == "pipelined" else 4) for c, b in zip(world.ctxs, before))
+            assert all(torch.equal(bits(g), w) for g, w in zip(got, want))
+            assert all(torch.equal(a, b) for a, b in zip(state(world), tables))
+        world.ctxs[1].trace_enable()  # traced contexts are launched one by one
+        got = grouped(rds)
+        assert all(torch.equal(bits(g), w) for g, w in zip(got, want))
+        assert bool((world.ctxs[1].trace_read()[:, 1] != 0).all())
+        world.check()
+    finally:
+        world.close()
+
+
+def test_nothing_begins_when_one_rank_is_refused():
+    cfg = pkg.MoEConfig(8, 2, 64, 4)
+    datas = [pkg.generate_input(8, 2, 64, 4, seed=1, rank=r, world_size=2) for r in range(2)]
+    rds = [d[1].to(DEV) for d in datas]
+    world = LocalWorld(cfg, 2, payload="dedup", schedule="pipelined", combine="push")
+    try:
+        want = [bits(y) for y in world.forward_pipelined(rds)]
+        bad = [rds[0], rds[1].to(DEV)]
+        bad[1].weights = bad[1].weights.double()
+        with pytest.raises(A2AError):
+            world.forward_pipelined(bad)
+        lib, before = world.ctxs[0].lib, [c.launches for c in world.ctxs]
+        handles = (C.c_void_p * 2)(*[c._h for c in world.ctxs])
+        calls = (_lib.Call * 2)()
+        for call, rd in zip(calls, rds):
+            call.x, call.topk_idx, call.topk_weights = rd.x.data_ptr(), rd.indices.data_ptr(), rd.weights.data_ptr()
+            call.y, call.num_tokens = rd.x.data_ptr(), 4
+        calls[1].num_tokens = 5  # more than the contexts were made for
+        assert lib.a2a_group_step(handles, _lib.GROUP_PHASE["pipe_send"], calls, None) == _lib.A2A_ERR_CONFIG
+        assert lib.a2a_group_step(handles, _lib.GROUP_PHASE["pipe_send"], None, None) == _lib.A2A_ERR_CONFIG
+        assert lib.a2a_group_step((C.c_void_p * 2)(handles[1], handles[0]), 0, calls, None) == _lib.A2A_ERR_CONFIG
+        assert lib.a2a_group_step(handles, 8, calls, None) == _lib.A2A_ERR_CONFIG
+        assert [c.launches for c in world.ctxs] == before
+        got = world.forward_pipelined(rds)  # the ranks' call counters are still level
+        assert all(torch.equal(bits(g), w) for g, w in zip(got, want))
+        world.check()
+    finally:
+        world.close()
