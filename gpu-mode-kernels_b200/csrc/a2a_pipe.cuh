@@ -565,35 +565,41 @@ __device__ __forceinline__ uint4 fp8_round_trip(const uint4& q, bool valid) {
     return pack8<T>(f);
 }
 
-// One 128-vector (2 KB) chunk of a wire row as four 16-byte vectors of T per lane.
-// Own rows are read from x (FP8: through the same quantise / dequantise arithmetic the wire applies).
+// One 128-vector (2 KB) chunk of a row as this rank received it, four 16-byte vectors of T per lane, in two
+// halves so that the bytes can be on their way while something else is worked on: the loads (an FP8 wire
+// row gives eight bytes and a scale per vector), and the conversion.
 template <typename T, int PAYLOAD>
 __device__ __forceinline__ void load_wire_chunk(const DevParams& p, bool own, const uint8_t* src, int v0, int nvec, uint4 (&q)[4]) {
     const int lane = threadIdx.x & 31;
-    if (PAYLOAD != A2A_PAYLOAD_FP8) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = v0 + u * 32 + lane;
-            if (v < nvec) q[u] = own ? ld_input(reinterpret_cast<const uint4*>(src) + v) : ld_stream(reinterpret_cast<const uint4*>(src) + v);
-        }
-    } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = v0 + u * 32 + lane;
-            float f[8];
-            if (own) {  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
-                uint4 own_q = make_uint4(0u, 0u, 0u, 0u);
-                if (v < nvec) own_q = ld_input(reinterpret_cast<const uint4*>(src) + v);
-                q[u] = fp8_round_trip<T>(own_q, v < nvec);
-            } else if (v < nvec) {
-                unpack8_e4m3(ld_stream(reinterpret_cast<const uint2*>(src) + v), f);
-                const float sc = ld_stream(reinterpret_cast<const float*>(src + p.H) + (v >> 4));
-#pragma unroll
-                for (int i = 0; i < 8; ++i) f[i] *= sc;
-                q[u] = pack8<T>(f);
-            }
+    for (int u = 0; u < 4; ++u) {
+        const int v = v0 + u * 32 + lane;
+        if (v >= nvec) continue;
+        if (own) {
+            q[u] = ld_input(reinterpret_cast<const uint4*>(src) + v);
+        } else if (PAYLOAD != A2A_PAYLOAD_FP8) {
+            q[u] = ld_stream(reinterpret_cast<const uint4*>(src) + v);
+        } else {
+            const uint2 bytes = ld_stream(reinterpret_cast<const uint2*>(src) + v);
+            q[u].x = bytes.x;
+            q[u].y = bytes.y;
+            q[u].z = __float_as_uint(ld_stream(reinterpret_cast<const float*>(src + p.H) + (v >> 4)));
         }
     }
+}
+
+// One vector of what load_wire_chunk read, as T.  FP8: own rows go through the same quantise / dequantise
+// arithmetic the wire applies.  Every lane of the warp calls it.
+template <typename T, int PAYLOAD>
+__device__ __forceinline__ uint4 wire_vector(bool own, const uint4& q, bool valid) {
+    if (PAYLOAD != A2A_PAYLOAD_FP8) return q;
+    if (own) return fp8_round_trip<T>(q, valid);  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
+    float f[8];
+    unpack8_e4m3(make_uint2(q.x, q.y), f);
+    const float sc = __uint_as_float(q.z);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] *= sc;
+    return pack8<T>(f);
 }
 
 // ---------------------------------------------------------------------------
@@ -613,7 +619,13 @@ __device__ __forceinline__ void load_wire_chunk(const DevParams& p, bool own, co
 //           home through the copy engine -- packed into one of the warp's two 2 KB shared-memory
 //           slots and bulk-stored -- so that the back-pressure of the link never sits in the load /
 //           store path of the SM in front of the slab stores and the next item's loads; such a source
-//           is booked one source later (by then its bulk stores have long completed), the last at once.
+//           is booked one source later (by then its bulk stores have long completed), the last, and one
+//           whose successor is not here yet, at once.
+// What bounds it: not the memory but a warp's own instructions per item (at two blocks per SM twelve workers
+// share an SM; 900 instructions and six cycles each made 2.8 us an item).  Hence the next item's loads ahead of
+// this one's work, packed products and multiply-adds, one accumulator vector at a time, no division per item.
+// Eight ranks in one launch, 256 tokens of 7168, top-8 of 256 experts: 134 -> 109 us, FP8 wire rows 209 -> 135;
+// three blocks per SM would leave 80 registers, and spill: 115 and 188.
 // ---------------------------------------------------------------------------
 constexpr int kExpertWorkers = kThreads / 32 - 2;
 
@@ -686,128 +698,191 @@ __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, i
         __threadfence_block();
         atomicAdd(&s_done[i], 1);
     };
-    long long cursor = 0;
-    int pending = -1;         // lane 0: a source whose bulk stores are still to be waited for
-    long long groups = 0;     // lane 0: bulk groups this warp has committed so far
-    long long pending_groups = 0;
-    for (int i = 0; i < p.ws; ++i) {
-        int seen;
-        while ((seen = s_seen[i]) == 0) __nanosleep(40);  // bounded by the poller's own bounded wait
-        if (seen < 0) {
-            // nothing further is processed or published; the completers are still owed this warp's bookings
-            if (lane == 0) {
-                s_dead = 1;
-                __threadfence_block();
-                bulk_wait_done(0);
-                if (pending >= 0) atomicAdd(&s_done[pending], 1);
-                for (int j = i; j < p.ws; ++j) atomicAdd(&s_done[j], 1);
+    int done = 0;             // source positions this warp is through with
+    int pending = -1;         // lane 0: one of them whose bulk stores are still to be waited for
+    int groups = 0;           // bulk groups this warp has committed so far
+    int pending_groups = 0;
+    auto flush = [&] {  // lane 0: wait for the pending source's bulk stores and book it
+        if (pending < 0) return;
+        bulk_wait_done(min(groups - pending_groups, 5));
+        fence_async_global();
+        book(pending);
+        pending = -1;
+    };
+    auto finish = [&](int upto) {  // every item this warp has of the positions before `upto` is processed
+        if (done >= upto) return;
+        __syncwarp();  // every lane's stores of these sources precede lane 0's fence and booking
+        for (; done < upto; ++done) {
+            if (lane != 0) continue;
+            flush();  // the source before: its bulk stores are at least this source's items old
+            if (PUSH && (p.rank - done + p.ws) % p.ws != p.rank) {
+                pending = done;
+                pending_groups = groups;
+                if (done + 1 == p.ws) flush();  // the last source: nothing comes after it to hide the wait behind
+            } else {
+                book(done);
             }
-            return;
         }
-        const int s = (p.rank - i + p.ws) % p.ws;
-        const int n_s = s_rows[i];
-        const int* rec_tok = reinterpret_cast<const int*>(self + p.off_rec_tok) + (size_t)s * p.T_max;
-        const unsigned* rec_ent = reinterpret_cast<const unsigned*>(self + p.off_rec_ent) + (size_t)s * p.T_max * K;
-        const float* rec_w = reinterpret_cast<const float*>(self + p.off_rec_w) + (size_t)s * p.T_max * K;
+    };
+    // A position in this warp's sequence of items: chunk `ch` of wire row `n` of the source at position `i`, rank
+    // `s`; the warp's first item there is number `first`.  `open`: the source's rows are known to be here.
+    const int step_n = nxw / nchunk, step_ch = nxw - step_n * nchunk;
+    struct Cursor {
+        int i, s, n, ch, n_s, first;
+        bool open;
+    };
+    auto advance = [&](Cursor& c) {
+        c.n += step_n;
+        c.ch += step_ch;
+        if (c.ch >= nchunk) {
+            c.ch -= nchunk;
+            ++c.n;
+        }
+    };
+    enum { kItem, kNotYet, kEnd, kGaveUp };
+    auto seek = [&](Cursor& c) {  // the first item at or after c, as far as sources have arrived
+        while (true) {
+            if (!c.open) {
+                if (c.i == p.ws) return kEnd;
+                const int seen = __shfl_sync(0xffffffffu, s_seen[c.i], 0);  // one lane's view, or the warp could part
+                if (seen == 0) return kNotYet;
+                if (seen < 0) return kGaveUp;
+                __threadfence_block();  // with the poller's: what it saw arrive is visible here
+                c.n_s = s_rows[c.i];
+                c.n = c.first / nchunk;
+                c.ch = c.first - c.n * nchunk;
+                c.open = true;
+            }
+            if (c.n < c.n_s) return kItem;
+            // all warps go on where this source's items end
+            c.first = (int)((c.first - (long long)c.n_s * nchunk) % nxw);
+            if (c.first < 0) c.first += nxw;
+            ++c.i;
+            c.s = c.s == 0 ? p.ws - 1 : c.s - 1;
+            c.open = false;
+        }
+    };
+    struct Item {
+        uint4 q[4];
+        unsigned ent;  // lane k: record entry of pair k
+        float w;       //         and its weight
+        int t;         // token
+    };
+    auto load = [&](const Cursor& c, Item& m) {
+        const int s = c.s, n = c.n, v0 = c.ch * 128;
+        const bool own = (s == p.rank);
+        const size_t rec = (size_t)s * p.T_max + n;
+        m.t = ld_stream(reinterpret_cast<const int*>(self + p.off_rec_tok) + rec);
+        m.ent = lane < K ? (unsigned)ld_stream(reinterpret_cast<const int*>(self + p.off_rec_ent) + rec * K + lane) : kNoEntry;
+        m.w = (PUSH && lane < K) ? ld_stream(reinterpret_cast<const float*>(self + p.off_rec_w) + rec * K + lane) : 0.f;
+        // a peer's row lies where its number says; only an own row has to be looked for
+        const uint8_t* src = self + p.off_stage + rec * p.stage_row_bytes;
+        if (own) {
+            if (m.t < 0 || m.t >= p.T_max) return;
+            src = reinterpret_cast<const uint8_t*>(p.x) + (size_t)m.t * p.H * 2;
+        }
+        load_wire_chunk<T, PAYLOAD>(p, own, src, v0, nvec, m.q);
+    };
+    auto process = [&](const Cursor& c, const Item& m) {
+        const int s = c.s, v0 = c.ch * 128, t = m.t;
         const bool own = (s == p.rank);
         const bool via_engine = PUSH && !own;  // the home rank is a peer: return through the copy engine
-        const long long items = (long long)n_s * nchunk;
-        for (long long it = (xw - cursor % nxw + nxw) % nxw; it < items; it += nxw) {
-            const int n = (int)(it / nchunk), v0 = (int)(it - (long long)n * nchunk) * 128;
-            const int t = ld_stream(rec_tok + n);
-            const unsigned my_ent = lane < K ? (unsigned)ld_stream(reinterpret_cast<const int*>(rec_ent) + (size_t)n * K + lane) : kNoEntry;
-            const float my_w = (PUSH && lane < K) ? ld_stream(rec_w + (size_t)n * K + lane) : 0.f;
-            if (t < 0 || t >= p.T_max) {
-                record_error(p.status, A2A_ERR_CAPACITY, p.rank, s, kPhaseRecv, p.epoch, t);
-                continue;
-            }
-            const uint8_t* src = own ? reinterpret_cast<const uint8_t*>(p.x) + (size_t)t * p.H * 2
-                                     : self + p.off_stage + ((size_t)s * p.T_max + n) * p.stage_row_bytes;
-            uint4 q[4];
-            load_wire_chunk<T, PAYLOAD>(p, own, src, v0, nvec, q);
-            float acc[4][8];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                q[u] = scale8<T>(q[u], scale);  // the placeholder expert op: T(float(row) * (1 + rank))
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[u][e] = 0.f;
-            }
-            for (int k = 0; k < K; ++k) {
-                const unsigned ent = __shfl_sync(0xffffffffu, my_ent, k);
-                const float w = __shfl_sync(0xffffffffu, my_w, k);
-                if (ent == kNoEntry) continue;
-                const int l = (int)(ent >> 16), j = (int)(ent & 0xffffu);
-                if (l >= p.L || j >= p.T_max) {
-                    record_error(p.status, A2A_ERR_CAPACITY, p.rank, s, kPhaseExpert, p.epoch, (int)ent);
-                    continue;
-                }
-                uint4* row = rows + (((size_t)l * p.ws + s) * p.T_max + j) * nvec;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int v = v0 + u * 32 + lane;
-                    if (v < nvec) {
-                        st_stream(row + v, q[u]);
-                        if (PUSH) {
-                            float f[8];
-                            unpack8<T>(q[u], f);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) acc[u][e] = fmaf(f[e], w, acc[u][e]);
-                        }
-                    }
-                }
-            }
-            if (PUSH && !via_engine) {
-                // one rank: the partial row IS the token's output -- no return buffer, no combine pass;
-                // own tokens of several ranks: the return buffer is local memory
-                uint4* home = p.ws == 1 ? reinterpret_cast<uint4*>(p.y) + (size_t)t * nvec
-                                        : reinterpret_cast<uint4*>(self + p.off_ret) + ((size_t)p.rank * p.T_max + t) * nvec;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int v = v0 + u * 32 + lane;
-                    if (v < nvec) st_stream(home + v, pack8<T>(acc[u]));
-                }
-            }
-            if (via_engine) {
-                uint8_t* slot = slots + (size_t)(groups & 1) * kReturnSlotBytes;  // `groups` is warp-uniform: every lane counts
-                if (groups >= 2) {
-                    if (lane == 0) bulk_wait_read<1>();  // the store that used this slot two items ago has read it
-                    __syncwarp();
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int v = v0 + u * 32 + lane;
-                    if (v < nvec) reinterpret_cast<uint4*>(slot)[u * 32 + lane] = pack8<T>(acc[u]);
-                }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    uint8_t* home = p.peer[s] + p.off_ret + (((size_t)p.rank * p.T_max + t) * nvec + v0) * 16;
-                    bulk_store(home, smem_addr(slot), (uint32_t)(min(128, nvec - v0) * 16));
-                    bulk_commit();
-                }
-                ++groups;
+        if (t < 0 || t >= p.T_max) {
+            record_error(p.status, A2A_ERR_CAPACITY, p.rank, s, kPhaseRecv, p.epoch, t);
+            return;
+        }
+        // lane k: the slab row of pair k here
+        int my_row = 0;
+        bool here = m.ent != kNoEntry;
+        if (here) {
+            const int l = (int)(m.ent >> 16), j = (int)(m.ent & 0xffffu);
+            my_row = (l * p.ws + s) * p.T_max + j;
+            if (l >= p.L || j >= p.T_max) {
+                record_error(p.status, A2A_ERR_CAPACITY, p.rank, s, kPhaseExpert, p.epoch, (int)m.ent);
+                here = false;
             }
         }
-        cursor += items;
-        __syncwarp();  // every lane's stores of this source precede lane 0's fence and booking
-        if (lane == 0) {
-            if (pending >= 0) {  // the source before: its bulk stores are at least this source's items old
-                bulk_wait_done((int)min(groups - pending_groups, 5LL));
-                fence_async_global();
-                book(pending);
-                pending = -1;
+        const unsigned pairs = __ballot_sync(0xffffffffu, here);
+        uint8_t* slot = slots + (size_t)(groups & 1) * kReturnSlotBytes;  // `groups` is warp-uniform: every lane counts
+        if (via_engine && groups >= 2) {
+            if (lane == 0) bulk_wait_read<1>();  // the store that used this slot two items ago has read it
+            __syncwarp();
+        }
+        // one rank: the partial row IS the token's output -- no return buffer, no combine pass;
+        // own tokens of several ranks: the return buffer is local memory
+        uint4* home = p.ws == 1 ? reinterpret_cast<uint4*>(p.y) + (size_t)t * nvec
+                                : reinterpret_cast<uint4*>(self + p.off_ret) + ((size_t)p.rank * p.T_max + t) * nvec;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int v = v0 + u * 32 + lane;
+            if (v - lane >= nvec) break;  // the whole warp is past the row's end
+            const uint4 out = scale8<T>(wire_vector<T, PAYLOAD>(own, m.q[u], v < nvec), scale);  // the placeholder expert op
+            float f[8], acc[8];
+            unpack8<T>(out, f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+            for (unsigned left = pairs; left != 0u; left &= left - 1u) {  // k ascending
+                const int k = __ffs(left) - 1;
+                const int r = __shfl_sync(0xffffffffu, my_row, k);
+                const float w = __shfl_sync(0xffffffffu, m.w, k);
+                if (v < nvec) st_stream(rows + (size_t)r * nvec + v, out);
+                if (PUSH) fma8(f, w, acc);
             }
-            if (via_engine && i + 1 < p.ws) {
-                pending = i;
-                pending_groups = groups;
-            } else {
-                if (via_engine) {  // the last source: nothing comes after it to hide the wait behind
-                    bulk_wait_done(0);
-                    fence_async_global();
-                }
-                book(i);
+            if (PUSH && v < nvec) {
+                if (via_engine) reinterpret_cast<uint4*>(slot)[u * 32 + lane] = pack8<T>(acc);
+                else st_stream(home + v, pack8<T>(acc));
             }
         }
+        if (via_engine) {
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                uint8_t* dst = p.peer[s] + p.off_ret + (((size_t)p.rank * p.T_max + t) * nvec + v0) * 16;
+                bulk_store(dst, smem_addr(slot), (uint32_t)(min(128, nvec - v0) * 16));
+                bulk_commit();
+            }
+            ++groups;
+        }
+    };
+    auto arrived = [&](Cursor& c) {  // waits for sources; books what this warp has nothing of first
+        while (true) {
+            const int st = seek(c);
+            finish(st == kEnd ? p.ws : c.i);
+            if (st != kNotYet) return st;
+            if (lane == 0) flush();
+            while (s_seen[c.i] == 0) __nanosleep(40);  // bounded by the poller's own bounded wait
+            __syncwarp();
+        }
+    };
+    // The row and record of the next item are requested before this one's stores are issued, across sources
+    // too where the next one's rows are already here.
+    Cursor cur = {0, p.rank, 0, 0, 0, xw, false};
+    Item m;
+    int st = arrived(cur);
+    if (st == kItem) load(cur, m);
+    while (st == kItem) {
+        Cursor next = cur;
+        advance(next);
+        Item mn;
+        st = seek(next);
+        if (st == kItem) load(next, mn);
+        process(cur, m);
+        if (st == kNotYet) {
+            st = arrived(next);
+            if (st == kItem) load(next, mn);
+        } else {
+            finish(st == kEnd ? p.ws : next.i);
+        }
+        cur = next;
+        m = mn;
+    }
+    if (st == kGaveUp && lane == 0) {
+        // nothing further is processed or published; the completers are still owed this warp's bookings
+        s_dead = 1;
+        __threadfence_block();
+        bulk_wait_done(0);
+        if (pending >= 0) atomicAdd(&s_done[pending], 1);
+        for (int j = done; j < p.ws; ++j) atomicAdd(&s_done[j], 1);
     }
 }
 

@@ -151,8 +151,7 @@ __global__ void __launch_bounds__(kThreads) solo_kernel(const __grid_constant__ 
                         st_stream(row + v, q[u]);
                         float f[8];
                         unpack8<T>(q[u], f);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) acc[u][e] = fmaf(f[e], w, acc[u][e]);
+                        fma8(f, w, acc[u]);
                     }
                 }
             }

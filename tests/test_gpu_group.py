@@ -100,3 +100,32 @@ def test_nothing_begins_when_one_rank_is_refused():
         world.check()
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("schedule,payload,combine", [("pipelined", "dedup", "push"), ("phased", "direct", "pull")])
+def test_expert_op_on_every_bit_pattern(dtype, schedule, payload, combine):
+    """Subnormals, overflow, infinities and signed zeros included: dtype(float(x) * (1 + rank)) to the bit on all
+    eight ranks (a NaN stays one, whatever its payload)."""
+    ws, T, H = 8, 64, 1024
+    x = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(dtype).view(T, H)
+    idx = torch.arange(ws, dtype=torch.int32).expand(T, ws).contiguous()  # every token to every rank's one expert
+    w = torch.ones(T, ws)
+    world = LocalWorld(pkg.MoEConfig(ws, ws, H, T, dtype, dtype), ws, payload=payload, schedule=schedule, combine=combine)
+    try:
+        rds = []
+        for _ in range(ws):
+            rd = object.__new__(pkg.RankTestData)
+            rd.num_tokens, rd.x, rd.indices, rd.weights = T, x.to(DEV), idx.to(DEV), w.to(DEV)
+            rds.append(rd)
+        (world.forward_pipelined if schedule == "pipelined" else world.forward_phases)(rds)
+        for r, c in enumerate(world.ctxs):
+            _, rows, _ = c.export_dispatch()
+            want = (x.float() * (1.0 + r)).to(dtype)
+            for s in range(ws):  # the rows of source s, tokens in order
+                got = rows[0, s * T:(s + 1) * T].cpu()
+                assert torch.equal(got.isnan(), want.isnan())
+                assert torch.equal(bits(got)[~got.isnan()], bits(want)[~want.isnan()])
+        world.check()
+    finally:
+        world.close()
