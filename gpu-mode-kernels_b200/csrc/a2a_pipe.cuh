@@ -41,13 +41,13 @@ namespace a2a {
 enum PipeTicket : int { kPipeTicketDest = 0, kPipeTicketSource = 1 };
 
 // ---- shared memory of a block, carved per role --------------------------------------------
-// sender: ring [kStages][kStageBytes] | mbarriers [kStages] u64 | descriptors | list [ws][per] u16 | warp totals
+// sender: ring [kStages][kStageBytes] | mbarriers [kMaxStages] u64 | descriptors | list [ws][per] u16 | warp totals
 // router: bits [Wc][L] | wpre [Wc][L] | cnt [L] | warp totals | wire row of each token of a round
 __host__ __device__ inline int pipe_list_per(int T_max, int senders) { return (T_max + senders - 1) / (senders > 0 ? senders : 1); }
 
 __host__ __device__ inline size_t pipe_sender_smem(int T_max, int ws, int senders) {
     size_t b = (size_t)kStages * kStageBytes + 128;                       // ring + barriers
-    b += (size_t)kStages * 32;                                            // descriptors
+    b += (size_t)kMaxStages * 16;                                         // descriptors
     b += ((size_t)ws * pipe_list_per(T_max, senders) * 2 + 15) / 16 * 16; // token lists
     b += 8 * A2A_MAX_WORLD * 4;                                           // warp totals
     return b;
@@ -58,6 +58,7 @@ __host__ __device__ inline size_t pipe_router_smem(int T_max, int L) {
     return (2 * W * L + L + 16 + 256) * 4;  // bitmap, prefix, counts, warp totals, wire row of a round's tokens
 }
 
+static_assert(kMaxStages * 8 <= 128, "mbarriers of the sender ring");
 struct SendDesc {
     unsigned long long dst;  // destination address of the piece
     unsigned bytes;
@@ -121,7 +122,9 @@ struct SenderSmem {
     uint8_t* ring;
     unsigned long long* bars;
     SendDesc* desc;
-    unsigned short* list;  // [ws][per]: this block's share of every destination's token list
+    // 16-bit payload [ws][per]: this block's share of every destination's token list;
+    // FP8 [per][ws]: the wire rows of this block's tokens
+    unsigned short* list;
     int* wt;
     int per;
 };
@@ -132,14 +135,16 @@ __device__ __forceinline__ SenderSmem carve_sender(const DevParams& p, uint8_t* 
     m.ring = smem;
     m.bars = reinterpret_cast<unsigned long long*>(smem + (size_t)kStages * kStageBytes);
     m.desc = reinterpret_cast<SendDesc*>(smem + (size_t)kStages * kStageBytes + 128);
-    m.list = reinterpret_cast<unsigned short*>(m.desc + 2 * kStages);
+    m.list = reinterpret_cast<unsigned short*>(m.desc + kMaxStages);
     m.wt = reinterpret_cast<int*>(smem + pipe_sender_smem(p.T_max, p.ws, ns) - 8 * A2A_MAX_WORLD * 4);
     return m;
 }
 
-// All threads: this block's share (wire rows n with n % ns == sb) of every destination's token
-// list by ballot / popc compaction, and the total number of wire rows per destination in cnt[].
-__device__ __forceinline__ void build_send_lists(const DevParams& p, const SenderSmem& m, int sb, int ns, int* cnt) {
+// All threads: the wire row every token of this rank has at every destination, found by ballot / popc
+// compaction; take(t, d, n) is called for token t, destination d and row n by the thread that has t.  The
+// total number of wire rows per destination goes to cnt[].
+template <typename Take>
+__device__ __forceinline__ void number_wire_rows(const DevParams& p, const SenderSmem& m, int* cnt, Take take) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int base[A2A_MAX_WORLD];
 #pragma unroll
@@ -162,10 +167,7 @@ __device__ __forceinline__ void build_send_lists(const DevParams& p, const Sende
                 if (w < warp) before += c;
                 total += c;
             }
-            if ((mask >> d) & 1u) {
-                const int n = base[d] + before + __popc(b & ((1u << lane) - 1u));
-                if (n % ns == sb) m.list[d * m.per + n / ns] = (unsigned short)t;
-            }
+            if ((mask >> d) & 1u) take(t, d, base[d] + before + __popc(b & ((1u << lane) - 1u)));
             base[d] += total;
         }
         __syncthreads();
@@ -213,82 +215,113 @@ struct PendingDests {
     }
 };
 
-// Sender block `sb` of `ns`, 16-bit payload: all threads build the block's token lists; then
-// thread 0 drives the copy engine (rows go HBM -> shared-memory ring -> peer without touching a
-// register) while, if `watch_kind` >= 0, warps 1.. watch the peers' flags of that kind (they
-// start only after the set-up barrier: a watcher may wait for a long time).
+// Sender block `sb` of `ns`, 16-bit payload: all threads build the block's token lists (wire rows n with
+// n % ns == sb of every destination); then thread 0 drives the copy engine (rows go HBM -> shared-memory
+// ring -> peer without touching a register) while, if `watch_kind` >= 0, warps 1.. watch the peers' flags of
+// that kind (they start only after the set-up barrier: a watcher may wait for a long time).  In the blocks
+// without watchers a lane of warp 1 per destination draws the block's ticket for it: a fence and an atomic of
+// a microsecond each that the copies would otherwise stand still for, once per destination.
+// LOCAL: every peer's memory is on this GPU (a group stepped here).  Eight ranks of 256 tokens in one launch:
+// rows of 7168 62 -> 46 us, of 2048 (top-6 of 64) 54 -> 28.
+template <bool LOCAL>
 __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, int sb, int ns, int watch_kind,
                                             int watch_phase) {
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const SenderSmem m = carve_sender(p, smem, ns);
     uint8_t* ring = m.ring;
     unsigned long long* bars = m.bars;
     SendDesc* desc = m.desc;
     unsigned short* list = m.list;
     const int per = m.per;
+    const int row_bytes = p.H * 2;
+    // A bulk store to a peer holds its stage until the peer has acknowledged the write (measured: with two
+    // store stages a block moves 28 KB per ~1.5 us round trip whatever the link could take), local loads
+    // complete in about a microsecond: two loads ahead, four stores in flight.  Stores to this GPU's own memory
+    // are through sooner than loads: two thirds of the ring load ahead, and it is cut into as many stages as
+    // there are rows it can hold.
+    const int stage_bytes = LOCAL ? min(kStageBytes, (row_bytes + 127) / 128 * 128) : kStageBytes;
+    const int stages = LOCAL ? min(kMaxStages, kStages * kStageBytes / stage_bytes) : kStages;
+    const int look = LOCAL ? 2 * stages / 3 : 2;
     __shared__ int s_cnt[A2A_MAX_WORLD];
+    __shared__ volatile int s_through[A2A_MAX_WORLD];  // per destination: 1 its last store is complete, -1 given up
     if (tid == 0) {  // before the lists: thread 0 can issue its first loads the moment they are built
-        for (int s = 0; s < kStages; ++s) mbar_init(smem_addr(bars + s), 1);
+        for (int s = 0; s < stages; ++s) mbar_init(smem_addr(bars + s), 1);
         mbar_fence_init();
     }
-    build_send_lists(p, m, sb, ns, s_cnt);
+    if (tid < A2A_MAX_WORLD) s_through[tid] = 0;
+    number_wire_rows(p, m, s_cnt, [&](int t, int d, int n) {
+        if (n % ns == sb) list[d * per + n / ns] = (unsigned short)t;
+    });
     __syncthreads();
     stamp(p, kStampSetup + 0);
+    const uint32_t expected = (uint32_t)(ns + p.routers);  // every sender block + the destination's router blocks
+    const bool helped = watch_kind < 0;
     if (tid != 0) {
-        if (watch_kind >= 0 && warp > 0) watcher_role(p, watch_kind, watch_phase, warp - 1);
+        if (!helped) {
+            if (warp > 0) watcher_role(p, watch_kind, watch_phase, warp - 1);
+        } else if (warp == 1 && lane < p.ws && lane != p.rank) {
+            // bounded by thread 0's own bounded waits; inside the loop, so that no lane waits for another to leave it
+            for (int seen = 0; seen == 0;) {
+                seen = s_through[lane];
+                if (seen > 0) {
+                    arrive_dest(p, lane, expected);
+                    stamp_by(p, kStampDestDone + (lane - p.rank + p.ws) % p.ws, true);
+                } else {
+                    __nanosleep(40);
+                }
+            }
+        }
         return;
     }
 
     // ---- one thread drives the copy engine ----------------------------------------------
-    const uint32_t expected = (uint32_t)(ns + p.routers);  // every sender block + the destination's router blocks
     auto arrive = [&](int d) {
-        arrive_dest(p, d, expected);
-        stamp(p, kStampDestDone + (d - p.rank + p.ws) % p.ws);
+        if (helped) {
+            fence_async_global();
+            __threadfence_block();
+            s_through[d] = 1;
+        } else {
+            arrive_dest(p, d, expected);
+            stamp(p, kStampDestDone + (d - p.rank + p.ws) % p.ws);
+        }
     };
-    const int row_bytes = p.H * 2;
-    const int pieces = (row_bytes + kStageBytes - 1) / kStageBytes;
-    long long total = 0;
+    const int pieces = (row_bytes + stage_bytes - 1) / stage_bytes;
+    int total = 0;
     for (int i = 1; i < p.ws; ++i) {
         const int d = (p.rank + i) % p.ws;
         const int mine = s_cnt[d] > sb ? (s_cnt[d] - sb + ns - 1) / ns : 0;
         if (mine == 0) arrive(d);  // nothing of ours goes there
-        total += (long long)mine * pieces;
+        total += mine * pieces;
     }
-    // A bulk store to a peer holds its stage until the peer has acknowledged the write (measured: with two
-    // store stages a block moves 28 KB per ~1.5 us round trip whatever the link could take), local loads
-    // complete in about a microsecond: two loads ahead, four stores in flight.
-    constexpr int kLook = 2;
-    int g_step = 1, g_i = 0, g_piece = 0;  // generator of the next piece to load
+    // generator of the next piece to load: row g_i of g_mine of destination g_d, the g_step-th from here
+    int g_step = 0, g_d = p.rank, g_i = 0, g_mine = 0, g_piece = 0;
     auto skip_empty = [&] {
-        while (g_step < p.ws) {
-            const int d = (p.rank + g_step) % p.ws;
-            const int mine = s_cnt[d] > sb ? (s_cnt[d] - sb + ns - 1) / ns : 0;
-            if (g_i < mine) break;
-            ++g_step;
+        while (g_i >= g_mine && ++g_step < p.ws) {
+            g_d = g_d + 1 == p.ws ? 0 : g_d + 1;
+            g_mine = s_cnt[g_d] > sb ? (s_cnt[g_d] - sb + ns - 1) / ns : 0;
             g_i = 0;
         }
     };
     skip_empty();
     PendingDests pending;
     bool failed = false;
-    for (long long q = 0; q < total + kLook && !failed; ++q) {
+    int st_in = 0, st_out = 0;  // stage of the next load and of the next store
+    uint32_t parity = 0;
+    for (int q = 0; q < total + look && !failed; ++q) {
         if (q < total) {
-            const int st = (int)(q % kStages);
-            if (q >= kStages) bulk_wait_read<kStages - kLook - 1>();  // the store that used this stage has read it
-            const int d = (p.rank + g_step) % p.ws;
-            const int mine = (s_cnt[d] - sb + ns - 1) / ns;
+            if (q >= stages) bulk_wait_read(stages - look - 1);  // the store that used this stage has read it
             const int n = sb + g_i * ns;  // wire row index at the destination
-            const int t = list[d * per + g_i];
-            const int off = g_piece * kStageBytes;
-            const unsigned bytes = (unsigned)min(kStageBytes, row_bytes - off);
+            const int t = list[g_d * per + g_i];
+            const int off = g_piece * stage_bytes;
+            const unsigned bytes = (unsigned)min(stage_bytes, row_bytes - off);
             const uint8_t* src = reinterpret_cast<const uint8_t*>(p.x) + (size_t)t * row_bytes + off;
-            uint8_t* dst = p.peer[d] + p.off_stage + ((size_t)p.rank * p.T_max + n) * p.stage_row_bytes + off;
+            uint8_t* dst = p.peer[g_d] + p.off_stage + ((size_t)p.rank * p.T_max + n) * p.stage_row_bytes + off;
             const bool last_piece = (g_piece == pieces - 1);
-            desc[st].dst = reinterpret_cast<unsigned long long>(dst);
-            desc[st].bytes = bytes;
-            desc[st].dest_done = (last_piece && g_i == mine - 1) ? d : -1;
-            mbar_expect_tx(smem_addr(bars + st), bytes);
-            bulk_load(smem_addr(ring + (size_t)st * kStageBytes), src, bytes, smem_addr(bars + st));
+            mbar_expect_tx(smem_addr(bars + st_in), bytes);
+            bulk_load(smem_addr(ring + (size_t)st_in * stage_bytes), src, bytes, smem_addr(bars + st_in));
+            desc[st_in].dst = reinterpret_cast<unsigned long long>(dst);
+            desc[st_in].bytes = bytes;
+            desc[st_in].dest_done = (last_piece && g_i == g_mine - 1) ? g_d : -1;
             if (q == 0) stamp(p, kStampSetup + 1);
             if (last_piece) {
                 g_piece = 0;
@@ -297,14 +330,12 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
             } else {
                 ++g_piece;
             }
+            st_in = st_in + 1 == stages ? 0 : st_in + 1;
         }
-        if (q >= kLook) {
-            const long long it = q - kLook;
-            const int st = (int)(it % kStages);
-            const uint32_t parity = (uint32_t)((it / kStages) & 1);
+        if (q >= look) {
             // the load is local and cannot be late by more than microseconds; bounded all the same
             long long t0 = 0;
-            for (int spins = 0; !mbar_try_wait(smem_addr(bars + st), parity); ++spins) {
+            for (int spins = 0; !mbar_try_wait(smem_addr(bars + st_out), parity); ++spins) {
                 if (spins == 0) t0 = global_ns();
                 else if (global_ns() - t0 > p.timeout_ns) {
                     record_timeout(p, kPhaseSend, -1, p.epoch);
@@ -313,99 +344,123 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
                 }
             }
             if (failed) break;
-            bulk_store(reinterpret_cast<void*>(desc[st].dst), smem_addr(ring + (size_t)st * kStageBytes), desc[st].bytes);
+            bulk_store(reinterpret_cast<void*>(desc[st_out].dst), smem_addr(ring + (size_t)st_out * stage_bytes), desc[st_out].bytes);
             bulk_commit();
-            if (it == 0) stamp(p, kStampSetup + 2);
-            if (desc[st].dest_done >= 0) pending.push(desc[st].dest_done, it);  // group `it` was the destination's last
-            pending.drain(it + 1, kArrivalLag, arrive);
+            if (q == look) stamp(p, kStampSetup + 2);
+            if (desc[st_out].dest_done >= 0) pending.push(desc[st_out].dest_done, q - look);  // that group was the destination's last
+            pending.drain(q - look + 1, kArrivalLag, arrive);
+            if (++st_out == stages) {
+                st_out = 0;
+                parity ^= 1u;
+            }
         }
     }
     bulk_wait_done(0);  // nothing of ours is in flight when the block moves on
     if (!failed)
         while (!pending.empty()) pending.drain(1LL << 40, 0, arrive);
+    else
+        for (int d = 0; d < p.ws; ++d)
+            if (s_through[d] == 0) s_through[d] = -1;
 }
 
-// Sender block `sb` of `ns`, FP8 payload: the whole block quantises one wire row at a time (the
-// arithmetic -- an IEEE division per value -- is the cost here, so all eight warps share a row):
-// 16-byte loads, amax over the 16 lanes of a 128-value block, e4m3 bytes and fp32 scales into one of
-// eight 12 KB stages of the ring, then thread 0 hands the finished wire row to the copy engine and
-// the block goes on to the next row while up to seven stores are still on their way.
+// Sender block `sb` of `ns`, FP8 payload: the tokens t with t % ns == sb, one after the other.  The whole
+// block quantises a token's row ONCE (the arithmetic -- an IEEE division per value -- is the cost here: a row
+// goes to four or five ranks of eight, and quantising it for each took 131 us where this takes 44, eight ranks of 256 tokens of 7168 in one launch):
+// 16-byte loads, requested a row ahead, amax over the 16 lanes of a 128-value block, e4m3 bytes and fp32
+// scales into one of eight 12 KB stages of the ring; then thread 0 hands the finished wire row to the copy
+// engine once per destination and the block goes on to the next row while up to six rows are still on their
+// way.  All destinations are through at the end, each booked by a thread of its own.
 constexpr int kFp8Stages = 8;
 constexpr int kWarpStageBytes = kStages * kStageBytes / kFp8Stages;  // 12 KB: the largest FP8 wire row
 
 template <typename T>
 __device__ __forceinline__ void sender_role_fp8(const DevParams& p, uint8_t* smem, int sb, int ns) {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, ws = p.ws;
     const SenderSmem m = carve_sender(p, smem, ns);
     __shared__ int s_cnt[A2A_MAX_WORLD];
-    build_send_lists(p, m, sb, ns, s_cnt);
+    const int mine = p.T > sb ? (p.T - sb + ns - 1) / ns : 0;
+    for (int i = tid; i < mine * ws; i += kThreads) m.list[i] = 0xffffu;  // no row there: rows end at 65534
+    __syncthreads();
+    number_wire_rows(p, m, s_cnt, [&](int t, int d, int n) {
+        if (t % ns == sb && d != p.rank) m.list[t / ns * ws + d] = (unsigned short)n;
+    });
     __syncthreads();
     stamp(p, kStampSetup + 0);
-    const uint32_t expected = (uint32_t)(ns + p.routers);
-    auto arrive = [&](int d) {  // thread 0 only
-        arrive_dest(p, d, expected);
-        stamp(p, kStampDestDone + (d - p.rank + p.ws) % p.ws);
-    };
     const int nvec = p.H >> 3;
-    PendingDests pending;  // thread 0's bookkeeping, as in the 16-bit sender
-    long long q = 0;       // rows this block has sent so far
-    for (int i = 1; i < p.ws; ++i) {
-        const int d = (p.rank + i) % p.ws;
-        const int mine = s_cnt[d] > sb ? (s_cnt[d] - sb + ns - 1) / ns : 0;
-        if (mine == 0) {
-            if (tid == 0) arrive(d);  // nothing of ours goes there
-            continue;
+    auto next_token = [&](int g) {  // the first of this block's tokens after the g-th that has to travel
+        while (++g < mine) {
+            bool any = false;
+            for (int d = 0; d < ws; ++d) any |= m.list[g * ws + d] != 0xffffu;
+            if (any) break;
         }
-        for (int g = 0; g < mine; ++g, ++q) {
-            const int n = sb + g * ns;
-            const int t = m.list[d * m.per + g];
-            uint8_t* stage = m.ring + (size_t)(q % kFp8Stages) * kWarpStageBytes;
-            if (tid == 0 && q >= kFp8Stages) bulk_wait_read<kFp8Stages - 1>();  // the store that used this stage has read it
-            __syncthreads();
-            const uint4* src = reinterpret_cast<const uint4*>(p.x) + (size_t)t * nvec;
-            for (int v0 = 0; v0 < nvec; v0 += 4 * kThreads) {
-                uint4 qv[4];
+        return g;
+    };
+    constexpr int kAhead = 4;  // vectors per thread that are requested together
+    auto load = [&](int g, int v0, uint4 (&q)[kAhead]) {
+        const uint4* src = reinterpret_cast<const uint4*>(p.x) + (size_t)(sb + g * ns) * nvec;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int v = v0 + u * kThreads + tid;
-                    if (v < nvec) qv[u] = ld_input(src + v);
+        for (int u = 0; u < kAhead; ++u) {
+            const int v = v0 + u * kThreads + tid;
+            if (v < nvec) q[u] = ld_input(src + v);
+        }
+    };
+    int g = next_token(-1);
+    uint4 q[kAhead], qn[kAhead];
+    if (g < mine) load(g, 0, q);
+    for (int stage_no = 0; g < mine; stage_no = (stage_no + 1) % kFp8Stages) {
+        const int gn = next_token(g);
+        if (gn < mine) load(gn, 0, qn);
+        uint8_t* stage = m.ring + (size_t)stage_no * kWarpStageBytes;
+        for (int v0 = 0; v0 < nvec; v0 += kAhead * kThreads) {
+            if (v0 > 0) load(g, v0, q);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int v = v0 + u * kThreads + tid;  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
+                float f[8];
+                float amax = 0.f;
+                if (v < nvec) {
+                    unpack8<T>(q[u], f);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int v = v0 + u * kThreads + tid;  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
-                    float f[8];
-                    float amax = 0.f;
-                    if (v < nvec) {
-                        unpack8<T>(qv[u], f);
+                for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                if (v < nvec) {
+                    const float sc = amax > 0.f ? amax / 448.f : 1.f;
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
-                    }
-#pragma unroll
-                    for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                    if (v < nvec) {
-                        const float sc = amax > 0.f ? amax / 448.f : 1.f;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) f[e] = f[e] / sc;
-                        reinterpret_cast<uint2*>(stage)[v] = pack8_e4m3(f);
-                        if ((v & 15) == 0) reinterpret_cast<float*>(stage + p.H)[v >> 4] = sc;
-                    }
+                    for (int e = 0; e < 8; ++e) f[e] = f[e] / sc;
+                    reinterpret_cast<uint2*>(stage)[v] = pack8_e4m3(f);
+                    if ((v & 15) == 0) reinterpret_cast<float*>(stage + p.H)[v >> 4] = sc;
                 }
             }
-            fence_async_smem();  // every thread's ordinary stores to the stage, before the copy engine reads it
-            __syncthreads();
-            if (tid == 0) {
+        }
+        fence_async_smem();  // every thread's ordinary stores to the stage, before the copy engine reads it
+        // the row that used the next stage, eight rows before the next one, has been read: six may be unread
+        if (tid == 0) bulk_wait_read<kFp8Stages - 2>();
+        __syncthreads();
+        if (tid == 0) {
+            for (int i = 1; i < ws; ++i) {
+                const int d = (p.rank + i) % ws;
+                const int n = m.list[g * ws + d];
+                if (n == 0xffff) continue;
                 uint8_t* dst = p.peer[d] + p.off_stage + ((size_t)p.rank * p.T_max + n) * p.stage_row_bytes;
                 bulk_store(dst, smem_addr(stage), (uint32_t)p.stage_row_bytes);
-                bulk_commit();
-                if (q == 0) stamp(p, kStampSetup + 2);
-                if (g == mine - 1) pending.push(d, q);  // the block's last row for d
-                pending.drain(q + 1, kArrivalLag, arrive);
             }
+            bulk_commit();
         }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) q[u] = qn[u];
+        g = gn;
     }
     if (tid == 0) {
         bulk_wait_done(0);
-        while (!pending.empty()) pending.drain(1LL << 40, 0, arrive);
+        fence_async_global();
+    }
+    __syncthreads();
+    if (tid > 0 && tid < ws) {
+        const int d = (p.rank + tid) % ws;
+        arrive_dest(p, d, (uint32_t)(ns + p.routers));
+        stamp_by(p, kStampDestDone + tid, true);
     }
 }
 
@@ -1023,7 +1078,7 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
             sender_role_fp8<T>(p, a2a_pipe_smem, b - nw, ns);
         } else {
             stamp_value(p, kStampRole, b < 2 ? (kRoleSender | kRoleWatcher) : kRoleSender);
-            sender_role(p, a2a_pipe_smem, b, ns, b == 0 ? kFlagDispatch : (b == 1 ? kFlagExpert : -1),
+            sender_role<false>(p, a2a_pipe_smem, b, ns, b == 0 ? kFlagDispatch : (b == 1 ? kFlagExpert : -1),
                         b == 0 ? kPhaseRecv : kPhaseCombine);
         }
         stamp(p, kStampSent);
@@ -1060,7 +1115,8 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_con
     if (ROLE == 0) {
         if (b < ns) {
             if (PAYLOAD == A2A_PAYLOAD_FP8) sender_role_fp8<T>(p, a2a_pipe_smem, b, ns);
-            else sender_role(p, a2a_pipe_smem, b, ns, -1, 0);
+            else if (g.n > 1) sender_role<true>(p, a2a_pipe_smem, b, ns, -1, 0);
+            else sender_role<false>(p, a2a_pipe_smem, b, ns, -1, 0);
         } else {
             const int rb = b - ns, d = (p.rank + 1 + rb % p.ws) % p.ws;
             router_role(p, a2a_pipe_smem, d, rb / p.ws, p.routers, rb == 0, (uint32_t)(d == p.rank ? 0 : ns) + p.routers);
