@@ -9,6 +9,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch
+
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "liba2a.so")
 
@@ -88,6 +90,8 @@ SIGNATURES = {
 }
 
 _lib = None
+# torch.cuda.current_stream() builds a Stream object first: 1 us a call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
 
 
 def load() -> C.CDLL:
@@ -105,6 +109,11 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def current_stream() -> int:
+    """The current CUDA stream of the current device, as the C ABI takes it."""
+    return _raw_stream(torch.cuda.current_device())
 
 
 def strerror(code: int) -> str:

@@ -141,7 +141,15 @@ class A2AContext:
 
     def _check_inputs(self, x, indices, weights, y, on_device: bool) -> int:
         """The library reads raw pointers: refuse anything whose bytes would be misread."""
-        n, K, H = x.shape[0], self.cfg.experts_per_token, self.cfg.hidden_dim
+        cfg, place = self.cfg, self.device_index if on_device else -1  # get_device(): -1 for a host tensor
+        n, K, H = x.shape[0], cfg.experts_per_token, cfg.hidden_dim
+        if (y is None and x.dtype is cfg.in_dtype and indices.dtype is torch.int32 and weights.dtype is torch.float32
+                and x.shape == (n, H) and indices.shape == (n, K) and weights.shape == (n, K)
+                and x.is_contiguous() and indices.is_contiguous() and weights.is_contiguous()
+                and x.get_device() == place and indices.get_device() == place and weights.get_device() == place
+                and x.is_cuda is on_device and indices.is_cuda is on_device and weights.is_cuda is on_device):
+            return n
+        # something is wrong, or unusual: look again, one thing at a time
         bad = None
         if x.dtype != self.cfg.in_dtype or tuple(x.shape) != (n, H):
             bad = f"x must be [{n}, {H}] {self.cfg.in_dtype}, got {tuple(x.shape)} {x.dtype}"
@@ -172,7 +180,10 @@ class A2AContext:
         if y is None:
             y = torch.empty(n, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=self.device)
         self._num_tokens = n
-        _lib.check(self.lib.a2a_forward(self._h, _ptr(x), _ptr(indices), _ptr(weights), _ptr(y), n, self._stream()))
+        rc = self.lib.a2a_forward(self._h, x.data_ptr(), indices.data_ptr(), weights.data_ptr(), y.data_ptr(), n,
+                                  _lib.current_stream())
+        if rc != 0:
+            _lib.check(rc)
         return y
 
     def pipe_step(self, role: int, x=None, indices=None, weights=None, y=None) -> Optional[torch.Tensor]:
@@ -255,7 +266,7 @@ class A2AContext:
 
     def peek(self) -> int:
         """The recorded error code (0 = none) without any CUDA call: a read of mapped host memory."""
-        return int(self.lib.a2a_status_peek(self._h))
+        return self.lib.a2a_status_peek(self._h)
 
     def raise_and_clear_if_failed(self) -> None:
         """What the plugin entry does before every call: if an earlier call recorded an error,
@@ -372,14 +383,16 @@ def custom_kernel(data: input_t, payload: Optional[str] = None, schedule: Option
     payload = payload or DEFAULT_PAYLOAD
     schedule = schedule or DEFAULT_SCHEDULE
     combine = combine or DEFAULT_COMBINE
-    device_index = x.device.index if x.is_cuda else torch.cuda.current_device()
+    on_device = x.is_cuda
+    device_index = x.get_device() if on_device else torch.cuda.current_device()
     ctx = _context_for(cfg, rank, world_size, device_index, payload, schedule, combine)
-    ctx.raise_and_clear_if_failed()
-    if idx.dtype != torch.int32:
+    if ctx.peek():
+        ctx.raise_and_clear_if_failed()
+    if idx.dtype is not torch.int32:
         idx = idx.to(torch.int32)
-    if w.dtype != torch.float32:
+    if w.dtype is not torch.float32:
         w = w.to(torch.float32)
-    if x.is_cuda:
+    if on_device:
         return ctx.forward(x.contiguous(), idx.contiguous(), w.contiguous())
     y = ctx.forward_host(x.contiguous(), idx.contiguous(), w.contiguous())
     torch.cuda.current_stream().synchronize()

@@ -8,7 +8,6 @@ there is no CPU or PyTorch fallback.
 """
 from __future__ import annotations
 
-import ctypes as C
 from typing import Tuple
 
 import torch
@@ -20,15 +19,18 @@ NUM_BINS = 256
 
 def histogram256(data: torch.Tensor, output: torch.Tensor) -> torch.Tensor:
     """Counts of the byte values of ``data`` into ``output`` on the current stream; returns ``output``."""
-    if data.dtype != torch.uint8 or not data.is_cuda or not data.is_contiguous() or data.dim() != 1:
+    if data.dtype is not torch.uint8 or not data.is_cuda or not data.is_contiguous() or data.dim() != 1:
         raise _lib.A2AError(_lib.A2A_ERR_CONFIG, f"data must be a contiguous 1-D uint8 CUDA tensor, got {data.dtype} {tuple(data.shape)} on {data.device}")
-    if (output.dtype != torch.int64 or output.numel() != NUM_BINS or not output.is_contiguous()
-            or output.device != data.device):
+    device = data.get_device()
+    if (output.dtype is not torch.int64 or output.numel() != NUM_BINS or not output.is_contiguous()
+            or not output.is_cuda or output.get_device() != device):
         raise _lib.A2AError(_lib.A2A_ERR_CONFIG, f"output must be a contiguous int64 [{NUM_BINS}] tensor on {data.device}")
-    lib = _lib.load()
-    with torch.cuda.device(data.device):
-        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
-        _lib.check(lib.a2a_histogram256(C.c_void_p(data.data_ptr()), data.numel(), C.c_void_p(output.data_ptr()), stream))
+    if device != torch.cuda.current_device():
+        with torch.cuda.device(device):
+            return histogram256(data, output)
+    rc = _lib.load().a2a_histogram256(data.data_ptr(), data.numel(), output.data_ptr(), _lib.current_stream())
+    if rc != 0:
+        _lib.check(rc)
     return output
 
 

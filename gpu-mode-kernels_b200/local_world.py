@@ -32,8 +32,8 @@ class LocalWorld:
         A2AContext.attach_local(self.ctxs)
 
     def _step(self, phase: str, calls=None) -> None:
-        handles = (C.c_void_p * self.world_size)(*[c._h for c in self.ctxs])
-        _lib.check(self.ctxs[0].lib.a2a_group_step(handles, _lib.GROUP_PHASE[phase], calls, A2AContext._stream()))
+        handles = (C.c_void_p * self.world_size)(*[c._h.value for c in self.ctxs])
+        _lib.check(self.ctxs[0].lib.a2a_group_step(handles, _lib.GROUP_PHASE[phase], calls, _lib.current_stream()))
 
     def _send(self, rank_datas: Sequence) -> None:
         """route + dispatch_send on every rank, in one launch."""
