@@ -1,6 +1,7 @@
 // liba2a.so -- host side of the C ABI declared in include/a2a.h: context life cycle,
 // symmetric-region layout, CUDA-IPC peer mapping and kernel launches.  No torch
 // types, no allocation and no host synchronisation on the data path.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -344,14 +345,45 @@ int launch_ranks(a2a_ctx* const* cs, int n, GroupFn fn, int blocks, int smem, cu
 // more warps with less to do each finish sooner (one token of 2048: 4.1 against 4.2 and 4.6 us).  Two
 // blocks per SM: with a third or fourth that does not fit beside them a second, nearly empty wave of
 // blocks starts after the first (headline 13.2 us).
-int launch_solo(a2a_ctx* c, cudaStream_t st) {
-    const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = 2LL * c->num_sms;
+// Rows in host memory: half an SM's worth of warps fills the link, and more only get in each other's way
+// (3.7 MB read and as much written by 74 / 148 / 296 blocks: 100 / 107 / 118 us).
+int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
+    const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = host_rows ? c->num_sms / 2 : 2LL * c->num_sms;
     const long long two = c->cur_tokens * ((nvec + 63) / 64), one = c->cur_tokens * ((nvec + 31) / 32);
     const bool wide = two >= cap * warps;
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     return launch(c, wide ? solo_fn<2>(c) : solo_fn<1>(c), (int)blocks, 0, st);
+}
+
+// The device address of host memory that kernels can reach -- pinned, all `bytes` of it in one allocation or
+// registration -- or nullptr.
+void* mapped_address(const void* host, size_t bytes) {
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 12000, cudaEnableDefault, &found);
+        return reinterpret_cast<Query>(e == cudaSuccess && found == cudaDriverEntryPointSuccess ? fn : nullptr);
+    }();
+    if (query == nullptr) return nullptr;
+    unsigned type = 0;
+    CUdeviceptr device = 0, start = 0;
+    size_t size = 0;
+    // attributes of memory the driver does not know come back as zeros
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* into[] = {&type, &device, &start, &size};
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(host);
+    if (query(4, what, into, at) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || device == 0) return nullptr;
+    if (at < start || at + bytes > start + size) return nullptr;
+    return reinterpret_cast<void*>(device);
+}
+
+inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
 }
 
 int check_call(const a2a_ctx* c, const int32_t* idx, int T) {
@@ -864,6 +896,27 @@ int a2a_forward_host(a2a_ctx* c, const void* x, const int32_t* idx, const float*
     DeviceGuard guard(c->cfg.device);
     cudaStream_t st = as_stream(stream);
     const size_t row = (size_t)c->cfg.hidden_dim * 2, tk = (size_t)T * c->cfg.experts_per_token * 4;
+    if (T > 0 && c->cfg.world_size == 1 && c->cfg.schedule == A2A_SCHEDULE_PIPELINED) {
+        // One rank reads every row once and writes every output once: where the kernel can reach the caller's
+        // memory it does so itself, and the link carries both directions at the same time instead of one copy
+        // after the other (256 tokens of 7168: 135 us a call, 192 with copies around the kernel).  The indices, which
+        // every block reads, are copied.
+        void *dx, *dw, *dy;
+        if (!overlap(y, row * T, x, row * T) && !overlap(y, row * T, w, tk) && !overlap(y, row * T, idx, tk) &&
+            (dx = mapped_address(x, row * T)) != nullptr && (dw = mapped_address(w, tk)) != nullptr &&
+            (dy = mapped_address(y, row * T)) != nullptr && rows_aligned(dx) && rows_aligned(dy) &&
+            reinterpret_cast<uintptr_t>(dw) % 4 == 0) {
+            CUDA_TRY(cudaMemcpyAsync(c->h_idx, idx, tk, cudaMemcpyHostToDevice, st));
+            const int r = begin_call(c, c->h_idx, T);
+            if (r != A2A_OK) return r;
+            c->p.x = dx;
+            c->p.w = static_cast<const float*>(dw);
+            c->p.y = dy;
+            const int rc = launch_solo(c, st, /*host_rows=*/true);
+            if (rc == A2A_OK) c->sent = true;
+            return rc;
+        }
+    }
     if (T > 0) {
         CUDA_TRY(cudaMemcpyAsync(c->h_idx, idx, tk, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(c->h_x, x, row * T, cudaMemcpyHostToDevice, st));

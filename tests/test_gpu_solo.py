@@ -104,3 +104,48 @@ def test_dropped_pairs_match_the_stepped_roles_and_phases_can_follow():
     finally:
         ctx.close()
         world.close()
+
+
+@pytest.mark.parametrize("place", ["pinned", "pageable", "pinned_x_only", "off_alignment", "in_place", "spans_two"])
+@pytest.mark.parametrize("K,H,T,n,payload", [(2, 8, 1, 1, "dedup"), (6, 2056, 93, 80, "dedup"), (8, 1024, 300, 300, "fp8")])
+def test_host_tensors_wherever_they_live(place, K, H, T, n, payload):
+    """Pinned rows are read and written by the kernel itself, all others copied: the bits of the device call
+    either way."""
+    cfg, rd, _, _ = pkg.generate_input(16, K, H, T, seed=21, rank=0, world_size=1, weights="rand")
+    x, idx, w = rd.x[:n].contiguous(), rd.indices[:n].contiguous(), rd.weights[:n].contiguous()
+    ctx = A2AContext(cfg, 0, 1, device=0, payload=payload, schedule="pipelined", combine="push")
+    pinned = []
+    try:
+        want = bits(ctx.forward(x.to(DEV), idx.to(DEV), w.to(DEV))).cpu()
+        y = torch.empty(n, H, dtype=cfg.out_dtype, pin_memory=place != "pageable")
+        if place != "pageable":
+            x = x.pin_memory()
+        if place in ("pinned", "in_place"):
+            idx, w = idx.pin_memory(), w.pin_memory()
+        if place == "off_alignment":  # two bytes past a 16-byte boundary
+            base = torch.empty(n * H + 8, dtype=x.dtype, pin_memory=True)
+            x = base[1:1 + n * H].view(n, H).copy_(x)
+        if place == "in_place":
+            y = x
+        if place == "spans_two":  # only the first page of the rows is registered
+            base = torch.empty(n * H * 2 + 8192, dtype=torch.uint8)
+            at = -base.data_ptr() % 4096
+            x = base[at:at + n * H * 2].view(x.dtype).view(n, H).copy_(x)
+            assert torch.cuda.cudart().cudaHostRegister(x.data_ptr(), 4096, 0) == torch.cuda.cudart().cudaError.success
+            pinned.append(x.data_ptr())
+        if place == "spans_two" and n * H * 2 > 4096:  # the copy refuses such rows; so does what replaces it
+            with pytest.raises(_lib.A2AError):
+                ctx.forward_host(x, idx, w, y)
+            return
+        got = ctx.forward_host(x, idx, w, y)
+        torch.cuda.synchronize()
+        ctx.check()
+        assert torch.equal(bits(got), want)
+        again = torch.empty(n, H, dtype=cfg.out_dtype, device=DEV)  # the phases after it find what they need
+        _lib.check(ctx.lib.a2a_combine(ctx._h, w.to(DEV).data_ptr(), again.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(bits(again).cpu(), want)
+    finally:
+        torch.cuda.synchronize()
+        for ptr in pinned:
+            torch.cuda.cudart().cudaHostUnregister(ptr)
+        ctx.close()
