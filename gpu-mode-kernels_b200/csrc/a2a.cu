@@ -322,6 +322,7 @@ int launch_ranks(a2a_ctx* const* cs, int n, GroupFn fn, int blocks, int smem, cu
     GroupParams g;
     for (int r = 0; r < n; ++r) {
         g.p[r] = call_params(cs[r]);
+        g.p[r].local = n > 1;
         adjust(g.p[r]);
         cs[r]->launches++;
     }
@@ -518,15 +519,15 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
     return rc;
 }
 
-// Roles 1 and 2: a watcher block and this rank's share of two blocks per SM (of four or eight, where a
-// group shares the launch: 134 us against 145 and 159 for role 1 of the workload named above).
+// Roles 1 and 2: this rank's share of two blocks per SM (of four or eight, where a group shares the launch:
+// 134 us against 145 and 159 for role 1 of the workload named above) and, for peers elsewhere, a watcher block.
 int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
     for (int r = 0; r < n; ++r)
         if (!cs[r]->sent) return A2A_ERR_STATE;
     const a2a_ctx* c = cs[0];
     const int blocks = c->num_sms * 2 / n;
     const int smem = role == 1 && c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
-    return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), 1 + (blocks < 1 ? 1 : blocks), smem, st);
+    return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), n > 1 ? blocks : 1 + blocks, smem, st);
 }
 
 // The contexts of every rank of one group, all on one GPU?

@@ -93,6 +93,7 @@ struct DevParams {
     int chunks;             // token chunks per call, 1..kMaxChunks (same on every rank)
     int wpc;                // 32-token bitmap words per chunk: chunk c = tokens [32*c*wpc, 32*(c+1)*wpc)
     uint32_t epoch;
+    int local;              // a group stepped on this GPU: every peer's memory is here, and its phases ran or run here
     long long timeout_ns;
     // local scratch of this rank
     int* slot;              // [T_max*K] slot of pair (t,k) inside slab (expert, this rank), -1 = dropped
@@ -286,6 +287,19 @@ __device__ __forceinline__ int chunk_end(const DevParams& p, int c) {
 
 __device__ __forceinline__ uint32_t* seen_ptr(const DevParams& p, int kind, int index) {
     return p.seen + ((size_t)kind * A2A_MAX_WORLD + index) * kFlagStride;
+}
+
+// What the blocks of this GPU wait on for rank `index`'s flag of `kind`: the word a watcher hands on, or,
+// where the writer's blocks are on this GPU too, the flag itself (gpu scope is enough between them, and
+// there is no watcher to wait for: two memory round trips and a system fence less).
+__device__ __forceinline__ const uint32_t* await_ptr(const DevParams& p, int kind, int index) {
+    return p.local && index != p.rank ? flag_ptr(p.peer[p.rank], p.off_flags, kind, index) : seen_ptr(p, kind, index);
+}
+
+// Fence in front of a flag a peer reads.
+__device__ __forceinline__ void fence_for_peers(const DevParams& p) {
+    if (p.local) fence_acq_rel_gpu();
+    else fence_acq_rel_sys();
 }
 
 // Watcher duty: wait for peer `index`'s flag of `kind` at system scope, then hand it to

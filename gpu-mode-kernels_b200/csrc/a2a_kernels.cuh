@@ -116,7 +116,7 @@ __device__ __forceinline__ void publish_flags(const DevParams& p, int kind, uint
     __syncthreads();  // whatever the block wrote for this publication has been issued
     if (tid == 0) st_release_gpu(seen_ptr(p, kind, p.rank), value);  // fence.gpu + store
     if (p.ws > 1) {
-        if (tid == 0) __threadfence_system();  // orders every block's rows (seen through the tickets) for the peers
+        if (tid == 0) fence_for_peers(p);  // orders every block's rows (seen through the tickets) for the peers
         __syncthreads();
         if (tid < p.ws && tid != p.rank) st_relaxed_sys(flag_ptr(p.peer[tid], p.off_flags, kind, p.rank), value);
     }
@@ -356,9 +356,9 @@ __device__ __forceinline__ void expert_chunk(const DevParams& p, const BlockSmem
             // part 0 watches a peer's flag at system scope and hands it on; the rest, and everybody
             // for our own rank (whose publisher writes the local word itself), wait locally
             if (tid == 0)
-                s_seen = (part == 0 && s != p.rank
+                s_seen = (part == 0 && s != p.rank && !p.local
                               ? watch_and_republish(p, kFlagDispatch, s, kPhaseRecv, want)
-                              : wait_flag_gpu(seen_ptr(p, kFlagDispatch, s), want, p, kPhaseRecv, s)) ? 1 : 0;
+                              : wait_flag_gpu(await_ptr(p, kFlagDispatch, s), want, p, kPhaseRecv, s)) ? 1 : 0;
             __syncthreads();
             const int seen = s_seen;
             __syncthreads();
@@ -409,7 +409,7 @@ __device__ __forceinline__ void combine_phase(const DevParams& p, int cb, int nc
     const int items = (tb - ta) * nseg;
     // warp d of the grid watches rank d's flag for this chunk before its own items (unless the
     // caller has watchers of its own)
-    if (own_watchers && warp < p.ws && warp != p.rank && lane == 0)
+    if (own_watchers && !p.local && warp < p.ws && warp != p.rank && lane == 0)
         watch_and_republish(p, kFlagExpert, warp, kPhaseCombine, want);
     __syncwarp();
     unsigned ready = 0u;  // ranks this lane has already seen ready for this chunk
@@ -428,7 +428,7 @@ __device__ __forceinline__ void combine_phase(const DevParams& p, int cb, int nc
                 // other blocks of this grid may still be writing) was complete when the rows left.
                 const int d = e / p.L, l = e - d * p.L;
                 if (!((ready >> d) & 1u)) {
-                    ok = wait_flag_gpu(seen_ptr(p, kFlagExpert, d), want, p, kPhaseCombine, d);
+                    ok = wait_flag_gpu(await_ptr(p, kFlagExpert, d), want, p, kPhaseCombine, d);
                     ready |= 1u << d;
                 }
                 const int j = ok ? ld_stream(p.slot + pair) : -1;

@@ -99,7 +99,7 @@ __device__ __forceinline__ void arrive_dest(const DevParams& p, int d, uint32_t 
         if (d == p.rank) {
             st_release_gpu(seen_ptr(p, kFlagDispatch, p.rank), flag_value(p, 0));
         } else {
-            fence_acq_rel_sys();
+            fence_for_peers(p);
             st_relaxed_sys(flag_ptr(p.peer[d], p.off_flags, kFlagDispatch, p.rank), flag_value(p, 0));
         }
     }
@@ -707,7 +707,7 @@ __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, i
     if (warp == 0) {
         if (lane < p.ws) {
             const int i = lane, s = (p.rank - i + p.ws) % p.ws;
-            const bool ok = wait_flag_gpu(seen_ptr(p, kFlagDispatch, s), want, p, kPhaseRecv, s);
+            const bool ok = wait_flag_gpu(await_ptr(p, kFlagDispatch, s), want, p, kPhaseRecv, s);
             int n_s = 0;
             if (ok) {
                 n_s = ld_stream(reinterpret_cast<const int*>(self + p.off_hdr) + s * 8);
@@ -735,7 +735,7 @@ __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, i
                     if (s == p.rank) {
                         st_release_gpu(seen_ptr(p, kFlagExpert, p.rank), want);
                     } else {
-                        fence_acq_rel_sys();
+                        fence_for_peers(p);
                         st_relaxed_sys(flag_ptr(p.peer[s], p.off_flags, kFlagExpert, p.rank), want);
                     }
                 }
@@ -977,7 +977,7 @@ __device__ __forceinline__ void combine_home_role(const DevParams& p, int cb, in
         return;
     }
     if (tid < 32) {  // lane d waits for rank d's flag: all of them at once, not one after the other
-        const bool ok = tid >= p.ws || wait_flag_gpu(seen_ptr(p, kFlagExpert, tid), want, p, kPhaseCombine, tid);
+        const bool ok = tid >= p.ws || wait_flag_gpu(await_ptr(p, kFlagExpert, tid), want, p, kPhaseCombine, tid);
         const bool all = __all_sync(0xffffffffu, ok);
         if (tid == 0) s_ok = all ? 1 : 0;
     }
@@ -1047,7 +1047,7 @@ __device__ __forceinline__ void combine_home_role(const DevParams& p, int cb, in
 __device__ __forceinline__ void wait_all_experts(const DevParams& p, int b) {
     if (b == 0 && threadIdx.x == 0)
         for (int d = 0; d < p.ws; ++d)
-            if (!wait_flag_gpu(seen_ptr(p, kFlagExpert, d), flag_value(p, 0), p, kPhaseCombine, d)) break;
+            if (!wait_flag_gpu(await_ptr(p, kFlagExpert, d), flag_value(p, 0), p, kPhaseCombine, d)) break;
 }
 
 // ---------------------------------------------------------------------------
@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_con
     if (ROLE == 0) {
         if (b < ns) {
             if (PAYLOAD == A2A_PAYLOAD_FP8) sender_role_fp8<T>(p, a2a_pipe_smem, b, ns);
-            else if (g.n > 1) sender_role<true>(p, a2a_pipe_smem, b, ns, -1, 0);
+            else if (p.local) sender_role<true>(p, a2a_pipe_smem, b, ns, -1, 0);
             else sender_role<false>(p, a2a_pipe_smem, b, ns, -1, 0);
         } else {
             const int rb = b - ns, d = (p.rank + 1 + rb % p.ws) % p.ws;
@@ -1123,16 +1123,18 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_con
         }
         stamp(p, kStampSent);
     } else if (ROLE == 1) {
-        if (b == 0) watcher_role(p, kFlagDispatch, kPhaseRecv, (int)(threadIdx.x >> 5));
-        else expert_role<T, PAYLOAD, PUSH>(p, a2a_pipe_smem, b - 1, G - 1);
+        const int first = p.local ? 0 : 1;
+        if (b < first) watcher_role(p, kFlagDispatch, kPhaseRecv, (int)(threadIdx.x >> 5));
+        else expert_role<T, PAYLOAD, PUSH>(p, a2a_pipe_smem, b - first, G - first);
         stamp(p, kStampExpertDone);
     } else {
-        if (b == 0) {
+        const int first = p.local ? 0 : 1;
+        if (b < first) {
             watcher_role(p, kFlagExpert, kPhaseCombine, (int)(threadIdx.x >> 5));
         } else if (PUSH) {
-            combine_home_role<T>(p, b - 1, G - 1);
+            combine_home_role<T>(p, b - first, G - first);
         } else {
-            combine_phase<T>(p, b - 1, G - 1, /*own_watchers=*/false);
+            combine_phase<T>(p, b - first, G - first, /*own_watchers=*/false);
         }
         if (!PUSH) wait_all_experts(p, b);
     }
