@@ -452,9 +452,12 @@ int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st) {
     }
     for (int r = 0; r < n; ++r) cs[r]->p.x = x[r];
     const a2a_ctx* c = cs[0];
-    const long long items = (long long)most_tokens(cs, n) *
-        (c->cfg.payload == A2A_PAYLOAD_DIRECT ? c->cfg.experts_per_token : c->cfg.world_size);
-    const int rc = launch_ranks(cs, n, select_tp<SendSel>(c), grid_for_ranks(c, n, items, 8), c->smem_bytes, st);
+    // DIRECT: a warp per pair and 2 KB, no more blocks than four per SM, each of which builds the routing tables;
+    // staged payloads: a block per (token, destination)
+    const bool direct = c->cfg.payload == A2A_PAYLOAD_DIRECT;
+    const long long T = most_tokens(cs, n), pieces = (c->cfg.hidden_dim / 8 + 127) / 128, warps = kThreads / 32;
+    const long long items = direct ? (T * c->cfg.experts_per_token * pieces + warps - 1) / warps : T * c->cfg.world_size;
+    const int rc = launch_ranks(cs, n, select_tp<SendSel>(c), grid_for_ranks(c, n, items, direct ? 4 : 8), c->smem_bytes, st);
     if (rc == A2A_OK)
         for (int r = 0; r < n; ++r) cs[r]->sent = true;
     return rc;

@@ -165,7 +165,7 @@ __device__ __forceinline__ void copy_row(const uint4* __restrict__ src, uint4* _
 
 // ---------------------------------------------------------------------------
 // Dispatch, sending half.  Never waits.
-// DIRECT: one block per (token, k) pair at a time; the row goes straight into slab
+// DIRECT: one warp per (token, k) pair and 2 KB of the row at a time; the row goes straight into slab
 //   (expert, this rank) on the expert's rank (NVLink for a peer, HBM for ourselves).
 // DEDUP / FP8: one block per (token, destination rank); the row crosses the wire
 //   once per destination into stage[src][t] (FP8: quantised on the fly, one fp32
@@ -179,17 +179,32 @@ __device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& 
     const int K = p.K, nvec = p.H >> 3;
     const int ta = chunk_begin(p, c), tb = chunk_end(p, c);  // this chunk's tokens
     if (PAYLOAD == A2A_PAYLOAD_DIRECT) {
-        for (int pair = ta * K + b; pair < tb * K; pair += G) {
+        // a warp per (pair, 2 KB of its row): no block-wide step between one row and the next
+        const int lane = tid & 31, npiece = (nvec + 127) >> 7;
+        const int items = (tb - ta) * K * npiece;
+        for (int it = b * (kThreads / 32) + (tid >> 5); it < items; it += G * (kThreads / 32)) {
+            const int pair = ta * K + it / npiece, v0 = it % npiece * 128;
             const int t = pair / K, k = pair - t * K;
+            const uint4* src = reinterpret_cast<const uint4*>(p.x) + (size_t)t * nvec;
+            uint4 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int v = v0 + u * 32 + lane;
+                if (v < nvec) q[u] = ld_input(src + v);
+            }
             const int e = s.idx[pair];
             const int j = pair_slot(p, s, t, k, e);
-            if (tid == 0) p.slot[pair] = j;
+            if (lane == 0 && v0 == 0) p.slot[pair] = j;
             if (j < 0) continue;
             const int d = e / p.L, l = e - d * p.L;
             const size_t row = ((size_t)l * p.ws + p.rank) * p.T_max + j;
-            copy_row(reinterpret_cast<const uint4*>(p.x) + (size_t)t * nvec,
-                     reinterpret_cast<uint4*>(p.peer[d] + p.off_rows) + row * nvec, nvec);
-            if (tid == 0) reinterpret_cast<int*>(p.peer[d] + p.off_meta)[row] = (t << 8) | k;
+            uint4* dst = reinterpret_cast<uint4*>(p.peer[d] + p.off_rows) + row * nvec;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int v = v0 + u * 32 + lane;
+                if (v < nvec) st_stream(dst + v, q[u]);
+            }
+            if (lane == 0 && v0 == 0) reinterpret_cast<int*>(p.peer[d] + p.off_meta)[row] = (t << 8) | k;
         }
     } else {
         for (int it = ta * p.ws + b; it < tb * p.ws; it += G) {
@@ -266,7 +281,7 @@ __device__ __forceinline__ void send_phase(const DevParams& p, const BlockSmem& 
 //   PUBLISH tell every home rank that this rank's expert outputs are ready
 // ---------------------------------------------------------------------------
 // The valid rows of source s, flattened over the local experts with a prefix sum of the
-// counts so that skewed routing does not idle blocks; one block per row at a time.
+// counts so that skewed routing does not idle blocks; one warp per row and 2 KB of it at a time.
 //   FANOUT (staged payloads): the row's content comes from the wire row of its token
 //          (found through the row's (token, k) word), FP8: dequantised and rounded to T;
 //   SCALE: the placeholder expert op, T(float(row) * (1 + rank)), on the way.
@@ -296,7 +311,10 @@ __device__ __forceinline__ void rows_of_source(const DevParams& p, int* pre, int
     const float scale = (float)(1 + p.rank);
     uint4* rows = reinterpret_cast<uint4*>(self + p.off_rows);
     const int* meta = reinterpret_cast<const int*>(self + p.off_meta);
-    for (int r = part; r < total; r += nparts) {
+    const int lane = tid & 31, npiece = (nvec + 127) >> 7;
+    const int items = total * npiece;
+    for (int it = part * (kThreads / 32) + (tid >> 5); it < items; it += nparts * (kThreads / 32)) {
+        const int r = it / npiece, v0 = (it - r * npiece) * 128;
         const int l = upper_slab(pre, p.L, r);
         const int j = base[l] + r - pre[l];
         const size_t ri = ((size_t)l * p.ws + s) * p.T_max + j;
@@ -310,31 +328,33 @@ __device__ __forceinline__ void rows_of_source(const DevParams& p, int* pre, int
             }
             wire = self + p.off_stage + ((size_t)s * p.T_max + t) * p.stage_row_bytes;
         }
-        for (int v0 = 0; v0 < nvec; v0 += kThreads * 4) {
-            uint4 q[4];
+        uint4 q[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int v = v0 + u * kThreads + tid;
-                if (v < nvec) {
-                    if (fp8) {
-                        float f[8];
-                        unpack8_e4m3(ld_stream(reinterpret_cast<const uint2*>(wire) + v), f);
-                        const float sc = ld_stream(reinterpret_cast<const float*>(wire + p.H) + (v >> 4));
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) f[i] *= sc;
-                        q[u] = pack8<T>(f);  // the received row, rounded to T as the receiver stores it
-                    } else if (from_wire) {
-                        q[u] = ld_stream(reinterpret_cast<const uint4*>(wire) + v);
-                    } else {
-                        q[u] = ld_stream(row + v);
-                    }
-                }
+        for (int u = 0; u < 4; ++u) {
+            const int v = v0 + u * 32 + lane;
+            if (v >= nvec) continue;
+            if (fp8) {
+                const uint2 bytes = ld_stream(reinterpret_cast<const uint2*>(wire) + v);
+                q[u].x = bytes.x;
+                q[u].y = bytes.y;
+                q[u].z = __float_as_uint(ld_stream(reinterpret_cast<const float*>(wire + p.H) + (v >> 4)));
+            } else {
+                q[u] = ld_stream((from_wire ? reinterpret_cast<const uint4*>(wire) : row) + v);
             }
+        }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int v = v0 + u * kThreads + tid;
-                if (v < nvec) st_stream(row + v, SCALE ? scale8<T>(q[u], scale) : q[u]);
+        for (int u = 0; u < 4; ++u) {
+            const int v = v0 + u * 32 + lane;
+            if (v >= nvec) continue;
+            if (fp8) {
+                float f[8];
+                unpack8_e4m3(make_uint2(q[u].x, q[u].y), f);
+                const float sc = __uint_as_float(q[u].z);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) f[i] *= sc;
+                q[u] = pack8<T>(f);  // the received row, rounded to T as the receiver stores it
             }
+            st_stream(row + v, SCALE ? scale8<T>(q[u], scale) : q[u]);
         }
     }
 }
