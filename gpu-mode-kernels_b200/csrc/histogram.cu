@@ -154,8 +154,11 @@ extern "C" int a2a_histogram256(const uint8_t* data, size_t n, int64_t* out, voi
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return -(int)e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return -(int)e;
-    zero_counts_kernel<<<1, kBins, 0, st>>>(counts);
-    if ((e = cudaGetLastError()) != cudaSuccess) return -(int)e;
+    cudaLaunchConfig_t zero{};
+    zero.gridDim = dim3(1);
+    zero.blockDim = dim3(kBins);
+    zero.stream = st;
+    if ((e = cudaLaunchKernelEx(&zero, zero_counts_kernel, counts)) != cudaSuccess) return -(int)e;
     const size_t want = (n / 16 + kThreads - 1) / kThreads;
     const size_t room = (size_t)sms * (n < kFullBytes ? 1 : kBlocksPerSm);
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
