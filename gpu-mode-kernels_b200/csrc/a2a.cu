@@ -248,24 +248,35 @@ auto select_tp(const a2a_ctx* c, A... a) {
 }
 
 using KernelFn = void (*)(DevParams);
-using GroupFn = void (*)(GroupParams);
-template <typename T, int P> struct SendSel { static GroupFn get() { return send_kernel<T, P>; } };
+// a phase's kernel for one rank and for a group
+struct PhaseFn {
+    void (*one)(RankParams);
+    void (*group)(GroupParams);
+};
+template <typename T, int P> struct SendSel {
+    static PhaseFn get() { return {send_kernel<T, P, RankParams>, send_kernel<T, P, GroupParams>}; }
+};
 template <typename T, int P> struct ForwardSel { static KernelFn get() { return forward_kernel<T, P>; } };
 template <typename T, int P> struct ExpertSel {
+    template <bool WAIT, bool FANOUT, bool SCALE, bool PUBLISH>
+    static PhaseFn pair() {
+        return {expert_kernel<T, P, WAIT, FANOUT, SCALE, PUBLISH, RankParams>,
+                expert_kernel<T, P, WAIT, FANOUT, SCALE, PUBLISH, GroupParams>};
+    }
     // the receive-side launches of the public phases
-    static GroupFn get(bool wait, bool fanout, bool scale, bool publish) {
-        if (wait && fanout && scale && publish) return expert_kernel<T, P, true, true, true, true>;      // recv + expert fused
-        if (wait && fanout && !scale && !publish) return expert_kernel<T, P, true, true, false, false>;  // dispatch_recv
-        if (!wait && !fanout && scale && publish) return expert_kernel<T, P, false, false, true, true>;  // expert_placeholder
-        return expert_kernel<T, P, false, false, false, true>;                                           // expert_done
+    static PhaseFn get(bool wait, bool fanout, bool scale, bool publish) {
+        if (wait && fanout && scale && publish) return pair<true, true, true, true>();      // recv + expert fused
+        if (wait && fanout && !scale && !publish) return pair<true, true, false, false>();  // dispatch_recv
+        if (!wait && !fanout && scale && publish) return pair<false, false, true, true>();  // expert_placeholder
+        return pair<false, false, false, true>();                                           // expert_done
     }
 };
 // pipelined schedule: (element type, payload, push/pull) -> kernel
 template <typename T, int P, bool PUSH> struct PipeForward { static KernelFn get() { return pipe_forward_kernel<T, P, PUSH>; } };
 template <typename T, int P, bool PUSH> struct PipeRole {
-    static GroupFn get(int role) {
-        return role == 0 ? pipe_role_kernel<T, P, PUSH, 0> : role == 1 ? pipe_role_kernel<T, P, PUSH, 1> : pipe_role_kernel<T, P, PUSH, 2>;
-    }
+    template <int ROLE>
+    static PhaseFn pair() { return {pipe_role_kernel<T, P, PUSH, ROLE, RankParams>, pipe_role_kernel<T, P, PUSH, ROLE, GroupParams>}; }
+    static PhaseFn get(int role) { return role == 0 ? pair<0>() : role == 1 ? pair<1>() : pair<2>(); }
 };
 template <template <typename, int, bool> class F, typename T, typename... A>
 auto select_pipe_t(const a2a_ctx* c, A... a) {
@@ -288,8 +299,9 @@ KernelFn solo_fn(const a2a_ctx* c) {
     return bf ? solo_kernel<__nv_bfloat16, A2A_PAYLOAD_DEDUP, U> : solo_kernel<__half, A2A_PAYLOAD_DEDUP, U>;
 }
 
-GroupFn combine_fn(const a2a_ctx* c) {
-    return c->cfg.dtype == A2A_DTYPE_BF16 ? (GroupFn)combine_kernel<__nv_bfloat16> : (GroupFn)combine_kernel<__half>;
+PhaseFn combine_fn(const a2a_ctx* c) {
+    if (c->cfg.dtype == A2A_DTYPE_BF16) return {combine_kernel<__nv_bfloat16, RankParams>, combine_kernel<__nv_bfloat16, GroupParams>};
+    return {combine_kernel<__half, RankParams>, combine_kernel<__half, GroupParams>};
 }
 
 int launch(a2a_ctx* c, KernelFn fn, int grid, int smem, cudaStream_t st, bool cooperative = false) {
@@ -309,7 +321,7 @@ int launch(a2a_ctx* c, KernelFn fn, int grid, int smem, cudaStream_t st, bool co
 // this launch's blocks agree on (senders, routers).  A trace has a slot per block of the grid, so contexts
 // that are being traced are launched one by one.
 template <typename Adjust>
-int launch_ranks(a2a_ctx* const* cs, int n, GroupFn fn, int blocks, int smem, cudaStream_t st, Adjust adjust) {
+int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int smem, cudaStream_t st, Adjust adjust) {
     bool traced = false;
     for (int r = 0; r < n; ++r) traced |= cs[r]->p.trace != nullptr;
     if (traced && n > 1) {
@@ -319,24 +331,33 @@ int launch_ranks(a2a_ctx* const* cs, int n, GroupFn fn, int blocks, int smem, cu
         }
         return A2A_OK;
     }
+    if (n == 1) {
+        a2a_ctx* c = cs[0];
+        RankParams g = {call_params(c)};
+        adjust(g.p);
+        if (traced) {
+            if (blocks > kTraceBlocks) g.p.trace = nullptr;
+            else c->last_grid = blocks;
+        }
+        c->launches++;
+        void* args[] = {&g};
+        const cudaError_t e = cudaLaunchKernel((const void*)fn.one, dim3(blocks), dim3(kThreads), args, smem, st);
+        return e == cudaSuccess ? A2A_OK : -(int)e;
+    }
     GroupParams g;
     for (int r = 0; r < n; ++r) {
         g.p[r] = call_params(cs[r]);
-        g.p[r].local = n > 1;
+        g.p[r].local = 1;
         adjust(g.p[r]);
         cs[r]->launches++;
     }
     g.n = n;
-    if (traced) {
-        if (blocks > kTraceBlocks) g.p[0].trace = nullptr;
-        else cs[0]->last_grid = blocks;
-    }
     void* args[] = {&g};
-    const cudaError_t e = cudaLaunchKernel((const void*)fn, dim3(n * blocks), dim3(kThreads), args, smem, st);
+    const cudaError_t e = cudaLaunchKernel((const void*)fn.group, dim3(n * blocks), dim3(kThreads), args, smem, st);
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
-int launch_ranks(a2a_ctx* const* cs, int n, GroupFn fn, int blocks, int smem, cudaStream_t st) {
+int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int smem, cudaStream_t st) {
     return launch_ranks(cs, n, fn, blocks, smem, st, [](DevParams&) {});
 }
 
@@ -680,15 +701,20 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     // Kernel attributes are per function and device, not per context: opt every routing-carrying
     // kernel in for the whole shared-memory budget, then size this context's own launches.
     c->smem_bytes = (int)(block_smem_ints(E, T, K) * sizeof(int));
-    const void* fns[] = {(const void*)route_kernel, (const void*)select_tp<SendSel>(c), (const void*)select_tp<ForwardSel>(c),
-                         (const void*)select_tp<ExpertSel>(c, true, true, true, true),
-                         (const void*)select_tp<ExpertSel>(c, true, true, false, false),
-                         (const void*)select_tp<ExpertSel>(c, false, false, true, true),
-                         (const void*)select_tp<ExpertSel>(c, false, false, false, true)};
-    for (const void* fn : fns) {
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
-        if (e != cudaSuccess) break;
-    }
+    auto opt_in = [&e](const void* fn) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
+    };
+    auto opt_in_both = [&opt_in](const PhaseFn& fn) {
+        opt_in((const void*)fn.one);
+        opt_in((const void*)fn.group);
+    };
+    opt_in((const void*)route_kernel);
+    opt_in((const void*)select_tp<ForwardSel>(c));
+    opt_in_both(select_tp<SendSel>(c));
+    opt_in_both(select_tp<ExpertSel>(c, true, true, true, true));
+    opt_in_both(select_tp<ExpertSel>(c, true, true, false, false));
+    opt_in_both(select_tp<ExpertSel>(c, false, false, true, true));
+    opt_in_both(select_tp<ExpertSel>(c, false, false, false, true));
     int coop = 0, occ = 0;
     const bool pipelined = cfg->schedule == A2A_SCHEDULE_PIPELINED;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, cfg->device);
@@ -696,9 +722,8 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     if (pipelined) {
         const size_t a = cfg->world_size > 1 ? pipe_sender_smem(T, cfg->world_size, p.senders) : 0, b = pipe_router_smem(T, L);
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
-        const void* roles[] = {(const void*)select_pipe<PipeForward>(c), (const void*)select_pipe<PipeRole>(c, 0)};
-        for (const void* fn : roles)
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes);
+        opt_in((const void*)select_pipe<PipeForward>(c));
+        opt_in_both(select_pipe<PipeRole>(c, 0));
         if (e == cudaSuccess && cfg->world_size == 1) {
             c->forward_grid = c->num_sms;
             c->fused = true;  // the solo kernel: no block waits for another

@@ -110,11 +110,22 @@ struct DevParams {
     void* y;
 };
 
-// The ranks one launch serves: a rank's own (n = 1) or, where a whole group lives on this GPU, all of them.
-// Block i works for rank position i % n as that rank's block i / n.
+// The ranks one launch serves: one, or, where a whole group lives on this GPU, all `n` of them: block i works
+// for rank position i % n as that rank's block i / n.  Two types, because parameters of eight ranks, looked up
+// by position, cost a launch for one rank half a microsecond and its blocks as much.
+struct RankParams {
+    DevParams p;
+    __device__ __forceinline__ const DevParams& rank() const { return p; }
+    __device__ __forceinline__ int block() const { return (int)blockIdx.x; }
+    __device__ __forceinline__ int blocks() const { return (int)gridDim.x; }
+};
+
 struct GroupParams {
     DevParams p[A2A_MAX_WORLD];
     int n;
+    __device__ __forceinline__ const DevParams& rank() const { return p[blockIdx.x % n]; }
+    __device__ __forceinline__ int block() const { return (int)blockIdx.x / n; }
+    __device__ __forceinline__ int blocks() const { return (int)gridDim.x / n; }
 };
 
 __device__ __forceinline__ long long global_ns() {

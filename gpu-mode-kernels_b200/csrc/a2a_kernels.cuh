@@ -522,22 +522,21 @@ __global__ void __launch_bounds__(kThreads) route_kernel(const __grid_constant__
     for (int e = threadIdx.x; e < p.E; e += kThreads) p.send_counts[e] = s.cnt[e];
 }
 
-template <typename T, int PAYLOAD>
-__global__ void __launch_bounds__(kThreads) send_kernel(const __grid_constant__ GroupParams g) {
-    const DevParams& p = g.p[blockIdx.x % g.n];
-    send_phase<T, PAYLOAD>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), (int)blockIdx.x / g.n, (int)gridDim.x / g.n);
+template <typename T, int PAYLOAD, class P>
+__global__ void __launch_bounds__(kThreads) send_kernel(const __grid_constant__ P g) {
+    const DevParams& p = g.rank();
+    send_phase<T, PAYLOAD>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), g.block(), g.blocks());
 }
 
-template <typename T, int PAYLOAD, bool WAIT, bool FANOUT, bool SCALE, bool PUBLISH>
-__global__ void __launch_bounds__(kThreads) expert_kernel(const __grid_constant__ GroupParams g) {
-    const DevParams& p = g.p[blockIdx.x % g.n];
-    expert_phase<T, PAYLOAD, WAIT, FANOUT, SCALE, PUBLISH>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), (int)blockIdx.x / g.n,
-                                                           (int)gridDim.x / g.n);
+template <typename T, int PAYLOAD, bool WAIT, bool FANOUT, bool SCALE, bool PUBLISH, class P>
+__global__ void __launch_bounds__(kThreads) expert_kernel(const __grid_constant__ P g) {
+    const DevParams& p = g.rank();
+    expert_phase<T, PAYLOAD, WAIT, FANOUT, SCALE, PUBLISH>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), g.block(), g.blocks());
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) combine_kernel(const __grid_constant__ GroupParams g) {
-    combine_phase<T>(g.p[blockIdx.x % g.n], (int)blockIdx.x / g.n, (int)gridDim.x / g.n, true);
+template <typename T, class P>
+__global__ void __launch_bounds__(kThreads) combine_kernel(const __grid_constant__ P g) {
+    combine_phase<T>(g.rank(), g.block(), g.blocks(), true);
 }
 
 // The whole path in one launch.  Launched cooperatively so that every block is

@@ -1106,10 +1106,10 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
 // that lives on ONE GPU -- a kernel that waits never shares the GPU with the kernel it waits for, so what
 // runs together is one role of every rank.  ROLE 0: senders + routers.  1: one watcher block + experts.
 // 2: one watcher block + combine.
-template <typename T, int PAYLOAD, bool PUSH, int ROLE>
-__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ GroupParams g) {
-    const DevParams& p = g.p[blockIdx.x % g.n];
-    const int G = (int)gridDim.x / g.n, b = (int)blockIdx.x / g.n;
+template <typename T, int PAYLOAD, bool PUSH, int ROLE, class P>
+__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ P g) {
+    const DevParams& p = g.rank();
+    const int G = g.blocks(), b = g.block();
     const int ns = p.ws > 1 ? p.senders : 0;
     stamp(p, kStampStart);
     if (ROLE == 0) {
