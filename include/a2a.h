@@ -205,7 +205,8 @@ int a2a_set_fused(a2a_ctx* ctx, int on);
 
 /* a2a_forward for HOST buffers (pinned for speed): copies x, topk_idx and
  * topk_weights to the device, runs the path, copies y back; all asynchronous
- * on `stream`.  This is the call a host-resident caller of custom_kernel makes. */
+ * on `stream`.  With one rank (pipelined schedule) and x, topk_weights and y pinned and not
+ * overlapping, the kernel reads and writes them in place.  This is the call a host-resident caller of custom_kernel makes. */
 int a2a_forward_host(a2a_ctx* ctx, const void* x_host, const int32_t* topk_idx_host,
                      const float* topk_weights_host, void* y_host, int num_tokens, void* stream);
 
