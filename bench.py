@@ -407,7 +407,9 @@ def main():
     all_idx = [pkg.workload_input(args.workload, r, ws)[1].indices for r in range(ws)] if ws > 1 else [rd_cpu.indices]
     tr = traffic.summarize(all_idx, cfg.num_experts, ws, H, payload, combine)
     if ws == 1:
-        alg = (3 * T * K + T) * 2 * H  # rows written and read in dispatch, read in combine, y written
+        # pipelined: rows read, dispatched and reduced in one pass, y written; phased: dispatched rows are written,
+        # read and written by the expert op and read again by the combine
+        alg = (T * K + 2 * T) * 2 * H if pipelined else (3 * T * K + T) * 2 * H
         achieved = alg / (ms * 1e-3) / 1e9
         roofline = {"bound": "hbm", "kernel": "one-launch forward (route + send + expert + combine)",
                     "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
@@ -519,7 +521,8 @@ def main():
             "metric": METRIC, "value": ms * 1e3, "unit": "us", "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": ms, "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
             "dtype": "bf16", "data": "synthetic", "config": workload_config(args.workload, ws, payload,
-                                      "one cooperative launch per forward" if fused else "one kernel per phase"),
+                                      ("one launch per forward" if pipelined and ws == 1 else
+                                       "one cooperative launch per forward") if fused else "one kernel per phase"),
             "roofline": roofline, "cpu_baseline": cpu_baseline,
             "e2e": {"value": e2e_ms * 1e3, "unit": "us", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": launches, "clocks": clocks.summary(),
@@ -639,9 +642,6 @@ def histogram_main(args, rank: int, ws: int):
 # kernel on this workload (a profiler cannot run inside the timed loop, so the figures are constants
 # of the kernel + workload, re-measured whenever the kernel changes).
 SINGLE_GPU_TRAFFIC = {
-    ("c4", "pipelined", "push"): {"dram_bytes": 5.26e6, "l2_bytes": 37.0e6,
-                                  "source": "ncu --set full, pipe_forward_kernel, c4 at world size 1: dram__bytes_read.sum 3.79 MB + "
-                                            "dram__bytes_write.sum 1.46 MB; L2 sectors from the SMs 3.93 MB read + 33.1 MB written"},
     ("c4", "phased", "pull"): {"dram_bytes": 7.76e6, "l2_bytes": 100.2e6,
                                "source": "ncu --set full, forward_kernel (phased schedule), c4 at world size 1: dram__bytes_read.sum "
                                          "4.16 MB + dram__bytes_write.sum 3.60 MB; L2 sectors from the SMs 63.4 MB read + 36.8 MB written"},
