@@ -86,6 +86,7 @@ struct a2a_ctx {
     void* ipc_mapped[A2A_MAX_WORLD];  // peers opened through CUDA IPC (to close on destroy)
     bool peers_ready;
     bool routed, sent;
+    bool recorded;          // this call's records are written: by role 0, or by the one launch of several ranks
     uint32_t epoch, barrier_epoch;
     int cur_tokens;
     int64_t launches;
@@ -422,7 +423,7 @@ int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
     c->cur_tokens = T;
     c->p.idx = idx;
     c->routed = true;
-    c->sent = false;
+    c->sent = c->recorded = false;
     return A2A_OK;
 }
 
@@ -539,15 +540,16 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
         p.routers = nr;
     });
     if (rc == A2A_OK)
-        for (int r = 0; r < n; ++r) cs[r]->sent = true;
+        for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->recorded = true;
     return rc;
 }
 
-// Roles 1 and 2: this rank's share of two blocks per SM (of four or eight, where a group shares the launch:
+// Roles 1 and 2, of a call whose records exist (the one launch of a single rank writes none: what role 1 would
+// find there belongs to an earlier call, and so may the tensors): this rank's share of two blocks per SM (of four or eight, where a group shares the launch:
 // 134 us against 145 and 159 for role 1 of the workload named above) and, for peers elsewhere, a watcher block.
 int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
     for (int r = 0; r < n; ++r)
-        if (!cs[r]->sent) return A2A_ERR_STATE;
+        if (!cs[r]->sent || !cs[r]->recorded) return A2A_ERR_STATE;
     const a2a_ctx* c = cs[0];
     const int blocks = c->num_sms * 2 / n;
     const int smem = role == 1 && c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
@@ -900,7 +902,10 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
         r = c->cfg.world_size == 1
             ? launch_solo(c, st)
             : launch(c, select_pipe<PipeForward>(c), c->forward_grid, c->pipe_smem, st, /*cooperative=*/true);
-        if (r == A2A_OK) c->sent = true;
+        if (r == A2A_OK) {
+            c->sent = true;
+            c->recorded = c->cfg.world_size > 1;
+        }
         return r;
     }
     if (c->fused) {
@@ -943,6 +948,8 @@ int a2a_forward_host(a2a_ctx* c, const void* x, const int32_t* idx, const float*
             c->p.y = dy;
             const int rc = launch_solo(c, st, /*host_rows=*/true);
             if (rc == A2A_OK) c->sent = true;
+            c->p.x = c->p.y = nullptr;  // the caller's host memory, which may be gone by the next launch
+            c->p.w = nullptr;
             return rc;
         }
     }

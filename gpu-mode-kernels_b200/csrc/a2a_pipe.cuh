@@ -833,7 +833,7 @@ __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, i
         // a peer's row lies where its number says; only an own row has to be looked for
         const uint8_t* src = self + p.off_stage + rec * p.stage_row_bytes;
         if (own) {
-            if (m.t < 0 || m.t >= p.T_max) return;
+            if (m.t < 0 || m.t >= p.T) return;
             src = reinterpret_cast<const uint8_t*>(p.x) + (size_t)m.t * p.H * 2;
         }
         load_wire_chunk<T, PAYLOAD>(p, own, src, v0, nvec, m.q);
@@ -842,7 +842,7 @@ __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, i
         const int s = c.s, v0 = c.ch * 128, t = m.t;
         const bool own = (s == p.rank);
         const bool via_engine = PUSH && !own;  // the home rank is a peer: return through the copy engine
-        if (t < 0 || t >= p.T_max) {
+        if (t < 0 || t >= (own ? p.T : p.T_max)) {  // own rows lie in the caller's tensors, a peer's in buffers of T_max
             record_error(p.status, A2A_ERR_CAPACITY, p.rank, s, kPhaseRecv, p.epoch, t);
             return;
         }

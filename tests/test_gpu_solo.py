@@ -149,3 +149,41 @@ def test_host_tensors_wherever_they_live(place, K, H, T, n, payload):
         for ptr in pinned:
             torch.cuda.cudart().cudaHostUnregister(ptr)
         ctx.close()
+
+
+@pytest.mark.parametrize("combine", ["push", "pull"])
+def test_roles_are_refused_where_the_call_was_not_begun_by_role_0(combine):
+    """The one launch writes none of the records that roles 1 and 2 work from: what lies there is of an earlier,
+    larger call."""
+    cfg, rd, _, _ = pkg.generate_input(8, 2, 64, 40, seed=31, rank=0, world_size=1)
+    big, n = rd.to(DEV), 5
+    few = [t[:n].contiguous() for t in (rd.x, rd.indices, rd.weights)]
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine=combine)
+    try:
+        def step_all():
+            ctx.pipe_step(0, big.x, big.indices, big.weights)
+            ctx.pipe_step(1)
+            return ctx.pipe_step(2)
+
+        want = bits(step_all())
+        assert torch.equal(bits(ctx.forward(big.x, big.indices, big.weights)), want)
+        by_phases = [t.to(DEV) for t in few]
+
+        def begin_phases():
+            ctx.route(by_phases[1])
+            ctx.dispatch_send(by_phases[0])
+
+        for begin in (lambda: ctx.forward(*by_phases), lambda: ctx.forward_host(*few),
+                      lambda: ctx.forward_host(*[t.pin_memory() for t in few]), begin_phases):
+            begin()
+            before = ctx.launches
+            for role in (1, 2):
+                with pytest.raises(_lib.A2AError) as refused:
+                    ctx.pipe_step(role)
+                assert refused.value.code == _lib.A2A_ERR_STATE
+            assert ctx.launches == before
+            assert torch.equal(bits(step_all()), want)
+        ctx.check()
+    finally:
+        torch.cuda.synchronize()
+        ctx.close()
