@@ -20,7 +20,10 @@ namespace {
 
 constexpr int kTraceBlocks = 2048;  // blocks the in-kernel trace buffer has room for
 constexpr size_t kMaxSmemBytes = 200 * 1024;  // routing bitmap budget per block (227 KB is the sm_100 limit)
-constexpr size_t kMaxPipeSmemBytes = 100 * 1024;  // pipelined kernel of several ranks: two blocks per SM must fit
+// Pipelined kernel of several ranks: two blocks per SM must fit (of 113 KB each).  A sender has 64 bytes more than a
+// router, the four descriptors by which its ring outgrew six stages; which configurations fit did not change by them.
+constexpr size_t kMaxPipeSmemBytes = 100 * 1024;
+constexpr size_t kMaxSenderSmemBytes = kMaxPipeSmemBytes + 64;
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -206,11 +209,11 @@ int validate(const a2a_config& c) {
         if (c.payload == A2A_PAYLOAD_FP8 && make_layout(c).stage_row_bytes > kWarpStageBytes) return A2A_ERR_CONFIG;
         if (c.chunks > 1) return A2A_ERR_CONFIG;
         // one rank has no senders and routes inside its one kernel; only its stepped roles need the tables
-        const size_t room = c.world_size == 1 ? kMaxSmemBytes : kMaxPipeSmemBytes;
+        const size_t router_room = c.world_size == 1 ? kMaxSmemBytes : kMaxPipeSmemBytes;
         const int senders = pipe_senders(c);
         if (c.world_size > 1 && senders < 2) return A2A_ERR_CONFIG;  // blocks 0 and 1 carry the watchers
-        if ((c.world_size > 1 && pipe_sender_smem(c.max_num_tokens, c.world_size, senders) > room) ||
-            pipe_router_smem(c.max_num_tokens, c.num_experts / c.world_size) > room)
+        if ((c.world_size > 1 && pipe_sender_smem(c.max_num_tokens, c.world_size, senders) > kMaxSenderSmemBytes) ||
+            pipe_router_smem(c.max_num_tokens, c.num_experts / c.world_size) > router_room)
             return A2A_ERR_CONFIG;
     }
     return A2A_OK;
@@ -443,7 +446,7 @@ void share_send_blocks(const a2a_ctx* c, int n, int tokens, int* senders, int* r
     int ns = 2 * c->num_sms / n - ws;
     if (ns > rows) ns = (int)rows;
     if (ns < 2) ns = 2;
-    if (pipe_sender_smem(T, ws, ns) > kMaxPipeSmemBytes) ns = c->p.senders;  // fewer blocks have longer token lists
+    if (pipe_sender_smem(T, ws, ns) > kMaxSenderSmemBytes) ns = c->p.senders;  // fewer blocks have longer token lists
     const size_t a = pipe_sender_smem(T, ws, ns), b = pipe_router_smem(T, c->p.L);
     *senders = ns;
     *routers = 1;

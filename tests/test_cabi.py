@@ -63,3 +63,17 @@ def test_null_arguments():
     assert lib.a2a_destroy(None) == 0
     assert lib.a2a_route(None, None, 0, None) == _lib.A2A_ERR_CONFIG
     assert lib.a2a_launch_count(None) == 0
+
+
+@pytest.mark.parametrize("world_size,senders,payload,largest", [
+    (2, 2, 1, 1760), (2, 7, 2, 6160), (8, 3, 1, 660), (8, 96, 2, 21120), (4, 48, 1, 21120),
+])
+def test_largest_token_count_of_the_pipelined_schedule(world_size, senders, payload, largest):
+    """100 KB + 64 bytes hold a sender's ring of 96 KB, its bookkeeping of 640 bytes, and 3520 bytes of token
+    lists: two bytes per destination and token of the block's share.  That is what callers may ask for."""
+    assert 2 * world_size * -(-largest // senders) == 3520
+    lib, out = _lib.load(), (C.c_uint8 * 128)()
+    for tokens, want in ((largest, 0), (largest + 1, _lib.A2A_ERR_CONFIG)):
+        cfg = _lib.Config(rank=0, world_size=world_size, device=0, num_experts=8, experts_per_token=1, hidden_dim=128,
+                          max_num_tokens=tokens, dtype=0, payload=payload, timeout_ms=100, schedule=1, combine=0, senders=senders)
+        assert lib.a2a_fingerprint(C.byref(cfg), out) == want, tokens

@@ -6,6 +6,8 @@ that a kernel that waits never shares the GPU with the kernel it waits for).  At
 the real one-launch kernel runs and must give the same bits as the stepped roles.  The
 one-process-per-GPU form is covered by test_x_gpu_multiprocess.py.
 """
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -139,6 +141,33 @@ def test_fp8_edge_shapes(combine):
                  for r in range(ws)]
         world, _ = run_case(datas[0][0], ws, [d[1] for d in datas], combine, payload="fp8")
         world.close()
+
+
+@pytest.mark.parametrize("payload", ["dedup", "fp8"])
+def test_largest_token_count_of_two_sender_blocks(payload):
+    """Token lists up to the last byte of a sender's shared memory, the roles called rank by rank."""
+    ws, senders = 2, 2
+    datas = [pkg.generate_input(8, 2, 128, 1760, seed=9, rank=r, world_size=ws) for r in range(ws)]
+    cfg, rds_cpu = datas[0][0], [d[1] for d in datas]
+    disp, ys = O.simulate(cfg, ws, rds_cpu)
+    ctxs = [A2AContext(cfg, r, ws, device=0, payload=payload, schedule="pipelined", combine="push", senders=senders,
+                       connect=False) for r in range(ws)]
+    try:
+        A2AContext.attach_local(ctxs)
+        rds = [rd.to(DEV) for rd in rds_cpu]
+        for c, rd in zip(ctxs, rds):
+            c.pipe_step(0, rd.x, rd.indices, rd.weights)
+        for c in ctxs:
+            c.pipe_step(1)
+        out = [c.pipe_step(2) for c in ctxs]
+        torch.cuda.synchronize()
+        for c in ctxs:
+            c.check()
+        check_pipelined_dispatch(SimpleNamespace(ctxs=ctxs), disp, cfg.in_dtype, payload)
+        check_y(cfg, ws, rds_cpu, out, ys, payload)
+    finally:
+        for c in ctxs:
+            c.close()
 
 
 @pytest.mark.parametrize("combine", COMBINES)
