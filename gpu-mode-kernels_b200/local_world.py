@@ -31,13 +31,19 @@ class LocalWorld:
         ]
         A2AContext.attach_local(self.ctxs)
 
+    def _calls(self, rank_datas: Sequence):
+        """One empty call per rank; a rank without data would pass for one that has no tokens."""
+        if len(rank_datas) < self.world_size:
+            raise _lib.A2AError(_lib.A2A_ERR_STATE, f"{self.world_size} ranks, but data for {len(rank_datas)}")
+        return (_lib.Call * self.world_size)()
+
     def _step(self, phase: str, calls=None) -> None:
         handles = (C.c_void_p * self.world_size)(*[c._h.value for c in self.ctxs])
         _lib.check(self.ctxs[0].lib.a2a_group_step(handles, _lib.GROUP_PHASE[phase], calls, _lib.current_stream()))
 
     def _send(self, rank_datas: Sequence) -> None:
         """route + dispatch_send on every rank, in one launch."""
-        calls = (_lib.Call * self.world_size)()
+        calls = self._calls(rank_datas)
         for call, c, rd in zip(calls, self.ctxs, rank_datas):
             assert rd.indices.dtype == torch.int32 and rd.indices.is_contiguous() and rd.indices.is_cuda
             assert rd.x.dtype == self.cfg.in_dtype and rd.x.is_contiguous() and rd.x.is_cuda
@@ -47,7 +53,7 @@ class LocalWorld:
             c._num_tokens, c._keep = rd.indices.shape[0], [rd.indices, rd.x]
 
     def _combine(self, rank_datas: Sequence) -> List[torch.Tensor]:
-        calls, ys = (_lib.Call * self.world_size)(), []
+        calls, ys = self._calls(rank_datas), []
         for call, c, rd in zip(calls, self.ctxs, rank_datas):
             assert rd.weights.dtype == torch.float32 and rd.weights.is_contiguous() and rd.weights.is_cuda
             ys.append(torch.empty(c._num_tokens, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=c.device))
@@ -76,7 +82,7 @@ class LocalWorld:
     def forward_pipelined(self, rank_datas: Sequence) -> List[torch.Tensor]:
         """The roles of the pipelined one-launch kernel as three launches, in lock-step:
         every rank's senders and routers, then every rank's expert blocks, then every rank's combine."""
-        calls, ys = (_lib.Call * self.world_size)(), []
+        calls, ys = self._calls(rank_datas), []
         for call, c, rd in zip(calls, self.ctxs, rank_datas):
             n = c._check_inputs(rd.x, rd.indices, rd.weights, None, on_device=True)
             ys.append(torch.empty(n, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=c.device))
