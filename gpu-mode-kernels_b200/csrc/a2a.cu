@@ -559,7 +559,9 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
     return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), n > 1 ? blocks : 1 + blocks, smem, st);
 }
 
-// The contexts of every rank of one group, all on one GPU?
+// The contexts of every rank of one group, all on one GPU, attached to one another and at the same call?  A launch
+// for all of them takes every rank's memory for this GPU's own, and none of its blocks watches for a rank that is
+// behind.
 int check_group(a2a_ctx* const* group) {
     if (group == nullptr || group[0] == nullptr) return A2A_ERR_CONFIG;
     const Fingerprint mine = fingerprint_of(group[0]->cfg);
@@ -568,8 +570,11 @@ int check_group(a2a_ctx* const* group) {
         if (c == nullptr || c->cfg.rank != r || c->cfg.device != group[0]->cfg.device) return A2A_ERR_CONFIG;
         const Fingerprint f = fingerprint_of(c->cfg);
         if (memcmp(&f, &mine, sizeof(f)) != 0) return A2A_ERR_CONFIG;
-        if (!c->peers_ready) return A2A_ERR_STATE;
+        if (!c->peers_ready || c->epoch != group[0]->epoch) return A2A_ERR_STATE;
     }
+    for (int r = 0; r < group[0]->cfg.world_size; ++r)
+        for (int s = 0; s < group[0]->cfg.world_size; ++s)
+            if (group[r]->p.peer[s] != group[s]->region) return A2A_ERR_CONFIG;
     return A2A_OK;
 }
 

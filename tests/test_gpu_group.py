@@ -102,6 +102,43 @@ def test_nothing_begins_when_one_rank_is_refused():
         world.close()
 
 
+@pytest.mark.parametrize("schedule,payload,combine", [("pipelined", "dedup", "push"), ("phased", "direct", "pull")])
+def test_contexts_that_are_no_group_are_refused(schedule, payload, combine):
+    """Contexts of two equal groups mixed, and ranks that are not at the same call."""
+    cfg = pkg.MoEConfig(8, 2, 64, 4)
+    rds = [pkg.generate_input(8, 2, 64, 4, seed=2, rank=r, world_size=2)[1].to(DEV) for r in range(2)]
+    worlds = [LocalWorld(cfg, 2, payload=payload, schedule=schedule, combine=combine) for _ in range(2)]
+
+    def forward(world):
+        return [bits(y) for y in (world.forward_pipelined if schedule == "pipelined" else world.forward_phases)(rds)]
+
+    def launches():
+        return [c.launches for w in worlds for c in w.ctxs]
+
+    try:
+        want = forward(worlds[0])
+        assert all(torch.equal(a, b) for a, b in zip(forward(worlds[1]), want))
+        mixed = object.__new__(LocalWorld)
+        mixed.cfg, mixed.world_size, mixed.ctxs = cfg, 2, [worlds[0].ctxs[0], worlds[1].ctxs[1]]
+        before = launches()
+        with pytest.raises(A2AError) as refused:
+            forward(mixed)
+        assert refused.value.code == _lib.A2A_ERR_CONFIG and launches() == before
+        for c in worlds[0].ctxs:  # one rank begins a call by itself, then the other
+            c.route(rds[0].indices)
+            if c.rank == 0:
+                before = launches()
+                with pytest.raises(A2AError) as refused:
+                    forward(worlds[0])
+                assert refused.value.code == _lib.A2A_ERR_STATE and launches() == before
+        for w in worlds:
+            assert all(torch.equal(a, b) for a, b in zip(forward(w), want))
+            w.check()
+    finally:
+        for w in worlds:
+            w.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("schedule,payload,combine", [("pipelined", "dedup", "push"), ("phased", "direct", "pull")])
 def test_expert_op_on_every_bit_pattern(dtype, schedule, payload, combine):
