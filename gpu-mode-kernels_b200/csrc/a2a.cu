@@ -547,9 +547,10 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
     return rc;
 }
 
-// Roles 1 and 2, of a call whose records exist (the one launch of a single rank writes none: what role 1 would
-// find there belongs to an earlier call, and so may the tensors): this rank's share of two blocks per SM (of four or eight, where a group shares the launch:
-// 134 us against 145 and 159 for role 1 of the workload named above) and, for peers elsewhere, a watcher block.
+// Roles 1 and 2, of a call whose records exist: the one launch of a single rank writes none, and what role 1 would
+// find there belongs to an earlier call.  This rank's share of two blocks per SM (of four or eight, where a group
+// shares the launch: 134 us against 145 and 159 for role 1 of the workload named above) and, for peers elsewhere,
+// a watcher block.
 int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
     for (int r = 0; r < n; ++r)
         if (!cs[r]->sent || !cs[r]->recorded) return A2A_ERR_STATE;
@@ -899,6 +900,16 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
     cudaStream_t st = as_stream(stream);
+    const size_t tk = T > 0 ? (size_t)T * c->cfg.experts_per_token * 4 : 0, rows = T > 0 ? (size_t)T * c->cfg.hidden_dim * 2 : 0;
+    if (c->cfg.schedule == A2A_SCHEDULE_PIPELINED && c->cfg.world_size == 1 && T > 0 &&
+        (overlap(y, rows, w, tk) || overlap(y, rows, idx, tk))) {
+        // An output laid over the weights: the one launch of a single rank reads them block by block while other
+        // blocks already write.  The roles read them all before the first row is written.
+        const a2a_call call = {x, idx, w, y, T};
+        int rc = do_pipe_send(&c, 1, &call, st);
+        for (int role = 1; role <= 2 && rc == A2A_OK; ++role) rc = do_pipe_rest(&c, 1, role, st);
+        return rc;
+    }
     int r = begin_call(c, idx, T);
     if (r != A2A_OK) return r;
     if (T > 0 && (x == nullptr || w == nullptr || y == nullptr)) return A2A_ERR_CONFIG;

@@ -187,3 +187,27 @@ def test_roles_are_refused_where_the_call_was_not_begun_by_role_0(combine):
     finally:
         torch.cuda.synchronize()
         ctx.close()
+
+
+@pytest.mark.parametrize("over", ["weights", "x"])
+@pytest.mark.parametrize("payload,H", [("dedup", 72), ("fp8", 128)])
+def test_output_laid_over_an_input(payload, H, over):
+    """More tokens than the blocks resolve at a time: the weights of a block's second round lie under output
+    rows of its first."""
+    T, K = 6000, 2
+    cfg, rd, _, _ = pkg.generate_input(8, K, H, T, seed=41, rank=0, world_size=1, weights="rand")
+    d = rd.to(DEV)
+    ctx = A2AContext(cfg, 0, 1, device=0, payload=payload, schedule="pipelined", combine="push")
+    try:
+        want = bits(ctx.forward(d.x, d.indices, d.weights))
+        y = torch.empty_like(d.x)
+        x, w = d.x, d.weights
+        if over == "x":
+            x = y.copy_(d.x)
+        else:
+            w = y.view(-1)[8:8 + 2 * T * K].view(torch.float32).view(T, K).copy_(d.weights)
+        assert torch.equal(bits(ctx.forward(x, d.indices, w, y)), want)
+        ctx.check()
+    finally:
+        torch.cuda.synchronize()
+        ctx.close()
