@@ -276,7 +276,9 @@ template <typename T, int P> struct ExpertSel {
     }
 };
 // pipelined schedule: (element type, payload, push/pull) -> kernel
-template <typename T, int P, bool PUSH> struct PipeForward { static KernelFn get() { return pipe_forward_kernel<T, P, PUSH>; } };
+template <typename T, int P, bool PUSH> struct PipeForward {
+    static PhaseFn get() { return {pipe_forward_kernel<T, P, PUSH, RankParams>, pipe_forward_kernel<T, P, PUSH, GroupParams>}; }
+};
 template <typename T, int P, bool PUSH> struct PipeRole {
     template <int ROLE>
     static PhaseFn pair() { return {pipe_role_kernel<T, P, PUSH, ROLE, RankParams>, pipe_role_kernel<T, P, PUSH, ROLE, GroupParams>}; }
@@ -308,14 +310,15 @@ PhaseFn combine_fn(const a2a_ctx* c) {
     return {combine_kernel<__half, RankParams>, combine_kernel<__half, GroupParams>};
 }
 
-int launch(a2a_ctx* c, KernelFn fn, int grid, int smem, cudaStream_t st, bool cooperative = false) {
+int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false) {
+    static_assert(sizeof(RankParams) == sizeof(DevParams), "a kernel of one rank takes either");
     DevParams p = call_params(c);
     if (p.trace != nullptr && grid > kTraceBlocks) p.trace = nullptr;
     if (p.trace != nullptr) c->last_grid = grid;
     void* args[] = {&p};
     cudaError_t e = (cooperative && !c->plain_launch)
-        ? cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(kThreads), args, smem, st)
-        : cudaLaunchKernel((const void*)fn, dim3(grid), dim3(kThreads), args, smem, st);
+        ? cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st)
+        : cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, smem, st);
     c->launches++;
     if (e != cudaSuccess) return -(int)e;
     return A2A_OK;
@@ -380,7 +383,7 @@ int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    return launch(c, wide ? solo_fn<2>(c) : solo_fn<1>(c), (int)blocks, 0, st);
+    return launch(c, (const void*)(wide ? solo_fn<2>(c) : solo_fn<1>(c)), (int)blocks, 0, st);
 }
 
 // The device address of host memory that kernels can reach -- pinned, all `bytes` of it in one allocation or
@@ -433,7 +436,7 @@ int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
 int do_route(a2a_ctx* c, const int32_t* idx, int T, cudaStream_t st) {
     int r = begin_call(c, idx, T);
     if (r != A2A_OK) return r;
-    return launch(c, route_kernel, 1, c->smem_bytes, st);
+    return launch(c, (const void*)route_kernel, 1, c->smem_bytes, st);
 }
 
 // Sender and router blocks per rank where `n` ranks share one launch on one GPU: two blocks per SM run at
@@ -518,8 +521,8 @@ int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y,
     return launch_ranks(cs, n, combine_fn(c), grid_for_ranks(c, n, (warps + kThreads / 32 - 1) / (kThreads / 32), 8), 0, st);
 }
 
-// Role 0 of the pipelined kernel: its tensors are checked and the call begun on every rank.
-int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st) {
+// The tensors of a pipelined call are checked and the call begun on every rank.
+int begin_pipe_call(a2a_ctx* const* cs, int n, const a2a_call* calls) {
     for (int r = 0; r < n; ++r) {
         const a2a_call& k = calls[r];
         const int rc = check_call(cs[r], k.topk_idx, k.num_tokens);
@@ -534,6 +537,13 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
         cs[r]->p.w = k.topk_weights;
         cs[r]->p.y = k.y;  // with one rank and the PUSH combine the expert blocks already write the output
     }
+    return A2A_OK;
+}
+
+// Role 0 of the pipelined kernel.
+int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st) {
+    const int begun = begin_pipe_call(cs, n, calls);
+    if (begun != A2A_OK) return begun;
     const a2a_ctx* c = cs[0];
     const int ws = c->cfg.world_size;
     int ns = c->p.senders, nr = c->p.routers, smem = c->pipe_smem;
@@ -558,6 +568,39 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
     const int blocks = c->num_sms * 2 / n;
     const int smem = role == 1 && c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
     return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), n > 1 ? blocks : 1 + blocks, smem, st);
+}
+
+// The one launch of all ranks of a group on one GPU, two blocks per SM shared out among them.  Unlike in the
+// phases above nothing is shortened for ranks that are near: this is the kernel a GPU per rank runs, and here so
+// that one GPU can hold it to the checker.  The cooperative launch keeps every block running, so no block waits
+// for one that is not, and each wait is bounded.  It needs room for the watchers, two senders, and twice the routers.
+int do_group_forward(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st) {
+    const a2a_ctx* c = cs[0];
+    const int blocks = 2 * c->num_sms / n, watchers = c->cfg.payload == A2A_PAYLOAD_FP8 ? 2 : 0;
+    int routers = blocks / (4 * n) < c->p.routers ? blocks / (4 * n) : c->p.routers;
+    if (routers < 1) routers = 1;
+    const int room = blocks - watchers - 2 * n * routers;
+    const int senders = room < c->p.senders ? room : c->p.senders;
+    if (n < 2 || senders < 2) return A2A_ERR_CONFIG;
+    const size_t a = pipe_sender_smem(c->cfg.max_num_tokens, n, senders), b = pipe_router_smem(c->cfg.max_num_tokens, c->p.L);
+    if (a > kMaxSenderSmemBytes) return A2A_ERR_CONFIG;
+    const int begun = begin_pipe_call(cs, n, calls);
+    if (begun != A2A_OK) return begun;
+    GroupParams g;
+    for (int r = 0; r < n; ++r) {
+        g.p[r] = call_params(cs[r]);
+        g.p[r].senders = senders;
+        g.p[r].routers = routers;
+        g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
+        cs[r]->launches++;
+    }
+    g.n = n;
+    void* args[] = {&g};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)select_pipe<PipeForward>(c).group, dim3(n * blocks),
+                                                      dim3(kThreads), args, align_up(a > b ? a : b, 128), st);
+    if (e != cudaSuccess) return -(int)e;
+    for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->recorded = true;
+    return A2A_OK;
 }
 
 // The contexts of every rank of one group, all on one GPU, attached to one another and at the same call?  A launch
@@ -733,13 +776,13 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     if (pipelined) {
         const size_t a = cfg->world_size > 1 ? pipe_sender_smem(T, cfg->world_size, p.senders) : 0, b = pipe_router_smem(T, L);
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
-        opt_in((const void*)select_pipe<PipeForward>(c));
+        opt_in_both(select_pipe<PipeForward>(c));
         opt_in_both(select_pipe<PipeRole>(c, 0));
         if (e == cudaSuccess && cfg->world_size == 1) {
             c->forward_grid = c->num_sms;
             c->fused = true;  // the solo kernel: no block waits for another
         } else if (e == cudaSuccess) {
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)select_pipe<PipeForward>(c), kThreads, c->pipe_smem);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)select_pipe<PipeForward>(c).one, kThreads, c->pipe_smem);
             if (occ > 2) occ = 2;
             c->forward_grid = c->num_sms * occ;
             c->fused = true;
@@ -920,7 +963,7 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
         c->p.y = y;
         r = c->cfg.world_size == 1
             ? launch_solo(c, st)
-            : launch(c, select_pipe<PipeForward>(c), c->forward_grid, c->pipe_smem, st, /*cooperative=*/true);
+            : launch(c, (const void*)select_pipe<PipeForward>(c).one, c->forward_grid, c->pipe_smem, st, /*cooperative=*/true);
         if (r == A2A_OK) {
             c->sent = true;
             c->recorded = c->cfg.world_size > 1;
@@ -931,7 +974,7 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
         c->p.x = x;
         c->p.w = w;
         c->p.y = y;
-        r = launch(c, select_tp<ForwardSel>(c), c->forward_grid, c->smem_bytes, st, /*cooperative=*/true);
+        r = launch(c, (const void*)select_tp<ForwardSel>(c), c->forward_grid, c->smem_bytes, st, /*cooperative=*/true);
         if (r == A2A_OK) c->sent = true;
         return r;
     }
@@ -1032,6 +1075,15 @@ int a2a_group_step(a2a_ctx* const* group, int phase, const a2a_call* calls, void
         case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st);
         default: return A2A_ERR_CONFIG;
     }
+}
+
+int a2a_group_forward(a2a_ctx* const* group, const a2a_call* calls, void* stream) {
+    const int rc = check_group(group);
+    if (rc != A2A_OK) return rc;
+    if (calls == nullptr) return A2A_ERR_CONFIG;
+    if (group[0]->cfg.schedule != A2A_SCHEDULE_PIPELINED) return A2A_ERR_STATE;
+    DeviceGuard guard(group[0]->cfg.device);
+    return do_group_forward(group, group[0]->cfg.world_size, calls, as_stream(stream));
 }
 
 int a2a_barrier(a2a_ctx* c, void* stream) {

@@ -1062,10 +1062,12 @@ extern __shared__ __align__(128) uint8_t a2a_pipe_smem[];
 template <int PAYLOAD>
 __device__ __forceinline__ int watcher_blocks(const DevParams& p) { return (PAYLOAD == A2A_PAYLOAD_FP8 && p.ws > 1) ? 2 : 0; }
 
-// The whole path in one cooperative launch.
-template <typename T, int PAYLOAD, bool PUSH>
-__global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_constant__ DevParams p) {
-    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+// The whole path in one cooperative launch: of one rank on a GPU of its own or, with the same blocks, flags and
+// watchers, of every rank of a group on one GPU.
+template <typename T, int PAYLOAD, bool PUSH, class P>
+__global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_constant__ P g) {
+    const DevParams& p = g.rank();
+    const int G = g.blocks(), b = g.block();
     const int ns = p.ws > 1 ? p.senders : 0;
     const int nw = watcher_blocks<PAYLOAD>(p);
     stamp(p, kStampStart);

@@ -3,8 +3,11 @@
 Kernels that wait on a peer must never share a GPU with the kernel they wait
 for, so the ranks here are stepped in lock-step: one launch runs a phase of every
 rank, the sending phase before any waiting one, on one stream, and each wait finds its
-flag already set.  The kernels, addresses, flags and epochs are exactly those of
-a real multi-GPU run; only CUDA IPC and true concurrency are not exercised.
+flag already set.  Routing, rows, records, flag values and epochs are those of a group
+with a GPU per rank; what depends on where a peer is, is not: flags are awaited at gpu
+scope without watchers, and 16-bit rows are sent with another ring depth.  The forms for distant peers
+run in ``forward_one_launch``, which puts every rank's blocks into one cooperative
+launch, and in the phases called context by context.
 Validation tool: parity tests and the smoke check use it to cover world sizes
 2, 4 and 8 on a single device.
 """
@@ -37,9 +40,11 @@ class LocalWorld:
             raise _lib.A2AError(_lib.A2A_ERR_STATE, f"{self.world_size} ranks, but data for {len(rank_datas)}")
         return (_lib.Call * self.world_size)()
 
+    def _handles(self):
+        return (C.c_void_p * self.world_size)(*[c._h.value for c in self.ctxs])
+
     def _step(self, phase: str, calls=None) -> None:
-        handles = (C.c_void_p * self.world_size)(*[c._h.value for c in self.ctxs])
-        _lib.check(self.ctxs[0].lib.a2a_group_step(handles, _lib.GROUP_PHASE[phase], calls, _lib.current_stream()))
+        _lib.check(self.ctxs[0].lib.a2a_group_step(self._handles(), _lib.GROUP_PHASE[phase], calls, _lib.current_stream()))
 
     def _send(self, rank_datas: Sequence) -> None:
         """route + dispatch_send on every rank, in one launch."""
@@ -82,18 +87,33 @@ class LocalWorld:
     def forward_pipelined(self, rank_datas: Sequence) -> List[torch.Tensor]:
         """The roles of the pipelined one-launch kernel as three launches, in lock-step:
         every rank's senders and routers, then every rank's expert blocks, then every rank's combine."""
+        calls, ys = self._whole_calls(rank_datas)
+        self._step("pipe_send", calls)
+        self._begun(rank_datas, ys)
+        self._step("pipe_expert")
+        self._step("pipe_combine")
+        return ys
+
+    def forward_one_launch(self, rank_datas: Sequence) -> List[torch.Tensor]:
+        """The pipelined one-launch kernel of every rank, as a group with a GPU per rank runs it, in one cooperative
+        launch: every block of every rank is running, so the waits of one rank for another are safe here."""
+        calls, ys = self._whole_calls(rank_datas)
+        _lib.check(self.ctxs[0].lib.a2a_group_forward(self._handles(), calls, _lib.current_stream()))
+        self._begun(rank_datas, ys)
+        return ys
+
+    def _whole_calls(self, rank_datas: Sequence):
         calls, ys = self._calls(rank_datas), []
         for call, c, rd in zip(calls, self.ctxs, rank_datas):
             n = c._check_inputs(rd.x, rd.indices, rd.weights, None, on_device=True)
             ys.append(torch.empty(n, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=c.device))
             call.x, call.topk_idx, call.topk_weights = rd.x.data_ptr(), rd.indices.data_ptr(), rd.weights.data_ptr()
             call.y, call.num_tokens = ys[-1].data_ptr(), n
-        self._step("pipe_send", calls)
+        return calls, ys
+
+    def _begun(self, rank_datas: Sequence, ys) -> None:
         for c, rd, y in zip(self.ctxs, rank_datas, ys):
             c._num_tokens, c._y, c._keep = y.shape[0], y, [rd.x, rd.indices, rd.weights, y]
-        self._step("pipe_expert")
-        self._step("pipe_combine")
-        return ys
 
     def check(self) -> None:
         for c in self.ctxs:

@@ -240,6 +240,12 @@ typedef struct a2a_call {
 } a2a_call;
 int a2a_group_step(a2a_ctx* const* group, int phase, const a2a_call* calls, void* stream);
 
+/* a2a_forward of every rank of such a group (two ranks or more, pipelined contexts) as ONE cooperative launch
+ * that holds the blocks of all ranks: the kernel, watchers, flags and fences that a group with a GPU per rank
+ * runs, for holding them to a checker where there is one GPU.  For speed on one GPU take the steps above.
+ * A2A_ERR_CONFIG where the group's blocks do not fit the device together. */
+int a2a_group_forward(a2a_ctx* const* group, const a2a_call* calls, void* stream);
+
 /* Cross-GPU rendezvous on the device: returns (on the stream) once every rank's
  * stream has reached it.  Bounded wait.  Used to align ranks before timing.
  * Plays the role of dist.barrier() around the timed call (my_eval.py:160-172). */
