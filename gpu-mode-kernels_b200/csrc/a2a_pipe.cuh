@@ -838,11 +838,12 @@ __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, i
         }
         load_wire_chunk<T, PAYLOAD>(p, own, src, v0, nvec, m.q);
     };
+    const int t_end = p.ws == 1 ? p.T : p.T_max;  // one rank's rows go into the caller's y, others into buffers of T_max
     auto process = [&](const Cursor& c, const Item& m) {
         const int s = c.s, v0 = c.ch * 128, t = m.t;
         const bool own = (s == p.rank);
         const bool via_engine = PUSH && !own;  // the home rank is a peer: return through the copy engine
-        if (t < 0 || t >= (own ? p.T : p.T_max)) {  // own rows lie in the caller's tensors, a peer's in buffers of T_max
+        if (t < 0 || t >= t_end) {
             record_error(p.status, A2A_ERR_CAPACITY, p.rank, s, kPhaseRecv, p.epoch, t);
             return;
         }
