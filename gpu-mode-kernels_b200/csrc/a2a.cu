@@ -205,8 +205,8 @@ int validate(const a2a_config& c) {
     if (c.schedule == A2A_SCHEDULE_PIPELINED) {
         // the senders move one wire row per (token, destination): the per-pair DIRECT payload has none
         if (c.payload != A2A_PAYLOAD_DEDUP && c.payload != A2A_PAYLOAD_FP8) return A2A_ERR_CONFIG;
-        // FP8: a warp assembles a whole wire row in its own stage of the sender ring
-        if (c.payload == A2A_PAYLOAD_FP8 && make_layout(c).stage_row_bytes > kWarpStageBytes) return A2A_ERR_CONFIG;
+        // FP8: a block assembles a whole wire row in one stage of the sender ring
+        if (c.payload == A2A_PAYLOAD_FP8 && make_layout(c).stage_row_bytes > kFp8StageBytes) return A2A_ERR_CONFIG;
         if (c.chunks > 1) return A2A_ERR_CONFIG;
         // one rank has no senders and routes inside its one kernel; only its stepped roles need the tables
         const size_t router_room = c.world_size == 1 ? kMaxSmemBytes : kMaxPipeSmemBytes;
@@ -280,9 +280,14 @@ template <typename T, int P, bool PUSH> struct PipeForward {
     static PhaseFn get() { return {pipe_forward_kernel<T, P, PUSH, RankParams>, pipe_forward_kernel<T, P, PUSH, GroupParams>}; }
 };
 template <typename T, int P, bool PUSH> struct PipeRole {
-    template <int ROLE>
-    static PhaseFn pair() { return {pipe_role_kernel<T, P, PUSH, ROLE, RankParams>, pipe_role_kernel<T, P, PUSH, ROLE, GroupParams>}; }
-    static PhaseFn get(int role) { return role == 0 ? pair<0>() : role == 1 ? pair<1>() : pair<2>(); }
+    template <int PP, bool PUSHP, int ROLE>
+    static PhaseFn pair() {
+        return {pipe_role_kernel<T, PP, PUSHP, ROLE, RankParams>, pipe_role_kernel<T, PP, PUSHP, ROLE, GroupParams>};
+    }
+    // what is sent does not depend on the combine, nor the combine on how rows travelled
+    static PhaseFn get(int role) {
+        return role == 0 ? pair<P, true, 0>() : role == 1 ? pair<P, PUSH, 1>() : pair<A2A_PAYLOAD_DEDUP, PUSH, 2>();
+    }
 };
 template <template <typename, int, bool> class F, typename T, typename... A>
 auto select_pipe_t(const a2a_ctx* c, A... a) {

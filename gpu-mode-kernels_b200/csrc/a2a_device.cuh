@@ -114,6 +114,7 @@ struct DevParams {
 // for rank position i % n as that rank's block i / n.  Two types, because parameters of eight ranks, looked up
 // by position, cost a launch for one rank half a microsecond and its blocks as much.
 struct RankParams {
+    static constexpr bool kGroup = false;
     DevParams p;
     __device__ __forceinline__ const DevParams& rank() const { return p; }
     __device__ __forceinline__ int block() const { return (int)blockIdx.x; }
@@ -121,6 +122,7 @@ struct RankParams {
 };
 
 struct GroupParams {
+    static constexpr bool kGroup = true;
     DevParams p[A2A_MAX_WORLD];
     int n;
     __device__ __forceinline__ const DevParams& rank() const { return p[blockIdx.x % n]; }

@@ -410,7 +410,7 @@ __device__ __forceinline__ void sender_role_fp8(const DevParams& p, uint8_t* sme
     for (int stage_no = 0; g < mine; stage_no = (stage_no + 1) % kFp8Stages) {
         const int gn = next_token(g);
         if (gn < mine) load(gn, 0, qn);
-        uint8_t* stage = m.ring + (size_t)stage_no * kWarpStageBytes;
+        uint8_t* stage = m.ring + (size_t)stage_no * kFp8StageBytes;
         for (int v0 = 0; v0 < nvec; v0 += kAhead * kThreads) {
             if (v0 > 0) load(g, v0, q);
 #pragma unroll
@@ -1060,17 +1060,14 @@ extern __shared__ __align__(128) uint8_t a2a_pipe_smem[];
 // their spare warps.  FP8: every warp of a sender block quantises, so blocks 0 and 1 only watch
 // and blocks [2, 2 + senders) send.  The next `ws` blocks route first, and every block after
 // the senders is an expert block.
-template <int PAYLOAD>
-__device__ __forceinline__ int watcher_blocks(const DevParams& p) { return (PAYLOAD == A2A_PAYLOAD_FP8 && p.ws > 1) ? 2 : 0; }
-
 // The whole path in one cooperative launch: of one rank on a GPU of its own or, with the same blocks, flags and
 // watchers, of every rank of a group on one GPU.
 template <typename T, int PAYLOAD, bool PUSH, class P>
 __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_constant__ P g) {
     const DevParams& p = g.rank();
     const int G = g.blocks(), b = g.block();
-    const int ns = p.ws > 1 ? p.senders : 0;
-    const int nw = watcher_blocks<PAYLOAD>(p);
+    const int ns = p.senders;
+    constexpr int nw = PAYLOAD == A2A_PAYLOAD_FP8 ? 2 : 0;
     stamp(p, kStampStart);
     if (b < nw) {
         stamp_value(p, kStampRole, kRoleWatcher);
@@ -1108,30 +1105,29 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
 // The same roles as separate launches: for callers that want the phases apart, and for stepping a group
 // that lives on ONE GPU -- a kernel that waits never shares the GPU with the kernel it waits for, so what
 // runs together is one role of every rank.  ROLE 0: senders + routers.  1: one watcher block + experts.
-// 2: one watcher block + combine.
+// 2: one watcher block + combine.  A group's launch has no watcher blocks.
 template <typename T, int PAYLOAD, bool PUSH, int ROLE, class P>
 __global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ P g) {
     const DevParams& p = g.rank();
     const int G = g.blocks(), b = g.block();
-    const int ns = p.ws > 1 ? p.senders : 0;
+    const int ns = p.senders;
     stamp(p, kStampStart);
     if (ROLE == 0) {
         if (b < ns) {
             if (PAYLOAD == A2A_PAYLOAD_FP8) sender_role_fp8<T>(p, a2a_pipe_smem, b, ns);
-            else if (p.local) sender_role<true>(p, a2a_pipe_smem, b, ns, -1, 0);
-            else sender_role<false>(p, a2a_pipe_smem, b, ns, -1, 0);
+            else sender_role<P::kGroup>(p, a2a_pipe_smem, b, ns, -1, 0);
         } else {
             const int rb = b - ns, d = (p.rank + 1 + rb % p.ws) % p.ws;
             router_role(p, a2a_pipe_smem, d, rb / p.ws, p.routers, rb == 0, (uint32_t)(d == p.rank ? 0 : ns) + p.routers);
         }
         stamp(p, kStampSent);
     } else if (ROLE == 1) {
-        const int first = p.local ? 0 : 1;
+        constexpr int first = P::kGroup ? 0 : 1;
         if (b < first) watcher_role(p, kFlagDispatch, kPhaseRecv, (int)(threadIdx.x >> 5));
         else expert_role<T, PAYLOAD, PUSH>(p, a2a_pipe_smem, b - first, G - first);
         stamp(p, kStampExpertDone);
     } else {
-        const int first = p.local ? 0 : 1;
+        constexpr int first = P::kGroup ? 0 : 1;
         if (b < first) {
             watcher_role(p, kFlagExpert, kPhaseCombine, (int)(threadIdx.x >> 5));
         } else if (PUSH) {
