@@ -175,8 +175,8 @@ int check_blobs(const a2a_config& cfg, const uint8_t* all, size_t nbytes, char* 
 // engine (two 14 KB loads ahead, four stores in flight).  Measured at 8 GPUs, the sending role alone
 // takes 52 us + 624 us / blocks (78 / 65 / 63 / 60 us with 24 / 48 / 64 / 96 blocks) and the whole
 // call 126.7 / 113.8 / 110.6 / 109.1 us: 96 blocks at 8 ranks, where there is most to send; 48 below,
-// where the call is a chain of latencies and the expert blocks are better served.  FP8: a block
-// quantises a row at a time and the arithmetic is the cost: 96.
+// where the call is a chain of latencies and the expert blocks are better served.  FP8: 96, chosen
+// when a block quantised a row for each of its destinations; not measured again since it does so once.
 int pipe_senders(const a2a_config& c) {
     if (c.world_size == 1) return 0;
     if (c.senders > 0) return c.senders;

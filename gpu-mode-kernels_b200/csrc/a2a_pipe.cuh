@@ -10,6 +10,8 @@
 //            needed for that, so rows move from the first microsecond.  When a
 //            destination's last store has completed the block draws a ticket; the last
 //            ticket (all senders + that destination's router) publishes the dispatch flag.
+//            FP8: token by token instead, each row quantised once by the whole block and
+//            stored to every rank that wants it; all tickets are drawn at the end.
 //   routers  (a few blocks per destination, then they join the experts)
 //            build the [token x expert] bitmap of the destination's experts only, derive
 //            the slot of every (token, k) row by popc, and write the destination its
@@ -29,6 +31,9 @@
 //            experts of t of their partial rows, read from local memory.  PULL: each
 //            (token, k) row is pulled from the expert's slab over NVLink and reduced with
 //            the token's weights at home (the phase-by-phase combine, started per peer).
+//
+// A group of two ranks or more runs it; a single rank has a2a_solo.cuh.  Stepped as launches of their own,
+// the roles also serve one rank, which has no senders then.
 //
 // Nothing here waits on work of its own role on another GPU, senders and routers never wait
 // at all, and every wait is bounded; see a2a_device.cuh for the flag protocol.
@@ -369,9 +374,13 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
 // 16-byte loads, requested a row ahead, amax over the 16 lanes of a 128-value block, e4m3 bytes and fp32
 // scales into one of eight 12 KB stages of the ring; then thread 0 hands the finished wire row to the copy
 // engine once per destination and the block goes on to the next row while up to six rows are still on their
-// way.  All destinations are through at the end, each booked by a thread of its own.
+// way.  All destinations are through at the end, each booked by a thread of its own: no receiver starts on
+// rows of this rank before, where it formerly started destination by destination.  With every role of every
+// rank overlapping in one launch on one GPU (256 tokens of 7168) that costs nothing at two ranks (72.2 us, per
+// destination 71.5; 768 tokens 182.6 / 177.7) and four (142 / 142), and gains at eight (314 / 332; rows of 2048
+// 116 / 145).  Over NVLink the two have not been compared.
 constexpr int kFp8Stages = 8;
-constexpr int kWarpStageBytes = kStages * kStageBytes / kFp8Stages;  // 12 KB: the largest FP8 wire row
+constexpr int kFp8StageBytes = kStages * kStageBytes / kFp8Stages;  // 12 KB: the largest FP8 wire row
 
 template <typename T>
 __device__ __forceinline__ void sender_role_fp8(const DevParams& p, uint8_t* smem, int sb, int ns) {

@@ -7,7 +7,7 @@
 // so an update is one pass over the banks whatever the data is -- random bytes and one value 90 % of
 // the time cost the same -- and the word's address comes out of the data with one shift and one
 // three-input logic operation.  Warps share the table (32 KB a block), so the updates are atomic, without
-// a result.  Measured on 512 MB, random bytes: 85 us = 6.3 TB/s (of 6.55 copied), against 303 us with a
+// a result.  Measured on 512 MB, random bytes: the launch 85 us = 6.3 TB/s (of 6.55 copied), against 303 us with a
 // 256-word table per warp, where 32 random bytes meet in a bank 3.5 deep and the frequent value needed
 // ballots; one byte counter per (value, thread) without atomics is two accesses a byte: 256 us.
 #include <cooperative_groups.h>
@@ -29,11 +29,12 @@ constexpr int kUnroll = 4;
 constexpr int kBins = 256;
 constexpr int kCluster = 8;
 // One cluster writes the counts itself: no zeroing in front, one launch.  128 KB 4.3 us against 6.3 as
-// zero + count; 512 KB 6.3 against 6.2, the reading of eight SMs being the longer part from there on.
+// zero + count; 512 KB 6.3 against 6.2.  A block takes 32 KB at a time, so below 256 KB only some of the
+// cluster's blocks count, and at 512 KB 16 blocks of the other launch do.
 constexpr size_t kClusterBytes = 256 * 1024;
 // Below this a block per SM: 256 sums per block meet at 256 global words, and with few bytes per block
-// that is what the call waits for (10 MB 6.3 us against 8.3 with three blocks per SM, 42 MB 12.4 / 12.2,
-// 168 MB 44 / 33).
+// that is what the call waits for.  Measured against the three blocks per SM that large buffers had then:
+// 10 MB 6.3 us / 8.3, 42 MB 12.4 / 12.2, 168 MB 44 / 33.
 constexpr size_t kFullBytes = 32 * 1024 * 1024;
 
 // `lane4` = 4 * lane: the byte offset of the lane's word in a row of 32.

@@ -1,10 +1,11 @@
 """GPU parity of the pipelined schedule (role-specialised one-launch kernel), both combine modes.
 
 World sizes above one are stepped role by role on a single GPU (``LocalWorld.forward_pipelined``:
-the same device code as the one-launch kernel, launched as senders+routers / experts / combine so
-that a kernel that waits never shares the GPU with the kernel it waits for).  At world size one
-the real one-launch kernel runs and must give the same bits as the stepped roles.  The
-one-process-per-GPU form is covered by test_x_gpu_multiprocess.py.
+launched as senders+routers / experts / combine so that a kernel that waits never shares the GPU with
+the kernel it waits for, in the forms for peers on this GPU).  The one-launch kernel itself and the forms for
+distant peers are held to the checker by test_gpu_one_launch.py.  At world size one the forward is a
+kernel of its own and must give the same bits as the stepped roles.  The one-process-per-GPU form is
+covered by test_x_gpu_multiprocess.py.
 """
 from types import SimpleNamespace
 
@@ -199,7 +200,7 @@ def test_reference_task_shapes_fp16(spec):
 
 @pytest.mark.parametrize("combine", COMBINES)
 def test_one_launch_equals_stepped_roles_single_rank(combine):
-    """World size 1 (no peer to wait for): the cooperative one-launch kernel gives the bits of the
+    """World size 1 (no peer to wait for): the one kernel of a single rank gives the bits of the
     three stepped launches, and both match the checker."""
     cfg, rd, _, _ = pkg.workload_input("c2", 0, 1)
     _, ys = O.simulate(cfg, 1, [rd])
