@@ -355,9 +355,12 @@ def main():
     h2d = hx.numel() * hx.element_size() + hi.numel() * 4 + hw.numel() * 4
     d2h = hy.numel() * hy.element_size()
 
-    # ---- per-kernel pass: events between the separate launches of the same device code ----
+    # ---- per-kernel pass: events between the separate launches of the same device code.  A single rank's forward
+    # is one kernel that shares none with the stepped roles: its line is that kernel ----
     ph_steps = min(args.steps, 200)
-    if pipelined:
+    if pipelined and ws == 1:
+        names, calls = ["solo"], [lambda: ctx.forward(rd.x, rd.indices, rd.weights, y)]
+    elif pipelined:
         names = ["send_route", "expert", "combine"]
         calls = [lambda: ctx.pipe_step(0, rd.x, rd.indices, rd.weights, y), lambda: ctx.pipe_step(1),
                  lambda: ctx.pipe_step(2)]
@@ -414,10 +417,11 @@ def main():
         roofline = {"bound": "hbm", "kernel": "one-launch forward (route + send + expert + combine)",
                     "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                     "traffic": SINGLE_GPU_TRAFFIC.get((args.workload, schedule, combine)),
-                    "peak_kind": f"of {peak_kind}", "algorithmic_bytes": alg, "kernel_us": ms * 1e3,
-                    "traffic_note": "bytes per launch from one ncu capture of this kernel on this workload "
-                                    "(dram__bytes_read.sum + dram__bytes_write.sum; L2 traffic beside it): the working set "
-                                    "fits the 126 MB L2, so DRAM sees far less than the algorithmic bytes"}
+                    "peak_kind": f"of {peak_kind}", "algorithmic_bytes": alg, "kernel_us": ms * 1e3}
+        if roofline["traffic"] is not None:
+            roofline["traffic_note"] = ("bytes per launch from one ncu capture of this kernel on this workload "
+                                        "(dram__bytes_read.sum + dram__bytes_write.sum; L2 traffic beside it): the working "
+                                        "set fits the 126 MB L2, so DRAM sees far less than the algorithmic bytes")
         nvlink = None
     else:
         achieved = tr["algorithmic_bytes"] / (ms * 1e-3) / 1e9

@@ -83,11 +83,16 @@ def test_ragged_sizes_and_unaligned_starts(size, offset):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("size", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1, 148 * 512 * 16 + 5, (1 << 25) - 1, 1 << 25, (1 << 25) + 31])
+@pytest.mark.parametrize("size", [
+    (1 << 18) - 1, 1 << 18, (1 << 18) + 1,
+    148 * 512 * 16 + 5,                             # a vector per thread of a block per SM; a third of the blocks count
+    148 * 512 * 4 * 16, 148 * 512 * 4 * 16 + 21,    # one round of that grid; one vector and five bytes more
+    (1 << 25) - 1, 1 << 25, (1 << 25) + 31,
+])
 @pytest.mark.parametrize("offset,frequent", [(0, 0.0), (9, 0.9)])
 def test_either_side_of_the_launch_rules(size, offset, frequent):
-    """One cluster / two launches, one block / three blocks per SM, one vector more than a grid holds; twice
-    into the same output, the second time on other data."""
+    """One cluster / two launches, one block / two blocks per SM, one vector more than a round of the grid takes;
+    twice into the same output, the second time on other data."""
     g = torch.Generator().manual_seed(size + offset)
     out = torch.full((256,), 3, dtype=torch.int64, device="cuda:0")
     from gpu_mode_kernels_b200.histogram import histogram256
