@@ -40,11 +40,9 @@ class LocalWorld:
             raise _lib.A2AError(_lib.A2A_ERR_STATE, f"{self.world_size} ranks, but data for {len(rank_datas)}")
         return (_lib.Call * self.world_size)()
 
-    def _handles(self):
-        return (C.c_void_p * self.world_size)(*[c._h.value for c in self.ctxs])
-
     def _step(self, phase: str, calls=None) -> None:
-        _lib.check(self.ctxs[0].lib.a2a_group_step(self._handles(), _lib.GROUP_PHASE[phase], calls, _lib.current_stream()))
+        handles = (C.c_void_p * self.world_size)(*[c._h.value for c in self.ctxs])
+        _lib.check(self.ctxs[0].lib.a2a_group_step(handles, _lib.GROUP_PHASE[phase], calls, _lib.current_stream()))
 
     def _send(self, rank_datas: Sequence) -> None:
         """route + dispatch_send on every rank, in one launch."""
@@ -58,7 +56,7 @@ class LocalWorld:
             c._num_tokens, c._keep = rd.indices.shape[0], [rd.indices, rd.x]
 
     def _combine(self, rank_datas: Sequence) -> List[torch.Tensor]:
-        calls, ys = self._calls(rank_datas), []
+        calls, ys = (_lib.Call * self.world_size)(), []
         for call, c, rd in zip(calls, self.ctxs, rank_datas):
             assert rd.weights.dtype == torch.float32 and rd.weights.is_contiguous() and rd.weights.is_cuda
             ys.append(torch.empty(c._num_tokens, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=c.device))
@@ -98,7 +96,8 @@ class LocalWorld:
         """The pipelined one-launch kernel of every rank, as a group with a GPU per rank runs it, in one cooperative
         launch: every block of every rank is running, so the waits of one rank for another are safe here."""
         calls, ys = self._whole_calls(rank_datas)
-        _lib.check(self.ctxs[0].lib.a2a_group_forward(self._handles(), calls, _lib.current_stream()))
+        handles = (C.c_void_p * self.world_size)(*[c._h.value for c in self.ctxs])
+        _lib.check(self.ctxs[0].lib.a2a_group_forward(handles, calls, _lib.current_stream()))
         self._begun(rank_datas, ys)
         return ys
 
