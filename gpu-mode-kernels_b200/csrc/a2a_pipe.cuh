@@ -685,8 +685,9 @@ __device__ __forceinline__ uint4 wire_vector(bool own, const uint4& q, bool vali
 //           store path of the SM in front of the slab stores and the next item's loads; such a source
 //           is booked one source later (by then its bulk stores have long completed), the last, and one
 //           whose successor is not here yet, at once.
-// What bounds it: not the memory but a warp's own instructions per item (at two blocks per SM twelve workers
-// share an SM; 900 instructions and six cycles each made 2.8 us an item).  Hence the next item's loads ahead of
+// What bounds it: not the memory (DRAM 43 % busy) nor the issue slots (46 %) but a warp's own chain of instructions
+// per item (at two blocks per SM twelve workers share an SM; 900 instructions and six cycles each made 2.8 us an
+// item).  Hence the next item's loads ahead of
 // this one's work, packed products and multiply-adds, one accumulator vector at a time, no division per item.
 // Eight ranks in one launch, 256 tokens of 7168, top-8 of 256 experts: 134 -> 109 us, FP8 wire rows 209 -> 135;
 // three blocks per SM would leave 80 registers, and spill: 115 and 188.
