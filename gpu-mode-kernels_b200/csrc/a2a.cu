@@ -577,7 +577,7 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
 
 // The one launch of all ranks of a group on one GPU, two blocks per SM shared out among them.  Unlike in the
 // phases above nothing is shortened for ranks that are near: this is the kernel a GPU per rank runs, and here so
-// that one GPU can hold it to the checker.  The cooperative launch keeps every block running, so no block waits
+// that one GPU can hold it to the oracle.  The cooperative launch keeps every block running, so no block waits
 // for one that is not, and each wait is bounded.  It needs room for the watchers, two senders, and twice the routers.
 int do_group_forward(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st) {
     const a2a_ctx* c = cs[0];

@@ -243,7 +243,7 @@ int a2a_group_step(a2a_ctx* const* group, int phase, const a2a_call* calls, void
 
 /* a2a_forward of every rank of such a group (two ranks or more, pipelined contexts) as ONE cooperative launch
  * that holds the blocks of all ranks: the kernel, watchers, flags and fences that a group with a GPU per rank
- * runs, for holding them to a checker where there is one GPU.  For speed on one GPU take the steps above.
+ * runs, for holding them to the oracle where there is one GPU.  For speed on one GPU take the steps above.
  * A2A_ERR_CONFIG where the group's blocks do not fit the device together. */
 int a2a_group_forward(a2a_ctx* const* group, const a2a_call* calls, void* stream);
 

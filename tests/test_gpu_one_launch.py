@@ -1,5 +1,5 @@
 """The kernel that a group with a GPU per rank runs -- senders in their form for distant peers, watchers, flags and
-fences at system scope, all roles at the same time -- held to the CPU checker on one GPU: every rank's blocks in one
+fences at system scope, all roles at the same time -- held to the oracle on one GPU: every rank's blocks in one
 cooperative launch, and the same roles rank by rank.  ``LocalWorld``'s steps, which the other tests call, run
 variants for peers on the same GPU."""
 import pytest
@@ -24,7 +24,7 @@ def bits(t):
 
 
 def run_case(cfg, ws, rds_cpu, how, payload, combine, calls=1):
-    """`calls` calls against the checker; the outputs bit for bit those of the roles in lock-step."""
+    """`calls` calls against the oracle; the outputs bit for bit those of the roles in lock-step."""
     disp, ys = O.simulate(cfg, ws, rds_cpu)
     rds = [rd.to(DEV) for rd in rds_cpu]
     world = LocalWorld(cfg, ws, payload=payload, schedule="pipelined", combine=combine)
