@@ -11,6 +11,7 @@
 
 #include "a2a.h"
 #include "a2a_kernels.cuh"
+#include "a2a_near.cuh"
 #include "a2a_pipe.cuh"
 #include "a2a_solo.cuh"
 
@@ -20,10 +21,7 @@ namespace {
 
 constexpr int kTraceBlocks = 2048;  // blocks the in-kernel trace buffer has room for
 constexpr size_t kMaxSmemBytes = 200 * 1024;  // routing bitmap budget per block (227 KB is the sm_100 limit)
-// Pipelined kernel of several ranks: two blocks per SM must fit (of 113 KB each).  A sender has 64 bytes more than a
-// router, the four descriptors by which its ring outgrew six stages; which configurations fit did not change by them.
-constexpr size_t kMaxPipeSmemBytes = 100 * 1024;
-constexpr size_t kMaxSenderSmemBytes = kMaxPipeSmemBytes + 64;
+constexpr size_t kMaxPipeSmemBytes = 100 * 1024;  // pipelined kernel of several ranks: two blocks per SM must fit (of 113 KB each)
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -90,6 +88,9 @@ struct a2a_ctx {
     bool peers_ready;
     bool routed, sent;
     bool recorded;          // this call's records are written: by role 0, or by the one launch of several ranks
+    bool near;              // its rows stayed where they are, for peers on this GPU: near_x, or FP8 the sources' own stages
+    const void* near_x[A2A_MAX_WORLD];  // input rows of every rank in this call
+    int near_T[A2A_MAX_WORLD];
     uint32_t epoch, barrier_epoch;
     int cur_tokens;
     int64_t launches;
@@ -212,7 +213,7 @@ int validate(const a2a_config& c) {
         const size_t router_room = c.world_size == 1 ? kMaxSmemBytes : kMaxPipeSmemBytes;
         const int senders = pipe_senders(c);
         if (c.world_size > 1 && senders < 2) return A2A_ERR_CONFIG;  // blocks 0 and 1 carry the watchers
-        if ((c.world_size > 1 && pipe_sender_smem(c.max_num_tokens, c.world_size, senders) > kMaxSenderSmemBytes) ||
+        if ((c.world_size > 1 && pipe_sender_smem(c.max_num_tokens, c.world_size, senders) > kMaxPipeSmemBytes) ||
             pipe_router_smem(c.max_num_tokens, c.num_experts / c.world_size) > router_room)
             return A2A_ERR_CONFIG;
     }
@@ -279,14 +280,17 @@ template <typename T, int P> struct ExpertSel {
 template <typename T, int P, bool PUSH> struct PipeForward {
     static PhaseFn get() { return {pipe_forward_kernel<T, P, PUSH, RankParams>, pipe_forward_kernel<T, P, PUSH, GroupParams>}; }
 };
+using NearFn = void (*)(NearParams);
 template <typename T, int P, bool PUSH> struct PipeRole {
-    template <int PP, bool PUSHP, int ROLE>
-    static PhaseFn pair() {
-        return {pipe_role_kernel<T, PP, PUSHP, ROLE, RankParams>, pipe_role_kernel<T, PP, PUSHP, ROLE, GroupParams>};
-    }
     // what is sent does not depend on the combine, nor the combine on how rows travelled
-    static PhaseFn get(int role) {
-        return role == 0 ? pair<P, true, 0>() : role == 1 ? pair<P, PUSH, 1>() : pair<A2A_PAYLOAD_DEDUP, PUSH, 2>();
+    static KernelFn get(int role) {
+        return role == 0 ? pipe_role_kernel<T, P, true, 0>
+                         : role == 1 ? pipe_role_kernel<T, P, PUSH, 1> : pipe_role_kernel<T, A2A_PAYLOAD_DEDUP, PUSH, 2>;
+    }
+};
+template <typename T, int P, bool PUSH> struct NearRole {
+    static NearFn get(int role) {
+        return role == 0 ? near_send_kernel<T, P> : role == 1 ? near_expert_kernel<T, P, PUSH> : near_combine_kernel<T, PUSH>;
     }
 };
 template <template <typename, int, bool> class F, typename T, typename... A>
@@ -329,48 +333,28 @@ int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool
     return A2A_OK;
 }
 
-// One phase of the `n` contexts in cs[] as one launch of `blocks` blocks for each; `adjust` may set what
-// this launch's blocks agree on (senders, routers).  A trace has a slot per block of the grid, so contexts
-// that are being traced are launched one by one.
-template <typename Adjust>
-int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int smem, cudaStream_t st, Adjust adjust) {
+// One phase of the `n` contexts in cs[] as one launch of `blocks` blocks for each.  A trace has a slot per block of
+// the grid, so contexts that are being traced are launched one by one.
+int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int smem, cudaStream_t st) {
     bool traced = false;
     for (int r = 0; r < n; ++r) traced |= cs[r]->p.trace != nullptr;
-    if (traced && n > 1) {
+    if (n == 1 || traced) {
         for (int r = 0; r < n; ++r) {
-            const int rc = launch_ranks(cs + r, 1, fn, blocks, smem, st, adjust);
+            const int rc = launch(cs[r], (const void*)fn.one, blocks, smem, st);
             if (rc != A2A_OK) return rc;
         }
         return A2A_OK;
-    }
-    if (n == 1) {
-        a2a_ctx* c = cs[0];
-        RankParams g = {call_params(c)};
-        adjust(g.p);
-        if (traced) {
-            if (blocks > kTraceBlocks) g.p.trace = nullptr;
-            else c->last_grid = blocks;
-        }
-        c->launches++;
-        void* args[] = {&g};
-        const cudaError_t e = cudaLaunchKernel((const void*)fn.one, dim3(blocks), dim3(kThreads), args, smem, st);
-        return e == cudaSuccess ? A2A_OK : -(int)e;
     }
     GroupParams g;
     for (int r = 0; r < n; ++r) {
         g.p[r] = call_params(cs[r]);
         g.p[r].local = 1;
-        adjust(g.p[r]);
         cs[r]->launches++;
     }
     g.n = n;
     void* args[] = {&g};
     const cudaError_t e = cudaLaunchKernel((const void*)fn.group, dim3(n * blocks), dim3(kThreads), args, smem, st);
     return e == cudaSuccess ? A2A_OK : -(int)e;
-}
-
-int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int smem, cudaStream_t st) {
-    return launch_ranks(cs, n, fn, blocks, smem, st, [](DevParams&) {});
 }
 
 // The forward of one rank.  A warp's item is one or two 16-byte vectors per lane of a token's row: two
@@ -434,7 +418,7 @@ int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
     c->cur_tokens = T;
     c->p.idx = idx;
     c->routed = true;
-    c->sent = c->recorded = false;
+    c->sent = c->recorded = c->near = false;
     return A2A_OK;
 }
 
@@ -442,23 +426,6 @@ int do_route(a2a_ctx* c, const int32_t* idx, int T, cudaStream_t st) {
     int r = begin_call(c, idx, T);
     if (r != A2A_OK) return r;
     return launch(c, (const void*)route_kernel, 1, c->smem_bytes, st);
-}
-
-// Sender and router blocks per rank where `n` ranks share one launch on one GPU: two blocks per SM run at
-// a time, and the launch should have no more.  One router per destination leaves the most senders: eight
-// ranks of 256 tokens of 7168, top-8 of 256 experts: 59 us with 29 senders and 8 routers each, 70 with 21
-// and 16; of 2048, top-6 of 64, skewed: 46 against 52.  No more senders than a rank has wire rows.
-void share_send_blocks(const a2a_ctx* c, int n, int tokens, int* senders, int* routers, int* smem) {
-    const int ws = c->cfg.world_size, K = c->cfg.experts_per_token, T = c->cfg.max_num_tokens;
-    const long long rows = (long long)tokens * (K < ws - 1 ? K : ws - 1);
-    int ns = 2 * c->num_sms / n - ws;
-    if (ns > rows) ns = (int)rows;
-    if (ns < 2) ns = 2;
-    if (pipe_sender_smem(T, ws, ns) > kMaxSenderSmemBytes) ns = c->p.senders;  // fewer blocks have longer token lists
-    const size_t a = pipe_sender_smem(T, ws, ns), b = pipe_router_smem(T, c->p.L);
-    *senders = ns;
-    *routers = 1;
-    *smem = (int)align_up(a > b ? a : b, 128);
 }
 
 // The phases below take the contexts of all ranks that share this launch: one, or a whole group on one GPU.
@@ -545,34 +512,87 @@ int begin_pipe_call(a2a_ctx* const* cs, int n, const a2a_call* calls) {
     return A2A_OK;
 }
 
-// Role 0 of the pipelined kernel.
+bool any_traced(a2a_ctx* const* cs, int n) {
+    for (int r = 0; r < n; ++r)
+        if (cs[r]->p.trace != nullptr) return true;
+    return false;
+}
+
+// A role of the pipelined schedule for one rank, in the form of a rank whose peers are on other GPUs.
+int launch_role(a2a_ctx* c, int role, int blocks, int smem, cudaStream_t st) {
+    return launch(c, (const void*)select_pipe<PipeRole>(c, role), blocks, smem, st);
+}
+
+// A role for ranks on one GPU, `blocks` in all; `ns` and `nr` are what role 0's blocks agree on.
+int launch_near(a2a_ctx* const* cs, int n, int role, int blocks, int smem, cudaStream_t st, int ns = 0, int nr = 0) {
+    NearParams g;
+    for (int r = 0; r < n; ++r) {
+        g.p[r] = call_params(cs[r]);
+        g.p[r].local = 1;
+        g.p[r].senders = ns;
+        g.p[r].routers = nr;
+        if (n > 1 || blocks > kTraceBlocks) g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
+        if (g.p[r].trace != nullptr) cs[r]->last_grid = blocks;
+        cs[r]->launches++;
+    }
+    memcpy(g.x, cs[0]->near_x, sizeof(g.x));
+    memcpy(g.T, cs[0]->near_T, sizeof(g.T));
+    g.n = n;
+    void* args[] = {&g};
+    const cudaError_t e = cudaLaunchKernel((const void*)select_pipe<NearRole>(cs[0], role), dim3(blocks), dim3(kThreads), args, smem, st);
+    return e == cudaSuccess ? A2A_OK : -(int)e;
+}
+
+// Role 0.  Contexts that are being traced are launched one by one, in the forms of a GPU per rank: a trace has a slot
+// per block of one rank's grid.
 int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st) {
     const int begun = begin_pipe_call(cs, n, calls);
     if (begun != A2A_OK) return begun;
     const a2a_ctx* c = cs[0];
     const int ws = c->cfg.world_size;
-    int ns = c->p.senders, nr = c->p.routers, smem = c->pipe_smem;
-    if (n > 1) share_send_blocks(c, n, most_tokens(cs, n), &ns, &nr, &smem);
-    const int rc = launch_ranks(cs, n, select_pipe<PipeRole>(c, 0), ns + ws * nr, smem, st, [=](DevParams& p) {
-        p.senders = ns;
-        p.routers = nr;
-    });
+    int rc = A2A_OK;
+    if (n == 1 || any_traced(cs, n)) {
+        for (int r = 0; r < n && rc == A2A_OK; ++r)
+            rc = launch_role(cs[r], 0, c->p.senders + ws * c->p.routers, c->pipe_smem, st);
+    } else {
+        for (int r = 0; r < n; ++r)
+            for (int s = 0; s < n; ++s) {
+                cs[r]->near_x[s] = calls[s].x;
+                cs[r]->near_T[s] = calls[s].num_tokens;
+            }
+        // Four routers per destination, as far as there are 32-token words for them: eight ranks of 256 tokens of 7168,
+        // top-8 of 256 experts 9.4 us (12 with one, 9.8 with two), of 2048, top-6 of 64 8.2 (10.1, 9.0); one or two
+        // tokens 5.3 whatever their number.  FP8: quantisers for two blocks per SM.
+        const long long pieces = (c->cfg.hidden_dim / 8 + 127) / 128, warps = kThreads / 32;
+        const int words = (c->cfg.max_num_tokens + 31) / 32, nr = words < 4 ? words : 4;
+        int ns = 0;
+        if (c->cfg.payload == A2A_PAYLOAD_FP8) ns = grid_for_ranks(c, n, (most_tokens(cs, n) * pieces + warps - 1) / warps, 2);
+        rc = launch_near(cs, n, 0, n * (ns + ws * nr), (int)pipe_router_smem(c->cfg.max_num_tokens, c->p.L), st, ns, nr);
+        if (rc == A2A_OK)
+            for (int r = 0; r < n; ++r) cs[r]->near = true;
+    }
     if (rc == A2A_OK)
         for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->recorded = true;
     return rc;
 }
 
 // Roles 1 and 2, of a call whose records exist: the one launch of a single rank writes none, and what role 1 would
-// find there belongs to an earlier call.  This rank's share of two blocks per SM (of four or eight, where a group
-// shares the launch: 134 us against 145 and 159 for role 1 of the workload named above) and, for peers elsewhere,
-// a watcher block.
+// find there belongs to an earlier call.  A call begun for ranks on one GPU goes on in that form, whoever asks for it.
 int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
-    for (int r = 0; r < n; ++r)
+    bool near = true;
+    for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent || !cs[r]->recorded) return A2A_ERR_STATE;
+        near = near && cs[r]->near;
+    }
     const a2a_ctx* c = cs[0];
-    const int blocks = c->num_sms * 2 / n;
-    const int smem = role == 1 && c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
-    return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), n > 1 ? blocks : 1 + blocks, smem, st);
+    const int blocks = c->num_sms * 2, push_smem = c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
+    if (n > 1 && !any_traced(cs, n) && near) return launch_near(cs, n, role, blocks, 0, st);
+    for (int r = 0; r < n; ++r) {
+        const int rc = cs[r]->near ? launch_near(cs + r, 1, role, blocks, 0, st)
+                                   : launch_role(cs[r], role, 1 + blocks, role == 1 ? push_smem : 0, st);
+        if (rc != A2A_OK) return rc;
+    }
+    return A2A_OK;
 }
 
 // The one launch of all ranks of a group on one GPU, two blocks per SM shared out among them.  Unlike in the
@@ -588,7 +608,7 @@ int do_group_forward(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStrea
     const int senders = room < c->p.senders ? room : c->p.senders;
     if (n < 2 || senders < 2) return A2A_ERR_CONFIG;
     const size_t a = pipe_sender_smem(c->cfg.max_num_tokens, n, senders), b = pipe_router_smem(c->cfg.max_num_tokens, c->p.L);
-    if (a > kMaxSenderSmemBytes) return A2A_ERR_CONFIG;
+    if (a > kMaxPipeSmemBytes) return A2A_ERR_CONFIG;
     const int begun = begin_pipe_call(cs, n, calls);
     if (begun != A2A_OK) return begun;
     GroupParams g;
@@ -782,7 +802,8 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
         const size_t a = cfg->world_size > 1 ? pipe_sender_smem(T, cfg->world_size, p.senders) : 0, b = pipe_router_smem(T, L);
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
         opt_in_both(select_pipe<PipeForward>(c));
-        opt_in_both(select_pipe<PipeRole>(c, 0));
+        opt_in((const void*)select_pipe<PipeRole>(c, 0));
+        opt_in((const void*)select_pipe<NearRole>(c, 0));
         if (e == cudaSuccess && cfg->world_size == 1) {
             c->forward_grid = c->num_sms;
             c->fused = true;  // the solo kernel: no block waits for another

@@ -47,7 +47,6 @@ constexpr int kFp8Block = 128;   // elements sharing one fp32 scale
 constexpr int kMaxChunks = 4;    // token chunks a call is pipelined in (whole 32-token bitmap words each)
 constexpr int kStageBytes = 16384;  // one stage of a sender block's shared-memory ring (a row piece)
 constexpr int kStages = 6;          // stages of that ring
-constexpr int kMaxStages = 16;      // smaller ones its bookkeeping has room for
 constexpr unsigned kNoEntry = 0xffffffffu;  // record entry of a (token, k) pair that has no row on the destination
 enum FlagKind : int { kFlagDispatch = 0, kFlagExpert = 1, kFlagBarrier = 2, kNumFlagKinds = 3 };
 enum Phase : int { kPhaseRoute = 1, kPhaseSend = 2, kPhaseRecv = 3, kPhaseExpert = 4, kPhaseCombine = 5, kPhaseBarrier = 6 };
@@ -436,18 +435,6 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 // At most N of this thread's most recent bulk groups may still be READING shared memory.
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-
-// ... or n of them, n >= 0 (a larger n than 5 waits as for 5).
-__device__ __forceinline__ void bulk_wait_read(int n) {
-    switch (n) {
-        case 0: bulk_wait_read<0>(); break;
-        case 1: bulk_wait_read<1>(); break;
-        case 2: bulk_wait_read<2>(); break;
-        case 3: bulk_wait_read<3>(); break;
-        case 4: bulk_wait_read<4>(); break;
-        default: bulk_wait_read<5>(); break;
-    }
-}
 
 // At most n (0..5; larger waits for 5) of this thread's most recent bulk groups may still be pending
 // at all: the older ones have written their destination.

@@ -32,8 +32,8 @@
 //            (token, k) row is pulled from the expert's slab over NVLink and reduced with
 //            the token's weights at home (the phase-by-phase combine, started per peer).
 //
-// A group of two ranks or more runs it; a single rank has a2a_solo.cuh.  Stepped as launches of their own,
-// the roles also serve one rank, which has no senders then.
+// A group of two ranks or more runs it; a single rank has a2a_solo.cuh, a group on one GPU steps through
+// a2a_near.cuh.  Stepped as launches of their own, the roles also serve one rank, which has no senders then.
 //
 // Nothing here waits on work of its own role on another GPU, senders and routers never wait
 // at all, and every wait is bounded; see a2a_device.cuh for the flag protocol.
@@ -46,13 +46,13 @@ namespace a2a {
 enum PipeTicket : int { kPipeTicketDest = 0, kPipeTicketSource = 1 };
 
 // ---- shared memory of a block, carved per role --------------------------------------------
-// sender: ring [kStages][kStageBytes] | mbarriers [kMaxStages] u64 | descriptors | list [ws][per] u16 | warp totals
+// sender: ring [kStages][kStageBytes] | mbarriers [kStages] u64 | descriptors | list [ws][per] u16 | warp totals
 // router: bits [Wc][L] | wpre [Wc][L] | cnt [L] | warp totals | wire row of each token of a round
 __host__ __device__ inline int pipe_list_per(int T_max, int senders) { return (T_max + senders - 1) / (senders > 0 ? senders : 1); }
 
 __host__ __device__ inline size_t pipe_sender_smem(int T_max, int ws, int senders) {
     size_t b = (size_t)kStages * kStageBytes + 128;                       // ring + barriers
-    b += (size_t)kMaxStages * 16;                                         // descriptors
+    b += (size_t)kStages * 2 * 16;                                        // descriptors (twice what the ring needs)
     b += ((size_t)ws * pipe_list_per(T_max, senders) * 2 + 15) / 16 * 16; // token lists
     b += 8 * A2A_MAX_WORLD * 4;                                           // warp totals
     return b;
@@ -63,7 +63,6 @@ __host__ __device__ inline size_t pipe_router_smem(int T_max, int L) {
     return (2 * W * L + L + 16 + 256) * 4;  // bitmap, prefix, counts, warp totals, wire row of a round's tokens
 }
 
-static_assert(kMaxStages * 8 <= 128, "mbarriers of the sender ring");
 struct SendDesc {
     unsigned long long dst;  // destination address of the piece
     unsigned bytes;
@@ -140,7 +139,7 @@ __device__ __forceinline__ SenderSmem carve_sender(const DevParams& p, uint8_t* 
     m.ring = smem;
     m.bars = reinterpret_cast<unsigned long long*>(smem + (size_t)kStages * kStageBytes);
     m.desc = reinterpret_cast<SendDesc*>(smem + (size_t)kStages * kStageBytes + 128);
-    m.list = reinterpret_cast<unsigned short*>(m.desc + kMaxStages);
+    m.list = reinterpret_cast<unsigned short*>(m.desc + 2 * kStages);
     m.wt = reinterpret_cast<int*>(smem + pipe_sender_smem(p.T_max, p.ws, ns) - 8 * A2A_MAX_WORLD * 4);
     return m;
 }
@@ -226,9 +225,6 @@ struct PendingDests {
 // that kind (they start only after the set-up barrier: a watcher may wait for a long time).  In the blocks
 // without watchers a lane of warp 1 per destination draws the block's ticket for it: a fence and an atomic of
 // a microsecond each that the copies would otherwise stand still for, once per destination.
-// LOCAL: every peer's memory is on this GPU (a group stepped here).  Eight ranks of 256 tokens in one launch:
-// rows of 7168 62 -> 46 us, of 2048 (top-6 of 64) 54 -> 28.
-template <bool LOCAL>
 __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, int sb, int ns, int watch_kind,
                                             int watch_phase) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -241,16 +237,12 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
     const int row_bytes = p.H * 2;
     // A bulk store to a peer holds its stage until the peer has acknowledged the write (measured: with two
     // store stages a block moves 28 KB per ~1.5 us round trip whatever the link could take), local loads
-    // complete in about a microsecond: two loads ahead, four stores in flight.  Stores to this GPU's own memory
-    // are through sooner than loads: two thirds of the ring load ahead, and it is cut into as many stages as
-    // there are rows it can hold.
-    const int stage_bytes = LOCAL ? min(kStageBytes, (row_bytes + 127) / 128 * 128) : kStageBytes;
-    const int stages = LOCAL ? min(kMaxStages, kStages * kStageBytes / stage_bytes) : kStages;
-    const int look = LOCAL ? 2 * stages / 3 : 2;
+    // complete in about a microsecond: two loads ahead, four stores in flight.
+    constexpr int look = 2;
     __shared__ int s_cnt[A2A_MAX_WORLD];
     __shared__ volatile int s_through[A2A_MAX_WORLD];  // per destination: 1 its last store is complete, -1 given up
     if (tid == 0) {  // before the lists: thread 0 can issue its first loads the moment they are built
-        for (int s = 0; s < stages; ++s) mbar_init(smem_addr(bars + s), 1);
+        for (int s = 0; s < kStages; ++s) mbar_init(smem_addr(bars + s), 1);
         mbar_fence_init();
     }
     if (tid < A2A_MAX_WORLD) s_through[tid] = 0;
@@ -290,7 +282,7 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
             stamp(p, kStampDestDone + (d - p.rank + p.ws) % p.ws);
         }
     };
-    const int pieces = (row_bytes + stage_bytes - 1) / stage_bytes;
+    const int pieces = (row_bytes + kStageBytes - 1) / kStageBytes;
     int total = 0;
     for (int i = 1; i < p.ws; ++i) {
         const int d = (p.rank + i) % p.ws;
@@ -314,16 +306,16 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
     uint32_t parity = 0;
     for (int q = 0; q < total + look && !failed; ++q) {
         if (q < total) {
-            if (q >= stages) bulk_wait_read(stages - look - 1);  // the store that used this stage has read it
+            if (q >= kStages) bulk_wait_read<kStages - look - 1>();  // the store that used this stage has read it
             const int n = sb + g_i * ns;  // wire row index at the destination
             const int t = list[g_d * per + g_i];
-            const int off = g_piece * stage_bytes;
-            const unsigned bytes = (unsigned)min(stage_bytes, row_bytes - off);
+            const int off = g_piece * kStageBytes;
+            const unsigned bytes = (unsigned)min(kStageBytes, row_bytes - off);
             const uint8_t* src = reinterpret_cast<const uint8_t*>(p.x) + (size_t)t * row_bytes + off;
             uint8_t* dst = p.peer[g_d] + p.off_stage + ((size_t)p.rank * p.T_max + n) * p.stage_row_bytes + off;
             const bool last_piece = (g_piece == pieces - 1);
             mbar_expect_tx(smem_addr(bars + st_in), bytes);
-            bulk_load(smem_addr(ring + (size_t)st_in * stage_bytes), src, bytes, smem_addr(bars + st_in));
+            bulk_load(smem_addr(ring + (size_t)st_in * kStageBytes), src, bytes, smem_addr(bars + st_in));
             desc[st_in].dst = reinterpret_cast<unsigned long long>(dst);
             desc[st_in].bytes = bytes;
             desc[st_in].dest_done = (last_piece && g_i == g_mine - 1) ? g_d : -1;
@@ -335,7 +327,7 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
             } else {
                 ++g_piece;
             }
-            st_in = st_in + 1 == stages ? 0 : st_in + 1;
+            st_in = st_in + 1 == kStages ? 0 : st_in + 1;
         }
         if (q >= look) {
             // the load is local and cannot be late by more than microseconds; bounded all the same
@@ -349,12 +341,12 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
                 }
             }
             if (failed) break;
-            bulk_store(reinterpret_cast<void*>(desc[st_out].dst), smem_addr(ring + (size_t)st_out * stage_bytes), desc[st_out].bytes);
+            bulk_store(reinterpret_cast<void*>(desc[st_out].dst), smem_addr(ring + (size_t)st_out * kStageBytes), desc[st_out].bytes);
             bulk_commit();
             if (q == look) stamp(p, kStampSetup + 2);
             if (desc[st_out].dest_done >= 0) pending.push(desc[st_out].dest_done, q - look);  // that group was the destination's last
             pending.drain(q - look + 1, kArrivalLag, arrive);
-            if (++st_out == stages) {
+            if (++st_out == kStages) {
                 st_out = 0;
                 parity ^= 1u;
             }
@@ -366,6 +358,26 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
     else
         for (int d = 0; d < p.ws; ++d)
             if (s_through[d] == 0) s_through[d] = -1;
+}
+
+// A vector of a row as e4m3 bytes, and the scale of its 128-value block, which 16 lanes share.  All 32 lanes call
+// it; a lane without a vector (`valid` false) only takes part in the shuffles.
+template <typename T>
+__device__ __forceinline__ uint2 quantise8(const uint4& q, bool valid, float& sc) {
+    float f[8];
+    float amax = 0.f;
+    if (valid) {
+        unpack8<T>(q, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
+    }
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    sc = amax > 0.f ? amax / 448.f : 1.f;
+    if (!valid) return make_uint2(0u, 0u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = f[i] / sc;
+    return pack8_e4m3(f);
 }
 
 // Sender block `sb` of `ns`, FP8 payload: the tokens t with t % ns == sb, one after the other.  The whole
@@ -425,20 +437,10 @@ __device__ __forceinline__ void sender_role_fp8(const DevParams& p, uint8_t* sme
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
                 const int v = v0 + u * kThreads + tid;  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
-                float f[8];
-                float amax = 0.f;
+                float sc;
+                const uint2 bytes = quantise8<T>(q[u], v < nvec, sc);
                 if (v < nvec) {
-                    unpack8<T>(q[u], f);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
-                }
-#pragma unroll
-                for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                if (v < nvec) {
-                    const float sc = amax > 0.f ? amax / 448.f : 1.f;
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) f[e] = f[e] / sc;
-                    reinterpret_cast<uint2*>(stage)[v] = pack8_e4m3(f);
+                    reinterpret_cast<uint2*>(stage)[v] = bytes;
                     if ((v & 15) == 0) reinterpret_cast<float*>(stage + p.H)[v >> 4] = sc;
                 }
             }
@@ -605,38 +607,27 @@ __device__ __forceinline__ void router_role(const DevParams& p, uint8_t* smem, i
     if (tid == 0) arrive_dest(p, d, expected);
 }
 
-// A vector of a row of this rank as it would look after crossing the wire in e4m3: the 16 lanes of a
-// 128-value block quantise it with its scale and dequantise it again.  All 32 lanes call it; a lane
-// without a vector (`valid` false) only takes part in the shuffles.
+// A vector of a row of this rank as it would look after crossing the wire in e4m3: quantised and dequantised again.
 template <typename T>
 __device__ __forceinline__ uint4 fp8_round_trip(const uint4& q, bool valid) {
-    float f[8];
-    float amax = 0.f;
-    if (valid) {
-        unpack8<T>(q, f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-    }
-#pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    float sc;
+    const uint2 bytes = quantise8<T>(q, valid, sc);
     if (!valid) return q;
-    const float sc = amax > 0.f ? amax / 448.f : 1.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = f[i] / sc;
-    unpack8_e4m3(pack8_e4m3(f), f);
+    float f[8];
+    unpack8_e4m3(bytes, f);
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] *= sc;
     return pack8<T>(f);
 }
 
-// One 128-vector (2 KB) chunk of a row as this rank received it, four 16-byte vectors of T per lane, in two
+// A chunk of a row as this rank received it, U 16-byte vectors of T per lane (four: 2 KB), in two
 // halves so that the bytes can be on their way while something else is worked on: the loads (an FP8 wire
 // row gives eight bytes and a scale per vector), and the conversion.
-template <typename T, int PAYLOAD>
-__device__ __forceinline__ void load_wire_chunk(const DevParams& p, bool own, const uint8_t* src, int v0, int nvec, uint4 (&q)[4]) {
+template <typename T, int PAYLOAD, int U>
+__device__ __forceinline__ void load_wire_chunk(const DevParams& p, bool own, const uint8_t* src, int v0, int nvec, uint4 (&q)[U]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
         const int v = v0 + u * 32 + lane;
         if (v >= nvec) continue;
         if (own) {
@@ -846,7 +837,7 @@ __device__ __forceinline__ void expert_role(const DevParams& p, uint8_t* smem, i
             if (m.t < 0 || m.t >= p.T) return;
             src = reinterpret_cast<const uint8_t*>(p.x) + (size_t)m.t * p.H * 2;
         }
-        load_wire_chunk<T, PAYLOAD>(p, own, src, v0, nvec, m.q);
+        load_wire_chunk<T, PAYLOAD, 4>(p, own, src, v0, nvec, m.q);
     };
     const int t_end = p.ws == 1 ? p.T : p.T_max;  // one rank's rows go into the caller's y, others into buffers of T_max
     auto process = [&](const Cursor& c, const Item& m) {
@@ -1088,7 +1079,7 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
             sender_role_fp8<T>(p, a2a_pipe_smem, b - nw, ns);
         } else {
             stamp_value(p, kStampRole, b < 2 ? (kRoleSender | kRoleWatcher) : kRoleSender);
-            sender_role<false>(p, a2a_pipe_smem, b, ns, b == 0 ? kFlagDispatch : (b == 1 ? kFlagExpert : -1),
+            sender_role(p, a2a_pipe_smem, b, ns, b == 0 ? kFlagDispatch : (b == 1 ? kFlagExpert : -1),
                         b == 0 ? kPhaseRecv : kPhaseCombine);
         }
         stamp(p, kStampSent);
@@ -1112,38 +1103,34 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
     }
 }
 
-// The same roles as separate launches: for callers that want the phases apart, and for stepping a group
-// that lives on ONE GPU -- a kernel that waits never shares the GPU with the kernel it waits for, so what
-// runs together is one role of every rank.  ROLE 0: senders + routers.  1: one watcher block + experts.
-// 2: one watcher block + combine.  A group's launch has no watcher blocks.
-template <typename T, int PAYLOAD, bool PUSH, int ROLE, class P>
-__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ P g) {
-    const DevParams& p = g.rank();
-    const int G = g.blocks(), b = g.block();
+// The same roles as separate launches: for callers that want the phases apart, and for stepping the ranks of a
+// group one by one.  ROLE 0: senders + routers.  1: one watcher block + experts.  2: one watcher block + combine.
+// A whole group on ONE GPU steps through the kernels of a2a_near.cuh.
+template <typename T, int PAYLOAD, bool PUSH, int ROLE>
+__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ DevParams p) {
+    const int G = (int)gridDim.x, b = (int)blockIdx.x;
     const int ns = p.senders;
     stamp(p, kStampStart);
     if (ROLE == 0) {
         if (b < ns) {
             if (PAYLOAD == A2A_PAYLOAD_FP8) sender_role_fp8<T>(p, a2a_pipe_smem, b, ns);
-            else sender_role<P::kGroup>(p, a2a_pipe_smem, b, ns, -1, 0);
+            else sender_role(p, a2a_pipe_smem, b, ns, -1, 0);
         } else {
             const int rb = b - ns, d = (p.rank + 1 + rb % p.ws) % p.ws;
             router_role(p, a2a_pipe_smem, d, rb / p.ws, p.routers, rb == 0, (uint32_t)(d == p.rank ? 0 : ns) + p.routers);
         }
         stamp(p, kStampSent);
     } else if (ROLE == 1) {
-        constexpr int first = P::kGroup ? 0 : 1;
-        if (b < first) watcher_role(p, kFlagDispatch, kPhaseRecv, (int)(threadIdx.x >> 5));
-        else expert_role<T, PAYLOAD, PUSH>(p, a2a_pipe_smem, b - first, G - first);
+        if (b == 0) watcher_role(p, kFlagDispatch, kPhaseRecv, (int)(threadIdx.x >> 5));
+        else expert_role<T, PAYLOAD, PUSH>(p, a2a_pipe_smem, b - 1, G - 1);
         stamp(p, kStampExpertDone);
     } else {
-        constexpr int first = P::kGroup ? 0 : 1;
-        if (b < first) {
+        if (b == 0) {
             watcher_role(p, kFlagExpert, kPhaseCombine, (int)(threadIdx.x >> 5));
         } else if (PUSH) {
-            combine_home_role<T>(p, b - first, G - first);
+            combine_home_role<T>(p, b - 1, G - 1);
         } else {
-            combine_phase<T>(p, b - first, G - first, /*own_watchers=*/false);
+            combine_phase<T>(p, b - 1, G - 1, /*own_watchers=*/false);
         }
         if (!PUSH) wait_all_experts(p, b);
     }

@@ -5,8 +5,8 @@ for, so the ranks here are stepped in lock-step: one launch runs a phase of ever
 rank, the sending phase before any waiting one, on one stream, and each wait finds its
 flag already set.  Routing, rows, records, flag values and epochs are those of a group
 with a GPU per rank; what depends on where a peer is, is not: flags are awaited at gpu
-scope without watchers, and 16-bit rows are sent with another ring depth.  The forms for distant peers
-run in ``forward_one_launch``, which puts every rank's blocks into one cooperative
+scope without watchers, and rows are read where they lie instead of being sent to a stage first
+(csrc/a2a_near.cuh).  The forms for distant peers run in ``forward_one_launch``, which puts every rank's blocks into one cooperative
 launch, and in the phases called context by context.
 Validation tool: parity tests and the smoke check use it to cover world sizes
 2, 4 and 8 on a single device.
@@ -84,7 +84,7 @@ class LocalWorld:
 
     def forward_pipelined(self, rank_datas: Sequence) -> List[torch.Tensor]:
         """The roles of the pipelined one-launch kernel as three launches, in lock-step:
-        every rank's senders and routers, then every rank's expert blocks, then every rank's combine."""
+        every rank's routers (and quantisers), then every rank's expert blocks, then every rank's combine."""
         calls, ys = self._whole_calls(rank_datas)
         self._step("pipe_send", calls)
         self._begun(rank_datas, ys)

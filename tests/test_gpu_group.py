@@ -166,3 +166,36 @@ def test_expert_op_on_every_bit_pattern(dtype, schedule, payload, combine):
         world.check()
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("payload,combine", [("dedup", "push"), ("dedup", "pull"), ("fp8", "push")])
+@pytest.mark.parametrize("together", [(True, False, False), (True, True, False), (True, False, True),
+                                      (False, True, True), (False, True, False), (False, False, True)])
+def test_a_call_goes_on_in_the_form_it_was_begun_in(payload, combine, together):
+    """Roles for the whole group and roles rank by rank, mixed inside one call: the same bits."""
+    ws, T, H = 3, 40, 2944
+    rds = [pkg.generate_input(12, 3, H, T, seed=5, rank=r, world_size=ws, ragged=True)[1].to(DEV) for r in range(ws)]
+    world = LocalWorld(pkg.MoEConfig(12, 3, H, T), ws, payload=payload, schedule="pipelined", combine=combine)
+    try:
+        want = [bits(y) for y in rank_by_rank(world, rds)]
+        tables = state(world)
+        for _ in range(2):
+            if together[0]:
+                calls, ys = world._whole_calls(rds)
+                world._step("pipe_send", calls)
+                world._begun(rds, ys)
+            else:
+                for c, rd in zip(world.ctxs, rds):
+                    c.pipe_step(0, rd.x, rd.indices, rd.weights)
+                ys = [c._y for c in world.ctxs]
+            for role, phase in ((1, "pipe_expert"), (2, "pipe_combine")):
+                if together[role]:
+                    world._step(phase)
+                else:
+                    for c in world.ctxs:
+                        c.pipe_step(role)
+            assert all(torch.equal(bits(y), w) for y, w in zip(ys, want))
+            assert all(torch.equal(a, b) for a, b in zip(state(world), tables))
+        world.check()
+    finally:
+        world.close()
