@@ -112,6 +112,22 @@ def load() -> C.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The compiled part of this layer (csrc/host.cpp), loaded once; raise if it is not there."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("_host.so is missing or does not load: build it with "
+                               "`python gpu-mode-kernels_b200/build.py`") from e
+        _host = module
+    return _host
+
+
 def current_stream() -> int:
     """The current CUDA stream of the current device, as the C ABI takes it."""
     return _raw_stream(torch.cuda.current_device())

@@ -58,11 +58,21 @@ class A2AContext:
                    _lib.SCHEDULE[schedule], _lib.COMBINE[combine], max(1, min(4, int(chunks))), int(senders))
         self._h = C.c_void_p()
         _lib.check(self.lib.a2a_create(C.byref(self._h), C.byref(c)))
+        self._native = _lib.host().Rank(self._h.value or 0, self.device_index, cfg.experts_per_token, cfg.hidden_dim,
+                                        cfg.in_dtype)
         self.num_local_experts = cfg.num_experts // world_size
         self.max_recv = cfg.max_num_tokens * world_size
-        self._num_tokens = 0
         if connect and world_size > 1:
             self._connect_over_group()
+
+    @property
+    def _num_tokens(self) -> int:
+        """Tokens of the current call."""
+        return self._native.tokens
+
+    @_num_tokens.setter
+    def _num_tokens(self, n: int) -> None:
+        self._native.tokens = n
 
     # ---- bootstrap ---------------------------------------------------------
     def export_handle(self) -> torch.Tensor:
@@ -176,6 +186,10 @@ class A2AContext:
     def forward(self, x: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor,
                 y: Optional[torch.Tensor] = None) -> torch.Tensor:
         """route + dispatch + expert placeholder + combine on the current stream (device tensors)."""
+        if y is None:
+            out = self._native.forward(x, indices, weights, False)
+            if out is not None:
+                return out if type(out) is not int else _lib.check(out)
         n = self._check_inputs(x, indices, weights, y, on_device=True)
         if y is None:
             y = torch.empty(n, self.cfg.hidden_dim, dtype=self.cfg.out_dtype, device=self.device)
@@ -306,6 +320,8 @@ class A2AContext:
 
     def close(self) -> None:
         if getattr(self, "_h", None) is not None and self._h.value:
+            if hasattr(self, "_native"):
+                self._native.close()
             self.lib.a2a_destroy(self._h)
             self._h = C.c_void_p()
 
@@ -386,6 +402,10 @@ def custom_kernel(data: input_t, payload: Optional[str] = None, schedule: Option
     on_device = x.is_cuda
     device_index = x.get_device() if on_device else torch.cuda.current_device()
     ctx = _context_for(cfg, rank, world_size, device_index, payload, schedule, combine)
+    if on_device:
+        y = ctx._native.forward(x, idx, w, True)  # None: an earlier error, or tensors that need a second look
+        if y is not None:
+            return y if type(y) is not int else _lib.check(y)
     if ctx.peek():
         ctx.raise_and_clear_if_failed()
     if idx.dtype is not torch.int32:

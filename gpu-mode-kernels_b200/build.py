@@ -1,14 +1,17 @@
-"""Build liba2a.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Build liba2a.so (the C-ABI CUDA library, nvcc for sm_100a) and _host.so (the compiled part of the Python
+layer, g++ against torch's headers) in-tree.
 
     python gpu-mode-kernels_b200/build.py [--verbose]
 
 nvcc cross-compiles without a GPU.  The library links the CUDA runtime
 statically, so it depends on nothing but the driver at run time.
 """
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG_DIR)
@@ -19,6 +22,8 @@ HEADERS = [os.path.join(CSRC, "a2a_kernels.cuh"), os.path.join(CSRC, "a2a_pipe.c
            os.path.join(CSRC, "a2a_solo.cuh"),
            os.path.join(CSRC, "a2a_device.cuh"),
            os.path.join(ROOT, "include", "a2a.h")]
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 
 
 def nvcc_path() -> str:
@@ -29,14 +34,35 @@ def nvcc_path() -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(HOST_PATH):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(f) > t for f in SOURCES + HEADERS + [os.path.abspath(__file__)])
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(HOST_PATH))
+    return any(os.path.getmtime(f) > t for f in SOURCES + HEADERS + [HOST_SOURCE, os.path.abspath(__file__)])
+
+
+def run(tool: str, cmd, verbose: bool) -> None:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{tool} failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    if verbose:
+        print(res.stdout + res.stderr)
+
+
+def build_host(verbose: bool = False) -> None:
+    torch_dir = importlib.util.find_spec("torch").submodule_search_locations[0]
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path())))
+    include = [os.path.join(ROOT, "include"), os.path.join(torch_dir, "include"),
+               os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
+               sysconfig.get_paths()["include"]]
+    run("g++", [
+        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", *("-I" + d for d in include), "-o", HOST_PATH,
+        HOST_SOURCE, "-L" + os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+        "-L" + PKG_DIR, "-la2a", "-Wl,-rpath,$ORIGIN",
+    ], verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources; return its path."""
+    """Compile both if one is missing or older than the sources; return the library's path."""
     if not force and not needs_build():
         return LIB_PATH
     cmd = [
@@ -47,11 +73,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     ]
     if verbose:
         cmd[1:1] = ["-Xptxas", "-v"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stdout + res.stderr)
+    run("nvcc", cmd, verbose)
+    build_host(verbose)
     return LIB_PATH
 
 

@@ -19,6 +19,10 @@ NUM_BINS = 256
 
 def histogram256(data: torch.Tensor, output: torch.Tensor) -> torch.Tensor:
     """Counts of the byte values of ``data`` into ``output`` on the current stream; returns ``output``."""
+    out = _lib.host().histogram(data, output)
+    if out is not None:
+        return out if type(out) is not int else _lib.check(out)
+    # something is wrong, or unusual: look again, one thing at a time
     if data.dtype is not torch.uint8 or not data.is_cuda or not data.is_contiguous() or data.dim() != 1:
         raise _lib.A2AError(_lib.A2A_ERR_CONFIG, f"data must be a contiguous 1-D uint8 CUDA tensor, got {data.dtype} {tuple(data.shape)} on {data.device}")
     device = data.get_device()

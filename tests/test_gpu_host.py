@@ -1,0 +1,143 @@
+"""The compiled part of the Python layer: the same answers and errors as the Python code behind it, for plain and
+for unusual inputs."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+import gpu_mode_kernels_b200 as pkg
+from gpu_mode_kernels_b200 import _lib, all2all, histogram
+from gpu_mode_kernels_b200.all2all import A2AContext, A2AError, custom_kernel, release_contexts
+from gpu_mode_kernels_b200.local_world import LocalWorld
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+class Sub(torch.Tensor):
+    pass
+
+
+def bits(t):
+    return t.contiguous().view(torch.int16)
+
+
+def data_of(rd, **changed):
+    return SimpleNamespace(**{**dict(num_tokens=rd.num_tokens, x=rd.x, indices=rd.indices, weights=rd.weights), **changed})
+
+
+FORMS = {
+    "plain": lambda rd: {},
+    "strided x": lambda rd: dict(x=rd.x.t().contiguous().t()),
+    "every second row": lambda rd: dict(x=rd.x.repeat_interleave(2, 0)[::2]),
+    "int64 indices": lambda rd: dict(indices=rd.indices.long()),
+    "strided indices": lambda rd: dict(indices=rd.indices.t().contiguous().t()),
+    "double weights": lambda rd: dict(weights=rd.weights.double()),
+    "a subclass": lambda rd: dict(x=rd.x.as_subclass(Sub)),
+    "needs a gradient": lambda rd: dict(x=rd.x.clone().requires_grad_()),
+    "no tokens": lambda rd: dict(x=rd.x[:0], indices=rd.indices[:0], weights=rd.weights[:0]),
+}
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_what_was_accepted_gives_the_same_bits(form):
+    cfg, rd, _, _ = pkg.generate_input(8, 3, 264, 9, seed=3, rank=0, world_size=1, device=DEV)
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push")
+    try:
+        d = data_of(rd, **FORMS[form](rd))
+        want = torch.empty(d.x.shape, dtype=rd.x.dtype, device=DEV)  # an output of its own: the code behind the compiled part
+        want = ctx.forward(d.x.contiguous(), d.indices.to(torch.int32).contiguous(), d.weights.float().contiguous(), want)
+        y = custom_kernel((cfg, d, 0, 1))
+        assert type(y) is torch.Tensor and y.dtype == want.dtype and not y.requires_grad and torch.equal(bits(y), bits(want))
+    finally:
+        ctx.close()
+        release_contexts(barrier=False)
+
+
+@pytest.mark.parametrize("wrong", [
+    dict(x=lambda t: t.half()), dict(x=lambda t: t[:, :-8]), dict(x=lambda t: t[0]), dict(x=lambda t: t.cpu(), indices=None),
+    dict(indices=lambda t: t[:-1].contiguous()), dict(weights=lambda t: t[:, :1].contiguous()), dict(weights=lambda t: t.cpu()),
+])
+def test_what_was_refused_is_refused(wrong):
+    cfg, rd, _, _ = pkg.generate_input(8, 3, 264, 9, seed=3, rank=0, world_size=1, device=DEV)
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push")
+    try:
+        d = data_of(rd, **{k: f(getattr(rd, k)) for k, f in wrong.items() if f})
+        for call in (lambda: ctx.forward(d.x, d.indices, d.weights), lambda: custom_kernel((cfg, d, 0, 1))):
+            with pytest.raises(A2AError) as refused:
+                call()
+            assert refused.value.code == _lib.A2A_ERR_CONFIG
+        with pytest.raises(A2AError) as refused:  # more tokens than the context was made for
+            ctx.forward(rd.x.repeat(2, 1), rd.indices.repeat(2, 1), rd.weights.repeat(2, 1))
+        assert refused.value.code == _lib.A2A_ERR_CONFIG
+        ctx.close()
+        with pytest.raises(A2AError):
+            ctx.forward(rd.x, rd.indices, rd.weights)
+    finally:
+        ctx.close()
+        release_contexts(barrier=False)
+
+
+@pytest.mark.parametrize("schedule,payload,combine", [("pipelined", "dedup", "push"), ("phased", "direct", "pull")])
+def test_a_group_with_unusual_data(schedule, payload, combine):
+    rds = [pkg.generate_input(8, 2, 264, 6, seed=4, rank=r, world_size=2)[1].to(DEV) for r in range(2)]
+    world = LocalWorld(pkg.MoEConfig(8, 2, 264, 6), 2, payload=payload, schedule=schedule, combine=combine)
+    forward = world.forward_pipelined if schedule == "pipelined" else world.forward_phases
+    try:
+        want = [bits(y) for y in forward(rds)]
+        kept = [[t.data_ptr() for t in c._keep] for c in world.ctxs]
+        odd = [data_of(rds[0], x=rds[0].x.as_subclass(Sub)), rds[1]]  # goes through the Python code
+        assert all(torch.equal(bits(y), w) for y, w in zip(forward(tuple(odd)), want))
+        assert [[t.data_ptr() for t in c._keep] for c in world.ctxs] == kept or schedule == "pipelined"
+        assert [c._num_tokens for c in world.ctxs] == [6, 6]
+        with pytest.raises(A2AError) as refused:
+            forward(rds[:1])
+        assert refused.value.code == _lib.A2A_ERR_STATE
+        before = [c.launches for c in world.ctxs]
+        with pytest.raises(A2AError):
+            big = data_of(rds[0], x=rds[0].x.repeat(2, 1), indices=rds[0].indices.repeat(2, 1), weights=rds[0].weights.repeat(2, 1))
+            forward([big, rds[1]])
+        assert [c.launches for c in world.ctxs] == before
+        assert all(torch.equal(bits(y), w) for y, w in zip(forward(rds), want))
+        world.check()
+    finally:
+        world.close()
+
+
+def test_histogram_of_unusual_tensors():
+    data = torch.randint(0, 256, (5000,), dtype=torch.uint8, device=DEV)
+    want = torch.bincount(data.cpu(), minlength=256)
+    out = torch.empty(256, dtype=torch.int64, device=DEV)
+    assert histogram.custom_kernel((data, out)) is out and torch.equal(out.cpu(), want)
+    assert torch.equal(histogram.custom_kernel((data.as_subclass(Sub), out.view(16, 16))).cpu().view(256), want)
+    for bad in ((data.cpu(), out), (data.int(), out), (data[::2], out), (data.view(50, 100), out), (data, out[:128]), (data, out.cpu())):
+        with pytest.raises(A2AError) as refused:
+            histogram.custom_kernel(bad)
+        assert refused.value.code == _lib.A2A_ERR_CONFIG
+
+
+def test_side_streams_and_threads():
+    """Calls go to the caller's current stream, from whichever thread."""
+    import threading
+
+    cfg, rd, _, _ = pkg.generate_input(8, 3, 264, 9, seed=3, rank=0, world_size=1, device=DEV)
+    ctxs = [A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push") for _ in range(3)]
+    got = [None] * 3
+    try:
+        want = bits(ctxs[0].forward(rd.x, rd.indices, rd.weights))
+        torch.cuda.synchronize()
+
+        def work(i):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(50):
+                    y = ctxs[i].forward(rd.x, rd.indices, rd.weights)
+                torch.cuda.current_stream().synchronize()
+                got[i] = y
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+        assert all(torch.equal(bits(y), want) for y in got)
+    finally:
+        [c.close() for c in ctxs]
+    assert all2all._CONTEXTS == {}
