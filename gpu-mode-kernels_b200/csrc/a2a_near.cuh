@@ -58,6 +58,7 @@ __device__ __forceinline__ void quantise_role(const DevParams& p, int b, int nb)
 // Blocks [0, senders) of a rank quantise (FP8 only), the others route: part rb / ws of destination rank + 1 + rb % ws.
 template <typename T, int PAYLOAD>
 __global__ void __launch_bounds__(kThreads) near_send_kernel(const __grid_constant__ NearParams g) {
+    begin_after_previous();
     const DevParams& p = g.p[blockIdx.x % g.n];
     const int b = (int)blockIdx.x / g.n, ns = p.senders;
     stamp(p, kStampStart);
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kThreads) near_send_kernel(const __grid_consta
 // ---------------------------------------------------------------------------
 template <typename T, int PAYLOAD, bool PUSH>
 __global__ void __launch_bounds__(kThreads, 2) near_expert_kernel(const __grid_constant__ NearParams g) {
+    begin_after_previous();
     constexpr int U = 4;
     __shared__ int s_pre[A2A_MAX_WORLD * A2A_MAX_WORLD + 1];
     __shared__ int s_whole;
@@ -443,6 +445,7 @@ __device__ __forceinline__ void near_combine_pull(const NearParams& g, int* s_pr
 
 template <typename T, bool PUSH>
 __global__ void __launch_bounds__(kThreads, 2) near_combine_kernel(const __grid_constant__ NearParams g) {
+    begin_after_previous();
     __shared__ int s_pre[A2A_MAX_WORLD + 1];
     stamp(g.p[0], kStampStart);
     if (PUSH) near_combine_push<T>(g, s_pre);

@@ -1108,6 +1108,7 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
 // A whole group on ONE GPU steps through the kernels of a2a_near.cuh.
 template <typename T, int PAYLOAD, bool PUSH, int ROLE>
 __global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ DevParams p) {
+    begin_after_previous();
     const int G = (int)gridDim.x, b = (int)blockIdx.x;
     const int ns = p.senders;
     stamp(p, kStampStart);

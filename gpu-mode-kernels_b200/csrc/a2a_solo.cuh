@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(kThreads) solo_kernel(const __grid_constant__ 
     __shared__ int s_idx[kSoloRound * A2A_MAX_TOPK];       // the round's indices,
     __shared__ float s_w[kSoloRound * A2A_MAX_TOPK];       // weights
     __shared__ int s_row[kSoloRound * A2A_MAX_TOPK];       // and slab rows (-1: dropped pair)
+    begin_after_previous();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int K = p.K, nvec = p.H >> 3;
     const int nchunk = (nvec + 32 * U - 1) / (32 * U);
