@@ -314,6 +314,15 @@ KernelFn solo_fn(const a2a_ctx* c) {
     return bf ? solo_kernel<__nv_bfloat16, A2A_PAYLOAD_DEDUP, U> : solo_kernel<__half, A2A_PAYLOAD_DEDUP, U>;
 }
 
+// its second launch where there are many tokens
+template <int U>
+KernelFn solo_rows_fn(const a2a_ctx* c) {
+    const bool bf = c->cfg.dtype == A2A_DTYPE_BF16;
+    if (c->cfg.payload == A2A_PAYLOAD_FP8)
+        return bf ? solo_rows_kernel<__nv_bfloat16, A2A_PAYLOAD_FP8, U> : solo_rows_kernel<__half, A2A_PAYLOAD_FP8, U>;
+    return bf ? solo_rows_kernel<__nv_bfloat16, A2A_PAYLOAD_DEDUP, U> : solo_rows_kernel<__half, A2A_PAYLOAD_DEDUP, U>;
+}
+
 PhaseFn combine_fn(const a2a_ctx* c) {
     if (c->cfg.dtype == A2A_DTYPE_BF16) return {combine_kernel<__nv_bfloat16, RankParams>, combine_kernel<__nv_bfloat16, GroupParams>};
     return {combine_kernel<__half, RankParams>, combine_kernel<__half, GroupParams>};
@@ -321,13 +330,14 @@ PhaseFn combine_fn(const a2a_ctx* c) {
 
 // A launch that, with `overlap`, may get ready while the one before it in the stream ends; its kernel begins with
 // begin_after_previous().
-cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** args, cudaStream_t st, bool overlap = true) {
+cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** args, cudaStream_t st, bool overlap = true,
+                                  int threads = kThreads) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
     cudaLaunchConfig_t launch{};
     launch.gridDim = dim3(grid);
-    launch.blockDim = dim3(kThreads);
+    launch.blockDim = dim3(threads);
     launch.dynamicSmemBytes = smem;
     launch.stream = st;
     launch.attrs = &attr;
@@ -342,13 +352,14 @@ cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** arg
 constexpr long long kOverlapBytes = 48LL << 20;
 bool overlaps(const a2a_ctx* c, long long tokens) { return tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 <= kOverlapBytes; }
 
-int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false, bool overlap = true) {
+int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false, bool overlap = true,
+           int threads = kThreads) {
     static_assert(sizeof(RankParams) == sizeof(DevParams), "a kernel of one rank takes either");
     DevParams p = call_params(c);
     if (p.trace != nullptr && grid > kTraceBlocks) p.trace = nullptr;
     if (p.trace != nullptr) c->last_grid = grid;
     void* args[] = {&p};
-    cudaError_t e = !cooperative ? launch_after_previous(fn, grid, smem, args, st, overlap)
+    cudaError_t e = !cooperative ? launch_after_previous(fn, grid, smem, args, st, overlap, threads)
         : c->plain_launch ? cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, smem, st)
                           : cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st);
     c->launches++;
@@ -388,9 +399,24 @@ int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int s
 // blocks starts after the first (headline 13.2 us).
 // Rows in host memory: half an SM's worth of warps fills the link, and more only get in each other's way
 // (3.7 MB read and as much written by 74 / 148 / 296 blocks: 100 / 107 / 118 us).
+// Many tokens in rows that outweigh a second launch: slots first, then rows in blocks of one item a warp, one vector a
+// lane, or two where fewer than six stores follow each load.  Back to back, against the one launch: 2048 tokens of
+// 7168, top-8 62.2 -> 57.1 us; of 2048, top-6 19.8 -> 17.0, top-2 12.4 -> 11.6; of 6144, top-2 23.3 both; 1300 tokens of
+// 4096, top-8 24.6 / 24.9, of 2880, top-4 13.4 / 12.9; 1024 of 2880 10.9 / 11.5, 400 of 2048, top-2 5.9 / 7.4.
+constexpr int kSoloManyTokens = 1280;
+constexpr long long kSoloManyBytes = 8LL << 20;
 int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = host_rows ? c->num_sms / 2 : 2LL * c->num_sms;
     const long long two = c->cur_tokens * ((nvec + 63) / 64), one = c->cur_tokens * ((nvec + 31) / 32);
+    const int K = c->cfg.experts_per_token;
+    if (!host_rows && c->p.trace == nullptr && c->cur_tokens >= kSoloManyTokens &&
+        (long long)c->cur_tokens * K * c->cfg.hidden_dim * 2 >= kSoloManyBytes) {
+        const bool narrow = K >= 6;
+        const int rc = launch(c, (const void*)solo_route_kernel, (c->cur_tokens + kRouteTokens - 1) / kRouteTokens, 0, st,
+                              /*cooperative=*/false, /*overlap=*/true, kRouteThreads);
+        return rc != A2A_OK ? rc : launch(c, (const void*)(narrow ? solo_rows_fn<1>(c) : solo_rows_fn<2>(c)),
+                                          (int)(((narrow ? one : two) + warps - 1) / warps), 0, st);
+    }
     const bool wide = two >= cap * warps;
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
     if (blocks > cap) blocks = cap;

@@ -141,3 +141,45 @@ def test_side_streams_and_threads():
     finally:
         [c.close() for c in ctxs]
     assert all2all._CONTEXTS == {}
+
+
+@pytest.mark.parametrize("what", ["one rank", "many tokens", "group", "phases", "histogram"])
+def test_calls_under_graph_capture(what):
+    """Captured launches, those that overlap included, replayed on other inputs."""
+    ws, E, K, H, T = 2, 8, 2, 2048, 1300 if what == "many tokens" else 40
+    sets = [[pkg.generate_input(E, K, H, T, seed=s, rank=r, world_size=ws)[1].to(DEV) for r in range(ws)] for s in (1, 2)]
+    cfg = pkg.MoEConfig(E, K, H, T)
+    data, counts = torch.zeros(300000, dtype=torch.uint8, device=DEV), torch.empty(256, dtype=torch.int64, device=DEV)
+    held = [data_of(rd, x=rd.x.clone(), indices=rd.indices.clone(), weights=rd.weights.clone()) for rd in sets[0]]
+    world = None
+    if what in ("group", "phases"):
+        world = LocalWorld(cfg, ws, payload="dedup" if what == "group" else "direct",
+                           schedule="pipelined" if what == "group" else "phased", combine="push" if what == "group" else "pull")
+    try:
+        def call():
+            if what == "histogram":
+                return [histogram.custom_kernel((data, counts))]
+            if world is None:
+                return [custom_kernel((cfg, held[0], 0, 1))]
+            return world.forward_pipelined(held) if what == "group" else world.forward_phases(held)
+
+        call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = [o for _ in range(3) for o in call()]
+        for rds in sets[::-1]:
+            for h, rd in zip(held, rds):
+                h.x.copy_(rd.x), h.indices.copy_(rd.indices), h.weights.copy_(rd.weights)
+            data.random_(0, 256)
+            graph.replay()
+            torch.cuda.synchronize()
+            got = [o.clone() for o in outs]
+            want = [o.clone() for o in call()] * 3
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+        if what == "histogram":
+            assert torch.equal(counts.cpu(), torch.bincount(data.cpu(), minlength=256))
+    finally:
+        if world is not None:
+            world.close()
+        release_contexts(barrier=False)

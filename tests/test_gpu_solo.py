@@ -76,6 +76,41 @@ def test_forward_against_the_checker_and_the_stepped_roles(E, K, H, T, n, dtype,
         world.close()
 
 
+@pytest.mark.parametrize("E,K,H,T,n,dtype,payload", [
+    (8, 2, 2048, 1280, 1280, torch.bfloat16, "dedup"),  # the fewest tokens, whole blocks of 64
+    (64, 6, 520, 2100, 2049, torch.float16, "dedup"),   # one token in the last routing block, rows that end inside a warp
+    (40, 32, 264, 1300, 1283, torch.bfloat16, "dedup"), # the most experts a token
+    (256, 8, 640, 1344, 1343, torch.bfloat16, "fp8"),
+    (8, 2, 2048, 1280, 1279, torch.bfloat16, "dedup"),  # one token fewer: one launch
+])
+def test_many_tokens_match_the_stepped_roles(E, K, H, T, n, dtype, payload):
+    """Routing and rows as two launches; repeated and out-of-range experts on both sides of a 32- and a 64-token edge."""
+    cfg, rd, _, _ = pkg.generate_input(E, K, H, T, seed=13, rank=0, world_size=1, dtype=dtype, weights="rand")
+    rd.num_tokens = n
+    rd.x, rd.indices, rd.weights = rd.x[:n], rd.indices[:n], rd.weights[:n]
+    for t in (31, 32, 63, 64, 127, n - 1):
+        rd.indices[t, K - 1] = rd.indices[t, 0]
+    rd.indices[95], rd.indices[96, 0] = -1, E
+    ctx = A2AContext(cfg, 0, 1, device=0, payload=payload, schedule="pipelined", combine="push", timeout_ms=500)
+    world = LocalWorld(cfg, 1, payload=payload, schedule="pipelined", combine="push")
+    try:
+        d = rd.to(DEV)
+        before = ctx.launches
+        y = ctx.forward(d.x, d.indices, d.weights)
+        assert ctx.launches == before + (2 if n >= 1280 else 1)
+        ref = world.forward_pipelined([d])[0]
+        got, want = ctx.route_tables() + ctx.export_dispatch(), world.ctxs[0].route_tables() + world.ctxs[0].export_dispatch()
+        again = torch.empty_like(y)  # a combine called on its own finds the flags up
+        _lib.check(ctx.lib.a2a_combine(ctx._h, d.weights.data_ptr(), again.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert ctx.peek() == _lib.A2A_ERR_ROUTING
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        assert torch.equal(bits(ref), bits(y)) and torch.equal(bits(again), bits(y)) and not y[95].any()
+    finally:
+        ctx.close()
+        world.close()
+
+
 def test_dropped_pairs_match_the_stepped_roles_and_phases_can_follow():
     """Indices out of range and repeated, the repeats also across the eight indices the kernel loads
     together and in tokens before the reading block's own; then a combine called on its own, which
