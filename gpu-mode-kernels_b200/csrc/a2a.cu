@@ -502,12 +502,13 @@ int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st) {
     }
     for (int r = 0; r < n; ++r) cs[r]->p.x = x[r];
     const a2a_ctx* c = cs[0];
-    // DIRECT: a warp per pair and 2 KB, no more blocks than four per SM, each of which builds the routing tables;
-    // staged payloads: a block per (token, destination)
+    // a warp per 2 KB of a pair's row (DIRECT) or 512 bytes of a token's, no more blocks than four per SM, each of which
+    // builds the routing tables (eight ranks, 200 tokens of 7168 by phases, direct: 145 us a call, 148 with three and 152
+    // with six; dedup 197, 200, 194; four ranks, 117 tokens of 4096, direct: 35.7, 37.2, 39.4)
     const bool direct = c->cfg.payload == A2A_PAYLOAD_DIRECT;
-    const long long T = most_tokens(cs, n), pieces = (c->cfg.hidden_dim / 8 + 127) / 128, warps = kThreads / 32;
-    const long long items = direct ? (T * c->cfg.experts_per_token * pieces + warps - 1) / warps : T * c->cfg.world_size;
-    const int rc = launch_ranks(cs, n, select_tp<SendSel>(c), grid_for_ranks(c, n, items, direct ? 4 : 8), c->smem_bytes, st);
+    const long long T = most_tokens(cs, n), nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32;
+    const long long items = direct ? T * c->cfg.experts_per_token * ((nvec + 127) / 128) : T * ((nvec + 31) / 32);
+    const int rc = launch_ranks(cs, n, select_tp<SendSel>(c), grid_for_ranks(c, n, (items + warps - 1) / warps, 4), c->smem_bytes, st);
     if (rc == A2A_OK)
         for (int r = 0; r < n; ++r) cs[r]->sent = true;
     return rc;
@@ -527,6 +528,36 @@ int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, boo
     return launch_ranks(cs, n, select_tp<ExpertSel>(cs[0], wait, fanout, scale, publish), grid, cs[0]->smem_bytes, st);
 }
 
+bool any_traced(a2a_ctx* const* cs, int n) {
+    for (int r = 0; r < n; ++r)
+        if (cs[r]->p.trace != nullptr) return true;
+    return false;
+}
+
+// A kernel for ranks on one GPU, `blocks` in all; `ns` and `nr` are what role 0's blocks agree on.
+int launch_near(a2a_ctx* const* cs, int n, NearFn fn, int blocks, int smem, cudaStream_t st, int ns = 0, int nr = 0) {
+    NearParams g;
+    for (int r = 0; r < n; ++r) {
+        g.p[r] = call_params(cs[r]);
+        g.p[r].local = 1;
+        g.p[r].senders = ns;
+        g.p[r].routers = nr;
+        if (n > 1 || blocks > kTraceBlocks) g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
+        if (g.p[r].trace != nullptr) cs[r]->last_grid = blocks;
+        cs[r]->launches++;
+    }
+    long long tokens = 0;
+    for (int r = 0; r < n; ++r) tokens += cs[r]->cur_tokens;
+    memcpy(g.x, cs[0]->near_x, sizeof(g.x));
+    memcpy(g.T, cs[0]->near_T, sizeof(g.T));
+    g.n = n;
+    void* args[] = {&g};
+    const cudaError_t e = launch_after_previous((const void*)fn, blocks, smem, args, st, overlaps(cs[0], tokens));
+    return e == cudaSuccess ? A2A_OK : -(int)e;
+}
+
+constexpr long long kNearCombineBytes = 16LL << 20;
+
 int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st) {
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent) return A2A_ERR_STATE;
@@ -538,6 +569,14 @@ int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y,
         cs[r]->p.y = y[r];
     }
     const a2a_ctx* c = cs[0];
+    // Many rows of a group: the combine of a2a_near.cuh, which looks up pairs two items ahead and shares the tokens of all
+    // ranks out among all blocks.  Calls by phases: 183 MB of expert rows 161 -> 145 us, 58 MB 90.2 -> 87.4, 31 MB 36.2 -> 35.7;
+    // 7 MB 27.1 -> 28.1, 1 MB 20.0 -> 21.7: more to set up.
+    long long tokens = 0;
+    for (int r = 0; r < n; ++r) tokens += cs[r]->cur_tokens;
+    if (n > 1 && c->p.chunks == 1 && !any_traced(cs, n) && tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 >= kNearCombineBytes)
+        return launch_near(cs, n, c->cfg.dtype == A2A_DTYPE_BF16 ? near_combine_kernel<__nv_bfloat16, false> : near_combine_kernel<__half, false>,
+                           2 * c->num_sms, 0, st);
     const int nseg = (c->cfg.hidden_dim / 8 + 63) / 64;  // a warp per (token, 1 KB segment)
     const long long warps = (long long)most_tokens(cs, n) * nseg;
     return launch_ranks(cs, n, combine_fn(c), grid_for_ranks(c, n, (warps + kThreads / 32 - 1) / (kThreads / 32), 8), 0, st);
@@ -562,37 +601,9 @@ int begin_pipe_call(a2a_ctx* const* cs, int n, const a2a_call* calls) {
     return A2A_OK;
 }
 
-bool any_traced(a2a_ctx* const* cs, int n) {
-    for (int r = 0; r < n; ++r)
-        if (cs[r]->p.trace != nullptr) return true;
-    return false;
-}
-
 // A role of the pipelined schedule for one rank, in the form of a rank whose peers are on other GPUs.
 int launch_role(a2a_ctx* c, int role, int blocks, int smem, cudaStream_t st) {
     return launch(c, (const void*)select_pipe<PipeRole>(c, role), blocks, smem, st);
-}
-
-// A role for ranks on one GPU, `blocks` in all; `ns` and `nr` are what role 0's blocks agree on.
-int launch_near(a2a_ctx* const* cs, int n, int role, int blocks, int smem, cudaStream_t st, int ns = 0, int nr = 0) {
-    NearParams g;
-    for (int r = 0; r < n; ++r) {
-        g.p[r] = call_params(cs[r]);
-        g.p[r].local = 1;
-        g.p[r].senders = ns;
-        g.p[r].routers = nr;
-        if (n > 1 || blocks > kTraceBlocks) g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
-        if (g.p[r].trace != nullptr) cs[r]->last_grid = blocks;
-        cs[r]->launches++;
-    }
-    long long tokens = 0;
-    for (int s = 0; s < cs[0]->cfg.world_size; ++s) tokens += cs[0]->near_T[s];
-    memcpy(g.x, cs[0]->near_x, sizeof(g.x));
-    memcpy(g.T, cs[0]->near_T, sizeof(g.T));
-    g.n = n;
-    void* args[] = {&g};
-    const cudaError_t e = launch_after_previous((const void*)select_pipe<NearRole>(cs[0], role), blocks, smem, args, st, overlaps(cs[0], tokens));
-    return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
 // Role 0.  Contexts that are being traced are launched one by one, in the forms of a GPU per rank: a trace has a slot
@@ -619,7 +630,7 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
         const int words = (c->cfg.max_num_tokens + 31) / 32, nr = words < 4 ? words : 4;
         int ns = 0;
         if (c->cfg.payload == A2A_PAYLOAD_FP8) ns = grid_for_ranks(c, n, (most_tokens(cs, n) * pieces + warps - 1) / warps, 2);
-        rc = launch_near(cs, n, 0, n * (ns + ws * nr), (int)pipe_router_smem(c->cfg.max_num_tokens, c->p.L), st, ns, nr);
+        rc = launch_near(cs, n, select_pipe<NearRole>(c, 0), n * (ns + ws * nr), (int)pipe_router_smem(c->cfg.max_num_tokens, c->p.L), st, ns, nr);
         if (rc == A2A_OK)
             for (int r = 0; r < n; ++r) cs[r]->near = true;
     }
@@ -638,9 +649,9 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
     }
     const a2a_ctx* c = cs[0];
     const int blocks = c->num_sms * 2, push_smem = c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
-    if (n > 1 && !any_traced(cs, n) && near) return launch_near(cs, n, role, blocks, 0, st);
+    if (n > 1 && !any_traced(cs, n) && near) return launch_near(cs, n, select_pipe<NearRole>(c, role), blocks, 0, st);
     for (int r = 0; r < n; ++r) {
-        const int rc = cs[r]->near ? launch_near(cs + r, 1, role, blocks, 0, st)
+        const int rc = cs[r]->near ? launch_near(cs + r, 1, select_pipe<NearRole>(c, role), blocks, 0, st)
                                    : launch_role(cs[r], role, 1 + blocks, role == 1 ? push_smem : 0, st);
         if (rc != A2A_OK) return rc;
     }

@@ -80,13 +80,19 @@ __device__ __forceinline__ void route_build(const DevParams& p, const BlockSmem&
         const int* row = p.idx + (size_t)t * K;
         const unsigned bit = 1u << (t & 31);
         unsigned* word = s.bits + (t >> 5) * E;
-        for (int k = 0; k < K; ++k) {
-            const int e = __ldg(row + k);
-            if (e < 0 || e >= E) {
-                record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
-            } else if (atomicOr(word + e, bit) & bit) {  // only this thread sets this bit: a repeat inside the token
-                record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
+        for (int k0 = 0; k0 < K; k0 += 8) {
+            int e8[8];
+            unsigned before[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) e8[u] = (k0 + u < K) ? __ldg(row + k0 + u) : 0;  // loaded together
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                before[u] = 0u;
+                if (k0 + u < K) before[u] = e8[u] >= 0 && e8[u] < E ? atomicOr(word + e8[u], bit) : bit;
             }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)  // out of range, or set already: only this thread sets this bit, so a repeat inside the token
+                if (before[u] & bit) record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e8[u]);
         }
     }
     __syncthreads();
@@ -145,20 +151,58 @@ __device__ __forceinline__ void publish_dispatch(const DevParams& p, const Block
     publish_flags(p, kFlagDispatch, flag_value(p, c));
 }
 
-// Copy one row of nvec 16-byte vectors with all 256 threads, up to four loads in flight each.
-__device__ __forceinline__ void copy_row(const uint4* __restrict__ src, uint4* __restrict__ dst, int nvec) {
-    const int tid = threadIdx.x;
-    for (int v0 = 0; v0 < nvec; v0 += kThreads * 4) {
-        uint4 r[4];
+// Staged payloads: a warp per token and U vectors per lane of its row, read and quantised once and stored to every rank
+// that wants it.
+template <typename T, int PAYLOAD, int U>
+__device__ __forceinline__ void send_staged(const DevParams& p, const BlockSmem& s, int ta, int tb, int b, int G) {
+    const int tid = threadIdx.x, lane = tid & 31, K = p.K, nvec = p.H >> 3, npiece = (nvec + 32 * U - 1) / (32 * U);
+    for (int it = b * (kThreads / 32) + (tid >> 5); it < (tb - ta) * npiece; it += G * (kThreads / 32)) {
+        const int t = ta + it / npiece, v0 = it % npiece * (32 * U);
+        const uint4* src = reinterpret_cast<const uint4*>(p.x) + (size_t)t * nvec;
+        uint4 q[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = v0 + u * kThreads + tid;
-            if (v < nvec) r[u] = ld_input(src + v);
+        for (int u = 0; u < U; ++u) {
+            const int v = v0 + u * 32 + lane;
+            if (v < nvec) q[u] = ld_input(src + v);
         }
+        // lane k: pair k's slab row gets its (token, k) word, through which the receiver finds the wire row
+        unsigned want = 0u;
+        if (lane < K) {
+            const int e = s.idx[t * K + lane];
+            const int j = pair_slot(p, s, t, lane, e);
+            if (v0 == 0) p.slot[(size_t)t * K + lane] = j;
+            if (j >= 0) {
+                const int d = e / p.L;
+                want = 1u << d;
+                if (v0 == 0)
+                    reinterpret_cast<int*>(p.peer[d] + p.off_meta)[((size_t)(e - d * p.L) * p.ws + p.rank) * p.T_max + j] = (t << 8) | lane;
+            }
+        }
+        want = __reduce_or_sync(0xffffffffu, want);
+        float sc[U];
+        if (PAYLOAD == A2A_PAYLOAD_FP8) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int v = v0 + u * kThreads + tid;
-            if (v < nvec) st_stream(dst + v, r[u]);
+            for (int u = 0; u < U; ++u) {
+                // nvec is a multiple of 16 (H % 128 == 0): the 16 lanes of a scale block are all in or all out
+                const uint2 bytes = quantise8<T>(q[u], v0 + u * 32 + lane < nvec, sc[u]);
+                q[u].x = bytes.x;
+                q[u].y = bytes.y;
+            }
+        }
+        for (; want != 0u; want &= want - 1u) {
+            const int d = __ffs(want) - 1;
+            uint8_t* wire = p.peer[d] + p.off_stage + ((size_t)p.rank * p.T_max + t) * p.stage_row_bytes;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int v = v0 + u * 32 + lane;
+                if (v >= nvec) continue;
+                if (PAYLOAD == A2A_PAYLOAD_FP8) {
+                    st_stream(reinterpret_cast<uint2*>(wire) + v, make_uint2(q[u].x, q[u].y));
+                    if ((v & 15) == 0) reinterpret_cast<float*>(wire + p.H)[v >> 4] = sc[u];
+                } else {
+                    st_stream(reinterpret_cast<uint4*>(wire) + v, q[u]);
+                }
+            }
         }
     }
 }
@@ -167,10 +211,10 @@ __device__ __forceinline__ void copy_row(const uint4* __restrict__ src, uint4* _
 // Dispatch, sending half.  Never waits.
 // DIRECT: one warp per (token, k) pair and 2 KB of the row at a time; the row goes straight into slab
 //   (expert, this rank) on the expert's rank (NVLink for a peer, HBM for ourselves).
-// DEDUP / FP8: one block per (token, destination rank); the row crosses the wire
-//   once per destination into stage[src][t] (FP8: quantised on the fly, one fp32
-//   scale per 128 values); every slab row that wants it gets its (token, k) word,
-//   through which the receiver finds the wire row when it fans out.
+// DEDUP / FP8: one warp per token and a piece of its row, which crosses the wire once per
+//   destination rank into stage[src][t] (FP8: quantised on the fly, one fp32 scale per
+//   128 values); every slab row that wants it gets its (token, k) word, through which the
+//   receiver finds the wire row when it fans out.
 // Work is done chunk of tokens by chunk; the block that finishes a chunk last publishes it.
 // ---------------------------------------------------------------------------
 template <typename T, int PAYLOAD>
@@ -207,53 +251,9 @@ __device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& 
             if (lane == 0 && v0 == 0) reinterpret_cast<int*>(p.peer[d] + p.off_meta)[row] = (t << 8) | k;
         }
     } else {
-        for (int it = ta * p.ws + b; it < tb * p.ws; it += G) {
-            const int t = it / p.ws, d = it - t * p.ws;
-            // which of the token's experts live on d: each of them gets its slab row's (token, k)
-            // word there; the row itself crosses the wire once
-            int hit = 0;
-            if (tid < K) {
-                const int e = s.idx[t * K + tid];
-                const bool in_range = (e >= 0 && e < p.E);
-                const int home = in_range ? e / p.L : 0;  // an out-of-range pair is booked (as dropped) by item d = 0
-                if (home == d) {
-                    const int j = pair_slot(p, s, t, tid, e);
-                    p.slot[(size_t)t * K + tid] = j;
-                    if (j >= 0) {
-                        const size_t row = ((size_t)(e - d * p.L) * p.ws + p.rank) * p.T_max + j;
-                        reinterpret_cast<int*>(p.peer[d] + p.off_meta)[row] = (t << 8) | tid;
-                        hit = 1;
-                    }
-                }
-            }
-            if (!__syncthreads_or(hit)) continue;  // nothing of this token lives on d
-            uint8_t* wire = p.peer[d] + p.off_stage + ((size_t)p.rank * p.T_max + t) * p.stage_row_bytes;
-            const uint4* src = reinterpret_cast<const uint4*>(p.x) + (size_t)t * nvec;
-            if (PAYLOAD == A2A_PAYLOAD_DEDUP) {
-                copy_row(src, reinterpret_cast<uint4*>(wire), nvec);
-            } else {
-                // nvec is a multiple of 16 (H % 128 == 0): the 16 lanes of a scale block are all in or all out
-                for (int v0 = 0; v0 < nvec; v0 += kThreads) {
-                    const int v = v0 + tid;
-                    float f[8];
-                    float amax = 0.f;
-                    if (v < nvec) {
-                        unpack8<T>(ld_input(src + v), f);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-                    }
-#pragma unroll
-                    for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                    if (v < nvec) {
-                        const float scale = amax > 0.f ? amax / 448.f : 1.f;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) f[i] = f[i] / scale;
-                        st_stream(reinterpret_cast<uint2*>(wire) + v, pack8_e4m3(f));
-                        if ((v & 15) == 0) reinterpret_cast<float*>(wire + p.H)[v >> 4] = scale;
-                    }
-                }
-            }
-        }
+        // 2 KB a warp, or 512 bytes where that still leaves every warp no more than one item
+        if ((tb - ta) * ((nvec + 31) >> 5) <= G * (kThreads / 32)) send_staged<T, PAYLOAD, 1>(p, s, ta, tb, b, G);
+        else send_staged<T, PAYLOAD, 4>(p, s, ta, tb, b, G);
     }
     if (grid_arrive_last(p.tickets + kTicketSend * kMaxChunks + c, G)) publish_dispatch(p, s, c);
 }

@@ -360,26 +360,6 @@ __device__ __forceinline__ void sender_role(const DevParams& p, uint8_t* smem, i
             if (s_through[d] == 0) s_through[d] = -1;
 }
 
-// A vector of a row as e4m3 bytes, and the scale of its 128-value block, which 16 lanes share.  All 32 lanes call
-// it; a lane without a vector (`valid` false) only takes part in the shuffles.
-template <typename T>
-__device__ __forceinline__ uint2 quantise8(const uint4& q, bool valid, float& sc) {
-    float f[8];
-    float amax = 0.f;
-    if (valid) {
-        unpack8<T>(q, f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-    }
-#pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    sc = amax > 0.f ? amax / 448.f : 1.f;
-    if (!valid) return make_uint2(0u, 0u);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = f[i] / sc;
-    return pack8_e4m3(f);
-}
-
 // Sender block `sb` of `ns`, FP8 payload: the tokens t with t % ns == sb, one after the other.  The whole
 // block quantises a token's row ONCE (the arithmetic -- an IEEE division per value -- is the cost here: a row
 // goes to four or five ranks of eight, and quantising it for each took 131 us where this takes 44, eight ranks of 256 tokens of 7168 in one launch):
