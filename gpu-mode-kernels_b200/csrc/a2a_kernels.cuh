@@ -72,7 +72,14 @@ __device__ __forceinline__ void route_build(const DevParams& p, const BlockSmem&
     const int tid = threadIdx.x;
     const int E = p.E, K = p.K, P = p.T * p.K;
     const int Wc = (p.T + 31) >> 5;
-    for (int pair = tid; pair < P; pair += kThreads) s.idx[pair] = __ldg(p.idx + pair);
+    for (int pair = tid; pair < P; pair += 4 * kThreads) {
+        int e4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e4[u] = pair + u * kThreads < P ? ld_input(p.idx + pair + u * kThreads) : 0;  // loaded together
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (pair + u * kThreads < P) s.idx[pair + u * kThreads] = e4[u];
+    }
     for (int i = tid; i < Wc * E; i += kThreads) s.bits[i] = 0u;
     __syncthreads();
     // one token per thread: no division, K consecutive indices (one or two 32-byte sectors)
@@ -84,7 +91,7 @@ __device__ __forceinline__ void route_build(const DevParams& p, const BlockSmem&
             int e8[8];
             unsigned before[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) e8[u] = (k0 + u < K) ? __ldg(row + k0 + u) : 0;  // loaded together
+            for (int u = 0; u < 8; ++u) e8[u] = (k0 + u < K) ? ld_input(row + k0 + u) : 0;  // loaded together
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 before[u] = 0u;
@@ -441,7 +448,7 @@ __device__ __forceinline__ void combine_phase(const DevParams& p, int cb, int nc
         bool ok = true;
         if (lane < K) {
             const size_t pair = (size_t)t * K + lane;
-            const int e = __ldg(p.idx + pair);
+            const int e = ld_input(p.idx + pair);
             if (e >= 0 && e < p.E) {
                 // The expert's rank is known from the caller's indices alone.  Its flag is awaited BEFORE
                 // the slot table is read: the flag implies that this rank's own routing of this call (which
@@ -453,7 +460,7 @@ __device__ __forceinline__ void combine_phase(const DevParams& p, int cb, int nc
                 }
                 const int j = ok ? ld_stream(p.slot + pair) : -1;
                 if (j >= 0) {
-                    my_w = __ldg(p.w + pair);
+                    my_w = ld_input(p.w + pair);
                     my_row = reinterpret_cast<unsigned long long>(
                         reinterpret_cast<const uint4*>(p.peer[d] + p.off_rows) +
                         (((size_t)l * p.ws + p.rank) * p.T_max + j) * nvec);

@@ -320,7 +320,7 @@ __device__ __forceinline__ void near_combine_push(const NearParams& g, int* s_pr
     if (!near_tokens(g, s_pre, (nvec + 127) >> 7, list)) return;  // timeout recorded; y is left untouched
     auto bit_of = [&](const NearTokens::At& a) {  // lane k: the rank of pair k
         if (a.row >= list.total || lane >= K) return 0u;
-        const int e = __ldg(g.p[g.n - 1 - a.at].idx + (size_t)(a.row - s_pre[a.at]) * K + lane);
+        const int e = ld_input(g.p[g.n - 1 - a.at].idx + (size_t)(a.row - s_pre[a.at]) * K + lane);
         return e >= 0 && e < p0.E ? 1u << (e / p0.L) : 0u;
     };
     NearTokens::At a0 = list.first();
@@ -385,9 +385,9 @@ __device__ __forceinline__ void near_combine_pull(const NearParams& g, int* s_pr
         if (a.row < list.total && lane < K) {
             const DevParams& p = g.p[g.n - 1 - a.at];
             const size_t i = (size_t)(a.row - s_pre[a.at]) * K + lane;
-            r.e = __ldg(p.idx + i);
+            r.e = ld_input(p.idx + i);
             r.j = ld_stream(p.slot + i);
-            r.w = __ldg(p.w + i);
+            r.w = ld_input(p.w + i);
         }
         return r;
     };

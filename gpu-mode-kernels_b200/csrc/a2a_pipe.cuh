@@ -75,7 +75,7 @@ __device__ __forceinline__ unsigned dest_mask(const DevParams& p, int t) {
     const int* row = p.idx + (size_t)t * p.K;
     if ((p.K & 3) == 0 && (reinterpret_cast<uintptr_t>(p.idx) & 15) == 0) {  // the row is 16-byte aligned: vector loads
         for (int k = 0; k < p.K; k += 4) {
-            const int4 e4 = __ldg(reinterpret_cast<const int4*>(row + k));
+            const int4 e4 = ld_input(reinterpret_cast<const int4*>(row + k));
             const int e[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
             for (int u = 0; u < 4; ++u)
@@ -84,7 +84,7 @@ __device__ __forceinline__ unsigned dest_mask(const DevParams& p, int t) {
         return m;
     }
     for (int k = 0; k < p.K; ++k) {
-        const int e = __ldg(row + k);
+        const int e = ld_input(row + k);
         if (e >= 0 && e < p.E) m |= 1u << (e / p.L);
     }
     return m;
@@ -481,7 +481,7 @@ __device__ __forceinline__ void router_role(const DevParams& p, uint8_t* smem, i
         for (int k0 = 0; k0 < K; k0 += 8) {
             int e8[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) e8[u] = (k0 + u < K) ? __ldg(row + k0 + u) : e0;  // loaded together
+            for (int u = 0; u < 8; ++u) e8[u] = (k0 + u < K) ? ld_input(row + k0 + u) : e0;  // loaded together
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int k = k0 + u, e = e8[u];
@@ -527,7 +527,7 @@ __device__ __forceinline__ void router_role(const DevParams& p, uint8_t* smem, i
         if (t < T) {
             const int* row = p.idx + (size_t)t * K;
             for (int k = 0; k < K; ++k) {
-                const int e = __ldg(row + k);
+                const int e = ld_input(row + k);
                 has |= (e >= e0 && e < e0 + L);
             }
         }
@@ -554,12 +554,12 @@ __device__ __forceinline__ void router_role(const DevParams& p, uint8_t* smem, i
             if (nn < 0) continue;
             const int tt = r0 + tl;
             const int* row = p.idx + (size_t)tt * K;
-            const int e = __ldg(row + k);
-            const float wk = __ldg(p.w + (size_t)tt * K + k);
+            const int e = ld_input(row + k);
+            const float wk = ld_input(p.w + (size_t)tt * K + k);
             unsigned ent = kNoEntry;
             if (e >= e0 && e < e0 + L) {
                 bool repeat = false;
-                for (int kk = 0; kk < k; ++kk) repeat |= (__ldg(row + kk) == e);
+                for (int kk = 0; kk < k; ++kk) repeat |= (ld_input(row + kk) == e);
                 int j = -1;
                 if (!repeat) {
                     const int l = e - e0, w = tt >> 5;
@@ -943,7 +943,7 @@ __device__ __forceinline__ void combine_home_role(const DevParams& p, int cb, in
             const int t = (int)(it / nchunk), v0 = (int)(it - (long long)t * nchunk) * 128;
             bool any = false;
             if (lane < K) {
-                const int e = __ldg(p.idx + (size_t)t * K + lane);
+                const int e = ld_input(p.idx + (size_t)t * K + lane);
                 any = (e >= 0 && e < p.E);
             }
             if (__any_sync(0xffffffffu, any)) continue;
@@ -975,7 +975,7 @@ __device__ __forceinline__ void combine_home_role(const DevParams& p, int cb, in
         const int t = (int)(it / nchunk), v0 = (int)(it - (long long)t * nchunk) * 128;
         unsigned bit = 0u;
         if (lane < K) {
-            const int e = __ldg(p.idx + (size_t)t * K + lane);
+            const int e = ld_input(p.idx + (size_t)t * K + lane);
             if (e >= 0 && e < p.E) bit = 1u << (e / p.L);
         }
         const unsigned mask = __reduce_or_sync(0xffffffffu, bit);

@@ -22,14 +22,14 @@ __device__ __forceinline__ void count_experts_before(const DevParams& p, int t_e
         for (int k0 = 0; k0 < K; k0 += 8) {
             int e8[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) e8[u] = (k0 + u < K) ? __ldg(row + k0 + u) : -1;
+            for (int u = 0; u < 8; ++u) e8[u] = (k0 + u < K) ? ld_input(row + k0 + u) : -1;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int e = e8[u];
                 bool ok = e >= 0 && e < p.E;
 #pragma unroll
                 for (int v = 0; v < u; ++v) ok = ok && e8[v] != e;
-                for (int kk = 0; ok && kk < k0; ++kk) ok = __ldg(row + kk) != e;
+                for (int kk = 0; ok && kk < k0; ++kk) ok = ld_input(row + kk) != e;
                 if (ok) atomicAdd(s_cnt + e, 1);
             }
         }
@@ -85,11 +85,17 @@ __global__ void __launch_bounds__(kThreads) solo_kernel(const __grid_constant__ 
     int* meta = reinterpret_cast<int*>(self + p.off_meta);
     const float scale = (float)(1 + p.rank);
 
-    // the first item's row is requested before anything else: it needs no routing
+    // the first item's row and the first round's pairs are requested before anything else: they need no routing
     long long it = lo + warp;
     int t = (int)(it / nchunk), c = (int)(it - (long long)t * nchunk);
     uint4 q[U];
     if (it < hi) load_own_chunk<T, PAYLOAD, U>(p, t, c * 32 * U, nvec, q);
+    int first_e = 0;
+    float first_w = 0.f;
+    if (tid < min(kSoloRound, t1 - t0) * K) {
+        first_e = ld_input(p.idx + (size_t)t0 * K + tid);
+        first_w = ld_input(p.w + (size_t)t0 * K + tid);
+    }
     for (int e = tid; e < p.E; e += kThreads) s_cnt[e] = 0;
     __syncthreads();
     count_experts_before<kThreads>(p, t0, s_cnt);
@@ -97,8 +103,11 @@ __global__ void __launch_bounds__(kThreads) solo_kernel(const __grid_constant__ 
     for (int r0 = t0; r0 < t1; r0 += kSoloRound) {
         const int nt = min(kSoloRound, t1 - r0), pairs = nt * K;
         for (int i = tid; i < pairs; i += kThreads) {
-            s_idx[i] = __ldg(p.idx + (size_t)r0 * K + i);
-            s_w[i] = __ldg(p.w + (size_t)r0 * K + i);
+            const bool first = r0 == t0 && i == tid;
+            const int e = first ? first_e : ld_input(p.idx + (size_t)r0 * K + i);
+            const float w = first ? first_w : ld_input(p.w + (size_t)r0 * K + i);
+            s_idx[i] = e;
+            s_w[i] = w;
         }
         __syncthreads();
         if (r0 == t0) stamp(p, kStampSourceSeen);
@@ -202,7 +211,7 @@ __global__ void __launch_bounds__(kRouteThreads) solo_route_kernel(const __grid_
     const int tid = threadIdx.x, K = p.K;
     const int t0 = (int)blockIdx.x * kRouteTokens, pairs = min(kRouteTokens, p.T - t0) * K;
     for (int e = tid; e < p.E; e += kRouteThreads) s_cnt[e] = s_bits[0][e] = s_bits[1][e] = 0;
-    for (int i = tid; i < pairs; i += kRouteThreads) s_idx[i] = __ldg(p.idx + (size_t)t0 * K + i);
+    for (int i = tid; i < pairs; i += kRouteThreads) s_idx[i] = ld_input(p.idx + (size_t)t0 * K + i);
     __syncthreads();
     count_experts_before<kRouteThreads>(p, t0, s_cnt);
     auto first_use = [&](int i) {  // pair i's expert is in range and of no earlier pair of its token
@@ -253,8 +262,8 @@ __global__ void __launch_bounds__(kThreads) solo_rows_kernel(const __grid_consta
     if (lane < K) {
         const size_t pair = (size_t)t * K + lane;
         const int j = ld_stream(p.slot + pair);
-        if (j >= 0) my_row = __ldg(p.idx + pair) * p.T_max + j;
-        my_w = __ldg(p.w + pair);
+        if (j >= 0) my_row = ld_input(p.idx + pair) * p.T_max + j;
+        my_w = ld_input(p.w + pair);
     }
     const float scale = (float)(1 + p.rank);
     uint4* rows = reinterpret_cast<uint4*>(p.peer[p.rank] + p.off_rows) + v0 + lane;
