@@ -535,7 +535,8 @@ bool any_traced(a2a_ctx* const* cs, int n) {
 }
 
 // A kernel for ranks on one GPU, `blocks` in all; `ns` and `nr` are what role 0's blocks agree on.
-int launch_near(a2a_ctx* const* cs, int n, NearFn fn, int blocks, int smem, cudaStream_t st, int ns = 0, int nr = 0) {
+int launch_near(a2a_ctx* const* cs, int n, NearFn fn, int blocks, int smem, cudaStream_t st, int ns = 0, int nr = 0,
+                bool every_rank = false) {
     NearParams g;
     for (int r = 0; r < n; ++r) {
         g.p[r] = call_params(cs[r]);
@@ -551,6 +552,7 @@ int launch_near(a2a_ctx* const* cs, int n, NearFn fn, int blocks, int smem, cuda
     memcpy(g.x, cs[0]->near_x, sizeof(g.x));
     memcpy(g.T, cs[0]->near_T, sizeof(g.T));
     g.n = n;
+    g.every_rank = every_rank ? 1 : 0;
     void* args[] = {&g};
     const cudaError_t e = launch_after_previous((const void*)fn, blocks, smem, args, st, overlaps(cs[0], tokens));
     return e == cudaSuccess ? A2A_OK : -(int)e;
@@ -649,9 +651,10 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
     }
     const a2a_ctx* c = cs[0];
     const int blocks = c->num_sms * 2, push_smem = c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
-    if (n > 1 && !any_traced(cs, n) && near) return launch_near(cs, n, select_pipe<NearRole>(c, role), blocks, 0, st);
+    // a role 2 is through when every rank is through with this call's records, whoever's rows its tokens want
+    if (n > 1 && !any_traced(cs, n) && near) return launch_near(cs, n, select_pipe<NearRole>(c, role), blocks, 0, st, 0, 0, true);
     for (int r = 0; r < n; ++r) {
-        const int rc = cs[r]->near ? launch_near(cs + r, 1, select_pipe<NearRole>(c, role), blocks, 0, st)
+        const int rc = cs[r]->near ? launch_near(cs + r, 1, select_pipe<NearRole>(c, role), blocks, 0, st, 0, 0, true)
                                    : launch_role(cs[r], role, 1 + blocks, role == 1 ? push_smem : 0, st);
         if (rc != A2A_OK) return rc;
     }

@@ -20,6 +20,7 @@ struct NearParams {
     const void* x[A2A_MAX_WORLD];  // input rows of rank s in this call
     int T[A2A_MAX_WORLD];          // and how many
     int n;
+    int every_rank;  // a PULL combine ends only when every rank's outputs are there, also those no token wants
 };
 
 // ---------------------------------------------------------------------------
@@ -291,13 +292,20 @@ struct NearTokens {
     }
 };
 
-// Waits for every expert flag of the ranks served; false where one gave up.
+// The list; with WAIT, once every expert flag of the ranks served is up.  False where one is not.
+template <bool WAIT>
 __device__ __forceinline__ bool near_tokens(const NearParams& g, int* s_pre, int nchunk, NearTokens& list) {
     const int tid = threadIdx.x, ws = g.p[0].ws, warps = (int)gridDim.x * (kThreads / 32);
     bool ok = true;
     if (tid < g.n * ws) {
         const DevParams& p = g.p[tid / ws];
-        ok = wait_flag_gpu(await_ptr(p, kFlagExpert, tid % ws), flag_value(p, 0), p, kPhaseCombine, tid % ws);
+        const uint32_t* flag = await_ptr(p, kFlagExpert, tid % ws);
+        if (WAIT) {
+            ok = wait_flag_gpu(flag, flag_value(p, 0), p, kPhaseCombine, tid % ws);
+        } else {
+            ok = (int32_t)(ld_relaxed_gpu(flag) - flag_value(p, 0)) >= 0;
+            fence_acq_rel_gpu();
+        }
     }
     if (tid == 0) {
         int sum = 0;
@@ -317,7 +325,7 @@ __device__ __forceinline__ void near_combine_push(const NearParams& g, int* s_pr
     const DevParams& p0 = g.p[0];
     const int K = p0.K, nvec = p0.H >> 3, T_max = p0.T_max;
     NearTokens list;
-    if (!near_tokens(g, s_pre, (nvec + 127) >> 7, list)) return;  // timeout recorded; y is left untouched
+    if (!near_tokens<true>(g, s_pre, (nvec + 127) >> 7, list)) return;  // timeout recorded; y is left untouched
     auto bit_of = [&](const NearTokens::At& a) {  // lane k: the rank of pair k
         if (a.row >= list.total || lane >= K) return 0u;
         const int e = ld_input(g.p[g.n - 1 - a.at].idx + (size_t)(a.row - s_pre[a.at]) * K + lane);
@@ -375,7 +383,9 @@ __device__ __forceinline__ void near_combine_pull(const NearParams& g, int* s_pr
     const DevParams& p0 = g.p[0];
     const int ws = p0.ws, K = p0.K, nvec = p0.H >> 3, T_max = p0.T_max;
     NearTokens list;
-    if (!near_tokens(g, s_pre, (nvec + 32 * U - 1) / (32 * U), list)) return;
+    // The launch before this one has raised the flags of the ranks whose expert phase ran.  Where one is missing, tokens
+    // wait for the ranks that have rows of theirs, and only for those: a rank without rows need not have run.
+    const bool all_up = near_tokens<false>(g, s_pre, (nvec + 32 * U - 1) / (32 * U), list);
     struct Pair {  // lane k: expert, slot and weight of pair k
         int e, j;
         float w;
@@ -393,6 +403,13 @@ __device__ __forceinline__ void near_combine_pull(const NearParams& g, int* s_pr
     };
     NearTokens::At a0 = list.first(), a1 = list.after(a0);
     Pair r0 = pair_of(a0), r1 = pair_of(a1);
+    auto go_on = [&](const NearTokens::At& a2, const Pair& r2) {
+        a0 = a1;
+        a1 = a2;
+        r0 = r1;
+        r1 = r2;
+    };
+    bool waited = false;
     while (a0.row < list.total) {
         const NearTokens::At a2 = list.after(a1);
         const Pair r2 = pair_of(a2);
@@ -400,6 +417,23 @@ __device__ __forceinline__ void near_combine_pull(const NearParams& g, int* s_pr
         const int t = a0.row - s_pre[a0.at], v0 = a0.ch * 32 * U + lane;
         const bool valid = r0.e >= 0 && r0.e < p0.E && r0.j >= 0;
         const int d = valid ? r0.e / p0.L : 0;
+        if (!all_up) {
+            const uint32_t* flag = await_ptr(p, kFlagExpert, d);
+            const uint32_t want = flag_value(p, 0);
+            bool ok = true;
+            if (valid && !waited) {
+                ok = wait_flag_gpu(flag, want, p, kPhaseCombine, d);
+            } else if (valid) {  // one budget is spent: the other ranks' tokens are told at once
+                ok = (int32_t)(ld_relaxed_gpu(flag) - want) >= 0;
+                if (!ok) record_timeout(p, kPhaseCombine, d, want);
+                fence_acq_rel_gpu();
+            }
+            if (!__all_sync(0xffffffffu, ok)) {  // timeout recorded; the token's output is left untouched
+                waited = true;
+                go_on(a2, r2);
+                continue;
+            }
+        }
         unsigned long long my_row = 0;
         if (valid)
             my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<const uint4*>(p0.peer[d] + p0.off_rows) +
@@ -436,10 +470,11 @@ __device__ __forceinline__ void near_combine_pull(const NearParams& g, int* s_pr
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (v0 + u * 32 < nvec) __stcs(y + u * 32, pack8<T>(acc[u]));
-        a0 = a1;
-        a1 = a2;
-        r0 = r1;
-        r1 = r2;
+        go_on(a2, r2);
+    }
+    if (!all_up && g.every_rank && blockIdx.x == 0 && threadIdx.x < g.n * ws) {
+        const DevParams& p = g.p[threadIdx.x / ws];
+        wait_flag_gpu(await_ptr(p, kFlagExpert, threadIdx.x % ws), flag_value(p, 0), p, kPhaseCombine, threadIdx.x % ws);
     }
 }
 

@@ -199,3 +199,32 @@ def test_a_call_goes_on_in_the_form_it_was_begun_in(payload, combine, together):
         world.check()
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("T", [8, 130])  # 1 MB of expert rows, and 18: the combine of many rows is another kernel
+def test_a_rank_without_rows_need_not_run_its_expert_phase(T):
+    """Phases called rank by rank by a program that steps only the ranks with rows; the combine for all ranks together."""
+    ws, E, K, H = 4, 16, 4, 4096
+    rds = [pkg.generate_input(E, K, H, T, seed=6, rank=r, world_size=ws)[1].to(DEV) for r in range(ws)]
+    for rd in rds:  # no expert of the last rank
+        rd.indices = torch.rand(T, E - E // ws, device=DEV).topk(K, dim=1).indices.int()
+    world = LocalWorld(pkg.MoEConfig(E, K, H, T), ws, payload="direct", timeout_ms=300)
+    try:
+        want = [bits(y) for y in world.forward_phases(rds)]
+        for run in (ws - 1, 0):
+            world._send(rds)
+            for c in world.ctxs[:run]:
+                c.dispatch_recv()
+                c.expert_placeholder()
+            ys = world._combine(rds)
+            torch.cuda.synchronize()
+            if run:
+                assert all(torch.equal(bits(y), w) for y, w in zip(ys, want))
+                world.check()
+        for c in world.ctxs:  # nobody's expert phase ran: every rank ran out of its budget, once
+            assert c.peek() == _lib.A2A_ERR_TIMEOUT
+            c.clear_status()
+        assert all(torch.equal(bits(y), w) for y, w in zip(world.forward_phases(rds), want))
+        world.check()
+    finally:
+        world.close()
