@@ -283,9 +283,13 @@ template <typename T, int P, bool PUSH> struct PipeForward {
 using NearFn = void (*)(NearParams);
 template <typename T, int P, bool PUSH> struct PipeRole {
     // what is sent does not depend on the combine, nor the combine on how rows travelled
-    static KernelFn get(int role) {
-        return role == 0 ? pipe_role_kernel<T, P, true, 0>
-                         : role == 1 ? pipe_role_kernel<T, P, PUSH, 1> : pipe_role_kernel<T, A2A_PAYLOAD_DEDUP, PUSH, 2>;
+    template <int PP, bool PUSHP, int ROLE>
+    static PhaseFn pair() {
+        return {pipe_role_kernel<T, PP, PUSHP, ROLE, RankParams>, pipe_role_kernel<T, PP, PUSHP, ROLE, GroupParams>};
+    }
+    static PhaseFn get(int role) {
+        if (role == 0) return {pipe_role_kernel<T, P, true, 0, RankParams>, nullptr};  // a group's role 0 is a near one
+        return role == 1 ? pair<P, PUSH, 1>() : pair<A2A_PAYLOAD_DEDUP, PUSH, 2>();
     }
 };
 template <typename T, int P, bool PUSH> struct NearRole {
@@ -605,7 +609,7 @@ int begin_pipe_call(a2a_ctx* const* cs, int n, const a2a_call* calls) {
 
 // A role of the pipelined schedule for one rank, in the form of a rank whose peers are on other GPUs.
 int launch_role(a2a_ctx* c, int role, int blocks, int smem, cudaStream_t st) {
-    return launch(c, (const void*)select_pipe<PipeRole>(c, role), blocks, smem, st);
+    return launch(c, (const void*)select_pipe<PipeRole>(c, role).one, blocks, smem, st);
 }
 
 // Role 0.  Contexts that are being traced are launched one by one, in the forms of a GPU per rank: a trace has a slot
@@ -650,12 +654,17 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
         near = near && cs[r]->near;
     }
     const a2a_ctx* c = cs[0];
-    const int blocks = c->num_sms * 2, push_smem = c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
-    // a role 2 is through when every rank is through with this call's records, whoever's rows its tokens want
-    if (n > 1 && !any_traced(cs, n) && near) return launch_near(cs, n, select_pipe<NearRole>(c, role), blocks, 0, st, 0, 0, true);
+    const int blocks = c->num_sms * 2, push_smem = role == 1 && c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
+    if (n > 1 && !any_traced(cs, n)) {
+        // a role 2 is through when every rank is through with this call's records, whoever's rows its tokens want
+        if (near) return launch_near(cs, n, select_pipe<NearRole>(c, role), blocks, 0, st, 0, 0, true);
+        // Begun rank by rank: one launch, in which each rank has its share of two blocks per SM.  Role 0 of eight ranks one by
+        // one and these two, 4 tokens of 2048 146 us (294 with a launch for each rank), 128 of 7168 222 (404).
+        return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), blocks / n, push_smem, st);
+    }
     for (int r = 0; r < n; ++r) {
         const int rc = cs[r]->near ? launch_near(cs + r, 1, select_pipe<NearRole>(c, role), blocks, 0, st, 0, 0, true)
-                                   : launch_role(cs[r], role, 1 + blocks, role == 1 ? push_smem : 0, st);
+                                   : launch_role(cs[r], role, 1 + blocks, push_smem, st);
         if (rc != A2A_OK) return rc;
     }
     return A2A_OK;
@@ -868,7 +877,7 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
         const size_t a = cfg->world_size > 1 ? pipe_sender_smem(T, cfg->world_size, p.senders) : 0, b = pipe_router_smem(T, L);
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
         opt_in_both(select_pipe<PipeForward>(c));
-        opt_in((const void*)select_pipe<PipeRole>(c, 0));
+        opt_in((const void*)select_pipe<PipeRole>(c, 0).one);
         opt_in((const void*)select_pipe<NearRole>(c, 0));
         if (e == cudaSuccess && cfg->world_size == 1) {
             c->forward_grid = c->num_sms;

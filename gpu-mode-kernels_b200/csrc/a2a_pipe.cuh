@@ -1085,11 +1085,14 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_forward_kernel(const __grid_
 
 // The same roles as separate launches: for callers that want the phases apart, and for stepping the ranks of a
 // group one by one.  ROLE 0: senders + routers.  1: one watcher block + experts.  2: one watcher block + combine.
-// A whole group on ONE GPU steps through the kernels of a2a_near.cuh.
-template <typename T, int PAYLOAD, bool PUSH, int ROLE>
-__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ DevParams p) {
+// A call that a whole group on ONE GPU began together steps through the kernels of a2a_near.cuh; one that its ranks
+// began one by one goes on here, roles 1 and 2 of all ranks in a launch without watcher blocks.
+template <typename T, int PAYLOAD, bool PUSH, int ROLE, class P>
+__global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_constant__ P g) {
     begin_after_previous();
-    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+    constexpr int first = P::kGroup ? 0 : 1;
+    const DevParams& p = g.rank();
+    const int G = g.blocks(), b = g.block();
     const int ns = p.senders;
     stamp(p, kStampStart);
     if (ROLE == 0) {
@@ -1102,16 +1105,16 @@ __global__ void __launch_bounds__(kThreads, 2) pipe_role_kernel(const __grid_con
         }
         stamp(p, kStampSent);
     } else if (ROLE == 1) {
-        if (b == 0) watcher_role(p, kFlagDispatch, kPhaseRecv, (int)(threadIdx.x >> 5));
-        else expert_role<T, PAYLOAD, PUSH>(p, a2a_pipe_smem, b - 1, G - 1);
+        if (b < first) watcher_role(p, kFlagDispatch, kPhaseRecv, (int)(threadIdx.x >> 5));
+        else expert_role<T, PAYLOAD, PUSH>(p, a2a_pipe_smem, b - first, G - first);
         stamp(p, kStampExpertDone);
     } else {
-        if (b == 0) {
+        if (b < first) {
             watcher_role(p, kFlagExpert, kPhaseCombine, (int)(threadIdx.x >> 5));
         } else if (PUSH) {
-            combine_home_role<T>(p, b - 1, G - 1);
+            combine_home_role<T>(p, b - first, G - first);
         } else {
-            combine_phase<T>(p, b - 1, G - 1, /*own_watchers=*/false);
+            combine_phase<T>(p, b - first, G - first, /*own_watchers=*/false);
         }
         if (!PUSH) wait_all_experts(p, b);
     }

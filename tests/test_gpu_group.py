@@ -228,3 +228,29 @@ def test_a_rank_without_rows_need_not_run_its_expert_phase(T):
         world.check()
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("payload,combine", [("dedup", "push"), ("dedup", "pull"), ("fp8", "push")])
+def test_a_call_begun_rank_by_rank_goes_on_in_one_launch_a_role(payload, combine):
+    from cuda.bindings import runtime
+
+    ws, T, H = 3, 40, 2944
+    rds = [pkg.generate_input(12, 3, H, T, seed=7, rank=r, world_size=ws, ragged=True)[1].to(DEV) for r in range(ws)]
+    world = LocalWorld(pkg.MoEConfig(12, 3, H, T), ws, payload=payload, schedule="pipelined", combine=combine)
+    try:
+        want = [bits(y) for y in rank_by_rank(world, rds)]
+        for c, rd in zip(world.ctxs, rds):
+            c.pipe_step(0, rd.x, rd.indices, rd.weights)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            world._step("pipe_expert")
+            world._step("pipe_combine")
+        status, _, nodes = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
+        assert int(status) == 0 and nodes == 2
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(bits(c._y), w) for c, w in zip(world.ctxs, want))
+        world.check()
+    finally:
+        world.close()
