@@ -1,15 +1,20 @@
 """ctypes binding of liba2a.so (the C ABI declared in include/a2a.h).
 
 There is no fallback: if the library is missing or does not load, the first use
-raises.  Build it with ``python gpu-mode-kernels_b200/build.py`` (or
+raises.  The compiled part of the Python layer in front of it (``host()``) is only a
+shorter way to the same library.  Build both with ``python gpu-mode-kernels_b200/build.py`` (or
 ``__graft_entry__.build()``).
 """
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
+import warnings
 
 import torch
+
+from .build import host_path
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "liba2a.so")
@@ -115,16 +120,43 @@ def load() -> C.CDLL:
 _host = None
 
 
+class Interpreted:
+    """Stands in for the compiled part where that is not built for this Python and torch: it takes no call, so every
+    call goes through the Python code, which can do them all."""
+
+    class Rank:
+        def __init__(self, *_):
+            self.tokens = 0
+
+        def forward(self, *_):
+            return None
+
+        def close(self):
+            pass
+
+    @staticmethod
+    def group_forward(*_):
+        return None
+
+    @staticmethod
+    def histogram(*_):
+        return None
+
+
 def host():
-    """The compiled part of this layer (csrc/host.cpp), loaded once; raise if it is not there."""
+    """The compiled part of this layer (csrc/host.cpp), loaded once, or its stand-in."""
     global _host
     if _host is None:
+        path = host_path()
         try:
-            from . import _host as module
+            spec = importlib.util.spec_from_file_location(__package__ + "._host", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            _host = module
         except ImportError as e:
-            raise RuntimeError("_host.so is missing or does not load: build it with "
-                               "`python gpu-mode-kernels_b200/build.py`") from e
-        _host = module
+            warnings.warn(f"{path} is missing or does not load ({e}): calls cost the host several microseconds more; "
+                          "build it with `python gpu-mode-kernels_b200/build.py`", RuntimeWarning)
+            _host = Interpreted
     return _host
 
 

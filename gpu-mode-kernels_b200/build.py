@@ -1,12 +1,12 @@
-"""Build liba2a.so (the C-ABI CUDA library, nvcc for sm_100a) and _host.so (the compiled part of the Python
+"""Build liba2a.so (the C-ABI CUDA library, nvcc for sm_100a) and _host (the compiled part of the Python
 layer, g++ against torch's headers) in-tree.
 
     python gpu-mode-kernels_b200/build.py [--verbose]
 
 nvcc cross-compiles without a GPU.  The library links the CUDA runtime
-statically, so it depends on nothing but the driver at run time.
+statically, so it depends on nothing but the driver at run time.  _host depends on
+the Python and the torch it was built against; its file name says which.
 """
-import importlib.util
 import os
 import shutil
 import subprocess
@@ -22,7 +22,6 @@ HEADERS = [os.path.join(CSRC, "a2a_kernels.cuh"), os.path.join(CSRC, "a2a_pipe.c
            os.path.join(CSRC, "a2a_solo.cuh"),
            os.path.join(CSRC, "a2a_device.cuh"),
            os.path.join(ROOT, "include", "a2a.h")]
-HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 
 
@@ -33,10 +32,17 @@ def nvcc_path() -> str:
     raise RuntimeError("nvcc not found (set NVCC=/path/to/nvcc)")
 
 
+def host_path() -> str:
+    """Where _host for this Python and this torch lies: another one's is neither loaded nor taken for up to date."""
+    import torch
+
+    return os.path.join(PKG_DIR, f"_host.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH) or not os.path.exists(HOST_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(host_path()):
         return True
-    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(HOST_PATH))
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(host_path()))
     return any(os.path.getmtime(f) > t for f in SOURCES + HEADERS + [HOST_SOURCE, os.path.abspath(__file__)])
 
 
@@ -49,14 +55,16 @@ def run(tool: str, cmd, verbose: bool) -> None:
 
 
 def build_host(verbose: bool = False) -> None:
-    torch_dir = importlib.util.find_spec("torch").submodule_search_locations[0]
+    import torch
+
+    torch_dir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path())))
     include = [os.path.join(ROOT, "include"), os.path.join(torch_dir, "include"),
                os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
                sysconfig.get_paths()["include"]]
     run("g++", [
-        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", *("-I" + d for d in include), "-o", HOST_PATH,
-        HOST_SOURCE, "-L" + os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + d for d in include), "-o", host_path(), HOST_SOURCE, "-L" + os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
         "-L" + PKG_DIR, "-la2a", "-Wl,-rpath,$ORIGIN",
     ], verbose)
 

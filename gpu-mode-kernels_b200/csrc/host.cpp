@@ -1,4 +1,4 @@
-// _host.so -- the calls of the Python layer whose inputs are plain, from the tensors to the launches: checks,
+// _host -- the calls of the Python layer whose inputs are plain, from the tensors to the launches: checks,
 // output tensors and liba2a.so's entry points without an interpreter in between.  What it finds unusual (another
 // type, shape, layout, place or device, a recorded error, a closed context) it leaves alone and answers None:
 // the Python code then looks again and converts, raises or runs it, so what is accepted and how errors read is
