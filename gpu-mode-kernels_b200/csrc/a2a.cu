@@ -349,11 +349,15 @@ cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** arg
     return cudaLaunchKernelExC(&launch, fn, args);
 }
 
-// Blocks that get ready early take the places that happen to be free, two on one SM and none on the next, which a long
-// launch pays for: expert rows of 235 MB, eight ranks 133.7 us a call without and 135.9 with, PULL, 183 MB 91 / 101, one
-// rank 63.4 / 64.2.  A short one gains the latency of its launch: 50 MB, eight ranks 45.1 / 44.4; 33 MB, one rank 10.8 / 9.6;
-// 54 MB 16.41 / 16.54.
-constexpr long long kOverlapBytes = 48LL << 20;
+// The one launch of a single rank and the roles of ranks on one GPU are grids that stay for the whole launch.  Blocks of
+// theirs that get ready early take the places that happen to be free, two on one SM and none on the next, which a long launch
+// pays for: expert rows of 235 MB, eight ranks 133.7 us a call without and 135.9 with, PULL, 183 MB 91 / 101, one rank
+// 63.4 / 64.2.  A short one gains the latency of its launch: 50.3 MB, eight ranks 45.1 / 44.4; 33 MB, one rank 10.8 / 9.6;
+// 54.5 MB 16.41 / 16.54.  The line lies between those last two sizes.
+// The other launches overlap at any size, and gain: phases of eight ranks, 183 MB, direct, 147.2 us a call without and 144.8 with
+// (dedup 199.7 / 199.6, 59 MB, fp8, 72.1 / 69.3), of one rank in launches of their own, 80 MB, 82.3 / 78.5 (direct 94.5 / 91.2);
+// roles of two ranks one by one, 59 MB each, 105.7 / 102.2; many tokens of one rank, 235 MB, 58.0 to 59.7 / 57.2.
+constexpr long long kOverlapBytes = 50LL << 20;
 bool overlaps(const a2a_ctx* c, long long tokens) { return tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 <= kOverlapBytes; }
 
 int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false, bool overlap = true,

@@ -52,7 +52,7 @@ __host__ __device__ inline int pipe_list_per(int T_max, int senders) { return (T
 
 __host__ __device__ inline size_t pipe_sender_smem(int T_max, int ws, int senders) {
     size_t b = (size_t)kStages * kStageBytes + 128;                       // ring + barriers
-    b += (size_t)kStages * 2 * 16;                                        // descriptors (twice what the ring needs)
+    b += (size_t)kStages * 2 * 16;  // descriptors, twice what the ring needs: which configurations fit is decided by this sum
     b += ((size_t)ws * pipe_list_per(T_max, senders) * 2 + 15) / 16 * 16; // token lists
     b += 8 * A2A_MAX_WORLD * 4;                                           // warp totals
     return b;
