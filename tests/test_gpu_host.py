@@ -85,10 +85,18 @@ def test_a_group_with_unusual_data(schedule, payload, combine):
     forward = world.forward_pipelined if schedule == "pipelined" else world.forward_phases
     try:
         want = [bits(y) for y in forward(rds)]
-        kept = [[t.data_ptr() for t in c._keep] for c in world.ctxs]
+        def kept(datas, ys):
+            for c, d, y in zip(world.ctxs, datas, ys):
+                held = [d.x, d.indices, d.weights, y] if schedule == "pipelined" else [d.indices, d.x, d.weights]
+                assert [t.data_ptr() for t in c._keep] == [t.data_ptr() for t in held]
+                assert schedule != "pipelined" or c._y is y
+
+        ys = forward(rds)
+        kept(rds, ys)
         odd = [data_of(rds[0], x=rds[0].x.as_subclass(Sub)), rds[1]]  # goes through the Python code
-        assert all(torch.equal(bits(y), w) for y, w in zip(forward(tuple(odd)), want))
-        assert [[t.data_ptr() for t in c._keep] for c in world.ctxs] == kept or schedule == "pipelined"
+        ys = forward(tuple(odd))
+        assert all(torch.equal(bits(y), w) for y, w in zip(ys, want))
+        kept(odd, ys)
         assert [c._num_tokens for c in world.ctxs] == [6, 6]
         with pytest.raises(A2AError) as refused:
             forward(rds[:1])

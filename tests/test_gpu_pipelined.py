@@ -1,8 +1,8 @@
 """GPU parity of the pipelined schedule (role-specialised one-launch kernel), both combine modes.
 
 World sizes above one are stepped role by role on a single GPU (``LocalWorld.forward_pipelined``:
-launched as senders+routers / experts / combine so that a kernel that waits never shares the GPU with
-the kernel it waits for, in the forms for peers on this GPU).  The one-launch kernel itself and the forms for
+launched as routers (and, FP8, quantisers) / experts / combine so that a kernel that waits never shares the GPU
+with the kernel it waits for, in the forms for peers on this GPU: 16-bit rows have no senders there).  The one-launch kernel itself and the forms for
 distant peers are held to the oracle by test_gpu_one_launch.py.  At world size one the forward is a
 kernel of its own and must give the same bits as the stepped roles.  The one-process-per-GPU form is
 covered by test_x_gpu_multiprocess.py.
