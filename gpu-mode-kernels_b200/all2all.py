@@ -203,7 +203,8 @@ class A2AContext:
     def pipe_step(self, role: int, x=None, indices=None, weights=None, y=None) -> Optional[torch.Tensor]:
         """One role of the pipelined kernel as its own launch: 0 senders + routers (takes x, indices,
         weights and optionally the output tensor), 1 experts, 2 combine (returns the output).  For
-        stepping several ranks on one GPU and for timing the roles apart."""
+        stepping several ranks on one GPU one by one and for timing the roles apart; a call that
+        ``LocalWorld.forward_pipelined`` began for all of them goes on in its forms for near peers."""
         if role == 0:
             n = self._check_inputs(x, indices, weights, y, on_device=True)
             if y is None:

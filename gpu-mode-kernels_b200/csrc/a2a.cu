@@ -408,9 +408,10 @@ int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int s
 // Rows in host memory: half an SM's worth of warps fills the link, and more only get in each other's way
 // (3.7 MB read and as much written by 74 / 148 / 296 blocks: 100 / 107 / 118 us).
 // Many tokens in rows that outweigh a second launch: slots first, then rows in blocks of one item a warp, one vector a
-// lane, or two where fewer than six stores follow each load.  Back to back, against the one launch: 2048 tokens of
-// 7168, top-8 62.2 -> 57.1 us; of 2048, top-6 19.8 -> 17.0, top-2 12.4 -> 11.6; of 6144, top-2 23.3 both; 1300 tokens of
-// 4096, top-8 24.6 / 24.9, of 2880, top-4 13.4 / 12.9; 1024 of 2880 10.9 / 11.5, 400 of 2048, top-2 5.9 / 7.4.
+// lane, or two where fewer than six stores follow each load.  Back to back, the one launch and the two, at 2048 tokens:
+// of 7168, top-8 61.6 / 57.0 us; of 4096, top-8 37.8 / 37.5; of 2048, top-6 19.0 / 16.9, top-2 12.1 / 11.4; of 2880, top-4
+// 18.9 / 18.7; of 6144, top-2 21.6 / 23.1.  At 1280: 39.5 / 39.0, 23.2 / 24.2, 13.3 / 11.7, 9.1 / 9.0, 12.8 / 12.5, 14.2 / 15.0; at
+// 1024 31.8 / 31.0, 18.7 / 19.4, 11.0 / 10.1, 7.9 / 7.6, 10.9 / 11.5, 12.1 / 12.1; at 400 13.0 / 13.3, 9.9 / 10.4, 7.2 / 7.4.
 constexpr int kSoloManyTokens = 1280;
 constexpr long long kSoloManyBytes = 8LL << 20;
 int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
@@ -1100,7 +1101,7 @@ int a2a_forward_host(a2a_ctx* c, const void* x, const int32_t* idx, const float*
     if (T > 0 && c->cfg.world_size == 1 && c->cfg.schedule == A2A_SCHEDULE_PIPELINED) {
         // One rank reads every row once and writes every output once: where the kernel can reach the caller's
         // memory it does so itself, and the link carries both directions at the same time instead of one copy
-        // after the other (256 tokens of 7168: 135 us a call, 192 with copies around the kernel).  The indices, which
+        // after the other (256 tokens of 7168: 128 us a call, 192 with copies around the kernel).  The indices, which
         // every block reads, are copied.
         void *dx, *dw, *dy;
         if (!overlap(y, row * T, x, row * T) && !overlap(y, row * T, w, tk) && !overlap(y, row * T, idx, tk) &&

@@ -214,7 +214,8 @@ int a2a_forward_host(a2a_ctx* ctx, const void* x_host, const int32_t* topk_idx_h
 /* The roles of the pipelined one-launch kernel as three separate launches (same device code):
  * role 0 = senders + routers (takes x, topk_idx, topk_weights, y and num_tokens; starts the call),
  * role 1 = dispatch watchers + expert blocks, role 2 = expert-flag watchers + combine; roles 1
- * and 2 take no tensors (NULL / 0): they use what role 0 was given, and are refused (A2A_ERR_STATE) where
+ * and 2 take no tensors (NULL / 0): they use what role 0 was given (where a2a_group_step began the call, role 1
+ * of any rank reads the x of every rank), and are refused (A2A_ERR_STATE) where
  * the current call was begun otherwise -- by a2a_forward with one rank, a2a_forward_host into pinned rows or
  * a2a_route, none of which writes what they read.  For stepping several ranks on one GPU -- a
  * kernel that waits for a peer never shares a GPU with the kernel it waits for -- and for
