@@ -66,6 +66,7 @@ SIGNATURES = {
     "a2a_check_handles": (_I, [C.POINTER(Config), _VP, C.c_size_t, C.c_char_p, C.c_size_t]),
     "a2a_pipe_step": (_I, [_VP, _I, _VP, _VP, _VP, _VP, _I, _VP]),
     "a2a_group_step": (_I, [C.POINTER(_VP), _I, C.POINTER(Call), _VP]),
+    "a2a_group_steps": (_I, [C.POINTER(_VP), C.POINTER(C.c_int32), _I, C.POINTER(Call), _VP, C.POINTER(C.c_int32)]),
     "a2a_group_forward": (_I, [C.POINTER(_VP), C.POINTER(Call), _VP]),
     "a2a_attach_local_peers": (_I, [_VP, C.POINTER(_VP)]),
     "a2a_route": (_I, [_VP, _VP, _I, _VP]),

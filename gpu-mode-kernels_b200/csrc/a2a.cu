@@ -87,9 +87,11 @@ struct a2a_ctx {
     void* ipc_mapped[A2A_MAX_WORLD];  // peers opened through CUDA IPC (to close on destroy)
     bool peers_ready;
     bool routed, sent;
-    bool recorded;          // this call's records are written: by role 0, or by the one launch of several ranks
-    bool near;              // its rows stayed where they are, for peers on this GPU: near_x, or FP8 the sources' own stages
+    bool recorded;          // roles 1 and 2 can follow: the call was begun by role 0, or by the one launch of several ranks
+    bool near;              // ... by role 0 of a group on this GPU: rows stay where they are
+    bool whole;             // ... and role 1 of the group has written the outputs too
     const void* near_x[A2A_MAX_WORLD];  // input rows of every rank in this call
+    const uint2* near_pairs[A2A_MAX_WORLD];
     int near_T[A2A_MAX_WORLD];
     uint32_t epoch, barrier_epoch;
     int cur_tokens;
@@ -280,7 +282,7 @@ template <typename T, int P> struct ExpertSel {
 template <typename T, int P, bool PUSH> struct PipeForward {
     static PhaseFn get() { return {pipe_forward_kernel<T, P, PUSH, RankParams>, pipe_forward_kernel<T, P, PUSH, GroupParams>}; }
 };
-using NearFn = void (*)(NearParams);
+
 template <typename T, int P, bool PUSH> struct PipeRole {
     // what is sent does not depend on the combine, nor the combine on how rows travelled
     template <int PP, bool PUSHP, int ROLE>
@@ -290,11 +292,6 @@ template <typename T, int P, bool PUSH> struct PipeRole {
     static PhaseFn get(int role) {
         if (role == 0) return {pipe_role_kernel<T, P, true, 0, RankParams>, nullptr};  // a group's role 0 is a near one
         return role == 1 ? pair<P, PUSH, 1>() : pair<A2A_PAYLOAD_DEDUP, PUSH, 2>();
-    }
-};
-template <typename T, int P, bool PUSH> struct NearRole {
-    static NearFn get(int role) {
-        return role == 0 ? near_send_kernel<T, P> : role == 1 ? near_expert_kernel<T, P, PUSH> : near_combine_kernel<T, PUSH>;
     }
 };
 template <template <typename, int, bool> class F, typename T, typename... A>
@@ -318,13 +315,24 @@ KernelFn solo_fn(const a2a_ctx* c) {
     return bf ? solo_kernel<__nv_bfloat16, A2A_PAYLOAD_DEDUP, U> : solo_kernel<__half, A2A_PAYLOAD_DEDUP, U>;
 }
 
-// its second launch where there are many tokens
-template <int U>
-KernelFn solo_rows_fn(const a2a_ctx* c) {
+// role 1 of ranks on one GPU
+template <typename T, int P, bool PUSH, int N>
+const void* rows_fn(bool narrow) {
+    return narrow ? (const void*)near_rows_kernel<T, P, PUSH, 1, N> : (const void*)near_rows_kernel<T, P, PUSH, 2, N>;
+}
+template <bool PUSH, int N>
+const void* rows_fn(const a2a_ctx* c, bool narrow) {
     const bool bf = c->cfg.dtype == A2A_DTYPE_BF16;
     if (c->cfg.payload == A2A_PAYLOAD_FP8)
-        return bf ? solo_rows_kernel<__nv_bfloat16, A2A_PAYLOAD_FP8, U> : solo_rows_kernel<__half, A2A_PAYLOAD_FP8, U>;
-    return bf ? solo_rows_kernel<__nv_bfloat16, A2A_PAYLOAD_DEDUP, U> : solo_rows_kernel<__half, A2A_PAYLOAD_DEDUP, U>;
+        return bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_FP8, PUSH, N>(narrow) : rows_fn<__half, A2A_PAYLOAD_FP8, PUSH, N>(narrow);
+    return bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_DEDUP, PUSH, N>(narrow) : rows_fn<__half, A2A_PAYLOAD_DEDUP, PUSH, N>(narrow);
+}
+
+// the combine of ranks on one GPU
+const void* near_combine_fn(const a2a_ctx* c, bool push) {
+    if (c->cfg.dtype == A2A_DTYPE_BF16)
+        return push ? (const void*)near_combine_kernel<__nv_bfloat16, true> : (const void*)near_combine_kernel<__nv_bfloat16, false>;
+    return push ? (const void*)near_combine_kernel<__half, true> : (const void*)near_combine_kernel<__half, false>;
 }
 
 PhaseFn combine_fn(const a2a_ctx* c) {
@@ -399,6 +407,63 @@ int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int s
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
+// What a launch for `n` ranks on one GPU is told.  The call's rows and pairs are those the contexts hold of every rank.
+NearGroup near_params(a2a_ctx* const* cs, int n) {
+    NearGroup g{};
+    for (int r = 0; r < n; ++r) {
+        g.p[r] = call_params(cs[r]);
+        g.p[r].local = 1;
+        if (n > 1) g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
+    }
+    memcpy(g.x, cs[0]->near_x, sizeof(g.x));
+    memcpy(g.pairs, cs[0]->near_pairs, sizeof(g.pairs));
+    memcpy(g.T, cs[0]->near_T, sizeof(g.T));
+    g.n = n;
+    return g;
+}
+
+template <int N>
+int launch_near(a2a_ctx* const* cs, NearParams<N>& g, const void* fn, int blocks, int smem, cudaStream_t st, bool overlap = true,
+                int threads = kThreads, int words = 0) {
+    if (blocks > kTraceBlocks) g.p[0].trace = nullptr;
+    if (g.p[0].trace != nullptr) cs[0]->last_grid = blocks;
+    for (int r = 0; r < g.n; ++r) cs[r]->launches++;
+    void* args[] = {&g, &words};
+    const cudaError_t e = launch_after_previous(fn, blocks, smem, args, st, overlap, threads);
+    return e == cudaSuccess ? A2A_OK : -(int)e;
+}
+
+// Role 0 of ranks on one GPU: 32 tokens a block (64: headline workload of eight ranks 56.5 us a call instead of 56.4, two ranks of
+// 200 tokens 15.4 / 15.1), or more where there are so many that counting the tokens before the block's shows (2048 tokens of one
+// rank, 32 / 64: 56.2 / 55.4).
+template <int N>
+int launch_near_route(a2a_ctx* const* cs, NearParams<N>& g, cudaStream_t st) {
+    int most = 1;
+    for (int r = 0; r < g.n; ++r) most = cs[r]->cur_tokens > most ? cs[r]->cur_tokens : most;
+    const int words = most > 8192 ? 8 : most > 1024 ? 2 : 1, nb = (most + 32 * words - 1) / (32 * words);
+    return launch_near(cs, g, (const void*)near_route_kernel<N>, g.n * nb, (int)near_route_smem(words, cs[0]->cfg.num_experts, cs[0]->cfg.experts_per_token),
+                       st, true, kRouteThreads, words);
+}
+
+// Role 1: a warp per 1 KB of a token's row, three blocks per SM, or per 512 bytes where that would be too few rounds of blocks:
+// two where six or more stores follow each load, one where fewer do.  Calls of a group, 512 bytes / 1 KB (rounds of the
+// latter): top-8 of 7168, 256 tokens, eight ranks 64.6 / 56.4 us (8.1), two ranks 18.6 / 19.6 (2.0), 200 tokens 15.1 / 16.5 (1.6); top-6 of 2048,
+// 256 tokens, eight ranks 21.4 / 19.8 (2.3); top-2 of 6144, 110 tokens, eight 17.4 / 15.5 (2.9), four 11.8 / 11.3 (1.5), 256, two 11.5 / 10.8
+// (1.7); top-4 of 2880, 110, eight 14.6 / 14.1 (1.5).
+template <int N>
+int launch_near_rows(a2a_ctx* const* cs, NearParams<N>& g, bool push, cudaStream_t st) {
+    const a2a_ctx* c = cs[0];
+    const long long nvec = c->cfg.hidden_dim / 8, wide = (nvec + 63) / 64, narrow = (nvec + 31) / 32, warps = kThreads / 32;
+    long long tokens = 0;
+    for (int s = 0; s < c->cfg.world_size; ++s) tokens += g.T[s];
+    const bool many = 2 * tokens * wide >= (c->cfg.experts_per_token >= 6 ? 13LL : 6LL) * c->num_sms * warps;
+    const long long items = tokens * (many ? wide : narrow), blocks = items > 0 ? (items + warps - 1) / warps : 1;
+    const void* fn = rows_fn<false, N>(c, !many);
+    if constexpr (N > 1)
+        if (push) fn = rows_fn<true, N>(c, !many);
+    return launch_near(cs, g, fn, (int)blocks, 0, st);
+}
+
 // The forward of one rank.  A warp's item is one or two 16-byte vectors per lane of a token's row: two
 // where that still gives every warp of two blocks per SM an item (headline workload, 256 tokens of 7168:
 // 9.4 us against 9.7 with one and 10.2 with four; 2048 tokens 61.0 / 62.1 / 61.5), one below that, where
@@ -420,11 +485,9 @@ int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     const int K = c->cfg.experts_per_token;
     if (!host_rows && c->p.trace == nullptr && c->cur_tokens >= kSoloManyTokens &&
         (long long)c->cur_tokens * K * c->cfg.hidden_dim * 2 >= kSoloManyBytes) {
-        const bool narrow = K >= 6;
-        const int rc = launch(c, (const void*)solo_route_kernel, (c->cur_tokens + kRouteTokens - 1) / kRouteTokens, 0, st,
-                              /*cooperative=*/false, /*overlap=*/true, kRouteThreads);
-        return rc != A2A_OK ? rc : launch(c, (const void*)(narrow ? solo_rows_fn<1>(c) : solo_rows_fn<2>(c)),
-                                          (int)(((narrow ? one : two) + warps - 1) / warps), 0, st);
+        NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, kOutputWhole, /*handed_on=*/1};
+        const int rc = launch_near_route(&c, g, st);
+        return rc != A2A_OK ? rc : launch_near_rows(&c, g, /*push=*/false, st);
     }
     const bool wide = two >= cap * warps;
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
@@ -477,7 +540,7 @@ int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
     c->cur_tokens = T;
     c->p.idx = idx;
     c->routed = true;
-    c->sent = c->recorded = c->near = false;
+    c->sent = c->recorded = c->near = c->whole = false;
     return A2A_OK;
 }
 
@@ -543,31 +606,14 @@ bool any_traced(a2a_ctx* const* cs, int n) {
     return false;
 }
 
-// A kernel for ranks on one GPU, `blocks` in all; `ns` and `nr` are what role 0's blocks agree on.
-int launch_near(a2a_ctx* const* cs, int n, NearFn fn, int blocks, int smem, cudaStream_t st, int ns = 0, int nr = 0,
-                bool every_rank = false) {
-    NearParams g;
-    for (int r = 0; r < n; ++r) {
-        g.p[r] = call_params(cs[r]);
-        g.p[r].local = 1;
-        g.p[r].senders = ns;
-        g.p[r].routers = nr;
-        if (n > 1 || blocks > kTraceBlocks) g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
-        if (g.p[r].trace != nullptr) cs[r]->last_grid = blocks;
-        cs[r]->launches++;
-    }
+constexpr long long kNearCombineBytes = 16LL << 20;
+int launch_near_combine(a2a_ctx* const* cs, int n, bool push, bool every_rank, cudaStream_t st) {
+    NearGroup g = near_params(cs, n);
+    g.every_rank = every_rank ? 1 : 0;
     long long tokens = 0;
     for (int r = 0; r < n; ++r) tokens += cs[r]->cur_tokens;
-    memcpy(g.x, cs[0]->near_x, sizeof(g.x));
-    memcpy(g.T, cs[0]->near_T, sizeof(g.T));
-    g.n = n;
-    g.every_rank = every_rank ? 1 : 0;
-    void* args[] = {&g};
-    const cudaError_t e = launch_after_previous((const void*)fn, blocks, smem, args, st, overlaps(cs[0], tokens));
-    return e == cudaSuccess ? A2A_OK : -(int)e;
+    return launch_near(cs, g, near_combine_fn(cs[0], push), 2 * cs[0]->num_sms, 0, st, overlaps(cs[0], tokens));
 }
-
-constexpr long long kNearCombineBytes = 16LL << 20;
 
 int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st) {
     for (int r = 0; r < n; ++r) {
@@ -586,8 +632,7 @@ int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y,
     long long tokens = 0;
     for (int r = 0; r < n; ++r) tokens += cs[r]->cur_tokens;
     if (n > 1 && c->p.chunks == 1 && !any_traced(cs, n) && tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 >= kNearCombineBytes)
-        return launch_near(cs, n, c->cfg.dtype == A2A_DTYPE_BF16 ? near_combine_kernel<__nv_bfloat16, false> : near_combine_kernel<__half, false>,
-                           2 * c->num_sms, 0, st);
+        return launch_near_combine(cs, n, /*push=*/false, /*every_rank=*/false, st);
     const int nseg = (c->cfg.hidden_dim / 8 + 63) / 64;  // a warp per (token, 1 KB segment)
     const long long warps = (long long)most_tokens(cs, n) * nseg;
     return launch_ranks(cs, n, combine_fn(c), grid_for_ranks(c, n, (warps + kThreads / 32 - 1) / (kThreads / 32), 8), 0, st);
@@ -618,30 +663,25 @@ int launch_role(a2a_ctx* c, int role, int blocks, int smem, cudaStream_t st) {
 }
 
 // Role 0.  Contexts that are being traced are launched one by one, in the forms of a GPU per rank: a trace has a slot
-// per block of one rank's grid.
-int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st) {
+// per block of one rank's grid.  `handed_on`: roles 1 and 2 of the call follow on this stream, with nothing in between.
+int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st, bool handed_on = false) {
     const int begun = begin_pipe_call(cs, n, calls);
     if (begun != A2A_OK) return begun;
     const a2a_ctx* c = cs[0];
-    const int ws = c->cfg.world_size;
     int rc = A2A_OK;
     if (n == 1 || any_traced(cs, n)) {
         for (int r = 0; r < n && rc == A2A_OK; ++r)
-            rc = launch_role(cs[r], 0, c->p.senders + ws * c->p.routers, c->pipe_smem, st);
+            rc = launch_role(cs[r], 0, c->p.senders + c->cfg.world_size * c->p.routers, c->pipe_smem, st);
     } else {
         for (int r = 0; r < n; ++r)
             for (int s = 0; s < n; ++s) {
                 cs[r]->near_x[s] = calls[s].x;
+                cs[r]->near_pairs[s] = cs[s]->p.pairs;
                 cs[r]->near_T[s] = calls[s].num_tokens;
             }
-        // Four routers per destination, as far as there are 32-token words for them: eight ranks of 256 tokens of 7168,
-        // top-8 of 256 experts 9.4 us (12 with one, 9.8 with two), of 2048, top-6 of 64 8.2 (10.1, 9.0); one or two
-        // tokens 5.3 whatever their number.  FP8: quantisers for two blocks per SM.
-        const long long pieces = (c->cfg.hidden_dim / 8 + 127) / 128, warps = kThreads / 32;
-        const int words = (c->cfg.max_num_tokens + 31) / 32, nr = words < 4 ? words : 4;
-        int ns = 0;
-        if (c->cfg.payload == A2A_PAYLOAD_FP8) ns = grid_for_ranks(c, n, (most_tokens(cs, n) * pieces + warps - 1) / warps, 2);
-        rc = launch_near(cs, n, select_pipe<NearRole>(c, 0), n * (ns + ws * nr), (int)pipe_router_smem(c->cfg.max_num_tokens, c->p.L), st, ns, nr);
+        NearGroup g = near_params(cs, n);
+        g.handed_on = handed_on;
+        rc = launch_near_route(cs, g, st);
         if (rc == A2A_OK)
             for (int r = 0; r < n; ++r) cs[r]->near = true;
     }
@@ -650,26 +690,63 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
     return rc;
 }
 
-// Roles 1 and 2, of a call whose records exist: the one launch of a single rank writes none, and what role 1 would
+// Does an output of the call lie over input rows?  Role 1 may then not write outputs while other warps still read rows.
+bool outputs_over_rows(const a2a_call* calls, int n, size_t row_bytes) {
+    for (int r = 0; r < n; ++r)
+        for (int s = 0; s < n; ++s)
+            if (overlap(calls[r].y, row_bytes * calls[r].num_tokens, calls[s].x, row_bytes * calls[s].num_tokens)) return true;
+    return false;
+}
+
+// Roles 1 and 2, of a call whose role 0 ran: the one launch of a single rank writes nothing for them, and what role 1 would
 // find there belongs to an earlier call.  A call begun for ranks on one GPU goes on in that form, whoever asks for it.
-int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st) {
-    bool near = true;
+int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool handed_on = false) {
+    bool near = true, whole = true;
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent || !cs[r]->recorded) return A2A_ERR_STATE;
         near = near && cs[r]->near;
+        whole = whole && cs[r]->whole;
     }
     const a2a_ctx* c = cs[0];
-    const int blocks = c->num_sms * 2, push_smem = role == 1 && c->cfg.combine == A2A_COMBINE_PUSH ? (int)kReturnSmemBytes : 0;
+    const bool push = c->cfg.combine == A2A_COMBINE_PUSH;
+    const int blocks = c->num_sms * 2, push_smem = role == 1 && push ? (int)kReturnSmemBytes : 0;
     if (n > 1 && !any_traced(cs, n)) {
-        // a role 2 is through when every rank is through with this call's records, whoever's rows its tokens want
-        if (near) return launch_near(cs, n, select_pipe<NearRole>(c, role), blocks, 0, st, 0, 0, true);
-        // Begun rank by rank: one launch, in which each rank has its share of two blocks per SM.  Role 0 of eight ranks one by
-        // one and these two, 4 tokens of 2048 146 us (294 with a launch for each rank), 128 of 7168 222 (404).
-        return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), blocks / n, push_smem, st);
+        if (!near)
+            // Begun rank by rank: one launch, in which each rank has its share of two blocks per SM.  Role 0 of eight ranks one by
+            // one and these two, 4 tokens of 2048 146 us (294 with a launch for each rank), 128 of 7168 222 (404).
+            return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), blocks / n, push_smem, st);
+        NearGroup g = near_params(cs, n);
+        g.handed_on = handed_on;
+        if (role == 1) {
+            a2a_call calls[A2A_MAX_WORLD];
+            for (int r = 0; r < n; ++r) calls[r] = {g.x[r], nullptr, nullptr, cs[r]->p.y, g.T[r]};
+            // PULL: between these roles the expert rows are the caller's
+            if (handed_on || (push && !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2))) g.output = kOutputWhole;
+            else if (push) g.output = kOutputPartial;
+            const int rc = launch_near_rows(cs, g, push, st);
+            if (rc == A2A_OK)
+                for (int r = 0; r < n; ++r) cs[r]->whole = g.output == kOutputWhole;
+            return rc;
+        }
+        // a role 2 is through when every rank is through with this call, whoever's rows its tokens want
+        if (whole) return launch_near(cs, g, (const void*)near_finish_kernel, 1, 0, st, true, A2A_MAX_WORLD * A2A_MAX_WORLD);
+        return launch_near_combine(cs, n, push, /*every_rank=*/true, st);
     }
     for (int r = 0; r < n; ++r) {
-        const int rc = cs[r]->near ? launch_near(cs + r, 1, select_pipe<NearRole>(c, role), blocks, 0, st, 0, 0, true)
-                                   : launch_role(cs[r], role, 1 + blocks, push_smem, st);
+        int rc;
+        if (!cs[r]->near) {
+            rc = launch_role(cs[r], role, 1 + blocks, push_smem, st);
+        } else if (role == 1) {
+            NearGroup g = near_params(cs + r, 1);
+            if (push) g.output = kOutputPartial;
+            else cs[r]->whole = false;  // the expert rows are written anew, and the caller's again
+            rc = launch_near_rows(cs + r, g, push, st);
+        } else if (cs[r]->whole) {
+            NearGroup g = near_params(cs + r, 1);
+            rc = launch_near(cs + r, g, (const void*)near_finish_kernel, 1, 0, st, true, A2A_MAX_WORLD * A2A_MAX_WORLD);
+        } else {
+            rc = launch_near_combine(cs + r, 1, push, /*every_rank=*/true, st);
+        }
         if (rc != A2A_OK) return rc;
     }
     return A2A_OK;
@@ -725,6 +802,45 @@ int check_group(a2a_ctx* const* group) {
         for (int s = 0; s < group[0]->cfg.world_size; ++s)
             if (group[r]->p.peer[s] != group[s]->region) return A2A_ERR_CONFIG;
     return A2A_OK;
+}
+
+// One phase of all ranks of a group that check_group has passed.
+int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStream_t st) {
+    const a2a_ctx* c = group[0];
+    const int n = c->cfg.world_size;
+    const bool pipe_phase = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_PIPE_EXPERT || phase == A2A_GROUP_PIPE_COMBINE;
+    if (pipe_phase && c->cfg.schedule != A2A_SCHEDULE_PIPELINED) return A2A_ERR_STATE;
+    const bool takes_tensors = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_SEND || phase == A2A_GROUP_COMBINE;
+    if (takes_tensors && calls == nullptr) return A2A_ERR_CONFIG;
+    const void* x[A2A_MAX_WORLD];
+    const float* w[A2A_MAX_WORLD];
+    void* y[A2A_MAX_WORLD];
+    for (int r = 0; takes_tensors && r < n; ++r) {
+        x[r] = calls[r].x;
+        w[r] = calls[r].topk_weights;
+        y[r] = calls[r].y;
+    }
+    switch (phase) {
+        case A2A_GROUP_PIPE_SEND: return do_pipe_send(group, n, calls, st);
+        case A2A_GROUP_PIPE_EXPERT: return do_pipe_rest(group, n, 1, st);
+        case A2A_GROUP_PIPE_COMBINE: return do_pipe_rest(group, n, 2, st);
+        case A2A_GROUP_SEND:
+            for (int r = 0; r < n; ++r) {
+                const int rc = check_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
+                if (rc != A2A_OK) return rc;
+                if (calls[r].num_tokens > 0 && x[r] == nullptr) return A2A_ERR_CONFIG;
+                if (!rows_aligned(x[r])) return A2A_ERR_CONFIG;
+            }
+            for (int r = 0; r < n; ++r) begin_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
+            return do_send(group, n, x, st);
+        case A2A_GROUP_RECV:
+            return do_expert(group, n, true, true, false, false,
+                             c->cfg.payload == A2A_PAYLOAD_DIRECT ? n : expert_grid(c, n, 4), st);
+        case A2A_GROUP_EXPERT: return do_expert(group, n, false, false, true, true, expert_grid(c, n, 4), st);
+        case A2A_GROUP_RECV_EXPERT: return do_expert(group, n, true, true, true, true, expert_grid(c, n, 4), st);
+        case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st);
+        default: return A2A_ERR_CONFIG;
+    }
 }
 
 }  // namespace
@@ -791,6 +907,7 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     // local scratch: slot | send_counts | tickets | seen words | status | trace | host-path staging
     size_t off = 0;
     const size_t o_slot = off;      off = align_up(off + (size_t)T * K * 4, 256);
+    const size_t o_pairs = off;     off = align_up(off + (size_t)T * K * sizeof(uint2), 256);
     const size_t o_send = off;      off = align_up(off + (size_t)E * 4, 256);
     const size_t o_tick = off;      off = align_up(off + 8 * 4, 256);
     const size_t o_ptick = off;     off = align_up(off + 2 * A2A_MAX_WORLD * 4, 256);
@@ -847,6 +964,7 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
         p.chunks = (Wmax + p.wpc - 1) / p.wpc;
     }
     p.slot = reinterpret_cast<int*>(c->scratch + o_slot);
+    p.pairs = reinterpret_cast<uint2*>(c->scratch + o_pairs);
     p.send_counts = reinterpret_cast<int*>(c->scratch + o_send);
     p.tickets = reinterpret_cast<uint32_t*>(c->scratch + o_tick);
     p.ptickets = reinterpret_cast<uint32_t*>(c->scratch + o_ptick);
@@ -883,7 +1001,8 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
         opt_in_both(select_pipe<PipeForward>(c));
         opt_in((const void*)select_pipe<PipeRole>(c, 0).one);
-        opt_in((const void*)select_pipe<NearRole>(c, 0));
+        opt_in((const void*)near_route_kernel<1>);
+        opt_in((const void*)near_route_kernel<A2A_MAX_WORLD>);
         if (e == cudaSuccess && cfg->world_size == 1) {
             c->forward_grid = c->num_sms;
             c->fused = true;  // the solo kernel: no block waits for another
@@ -1142,45 +1261,32 @@ int a2a_pipe_step(a2a_ctx* c, int role, const void* x, const int32_t* idx, const
 }
 
 int a2a_group_step(a2a_ctx* const* group, int phase, const a2a_call* calls, void* stream) {
+    const int rc = check_group(group);
+    if (rc != A2A_OK) return rc;
+    DeviceGuard guard(group[0]->cfg.device);
+    return group_phase(group, phase, calls, as_stream(stream));
+}
+
+int a2a_group_steps(a2a_ctx* const* group, const int32_t* phases, int num_phases, const a2a_call* calls, void* stream, int32_t* done) {
+    if (done == nullptr || num_phases < 0 || (num_phases > 0 && phases == nullptr)) return A2A_ERR_CONFIG;
+    *done = 0;
     int rc = check_group(group);
     if (rc != A2A_OK) return rc;
     const a2a_ctx* c = group[0];
     const int n = c->cfg.world_size;
-    const bool pipe_phase = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_PIPE_EXPERT || phase == A2A_GROUP_PIPE_COMBINE;
-    if (pipe_phase && c->cfg.schedule != A2A_SCHEDULE_PIPELINED) return A2A_ERR_STATE;
-    const bool takes_tensors = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_SEND || phase == A2A_GROUP_COMBINE;
-    if (takes_tensors && calls == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
     cudaStream_t st = as_stream(stream);
-    const void* x[A2A_MAX_WORLD];
-    const float* w[A2A_MAX_WORLD];
-    void* y[A2A_MAX_WORLD];
-    for (int r = 0; takes_tensors && r < n; ++r) {
-        x[r] = calls[r].x;
-        w[r] = calls[r].topk_weights;
-        y[r] = calls[r].y;
+    // The roles of a whole call: with nothing between them role 1 writes the outputs of a PULL combine too, and no launch
+    // waits for flags of the one before it.
+    const bool roles = num_phases == 3 && phases[0] == A2A_GROUP_PIPE_SEND && phases[1] == A2A_GROUP_PIPE_EXPERT && phases[2] == A2A_GROUP_PIPE_COMBINE;
+    if (roles && n > 1 && calls != nullptr && c->cfg.schedule == A2A_SCHEDULE_PIPELINED && !any_traced(group, n) &&
+        !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2)) {
+        rc = do_pipe_send(group, n, calls, st, /*handed_on=*/true);
+        for (; rc == A2A_OK && ++*done < 3;) rc = do_pipe_rest(group, n, *done, st, /*handed_on=*/true);
+        return rc;
     }
-    switch (phase) {
-        case A2A_GROUP_PIPE_SEND: return do_pipe_send(group, n, calls, st);
-        case A2A_GROUP_PIPE_EXPERT: return do_pipe_rest(group, n, 1, st);
-        case A2A_GROUP_PIPE_COMBINE: return do_pipe_rest(group, n, 2, st);
-        case A2A_GROUP_SEND:
-            for (int r = 0; r < n; ++r) {
-                rc = check_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
-                if (rc != A2A_OK) return rc;
-                if (calls[r].num_tokens > 0 && x[r] == nullptr) return A2A_ERR_CONFIG;
-                if (!rows_aligned(x[r])) return A2A_ERR_CONFIG;
-            }
-            for (int r = 0; r < n; ++r) begin_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
-            return do_send(group, n, x, st);
-        case A2A_GROUP_RECV:
-            return do_expert(group, n, true, true, false, false,
-                             c->cfg.payload == A2A_PAYLOAD_DIRECT ? n : expert_grid(c, n, 4), st);
-        case A2A_GROUP_EXPERT: return do_expert(group, n, false, false, true, true, expert_grid(c, n, 4), st);
-        case A2A_GROUP_RECV_EXPERT: return do_expert(group, n, true, true, true, true, expert_grid(c, n, 4), st);
-        case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st);
-        default: return A2A_ERR_CONFIG;
-    }
+    for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK) rc = group_phase(group, phases[*done], calls, st);
+    return rc;
 }
 
 int a2a_group_forward(a2a_ctx* const* group, const a2a_call* calls, void* stream) {

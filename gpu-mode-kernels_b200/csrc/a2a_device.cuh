@@ -96,6 +96,7 @@ struct DevParams {
     long long timeout_ns;
     // local scratch of this rank
     int* slot;              // [T_max*K] slot of pair (t,k) inside slab (expert, this rank), -1 = dropped
+    uint2* pairs;           // [T_max*K] the same pairs as the kernels of ranks on one GPU read them (a2a_near.cuh)
     int* send_counts;       // [E]
     uint32_t* tickets;      // [2][kMaxChunks] block-arrival counters, one per publishing phase and chunk
     uint32_t* ptickets;     // [2][A2A_MAX_WORLD] pipelined schedule: arrivals per destination / per source

@@ -194,102 +194,4 @@ __global__ void __launch_bounds__(kThreads) solo_kernel(const __grid_constant__ 
     stamp(p, kStampCombineDone);
 }
 
-// ---------------------------------------------------------------------------
-// Many tokens: two launches, the slots of all pairs and then the rows, a warp an item in blocks that take no second
-// one.  What bounds it is the memory the rows go to, and a fixed share for each resident block, as above, leaves the
-// SMs that are farther from it at work when the others are through; blocks handed out in order do not, and need the
-// slots before they start.  2048 tokens of 7168, top-8: 62.2 -> 57.1 us a call, 293 MB at 5.1 TB/s with the routing.
-// ---------------------------------------------------------------------------
-constexpr int kRouteThreads = 1024;
-constexpr int kRouteTokens = 64;  // tokens of a routing block: two bitmap words per expert
-
-__global__ void __launch_bounds__(kRouteThreads) solo_route_kernel(const __grid_constant__ DevParams p) {
-    __shared__ int s_cnt[A2A_MAX_EXPERTS];           // tokens before this block's that use expert e
-    __shared__ unsigned s_bits[2][A2A_MAX_EXPERTS];  // this block's tokens that do
-    __shared__ int s_idx[kRouteTokens * A2A_MAX_TOPK];
-    begin_after_previous();
-    const int tid = threadIdx.x, K = p.K;
-    const int t0 = (int)blockIdx.x * kRouteTokens, pairs = min(kRouteTokens, p.T - t0) * K;
-    for (int e = tid; e < p.E; e += kRouteThreads) s_cnt[e] = s_bits[0][e] = s_bits[1][e] = 0;
-    for (int i = tid; i < pairs; i += kRouteThreads) s_idx[i] = ld_input(p.idx + (size_t)t0 * K + i);
-    __syncthreads();
-    count_experts_before<kRouteThreads>(p, t0, s_cnt);
-    auto first_use = [&](int i) {  // pair i's expert is in range and of no earlier pair of its token
-        const int e = s_idx[i];
-        bool ok = e >= 0 && e < p.E;
-        for (int j = i / K * K; ok && j < i; ++j) ok = s_idx[j] != e;
-        return ok;
-    };
-    for (int i = tid; i < pairs; i += kRouteThreads)
-        if (first_use(i)) atomicOr(&s_bits[i / K >> 5][s_idx[i]], 1u << (i / K & 31));
-    __syncthreads();
-    uint8_t* self = p.peer[p.rank];
-    int* meta = reinterpret_cast<int*>(self + p.off_meta);
-    for (int i = tid; i < pairs; i += kRouteThreads) {
-        const int tl = i / K, e = s_idx[i];
-        int j = -1;
-        if (first_use(i)) {
-            j = s_cnt[e] + __popc(s_bits[tl >> 5][e] & ((1u << (tl & 31)) - 1u));
-            if (tl >= 32) j += __popc(s_bits[0][e]);
-            meta[(size_t)e * p.T_max + j] = ((t0 + tl) << 8) | (i - tl * K);
-        } else {
-            record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
-        }
-        p.slot[(size_t)t0 * K + i] = j;
-    }
-    if (blockIdx.x == gridDim.x - 1) {
-        int* counts = reinterpret_cast<int*>(self + p.off_counts);
-        for (int e = tid; e < p.E; e += kRouteThreads)
-            counts[e] = p.send_counts[e] = s_cnt[e] + __popc(s_bits[0][e]) + __popc(s_bits[1][e]);
-    }
-}
-
-template <typename T, int PAYLOAD, int U>
-__global__ void __launch_bounds__(kThreads) solo_rows_kernel(const __grid_constant__ DevParams p) {
-    begin_after_previous();
-    const int lane = threadIdx.x & 31, K = p.K, nvec = p.H >> 3, nchunk = (nvec + 32 * U - 1) / (32 * U);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // phases called on this context after the forward find its flags up
-        *seen_ptr(p, kFlagDispatch, p.rank) = flag_value(p, 0);
-        *seen_ptr(p, kFlagExpert, p.rank) = flag_value(p, 0);
-    }
-    const long long it = (long long)blockIdx.x * kSoloWarps + (threadIdx.x >> 5);
-    const int t = (int)(it / nchunk), v0 = (int)(it - (long long)t * nchunk) * 32 * U;
-    if (t >= p.T) return;
-    uint4 q[U];
-    load_own_chunk<T, PAYLOAD, U>(p, t, v0, nvec, q);
-    int my_row = -1;  // lane k: the slab row of pair k
-    float my_w = 0.f;
-    if (lane < K) {
-        const size_t pair = (size_t)t * K + lane;
-        const int j = ld_stream(p.slot + pair);
-        if (j >= 0) my_row = ld_input(p.idx + pair) * p.T_max + j;
-        my_w = ld_input(p.w + pair);
-    }
-    const float scale = (float)(1 + p.rank);
-    uint4* rows = reinterpret_cast<uint4*>(p.peer[p.rank] + p.off_rows) + v0 + lane;
-    float acc[U][8];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        q[u] = scale8<T>(q[u], scale);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[u][e] = 0.f;
-    }
-    for (unsigned left = __ballot_sync(0xffffffffu, my_row >= 0); left != 0u; left &= left - 1u) {  // k ascending
-        const int k = __ffs(left) - 1;
-        uint4* row = rows + (size_t)__shfl_sync(0xffffffffu, my_row, k) * nvec;
-        const float w = __shfl_sync(0xffffffffu, my_w, k);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (v0 + u * 32 + lane < nvec) st_stream(row + u * 32, q[u]);
-            float f[8];
-            unpack8<T>(q[u], f);
-            fma8(f, w, acc[u]);
-        }
-    }
-    uint4* y = reinterpret_cast<uint4*>(p.y) + (size_t)t * nvec + v0 + lane;
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-        if (v0 + u * 32 + lane < nvec) st_stream(y + u * 32, pack8<T>(acc[u]));
-}
-
 }  // namespace a2a

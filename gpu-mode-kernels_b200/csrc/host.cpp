@@ -133,7 +133,7 @@ PyObject* group_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const bool pipelined = args[3] == Py_True;
     if (n < 1 || n > A2A_MAX_WORLD || !(PyList_Check(args[1]) || PyTuple_Check(args[1])) || PySequence_Fast_GET_SIZE(args[1]) < n)
         Py_RETURN_NONE;
-    int phases[4];
+    int32_t phases[4];
     const Py_ssize_t num_phases = PyTuple_GET_SIZE(args[2]);
     if (num_phases > 4) Py_RETURN_NONE;
     for (Py_ssize_t i = 0; i < num_phases; ++i) {
@@ -161,10 +161,10 @@ PyObject* group_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     at::Tensor ys[A2A_MAX_WORLD];
     for (Py_ssize_t i = 0; i < n; ++i) ys[i] = output_of(reinterpret_cast<Rank*>(native[i].o), calls[i]);
     void* stream = c10::cuda::getCurrentCUDAStream().stream();
-    int rc = A2A_OK, through = 0;
+    int rc;
+    int32_t through = 0;
     Py_BEGIN_ALLOW_THREADS
-    for (; through < num_phases; ++through)
-        if ((rc = a2a_group_step(group, phases[through], calls, stream)) != A2A_OK) break;
+    rc = a2a_group_steps(group, phases, (int)num_phases, calls, stream, &through);
     Py_END_ALLOW_THREADS
     if (through == 0) return PyLong_FromLong(rc);  // nothing begun
     Ref out;

@@ -101,7 +101,8 @@ class LocalWorld:
 
     def forward_pipelined(self, rank_datas: Sequence) -> List[torch.Tensor]:
         """The roles of the pipelined one-launch kernel as three launches, in lock-step:
-        every rank's routers (and quantisers), then every rank's expert blocks, then every rank's combine."""
+        every rank's routers, then every rank's expert blocks, then every rank's combine.  Nothing of the caller's
+        runs in between, so the second writes the outputs too where they do not lie over inputs (csrc/a2a_near.cuh)."""
         ys = self._quick(rank_datas, _ROLES, True)
         if ys is not None:
             return ys

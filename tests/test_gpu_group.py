@@ -254,3 +254,74 @@ def test_a_call_begun_rank_by_rank_goes_on_in_one_launch_a_role(payload, combine
         world.check()
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("payload,combine", [("dedup", "push"), ("dedup", "pull"), ("fp8", "push"), ("fp8", "pull")])
+@pytest.mark.parametrize("E,K,H,T,ws", [
+    (12, 3, 640, 33, 3),     # one token more than a routing block takes, rows that end inside a warp's piece
+    (16, 7, 6144, 200, 8),   # the wide form of role 1, for many stores a load
+    (8, 2, 2816, 400, 4),    # and for few
+    (8, 2, 128, 1100, 2),    # routing blocks of 64 tokens
+    (8, 2, 128, 8200, 2),    # of 256
+])
+def test_a_whole_call_equals_its_roles(payload, combine, E, K, H, T, ws):
+    """Outputs from the expert pass, against the forms of distant ranks, to the bit: in one call, role by role, and with
+    outputs over inputs (of the same rank, of another, and across two), where partial rows are added up."""
+    rds = [pkg.generate_input(E, K, H, T, seed=8, rank=r, world_size=ws)[1].to(DEV) for r in range(ws)]
+    for name in ("x", "indices", "weights"):  # a rank without tokens, one with few
+        setattr(rds[1], name, getattr(rds[1], name)[:0].contiguous())
+        setattr(rds[-1], name, getattr(rds[-1], name)[:1 if ws > 2 else 0].contiguous())
+    rds[0].indices[0, :] = rds[0].indices[0, 0]  # repeats, and a token without a valid expert: dropped, zero
+    rds[0].indices[T - 1, :] = E
+    for rd in rds:
+        rd.num_tokens = rd.x.shape[0]
+    world = LocalWorld(pkg.MoEConfig(E, K, H, T), ws, payload=payload, schedule="pipelined", combine=combine)
+    phases = (C.c_int32 * 3)(*[_lib.GROUP_PHASE[name] for name in ("pipe_send", "pipe_expert", "pipe_combine")])
+    handles = (C.c_void_p * ws)(*[c._h.value for c in world.ctxs])
+
+    def clear():
+        for c in world.ctxs:
+            assert c.peek() in (0, _lib.A2A_ERR_ROUTING)
+            c.clear_status()
+
+    def steps(xs, ys, whole):
+        calls, done = (_lib.Call * ws)(), C.c_int32()
+        for call, rd, x, y in zip(calls, rds, xs, ys):
+            call.x, call.topk_idx, call.topk_weights = x.data_ptr(), rd.indices.data_ptr(), rd.weights.data_ptr()
+            call.y, call.num_tokens = y.data_ptr(), x.shape[0]
+        if whole:
+            _lib.check(world.ctxs[0].lib.a2a_group_steps(handles, phases, 3, calls, _lib.current_stream(), C.byref(done)))
+            assert done.value == 3
+        else:
+            for name in ("pipe_send", "pipe_expert", "pipe_combine"):
+                world._step(name, calls)
+        torch.cuda.synchronize()
+        clear()
+        for c, x in zip(world.ctxs, xs):
+            c._num_tokens = x.shape[0]
+        return [bits(y) for y in ys]
+
+    try:
+        want = [bits(y) for y in rank_by_rank(world, rds)]
+        clear()
+        tables = state(world)
+        for whole in (True, False):
+            got = steps([rd.x for rd in rds], [torch.full_like(rd.x, 3) for rd in rds], whole)
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+            assert all(torch.equal(a, b) for a, b in zip(state(world), tables))
+            xs = [rd.x.clone() for rd in rds]
+            assert all(torch.equal(a, b) for a, b in zip(steps(xs, xs, whole), want))
+            xs = [rd.x.clone() for rd in rds]
+            ys = [torch.empty_like(x) for x in xs]
+            ys[-1] = xs[0][:xs[-1].shape[0]]  # over rows of another rank
+            assert all(torch.equal(a, b) for a, b in zip(steps(xs, ys, whole), want))
+            room, xs, ys, at = torch.empty(sum(rd.x.numel() for rd in rds) + 8 * H, dtype=rds[0].x.dtype, device=DEV), [], [], 0
+            for rd in rds:  # outputs that begin three rows into the inputs: over rows of two ranks
+                n = rd.x.numel()
+                xs.append(room[at:at + n].view_as(rd.x).copy_(rd.x))
+                ys.append(room[at + 3 * H:at + 3 * H + n].view_as(rd.x))
+                at += n
+            assert all(torch.equal(a, b) for a, b in zip(steps(xs, ys, whole), want))
+            assert all(torch.equal(a, b) for a, b in zip(state(world), tables))
+    finally:
+        world.close()
