@@ -28,13 +28,14 @@ constexpr int kBlocksPerSm = 2;
 constexpr int kUnroll = 4;
 constexpr int kBins = 256;
 constexpr int kCluster = 8;
-// One cluster writes the counts itself: no zeroing in front, one launch.  128 KB 4.3 us against 6.3 as
-// zero + count; 512 KB 6.3 against 6.2.  A block takes 32 KB at a time, so below 256 KB only some of the
-// cluster's blocks count, and at 512 KB 16 blocks of the other launch do.
+// One cluster writes the counts itself: no zeroing in front, one launch, which gets ready while the launch before it ends.
+// Calls back to back, 30 KB 2.7 us (5.2 without the overlap, and with 32 KB a block one of eight at work), 256 KB 3.3 (6.2). Above, the
+// host needs 5 us for zero + count, 300 KB 5.2 to one cluster's 4.0, but the GPU 2.6 to 3.6, which is what a captured call takes.
 constexpr size_t kClusterBytes = 256 * 1024;
+// Up to half a row of 8 KB for a block per SM, rows a grid apart: 300 KB 2.6 us on the GPU, 3.3 with 32 KB a block; 2 MB 3.6 / 3.1.
+constexpr size_t kSpreadBytesPerSm = 4 * 1024;
 // Below this a block per SM: 256 sums per block meet at 256 global words, and with few bytes per block
-// that is what the call waits for.  Measured against the three blocks per SM that large buffers had then:
-// 10 MB 6.3 us / 8.3, 42 MB 12.4 / 12.2, 168 MB 44 / 33.
+// that is what the call waits for.  10 MB 4.5 us on the GPU, 20 MB 6.2, 31 MB 7.9; with two blocks from 16 MB on 6.4 and 8.2.
 constexpr size_t kFullBytes = 32 * 1024 * 1024;
 
 // `lane4` = 4 * lane: the byte offset of the lane's word in a row of 32.
@@ -54,17 +55,20 @@ __device__ __forceinline__ void count_vector(unsigned* table, const uint4& q, un
     }
 }
 
-__device__ __forceinline__ void load_vectors(const uint4* vec, size_t i, size_t nvec, uint4 (&q)[kUnroll]) {
+// Ordinary loads, past the L1: a launch that overlaps the end of the one before it may not promise that nobody writes the data.
+__device__ __forceinline__ void load_vectors(const uint4* vec, size_t i, size_t row, size_t nvec, uint4 (&q)[kUnroll]) {
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u)
-        if (i + u * kThreads < nvec) q[u] = __ldcs(vec + i + u * kThreads);
+        if (i + u * row < nvec) q[u] = __ldcg(vec + i + u * row);
 }
 
-// CLUSTER: the grid is one cluster and stores the counts.  Otherwise the blocks add theirs to `out`, which
-// the launch before this one zeroes while the blocks already count.
-template <bool CLUSTER>
-__global__ void __launch_bounds__(kThreads, kBlocksPerSm) histogram256_kernel(const uint8_t* __restrict__ data, size_t n,
-                                                                             unsigned long long* __restrict__ out) {
+// The grid is one cluster and stores the counts; or its blocks add theirs to `out`, which the launch before this one zeroes while
+// they already count: with no more than a round of data (kSpread) or with more.
+enum Form { kCluster8, kSpread, kRounds };
+
+template <Form FORM>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm) histogram256_kernel(const uint8_t* data, size_t n,
+                                                                             unsigned long long* out) {
     __shared__ __align__(16) unsigned table[kBins * 32];
     __shared__ unsigned long long sums[kBins];
     const int tid = threadIdx.x;
@@ -75,24 +79,31 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) histogram256_kernel(co
     if (head > n) head = n;
     const size_t nvec = (n - head) / 16;
     const uint4* vec = reinterpret_cast<const uint4*>(data + head);
-    // a block takes 32 KB at a time
-    const size_t step = (size_t)gridDim.x * kThreads * kUnroll;
-    size_t i = (size_t)blockIdx.x * kThreads * kUnroll + tid;
+    // A block takes kUnroll rows of 8 KB at a time: one after the other, 32 KB of the memory's pages (512 MB 88 us, 97 with a row from
+    // each of four places), or, where there is no more than a round, rows a grid apart, so that every block has some.
+    constexpr bool cluster = FORM == kCluster8, apart = FORM != kRounds;
+    const size_t row = apart ? (size_t)gridDim.x * kThreads : kThreads, step = (size_t)gridDim.x * kThreads * kUnroll;
+    size_t i = (size_t)blockIdx.x * kThreads * (apart ? 1 : kUnroll) + tid;
     uint4 q[kUnroll], next[kUnroll];
-    load_vectors(vec, i, nvec, q);
+    if (!cluster) load_vectors(vec, i, row, nvec, q);
     for (int v = tid; v < kBins * 8; v += kThreads) reinterpret_cast<uint4*>(table)[v] = make_uint4(0u, 0u, 0u, 0u);
+    if (cluster) {
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+        load_vectors(vec, i, row, nvec, q);
+    }
     __syncthreads();
     for (; i < nvec; i += step) {
-        load_vectors(vec, i + step, nvec, next);
+        load_vectors(vec, i + step, row, nvec, next);
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            if (i + u * kThreads < nvec) count_vector(table, q[u], lane4);
+            if (i + u * row < nvec) count_vector(table, q[u], lane4);
             q[u] = next[u];
         }
     }
     if (blockIdx.x == 0 && tid < 32) {  // the ragged ends: at most 15 + 15 bytes
         const size_t i = tid < 16 ? (size_t)tid : head + nvec * 16 + (tid - 16);
-        if (tid < 16 ? i < head : i < n) count_byte(table, data[i], lane4);
+        if (tid < 16 ? i < head : i < n) count_byte(table, __ldcg(data + i), lane4);
     }
     __syncthreads();
     {
@@ -104,28 +115,30 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) histogram256_kernel(co
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         if (half == 0) sums[bin] = sum;
     }
-    if (CLUSTER) {
-        const cg::cluster_group cluster = cg::this_cluster();
-        cluster.sync();
+    if (cluster) {
+        const cg::cluster_group blocks = cg::this_cluster();
+        blocks.sync();
         constexpr int kShare = kBins / kCluster;  // bins this block adds up over the cluster
-        const int bin = cluster.block_rank() * kShare + tid;
+        const int bin = blocks.block_rank() * kShare + tid;
         if (tid < kShare) {
             unsigned long long sum = 0;
 #pragma unroll
-            for (int b = 0; b < kCluster; ++b) sum += *cluster.map_shared_rank(sums + bin, b);
+            for (int b = 0; b < kCluster; ++b) sum += *blocks.map_shared_rank(sums + bin, b);
             out[bin] = sum;
         }
-        cluster.sync();  // no block leaves while its sums are read
+        blocks.sync();  // no block leaves while its sums are read
     } else {
         __syncthreads();
         cudaGridDependencySynchronize();  // `out` is zero
+        cudaTriggerProgrammaticLaunchCompletion();
         if (tid < kBins && sums[tid]) atomicAdd(out + tid, sums[tid]);
     }
 }
 
-// Starts the counting launch at once: by then everything before this launch in the stream has completed, so
-// the data is there, and only the adding to `out` waits for the zeros.
+// Gets ready while the launch before it ends, and starts the counting launch as soon as that has completed: the data is there then, and
+// only the adding to `out` waits for the zeros (10 MB 7.0 -> 5.2 us a call, 512 MB 87.6 -> 85.9).
 __global__ void __launch_bounds__(kBins) zero_counts_kernel(unsigned long long* out) {
+    cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
     out[threadIdx.x] = 0ull;
 }
@@ -137,19 +150,22 @@ extern "C" int a2a_histogram256(const uint8_t* data, size_t n, int64_t* out, voi
     if (reinterpret_cast<uintptr_t>(out) % 8 != 0) return A2A_ERR_CONFIG;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     unsigned long long* counts = reinterpret_cast<unsigned long long*>(out);
-    cudaLaunchAttribute attr{};
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t launch{};
     launch.blockDim = dim3(kThreads);
     launch.stream = st;
-    launch.attrs = &attr;
+    launch.attrs = attr;
     launch.numAttrs = 1;
     cudaError_t e;
     if (n <= kClusterBytes) {
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = kCluster;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = kCluster;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        launch.numAttrs = 2;
         launch.gridDim = dim3(kCluster);
-        e = cudaLaunchKernelEx(&launch, histogram256_kernel<true>, data, n, counts);
+        e = cudaLaunchKernelEx(&launch, histogram256_kernel<kCluster8>, data, n, counts);
         return e == cudaSuccess ? A2A_OK : -(int)e;
     }
     int dev = 0, sms = 0;
@@ -159,12 +175,12 @@ extern "C" int a2a_histogram256(const uint8_t* data, size_t n, int64_t* out, voi
     zero.gridDim = dim3(1);
     zero.blockDim = dim3(kBins);
     zero.stream = st;
+    zero.attrs = attr;
+    zero.numAttrs = 1;
     if ((e = cudaLaunchKernelEx(&zero, zero_counts_kernel, counts)) != cudaSuccess) return -(int)e;
     const size_t want = (n / 16 + kThreads - 1) / kThreads;
     const size_t room = (size_t)sms * (n < kFullBytes ? 1 : kBlocksPerSm);
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
     launch.gridDim = dim3((unsigned)(want < room ? want : room));
-    e = cudaLaunchKernelEx(&launch, histogram256_kernel<false>, data, n, counts);
+    e = cudaLaunchKernelEx(&launch, n <= (size_t)sms * kSpreadBytesPerSm ? histogram256_kernel<kSpread> : histogram256_kernel<kRounds>, data, n, counts);
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }

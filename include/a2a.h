@@ -308,7 +308,7 @@ int a2a_route_noalloc(const int32_t* topk_idx, int num_tokens, int num_experts, 
  * data[0..n) equal to b, for b = 0..255 -- torch.bincount(data, minlength=256) on uint8 input
  * (reference.py:6-19; native entry of its submission: submission_v1.py:20-113).  `data` is device
  * memory (any alignment, any n >= 0), `out` 256 int64 in device memory, overwritten.  Needs no
- * context; runs on the current device; enqueues a 2 KB memset and one kernel on `stream`. */
+ * context; runs on the current device; enqueues one kernel (up to 256 KB) or two on `stream`. */
 int a2a_histogram256(const uint8_t* data, size_t n, int64_t* out, void* stream);
 
 /* Read the first error recorded by a kernel since the last a2a_status_clear.  Waits for

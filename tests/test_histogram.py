@@ -126,3 +126,28 @@ def test_arguments_are_checked():
     lib = _lib.load()
     assert lib.a2a_histogram256(None, 16, C.c_void_p(out.data_ptr()), None) == _lib.A2A_ERR_CONFIG
     assert lib.a2a_histogram256(C.c_void_p(data.data_ptr()), 16, None, None) == _lib.A2A_ERR_CONFIG
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [2048, 200000, 148 * 4096, 148 * 4096 + 1, 5 << 20])
+def test_calls_that_overlap_read_what_the_stream_wrote(size):
+    """A call may be resident while the launch before it still writes its data -- a copy, or the call before, whose counts are
+    the next call's bytes; and while the call before it still adds to the same output."""
+    from gpu_mode_kernels_b200.histogram import histogram256
+
+    g = torch.Generator().manual_seed(size)
+    sets = [torch.randint(0, 256, (size,), dtype=torch.uint8, generator=g) for _ in range(3)]
+    want = [HO.ref_histogram(s) for s in sets]
+    want_of_counts = [HO.ref_histogram(w.view(torch.uint8)) for w in want]
+    on_gpu, data = [s.to("cuda:0") for s in sets], torch.empty(size, dtype=torch.uint8, device="cuda:0")
+    out = torch.empty(256, dtype=torch.int64, device="cuda:0")
+    got = []
+    for i in range(60):
+        data.copy_(on_gpu[i % 3])
+        histogram256(data, out)
+        chained = histogram256(out.view(torch.uint8), torch.empty_like(out))
+        got.append((out.clone(), chained))
+        histogram256(on_gpu[(i + 1) % 3], out)
+    torch.cuda.synchronize()
+    for i, (counts, chained) in enumerate(got):
+        assert torch.equal(counts.cpu(), want[i % 3]) and torch.equal(chained.cpu(), want_of_counts[i % 3])
