@@ -472,19 +472,21 @@ int launch_near_rows(a2a_ctx* const* cs, NearParams<N>& g, bool push, cudaStream
 // blocks starts after the first (headline 13.2 us).
 // Rows in host memory: half an SM's worth of warps fills the link, and more only get in each other's way
 // (3.7 MB read and as much written by 74 / 148 / 296 blocks: 100 / 107 / 118 us).
-// Many tokens in rows that outweigh a second launch: slots first, then rows in blocks of one item a warp, one vector a
-// lane, or two where fewer than six stores follow each load.  Back to back, the one launch and the two, at 2048 tokens:
-// of 7168, top-8 61.6 / 57.0 us; of 4096, top-8 37.8 / 37.5; of 2048, top-6 19.0 / 16.9, top-2 12.1 / 11.4; of 2880, top-4
-// 18.9 / 18.7; of 6144, top-2 21.6 / 23.1.  At 1280: 39.5 / 39.0, 23.2 / 24.2, 13.3 / 11.7, 9.1 / 9.0, 12.8 / 12.5, 14.2 / 15.0; at
-// 1024 31.8 / 31.0, 18.7 / 19.4, 11.0 / 10.1, 7.9 / 7.6, 10.9 / 11.5, 12.1 / 12.1; at 400 13.0 / 13.3, 9.9 / 10.4, 7.2 / 7.4.
-constexpr int kSoloManyTokens = 1280;
-constexpr long long kSoloManyBytes = 8LL << 20;
+// Many tokens, or rows that outweigh a second launch: the routing of a group of one and then its rows (a2a_near.cuh).  Back to back,
+// us a call, the one launch and the two, by MB of expert rows: top-8 of 7168, 400 tokens 13.0 / 13.0 (46), 512 16.4 / 15.7 (59), 1000
+// 30.9 / 28.0; top-8 of 4096, 512 11.3 / 11.6 (34), 640 13.6 / 12.9 (42), 1279 23.0 / 21.7; top-2 of 6144, 640 8.9 / 8.9 (16), 800 10.2 / 9.8
+// (20), 1279 14.2 / 13.9; top-6 of 2048, 640 8.8 / 8.8 (16), 800 9.7 / 9.3 (20), 1279 13.5 / 12.0; top-4 of 2880, 640 8.2 / 9.0 (15), 800
+// 9.7 / 9.4 (18), 1279 12.7 / 12.1; below 16 MB the host's two launches, 6.5, are what a call waits for until the counting in
+// every block of the one launch does: top-2 of 512, 800 6.5 / 6.3, 2048 10.5 / 7.4, of 2048, 800 7.2 / 7.0, 2048 11.4 / 10.4.
+bool solo_two_launches(const a2a_ctx* c) {
+    const long long mb = (long long)c->cur_tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 >> 20;
+    return mb >= 40 || (mb >= 16 && c->cur_tokens >= 800) || (mb >= 4 && c->cur_tokens >= 1280);
+}
+
 int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = host_rows ? c->num_sms / 2 : 2LL * c->num_sms;
     const long long two = c->cur_tokens * ((nvec + 63) / 64), one = c->cur_tokens * ((nvec + 31) / 32);
-    const int K = c->cfg.experts_per_token;
-    if (!host_rows && c->p.trace == nullptr && c->cur_tokens >= kSoloManyTokens &&
-        (long long)c->cur_tokens * K * c->cfg.hidden_dim * 2 >= kSoloManyBytes) {
+    if (!host_rows && c->p.trace == nullptr && solo_two_launches(c)) {
         NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, kOutputWhole, /*handed_on=*/1};
         const int rc = launch_near_route(&c, g, st);
         return rc != A2A_OK ? rc : launch_near_rows(&c, g, /*push=*/false, st);

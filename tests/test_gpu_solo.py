@@ -111,6 +111,31 @@ def test_many_tokens_match_the_stepped_roles(E, K, H, T, n, dtype, payload):
         world.close()
 
 
+@pytest.mark.parametrize("E,K,H,T,launches", [
+    (64, 8, 4096, 640, 2), (64, 8, 4096, 639, 1),    # 40 MB of expert rows, and a token less
+    (32, 6, 2048, 800, 2), (32, 6, 2048, 799, 1),    # 800 tokens of more than 16 MB, and 799
+    (16, 4, 2624, 800, 2), (16, 4, 2616, 800, 1),    # just above 16 MB, and below
+    (8, 2, 824, 1280, 2), (8, 2, 816, 1280, 1),      # 1280 tokens of 4 MB, and of less
+])
+def test_where_a_call_takes_two_launches(E, K, H, T, launches):
+    cfg, rd, _, _ = pkg.generate_input(E, K, H, T, seed=14, rank=0, world_size=1)
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push", timeout_ms=500)
+    world = LocalWorld(cfg, 1, payload="dedup", schedule="pipelined", combine="push")
+    try:
+        d = rd.to(DEV)
+        before = ctx.launches
+        y = ctx.forward(d.x, d.indices, d.weights)
+        assert ctx.launches == before + launches
+        ref = world.forward_pipelined([d])[0]
+        got, want = ctx.route_tables() + ctx.export_dispatch(), world.ctxs[0].route_tables() + world.ctxs[0].export_dispatch()
+        torch.cuda.synchronize()
+        ctx.check()
+        assert torch.equal(bits(ref), bits(y)) and all(torch.equal(a, b) for a, b in zip(got, want))
+    finally:
+        ctx.close()
+        world.close()
+
+
 def test_dropped_pairs_match_the_stepped_roles_and_phases_can_follow():
     """Indices out of range and repeated, the repeats also across the eight indices the kernel loads
     together and in tokens before the reading block's own; then a combine called on its own, which
