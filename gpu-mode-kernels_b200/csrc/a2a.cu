@@ -90,6 +90,8 @@ struct a2a_ctx {
     bool recorded;          // roles 1 and 2 can follow: the call was begun by role 0, or by the one launch of several ranks
     bool near;              // ... by role 0 of a group on this GPU: rows stay where they are
     bool whole;             // ... and role 1 of the group has written the outputs too
+    bool listed;            // every pair's place is in p.pairs
+    bool backwards;         // the last launch that wrote the expert rows of the group began with the last tokens
     const void* near_x[A2A_MAX_WORLD];  // input rows of every rank in this call
     const uint2* near_pairs[A2A_MAX_WORLD];
     int near_T[A2A_MAX_WORLD];
@@ -328,11 +330,25 @@ const void* rows_fn(const a2a_ctx* c, bool narrow) {
     return bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_DEDUP, PUSH, N>(narrow) : rows_fn<__half, A2A_PAYLOAD_DEDUP, PUSH, N>(narrow);
 }
 
-// the combine of ranks on one GPU
-const void* near_combine_fn(const a2a_ctx* c, bool push) {
-    if (c->cfg.dtype == A2A_DTYPE_BF16)
-        return push ? (const void*)near_combine_kernel<__nv_bfloat16, true> : (const void*)near_combine_kernel<__nv_bfloat16, false>;
-    return push ? (const void*)near_combine_kernel<__half, true> : (const void*)near_combine_kernel<__half, false>;
+// the kernels of the phases and the combine of ranks on one GPU: element type, U vectors a lane
+template <typename T, int U>
+const void* near_combine_fn(bool push) {
+    return push ? (const void*)near_combine_kernel<T, true, U> : (const void*)near_combine_kernel<T, false, U>;
+}
+template <typename T, int P>
+const void* near_wire_fn(bool scale) {
+    return scale ? (const void*)near_expert_kernel<T, P, true, true> : (const void*)near_expert_kernel<T, P, true, false>;
+}
+template <typename T>
+const void* near_expert_fn(int payload, bool fanout, bool scale) {
+    if (fanout && payload == A2A_PAYLOAD_FP8) return near_wire_fn<T, A2A_PAYLOAD_FP8>(scale);
+    if (fanout && payload == A2A_PAYLOAD_DEDUP) return near_wire_fn<T, A2A_PAYLOAD_DEDUP>(scale);
+    return fanout ? (const void*)near_expert_kernel<T, A2A_PAYLOAD_DIRECT, true, true> : (const void*)near_expert_kernel<T, A2A_PAYLOAD_DIRECT, false, true>;
+}
+template <typename T, int U>
+const void* near_dispatch_fn(int payload) {
+    if (payload == A2A_PAYLOAD_FP8) return (const void*)near_dispatch_kernel<T, A2A_PAYLOAD_FP8, U>;
+    return payload == A2A_PAYLOAD_DEDUP ? (const void*)near_dispatch_kernel<T, A2A_PAYLOAD_DEDUP, U> : (const void*)near_dispatch_kernel<T, A2A_PAYLOAD_DIRECT, U>;
 }
 
 PhaseFn combine_fn(const a2a_ctx* c) {
@@ -340,13 +356,11 @@ PhaseFn combine_fn(const a2a_ctx* c) {
     return {combine_kernel<__half, RankParams>, combine_kernel<__half, GroupParams>};
 }
 
-// A launch that, with `overlap`, may get ready while the one before it in the stream ends; its kernel begins with
-// begin_after_previous().
-cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** args, cudaStream_t st, bool overlap = true,
-                                  int threads = kThreads) {
+// A launch that may get ready while the one before it in the stream ends; its kernel begins with begin_after_previous().
+cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** args, cudaStream_t st, int threads = kThreads) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
+    attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t launch{};
     launch.gridDim = dim3(grid);
     launch.blockDim = dim3(threads);
@@ -357,25 +371,13 @@ cudaError_t launch_after_previous(const void* fn, int grid, int smem, void** arg
     return cudaLaunchKernelExC(&launch, fn, args);
 }
 
-// The one launch of a single rank and the roles of ranks on one GPU are grids that stay for the whole launch.  Blocks of
-// theirs that get ready early take the places that happen to be free, two on one SM and none on the next, which a long launch
-// pays for: expert rows of 235 MB, eight ranks 133.7 us a call without and 135.9 with, PULL, 183 MB 91 / 101, one rank
-// 63.4 / 64.2.  A short one gains the latency of its launch: 50.3 MB, eight ranks 45.1 / 44.4; 33 MB, one rank 10.8 / 9.6;
-// 54.5 MB 16.41 / 16.54.  The line lies between those last two sizes.
-// The other launches overlap at any size, and gain: phases of eight ranks, 183 MB, direct, 147.2 us a call without and 144.8 with
-// (dedup 199.7 / 199.6, 59 MB, fp8, 72.1 / 69.3), of one rank in launches of their own, 80 MB, 82.3 / 78.5 (direct 94.5 / 91.2);
-// roles of two ranks one by one, 59 MB each, 105.7 / 102.2; many tokens of one rank, 235 MB, 58.0 to 59.7 / 57.2.
-constexpr long long kOverlapBytes = 50LL << 20;
-bool overlaps(const a2a_ctx* c, long long tokens) { return tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 <= kOverlapBytes; }
-
-int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false, bool overlap = true,
-           int threads = kThreads) {
+int launch(a2a_ctx* c, const void* fn, int grid, int smem, cudaStream_t st, bool cooperative = false) {
     static_assert(sizeof(RankParams) == sizeof(DevParams), "a kernel of one rank takes either");
     DevParams p = call_params(c);
     if (p.trace != nullptr && grid > kTraceBlocks) p.trace = nullptr;
     if (p.trace != nullptr) c->last_grid = grid;
     void* args[] = {&p};
-    cudaError_t e = !cooperative ? launch_after_previous(fn, grid, smem, args, st, overlap, threads)
+    cudaError_t e = !cooperative ? launch_after_previous(fn, grid, smem, args, st)
         : c->plain_launch ? cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, smem, st)
                           : cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st);
     c->launches++;
@@ -407,29 +409,35 @@ int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int s
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
-// What a launch for `n` ranks on one GPU is told.  The call's rows and pairs are those the contexts hold of every rank.
-NearGroup near_params(a2a_ctx* const* cs, int n) {
+// What a launch for a group on one GPU is told, or for one rank of it in a call that the group began together.
+NearGroup near_params(a2a_ctx* const* cs, int n, bool handed_on = false) {
     NearGroup g{};
     for (int r = 0; r < n; ++r) {
         g.p[r] = call_params(cs[r]);
         g.p[r].local = 1;
         if (n > 1) g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
+        g.x[r] = cs[r]->p.x;
+        g.pairs[r] = cs[r]->p.pairs;
+        g.T[r] = cs[r]->cur_tokens;
     }
-    memcpy(g.x, cs[0]->near_x, sizeof(g.x));
-    memcpy(g.pairs, cs[0]->near_pairs, sizeof(g.pairs));
-    memcpy(g.T, cs[0]->near_T, sizeof(g.T));
+    if (n == 1) {
+        memcpy(g.x, cs[0]->near_x, sizeof(g.x));
+        memcpy(g.pairs, cs[0]->near_pairs, sizeof(g.pairs));
+        memcpy(g.T, cs[0]->near_T, sizeof(g.T));
+    }
     g.n = n;
+    g.handed_on = handed_on;
     return g;
 }
 
 template <int N>
-int launch_near(a2a_ctx* const* cs, NearParams<N>& g, const void* fn, int blocks, int smem, cudaStream_t st, bool overlap = true,
-                int threads = kThreads, int words = 0) {
+int launch_near(a2a_ctx* const* cs, NearParams<N>& g, const void* fn, int blocks, int smem, cudaStream_t st, int threads = kThreads,
+                int arg = 0) {
     if (blocks > kTraceBlocks) g.p[0].trace = nullptr;
     if (g.p[0].trace != nullptr) cs[0]->last_grid = blocks;
     for (int r = 0; r < g.n; ++r) cs[r]->launches++;
-    void* args[] = {&g, &words};
-    const cudaError_t e = launch_after_previous(fn, blocks, smem, args, st, overlap, threads);
+    void* args[] = {&g, &arg};
+    const cudaError_t e = launch_after_previous(fn, blocks, smem, args, st, threads);
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
@@ -442,7 +450,7 @@ int launch_near_route(a2a_ctx* const* cs, NearParams<N>& g, cudaStream_t st) {
     for (int r = 0; r < g.n; ++r) most = cs[r]->cur_tokens > most ? cs[r]->cur_tokens : most;
     const int words = most > 8192 ? 8 : most > 1024 ? 2 : 1, nb = (most + 32 * words - 1) / (32 * words);
     return launch_near(cs, g, (const void*)near_route_kernel<N>, g.n * nb, (int)near_route_smem(words, cs[0]->cfg.num_experts, cs[0]->cfg.experts_per_token),
-                       st, true, kRouteThreads, words);
+                       st, kRouteThreads, words);
 }
 
 // Role 1: a warp per 1 KB of a token's row, three blocks per SM, or per 512 bytes where that would be too few rounds of blocks:
@@ -462,6 +470,68 @@ int launch_near_rows(a2a_ctx* const* cs, NearParams<N>& g, bool push, cudaStream
     if constexpr (N > 1)
         if (push) fn = rows_fn<true, N>(c, !many);
     return launch_near(cs, g, fn, (int)blocks, 0, st);
+}
+
+// Blocks of a launch in which each warp has one item, `U` vectors a lane of a token's row.
+template <int N>
+int near_blocks(const a2a_ctx* c, const NearParams<N>& g, int U) {
+    const long long chunks = (c->cfg.hidden_dim / 8 + 32 * U - 1) / (32 * U);
+    long long items = 0;
+    for (int s = 0; s < c->cfg.world_size; ++s)
+        if (g.n > 1 || c->cfg.world_size == 1 || s == c->cfg.rank) items += g.T[s] * chunks;
+    const long long blocks = (items + kThreads / 32 - 1) / (kThreads / 32);
+    return blocks < 1 ? 1 : (int)blocks;
+}
+
+constexpr int kBothFlags = 1 << kFlagDispatch | 1 << kFlagExpert;
+
+// Where the expert rows are more than the L2 keeps, a phase begins with those that the one before it wrote last: eight ranks of 200
+// tokens of 7168, top-8 of 256 experts, 183 MB, staged 171 -> 161 us a call, direct 132 -> 131; 128 tokens, 117 MB, 81.4 / 80.6.  Below 64 MB
+// no difference.
+bool beyond_l2(const a2a_ctx* c, const NearGroup& g) {
+    long long tokens = 0;
+    for (int s = 0; s < c->cfg.world_size; ++s) tokens += g.T[s];
+    return tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 >= 64LL << 20;
+}
+
+// The combine: 512 bytes of a token's output a warp, 1 KB where fewer than six rows are added up (a call by
+// phases, us, 512 bytes / 1 KB: four ranks of 200 tokens of 6144, top-2, 26.2 / 25.6; two of 256 of 7168, top-8, 38.4 / 39.3).
+int launch_near_combine(a2a_ctx* const* cs, NearGroup& g, bool push, cudaStream_t st) {
+    g.backwards = !cs[0]->backwards && beyond_l2(cs[0], g);
+    const bool bf = cs[0]->cfg.dtype == A2A_DTYPE_BF16, wide = cs[0]->cfg.experts_per_token < 6;
+    const void* fn = wide ? (bf ? near_combine_fn<__nv_bfloat16, 2>(push) : near_combine_fn<__half, 2>(push))
+                          : (bf ? near_combine_fn<__nv_bfloat16, 1>(push) : near_combine_fn<__half, 1>(push));
+    return launch_near(cs, g, fn, near_blocks(cs[0], g, wide ? 2 : 1), 0, st);
+}
+
+// RECV, EXPERT and RECV_EXPERT: 512 bytes a warp (1 KB: two ranks of 256 tokens of 7168 39.2 us a call by phases instead of 38.4).
+int launch_near_expert(a2a_ctx* const* cs, NearGroup& g, bool fanout, bool scale, cudaStream_t st) {
+    const int payload = cs[0]->cfg.payload;
+    if (fanout && !scale && payload == A2A_PAYLOAD_DIRECT)  // the rows are in place
+        return launch_near(cs, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, 1 << kFlagDispatch);
+    const bool bf = cs[0]->cfg.dtype == A2A_DTYPE_BF16;
+    g.backwards = !fanout && !cs[0]->backwards && beyond_l2(cs[0], g);
+    for (int r = 0; r < g.n; ++r) cs[r]->backwards = g.backwards;
+    return launch_near(cs, g, bf ? near_expert_fn<__nv_bfloat16>(payload, fanout, scale) : near_expert_fn<__half>(payload, fanout, scale),
+                       near_blocks(cs[0], g, 1), 0, st);
+}
+
+// SEND: as many blocks as are resident together, three per SM, each of which counts the experts of the tokens before its own; a second round
+// of them costs 3 us (phases of two ranks, 256 tokens of 2048, 15.9 us a call with three, 19.3 with six).  1 KB a warp where every warp
+// has that much, else 512 bytes.
+int launch_near_dispatch(a2a_ctx* const* cs, NearGroup& g, cudaStream_t st) {
+    const a2a_ctx* c = cs[0];
+    int most = 0;
+    for (int r = 0; r < g.n; ++r) most = cs[r]->cur_tokens > most ? cs[r]->cur_tokens : most;
+    const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = (long long)c->num_sms * 3 / g.n;
+    const long long two = most * ((nvec + 63) / 64), one = most * ((nvec + 31) / 32);
+    const bool bf = c->cfg.dtype == A2A_DTYPE_BF16, wide = two >= cap * warps;
+    long long blocks = ((wide ? two : one) + warps - 1) / warps;
+    if (blocks > cap) blocks = cap;
+    if (blocks < 1) blocks = 1;
+    const void* fn = wide ? (bf ? near_dispatch_fn<__nv_bfloat16, 2>(c->cfg.payload) : near_dispatch_fn<__half, 2>(c->cfg.payload))
+                          : (bf ? near_dispatch_fn<__nv_bfloat16, 1>(c->cfg.payload) : near_dispatch_fn<__half, 1>(c->cfg.payload));
+    return launch_near(cs, g, fn, g.n * (int)blocks, 0, st);
 }
 
 // The forward of one rank.  A warp's item is one or two 16-byte vectors per lane of a token's row: two
@@ -487,7 +557,7 @@ int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = host_rows ? c->num_sms / 2 : 2LL * c->num_sms;
     const long long two = c->cur_tokens * ((nvec + 63) / 64), one = c->cur_tokens * ((nvec + 31) / 32);
     if (!host_rows && c->p.trace == nullptr && solo_two_launches(c)) {
-        NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, kOutputWhole, /*handed_on=*/1};
+        NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, /*backwards=*/0, kOutputWhole, /*handed_on=*/1};
         const int rc = launch_near_route(&c, g, st);
         return rc != A2A_OK ? rc : launch_near_rows(&c, g, /*push=*/false, st);
     }
@@ -495,8 +565,7 @@ int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    return launch(c, (const void*)(wide ? solo_fn<2>(c) : solo_fn<1>(c)), (int)blocks, 0, st,
-                  /*cooperative=*/false, overlaps(c, c->cur_tokens));
+    return launch(c, (const void*)(wide ? solo_fn<2>(c) : solo_fn<1>(c)), (int)blocks, 0, st);
 }
 
 // The device address of host memory that kernels can reach -- pinned, all `bytes` of it in one allocation or
@@ -542,7 +611,7 @@ int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
     c->cur_tokens = T;
     c->p.idx = idx;
     c->routed = true;
-    c->sent = c->recorded = c->near = c->whole = false;
+    c->sent = c->recorded = c->near = c->whole = c->listed = c->backwards = false;
     return A2A_OK;
 }
 
@@ -568,7 +637,16 @@ int grid_for_ranks(const a2a_ctx* c, int n, long long items, int per_sm) {
     return g < share ? g : (share < 1 ? 1 : share);
 }
 
-int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st) {
+bool any_traced(a2a_ctx* const* cs, int n) {
+    for (int r = 0; r < n; ++r)
+        if (cs[r]->p.trace != nullptr) return true;
+    return false;
+}
+
+// All ranks of a group on one GPU in a launch of a2a_near.cuh?
+bool near_phases(a2a_ctx* const* cs, int n) { return n > 1 && cs[0]->p.chunks == 1 && !any_traced(cs, n); }
+
+int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st, bool handed_on = false) {
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->routed || cs[r]->sent) return A2A_ERR_STATE;
         if (cs[r]->cur_tokens > 0 && x[r] == nullptr) return A2A_ERR_CONFIG;
@@ -576,15 +654,21 @@ int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st) {
     }
     for (int r = 0; r < n; ++r) cs[r]->p.x = x[r];
     const a2a_ctx* c = cs[0];
+    if (near_phases(cs, n)) {
+        NearGroup g = near_params(cs, n, handed_on);
+        const int rc = launch_near_dispatch(cs, g, st);
+        if (rc == A2A_OK)
+            for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->listed = true;
+        return rc;
+    }
     // a warp per 2 KB of a pair's row (DIRECT) or 512 bytes of a token's, no more blocks than four per SM, each of which
-    // builds the routing tables (eight ranks, 200 tokens of 7168 by phases, direct: 145 us a call, 148 with three and 152
-    // with six; dedup 197, 200, 194; four ranks, 117 tokens of 4096, direct: 35.7, 37.2, 39.4)
+    // builds the routing tables
     const bool direct = c->cfg.payload == A2A_PAYLOAD_DIRECT;
     const long long T = most_tokens(cs, n), nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32;
     const long long items = direct ? T * c->cfg.experts_per_token * ((nvec + 127) / 128) : T * ((nvec + 31) / 32);
     const int rc = launch_ranks(cs, n, select_tp<SendSel>(c), grid_for_ranks(c, n, (items + warps - 1) / warps, 4), c->smem_bytes, st);
     if (rc == A2A_OK)
-        for (int r = 0; r < n; ++r) cs[r]->sent = true;
+        for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->listed = true;
     return rc;
 }
 
@@ -596,28 +680,20 @@ int expert_grid(const a2a_ctx* c, int n, int per_sm) {
     return g < ws ? ws : g;
 }
 
-int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st) {
-    for (int r = 0; r < n; ++r)
+int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st, bool handed_on = false) {
+    bool listed = true;
+    for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent) return A2A_ERR_STATE;
+        listed = listed && cs[r]->listed;
+    }
+    if (listed && near_phases(cs, n)) {
+        NearGroup g = near_params(cs, n, handed_on);
+        return launch_near_expert(cs, g, fanout, scale, st);
+    }
     return launch_ranks(cs, n, select_tp<ExpertSel>(cs[0], wait, fanout, scale, publish), grid, cs[0]->smem_bytes, st);
 }
 
-bool any_traced(a2a_ctx* const* cs, int n) {
-    for (int r = 0; r < n; ++r)
-        if (cs[r]->p.trace != nullptr) return true;
-    return false;
-}
-
-constexpr long long kNearCombineBytes = 16LL << 20;
-int launch_near_combine(a2a_ctx* const* cs, int n, bool push, bool every_rank, cudaStream_t st) {
-    NearGroup g = near_params(cs, n);
-    g.every_rank = every_rank ? 1 : 0;
-    long long tokens = 0;
-    for (int r = 0; r < n; ++r) tokens += cs[r]->cur_tokens;
-    return launch_near(cs, g, near_combine_fn(cs[0], push), 2 * cs[0]->num_sms, 0, st, overlaps(cs[0], tokens));
-}
-
-int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st) {
+int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st, bool handed_on = false) {
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent) return A2A_ERR_STATE;
         if (cs[r]->cur_tokens > 0 && (w[r] == nullptr || y[r] == nullptr)) return A2A_ERR_CONFIG;
@@ -628,13 +704,12 @@ int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y,
         cs[r]->p.y = y[r];
     }
     const a2a_ctx* c = cs[0];
-    // Many rows of a group: the combine of a2a_near.cuh, which looks up pairs two items ahead and shares the tokens of all
-    // ranks out among all blocks.  Calls by phases: 183 MB of expert rows 161 -> 145 us, 58 MB 90.2 -> 87.4, 31 MB 36.2 -> 35.7;
-    // 7 MB 27.1 -> 28.1, 1 MB 20.0 -> 21.7: more to set up.
-    long long tokens = 0;
-    for (int r = 0; r < n; ++r) tokens += cs[r]->cur_tokens;
-    if (n > 1 && c->p.chunks == 1 && !any_traced(cs, n) && tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 >= kNearCombineBytes)
-        return launch_near_combine(cs, n, /*push=*/false, /*every_rank=*/false, st);
+    bool listed = true;
+    for (int r = 0; r < n; ++r) listed = listed && cs[r]->listed;
+    if (listed && near_phases(cs, n)) {
+        NearGroup g = near_params(cs, n, handed_on);
+        return launch_near_combine(cs, g, /*push=*/false, st);
+    }
     const int nseg = (c->cfg.hidden_dim / 8 + 63) / 64;  // a warp per (token, 1 KB segment)
     const long long warps = (long long)most_tokens(cs, n) * nseg;
     return launch_ranks(cs, n, combine_fn(c), grid_for_ranks(c, n, (warps + kThreads / 32 - 1) / (kThreads / 32), 8), 0, st);
@@ -681,11 +756,10 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
                 cs[r]->near_pairs[s] = cs[s]->p.pairs;
                 cs[r]->near_T[s] = calls[s].num_tokens;
             }
-        NearGroup g = near_params(cs, n);
-        g.handed_on = handed_on;
+        NearGroup g = near_params(cs, n, handed_on);
         rc = launch_near_route(cs, g, st);
         if (rc == A2A_OK)
-            for (int r = 0; r < n; ++r) cs[r]->near = true;
+            for (int r = 0; r < n; ++r) cs[r]->near = cs[r]->listed = true;
     }
     if (rc == A2A_OK)
         for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->recorded = true;
@@ -717,8 +791,7 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool hand
             // Begun rank by rank: one launch, in which each rank has its share of two blocks per SM.  Role 0 of eight ranks one by
             // one and these two, 4 tokens of 2048 146 us (294 with a launch for each rank), 128 of 7168 222 (404).
             return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), blocks / n, push_smem, st);
-        NearGroup g = near_params(cs, n);
-        g.handed_on = handed_on;
+        NearGroup g = near_params(cs, n, handed_on);
         if (role == 1) {
             a2a_call calls[A2A_MAX_WORLD];
             for (int r = 0; r < n; ++r) calls[r] = {g.x[r], nullptr, nullptr, cs[r]->p.y, g.T[r]};
@@ -731,8 +804,9 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool hand
             return rc;
         }
         // a role 2 is through when every rank is through with this call, whoever's rows its tokens want
-        if (whole) return launch_near(cs, g, (const void*)near_finish_kernel, 1, 0, st, true, A2A_MAX_WORLD * A2A_MAX_WORLD);
-        return launch_near_combine(cs, n, push, /*every_rank=*/true, st);
+        if (whole) return launch_near(cs, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, kBothFlags);
+        g.every_rank = 1;
+        return launch_near_combine(cs, g, push, st);
     }
     for (int r = 0; r < n; ++r) {
         int rc;
@@ -745,9 +819,11 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool hand
             rc = launch_near_rows(cs + r, g, push, st);
         } else if (cs[r]->whole) {
             NearGroup g = near_params(cs + r, 1);
-            rc = launch_near(cs + r, g, (const void*)near_finish_kernel, 1, 0, st, true, A2A_MAX_WORLD * A2A_MAX_WORLD);
+            rc = launch_near(cs + r, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, kBothFlags);
         } else {
-            rc = launch_near_combine(cs + r, 1, push, /*every_rank=*/true, st);
+            NearGroup g = near_params(cs + r, 1);
+            g.every_rank = 1;
+            rc = launch_near_combine(cs + r, g, push, st);
         }
         if (rc != A2A_OK) return rc;
     }
@@ -807,7 +883,7 @@ int check_group(a2a_ctx* const* group) {
 }
 
 // One phase of all ranks of a group that check_group has passed.
-int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStream_t st) {
+int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStream_t st, bool handed_on = false) {
     const a2a_ctx* c = group[0];
     const int n = c->cfg.world_size;
     const bool pipe_phase = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_PIPE_EXPERT || phase == A2A_GROUP_PIPE_COMBINE;
@@ -834,13 +910,13 @@ int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStr
                 if (!rows_aligned(x[r])) return A2A_ERR_CONFIG;
             }
             for (int r = 0; r < n; ++r) begin_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
-            return do_send(group, n, x, st);
+            return do_send(group, n, x, st, handed_on);
         case A2A_GROUP_RECV:
             return do_expert(group, n, true, true, false, false,
-                             c->cfg.payload == A2A_PAYLOAD_DIRECT ? n : expert_grid(c, n, 4), st);
-        case A2A_GROUP_EXPERT: return do_expert(group, n, false, false, true, true, expert_grid(c, n, 4), st);
-        case A2A_GROUP_RECV_EXPERT: return do_expert(group, n, true, true, true, true, expert_grid(c, n, 4), st);
-        case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st);
+                             c->cfg.payload == A2A_PAYLOAD_DIRECT ? n : expert_grid(c, n, 4), st, handed_on);
+        case A2A_GROUP_EXPERT: return do_expert(group, n, false, false, true, true, expert_grid(c, n, 4), st, handed_on);
+        case A2A_GROUP_RECV_EXPERT: return do_expert(group, n, true, true, true, true, expert_grid(c, n, 4), st, handed_on);
+        case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st, handed_on);
         default: return A2A_ERR_CONFIG;
     }
 }
@@ -1287,7 +1363,10 @@ int a2a_group_steps(a2a_ctx* const* group, const int32_t* phases, int num_phases
         for (; rc == A2A_OK && ++*done < 3;) rc = do_pipe_rest(group, n, *done, st, /*handed_on=*/true);
         return rc;
     }
-    for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK) rc = group_phase(group, phases[*done], calls, st);
+    static const int32_t four[] = {A2A_GROUP_SEND, A2A_GROUP_RECV, A2A_GROUP_EXPERT, A2A_GROUP_COMBINE}, three[] = {A2A_GROUP_SEND, A2A_GROUP_RECV_EXPERT, A2A_GROUP_COMBINE};
+    const bool handed_on = near_phases(group, n) && ((num_phases == 4 && memcmp(phases, four, sizeof(four)) == 0) ||
+                                                     (num_phases == 3 && memcmp(phases, three, sizeof(three)) == 0));
+    for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK) rc = group_phase(group, phases[*done], calls, st, handed_on);
     return rc;
 }
 

@@ -96,7 +96,6 @@ struct DevParams {
     long long timeout_ns;
     // local scratch of this rank
     int* slot;              // [T_max*K] slot of pair (t,k) inside slab (expert, this rank), -1 = dropped
-    uint2* pairs;           // [T_max*K] the same pairs as the kernels of ranks on one GPU read them (a2a_near.cuh)
     int* send_counts;       // [E]
     uint32_t* tickets;      // [2][kMaxChunks] block-arrival counters, one per publishing phase and chunk
     uint32_t* ptickets;     // [2][A2A_MAX_WORLD] pipelined schedule: arrivals per destination / per source
@@ -108,6 +107,7 @@ struct DevParams {
     const void* x;
     const float* w;
     void* y;
+    uint2* pairs;           // local scratch too, [T_max*K]: the pairs of `slot` by place (kNoPair, pair_place)
 };
 
 // The ranks one launch serves: one, or, where a whole group lives on this GPU, all `n` of them: block i works
@@ -137,6 +137,17 @@ struct GroupParams {
 __device__ __forceinline__ void begin_after_previous() {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
+}
+
+// A (token, k) pair as the kernels of ranks on one GPU read it: where its slab row lies, as (rank << 28 | row of that rank's slabs),
+// and, in a pipelined call, its weight.
+constexpr unsigned kNoPair = 0xffffffffu, kPairRow = 0x0fffffffu;
+static_assert((long long)A2A_MAX_EXPERTS * 65535 < 1 << 28 && A2A_MAX_WORLD <= 8, "a slab row fits 28 bits, a rank three");
+
+// Pair (t, k) of rank p with slot j of expert e.
+__device__ __forceinline__ unsigned pair_place(const DevParams& p, int e, int j) {
+    const int d = e / p.L;
+    return (unsigned)d << 28 | (unsigned)(((e - d * p.L) * p.ws + p.rank) * p.T_max + j);
 }
 
 __device__ __forceinline__ long long global_ns() {

@@ -177,12 +177,14 @@ __device__ __forceinline__ void send_staged(const DevParams& p, const BlockSmem&
         if (lane < K) {
             const int e = s.idx[t * K + lane];
             const int j = pair_slot(p, s, t, lane, e);
-            if (v0 == 0) p.slot[(size_t)t * K + lane] = j;
+            const unsigned place = j >= 0 ? pair_place(p, e, j) : kNoPair;
+            if (v0 == 0) {
+                p.slot[(size_t)t * K + lane] = j;
+                p.pairs[(size_t)t * K + lane] = make_uint2(place, 0u);
+            }
             if (j >= 0) {
-                const int d = e / p.L;
-                want = 1u << d;
-                if (v0 == 0)
-                    reinterpret_cast<int*>(p.peer[d] + p.off_meta)[((size_t)(e - d * p.L) * p.ws + p.rank) * p.T_max + j] = (t << 8) | lane;
+                want = 1u << (place >> 28);
+                if (v0 == 0) reinterpret_cast<int*>(p.peer[place >> 28] + p.off_meta)[place & kPairRow] = (t << 8) | lane;
             }
         }
         want = __reduce_or_sync(0xffffffffu, want);
@@ -245,10 +247,14 @@ __device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& 
             }
             const int e = s.idx[pair];
             const int j = pair_slot(p, s, t, k, e);
-            if (lane == 0 && v0 == 0) p.slot[pair] = j;
+            const unsigned place = j >= 0 ? pair_place(p, e, j) : kNoPair;
+            if (lane == 0 && v0 == 0) {
+                p.slot[pair] = j;
+                p.pairs[pair] = make_uint2(place, 0u);
+            }
             if (j < 0) continue;
-            const int d = e / p.L, l = e - d * p.L;
-            const size_t row = ((size_t)l * p.ws + p.rank) * p.T_max + j;
+            const unsigned d = place >> 28;
+            const size_t row = place & kPairRow;
             uint4* dst = reinterpret_cast<uint4*>(p.peer[d] + p.off_rows) + row * nvec;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {

@@ -10,7 +10,7 @@
 //     keep its own blocks busy while the others' are through.
 //   * every flag of the role before is up when a launch starts (it is awaited all the same, bounded, at gpu
 //     scope, unless the launch before it in the same call is that role).
-// One rank with many tokens is a group of one.
+// One rank with many tokens is a group of one, and the phases of a call (a2a_kernels.cuh) go by the same lists of pairs.
 #pragma once
 
 #include "a2a_solo.cuh"
@@ -28,15 +28,12 @@ struct NearParams {
     int T[N];               // and its tokens
     int n;
     int every_rank;  // a PULL combine ends only when every rank's outputs are there, also those no token wants
+    int backwards;   // blocks take the items from the end
     int output;      // role 1: kOutput...
     int handed_on;   // the launches of one call, one after the other on one stream: no flag is awaited or raised before the last
 };
 using NearGroup = NearParams<A2A_MAX_WORLD>;
 enum NearOutput : int { kOutputNone = 0, kOutputWhole = 1, kOutputPartial = 2 };
-
-// A pair as role 1 reads it: where its slab row lies, as (rank << 28 | row of that rank's slabs), and its weight.
-constexpr unsigned kNoPair = 0xffffffffu;
-static_assert((long long)A2A_MAX_EXPERTS * 65535 < 1 << 28 && A2A_MAX_WORLD <= 8, "a slab row fits 28 bits, a rank three");
 
 // ---------------------------------------------------------------------------
 // Role 0: routing.  A block takes `words` * 32 tokens of a rank: it counts the experts of the tokens before them once
@@ -85,9 +82,8 @@ __global__ void __launch_bounds__(kRouteThreads) near_route_kernel(const __grid_
                 j = s_cnt[e];
                 for (int w = 0; w < tl >> 5; ++w) j += __popc(s_bits[w * E + e]);
                 j += __popc(s_bits[(tl >> 5) * E + e] & ((1u << (tl & 31)) - 1u));
-                const int d = e / p.L, row = ((e - d * p.L) * p.ws + p.rank) * p.T_max + j;
-                place = (unsigned)d << 28 | (unsigned)row;
-                reinterpret_cast<int*>(p.peer[d] + p.off_meta)[row] = ((t0 + tl) << 8) | (i - tl * K);
+                place = pair_place(p, e, j);
+                reinterpret_cast<int*>(p.peer[place >> 28] + p.off_meta)[place & kPairRow] = ((t0 + tl) << 8) | (i - tl * K);
             } else {
                 record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
             }
@@ -109,10 +105,17 @@ __global__ void __launch_bounds__(kRouteThreads) near_route_kernel(const __grid_
     if (tid < p.ws) arrive_dest(p, tid, (uint32_t)nb);
 }
 
-// Rank p's expert outputs are there for the tokens of rank s; a fence before.
-__device__ __forceinline__ void raise_expert_flag(const DevParams& p, int s) {
-    uint32_t* flag = s == p.rank ? seen_ptr(p, kFlagExpert, s) : flag_ptr(p.peer[s], p.off_flags, kFlagExpert, p.rank);
-    st_relaxed_gpu(flag, flag_value(p, 0));
+// The flags of `kinds` of the ranks served go up, unless a wait of one of them gave up; called by a whole block, which has seen
+// what they stand for.
+__device__ __forceinline__ void raise_flags(const NearGroup& g, unsigned kinds) {
+    const int ws = g.p[0].ws, i = threadIdx.x / ws, s = threadIdx.x % ws;
+    const DevParams& p = g.p[i < g.n ? i : 0];
+    if (!__syncthreads_and(ld_volatile_i32(&p.status->code) != A2A_ERR_TIMEOUT) || i >= g.n) return;
+    fence_acq_rel_gpu();
+    if (kinds >> kFlagDispatch & 1u)  // rank s has sent to rank i
+        st_relaxed_gpu(const_cast<uint32_t*>(await_ptr(p, kFlagDispatch, s)), flag_value(p, 0));
+    if (kinds >> kFlagExpert & 1u)  // rank i's outputs are there for the tokens of rank s
+        st_relaxed_gpu(s == p.rank ? seen_ptr(p, kFlagExpert, s) : flag_ptr(p.peer[s], p.off_flags, kFlagExpert, p.rank), flag_value(p, 0));
 }
 
 // ---------------------------------------------------------------------------
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
         if (N > 1 && g.n != ws && my_rank != p0.rank) my_rank = -1;
         unsigned long long my_row = 0;
         if (my_rank >= 0)
-            my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[N == 1 ? 0 : my_rank] + p0.off_rows) + (size_t)(pair.x & 0x0fffffffu) * nvec);
+            my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[N == 1 ? 0 : my_rank] + p0.off_rows) + (size_t)(pair.x & kPairRow) * nvec);
         if (PAYLOAD == A2A_PAYLOAD_FP8) {
 #pragma unroll
             for (int u = 0; u < U; ++u) q[u] = fp8_round_trip<T>(q[u], v0 + u * 32 < nvec);  // nvec % 16 == 0: a scale block's lanes are all in or all out
@@ -233,263 +236,336 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
     } else if (grid_arrive_last(p0.ptickets + kPipeTicketSource * A2A_MAX_WORLD, (int)gridDim.x)) {
         // The block that arrives last tells every home rank that the expert outputs and partial rows are there, unless a
         // wait of one of the ranks gave up.  Every block arrives, whatever happened: the ticket is whole for the next call.
-        const DevParams& p = g.p[tid < g.n * ws ? tid / ws : 0];
-        const bool whole = __syncthreads_and(ld_volatile_i32(&p.status->code) != A2A_ERR_TIMEOUT);
-        fence_acq_rel_gpu();
-        if (whole && tid < g.n * ws) raise_expert_flag(p, tid % ws);
+        if constexpr (N > 1) raise_flags(g, 1u << kFlagExpert);
     }
     stamp(p0, kStampExpertDone);
 }
 
 // ---------------------------------------------------------------------------
-// Role 2 where role 1 has written the outputs.  In a call whose launches follow one another it raises the flags of both
-// phases, which nobody has needed until then; otherwise it ends when every rank's expert flag is up, as any combine.
+// Role 2 where role 1 has written the outputs, and RECV of rows that are in their slabs already.  In a call whose launches follow
+// one another it raises the flags that nobody has needed until then; otherwise it ends when those of the last kind are up.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(A2A_MAX_WORLD * A2A_MAX_WORLD) near_finish_kernel(const __grid_constant__ NearGroup g) {
+__global__ void __launch_bounds__(A2A_MAX_WORLD * A2A_MAX_WORLD) near_flags_kernel(const __grid_constant__ NearGroup g, int kinds) {
     begin_after_previous();
-    const int ws = g.p[0].ws, i = threadIdx.x / ws, s = threadIdx.x % ws;
-    const DevParams& p = g.p[i < g.n ? i : 0];
+    const int ws = g.p[0].ws, i = threadIdx.x / ws, s = threadIdx.x % ws, kind = kinds >> kFlagExpert & 1 ? kFlagExpert : kFlagDispatch;
     stamp(g.p[0], kStampStart);
-    if (!g.handed_on) {
-        if (i < g.n) wait_flag_gpu(await_ptr(p, kFlagExpert, s), flag_value(p, 0), p, kPhaseCombine, s);
-    } else if (__syncthreads_and(ld_volatile_i32(&p.status->code) != A2A_ERR_TIMEOUT) && i < g.n) {
-        fence_acq_rel_gpu();
-        st_relaxed_gpu(const_cast<uint32_t*>(await_ptr(p, kFlagDispatch, s)), flag_value(p, 0));
-        raise_expert_flag(p, s);
-    }
+    if (g.handed_on) raise_flags(g, (unsigned)kinds);
+    else if (i < g.n) wait_flag_gpu(await_ptr(g.p[i], kind, s), flag_value(g.p[i], 0), g.p[i], kind == kFlagExpert ? kPhaseCombine : kPhaseRecv, s);
     stamp(g.p[0], kStampCombineDone);
 }
 
 // ---------------------------------------------------------------------------
-// Role 2.  A warp's item is a piece of a token's output row; the tokens of all ranks are one list, the last rank's
-// first: what was written for them was written last and is still in the L2.  What an item reads first, the token's
-// experts, is requested one or two items ahead.
-//   PUSH: y[t] = T(sum over the ranks d holding experts of t, ascending, of float(partial[d][t])).
-//   PULL: y[t] = T(sum over k of w[t,k] * float(row k)), eight rows requested before the first is used.
-// Eight ranks of 256 tokens of 7168, top-8 of 256 experts, PUSH: 33 us (154 MB of partial rows read, some from the L2),
-// 44 with the ranks side by side and the experts looked up when needed; 200 tokens, PULL: 36, 53.  One vector a lane
-// at three or four blocks per SM: 37 and 41 (PULL); PUSH with two: 49 to 56.
+// The phases that a program with its own expert kernels calls, for all ranks of a group on one GPU: the same lists.  A token's place in
+// memory follows from its number and its pairs' places are looked up, so that no launch counts, scans or searches before its first row.
+// What bounds them: with tens of MB of rows the latencies (four ranks of 117 tokens of 4096, top-8, direct: SEND 9.7 us, RECV 3.0, EXPERT 8.8, COMBINE 7.1
+// by themselves, 25.8 together; 12.0, 2.9, 11.5, 8.6 and 33.3 by counts and bitmaps), with hundreds the memory (eight of 200 of 7168, staged:
+// 30, 48, 50 to 60, 31 to 37, 161 together; 33, 62, 68, 31 and 193).
 // ---------------------------------------------------------------------------
-struct NearTokens {
-    struct At {  // piece ch of token `row` of the list, one of the tokens of rank position n - 1 - at
-        int row, ch, at;
-    };
-    const int* pre;  // shared memory [n + 1]
-    int total, nchunk, step_row, step_ch;
-    __device__ __forceinline__ void settle(At& a) const {
-        while (a.row < total && a.row >= pre[a.at + 1]) ++a.at;
-    }
-    __device__ __forceinline__ At first() const {
-        const int w = (int)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-        At a = {w / nchunk, w % nchunk, 0};
-        settle(a);
-        return a;
-    }
-    __device__ __forceinline__ At after(const At& a) const {
-        At b = {a.row + step_row, a.ch + step_ch, a.at};
-        if (b.ch >= nchunk) {
-            b.ch -= nchunk;
-            ++b.row;
-        }
-        settle(b);
-        return b;
+// A warp's item in a launch whose blocks take no second one: U vectors a lane, from v0 on, of token t of rank s.
+template <int U>
+struct NearItem {
+    int s, t, v0;
+    bool there;
+    __device__ __forceinline__ explicit NearItem(const NearGroup& g) {
+        const int ws = g.p[0].ws, nvec = g.p[0].H >> 3, nchunk = (nvec + 32 * U - 1) / (32 * U);
+        const long long it = (long long)(g.backwards ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5);
+        long long row = it / nchunk;
+        v0 = (int)(it - row * nchunk) * 32 * U + (threadIdx.x & 31);
+        s = g.n == ws ? 0 : g.p[0].rank;  // the tokens of all ranks, or of the one served
+        const int end = g.n == ws ? ws : s + 1;
+        while (s < end && row >= g.T[s]) row -= g.T[s++];
+        there = s < end;
+        t = (int)row;
     }
 };
 
-// The list; with WAIT, once every expert flag of the ranks served is up.  False where one is not.
-template <bool WAIT>
-__device__ __forceinline__ bool near_tokens(const NearGroup& g, int* s_pre, int nchunk, NearTokens& list) {
-    const int tid = threadIdx.x, ws = g.p[0].ws, warps = (int)gridDim.x * (kThreads / 32);
-    bool ok = true;
-    if (tid < g.n * ws) {
-        const DevParams& p = g.p[tid / ws];
-        const uint32_t* flag = await_ptr(p, kFlagExpert, tid % ws);
-        if (WAIT) {
-            ok = wait_flag_gpu(flag, flag_value(p, 0), p, kPhaseCombine, tid % ws);
-        } else {
-            ok = (int32_t)(ld_relaxed_gpu(flag) - flag_value(p, 0)) >= 0;
-            fence_acq_rel_gpu();
-        }
-    }
-    if (tid == 0) {
-        int sum = 0;
-        for (int i = 0; i <= g.n; ++i) {
-            s_pre[i] = sum;
-            if (i < g.n) sum += g.p[g.n - 1 - i].T;
-        }
-    }
-    ok = __syncthreads_and(ok);
-    list = {s_pre, s_pre[g.n], nchunk, warps / nchunk, warps % nchunk};
-    return ok;
+// Lane k: where the slab row of the item's pair k lies (this lane's first vector of it), and at which rank; -1: nowhere.
+__device__ __forceinline__ unsigned long long near_row(const NearGroup& g, int s, int t, int v0, int& rank) {
+    const DevParams& p0 = g.p[0];
+    const int lane = threadIdx.x & 31;
+    unsigned place = kNoPair;
+    if (lane < p0.K) place = ld_stream(g.pairs[s] + (size_t)t * p0.K + lane).x;
+    rank = place == kNoPair ? -1 : (int)(place >> 28);
+    if (rank < 0) return 0;
+    return reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[rank] + p0.off_rows) + (size_t)(place & kPairRow) * (p0.H >> 3));
 }
 
-template <typename T>
-__device__ __forceinline__ void near_combine_push(const NearGroup& g, int* s_pre) {
-    const int lane = threadIdx.x & 31;
-    const DevParams& p0 = g.p[0];
-    const int K = p0.K, nvec = p0.H >> 3, T_max = p0.T_max;
-    NearTokens list;
-    if (!near_tokens<true>(g, s_pre, (nvec + 127) >> 7, list)) return;  // timeout recorded; y is left untouched
-    auto bit_of = [&](const NearTokens::At& a) {  // lane k: the rank of pair k
-        if (a.row >= list.total || lane >= K) return 0u;
-        const int e = ld_input(g.p[g.n - 1 - a.at].idx + (size_t)(a.row - s_pre[a.at]) * K + lane);
-        return e >= 0 && e < p0.E ? 1u << (e / p0.L) : 0u;
+// SEND: routing and sending in one launch.  A block takes a contiguous range of a rank's (token, chunk) items, as solo_kernel does.
+//   DIRECT: the row, read once, goes into the slab of every pair.  DEDUP / FP8: to the stage of every rank that wants it, FP8 quantised.
+template <typename T, int PAYLOAD, int U>
+__global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid_constant__ NearGroup g) {
+    __shared__ int s_cnt[A2A_MAX_EXPERTS];                  // tokens before the current round that use expert e
+    __shared__ int s_idx[kSoloRound * A2A_MAX_TOPK];        // the round's indices
+    __shared__ unsigned s_place[kSoloRound * A2A_MAX_TOPK]; // and where its pairs' rows go
+    begin_after_previous();
+    const DevParams& p = g.p[blockIdx.x % g.n];
+    const int b = (int)blockIdx.x / g.n, G = (int)gridDim.x / g.n;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int K = p.K, nvec = p.H >> 3, nchunk = (nvec + 32 * U - 1) / (32 * U);
+    const long long items = (long long)p.T * nchunk;
+    const long long lo = items * b / G, hi = items * (b + 1) / G;
+    const int t0 = (int)(lo / nchunk), t1 = (int)((hi + nchunk - 1) / nchunk);
+    auto load = [&](int t, int c, uint4 (&q)[U]) {
+        const uint4* src = reinterpret_cast<const uint4*>(p.x) + (size_t)t * nvec;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if ((c * U + u) * 32 + lane < nvec) q[u] = ld_input(src + (c * U + u) * 32 + lane);
     };
-    NearTokens::At a0 = list.first();
-    unsigned bit = bit_of(a0);
-    while (a0.row < list.total) {
-        const unsigned mask = __reduce_or_sync(0xffffffffu, bit);
-        const NearTokens::At a1 = list.after(a0);
-        bit = bit_of(a1);
-        const DevParams& p = g.p[g.n - 1 - a0.at];
-        const int t = a0.row - s_pre[a0.at], v0 = a0.ch * 128 + lane;
-        const uint4* ret = reinterpret_cast<const uint4*>(p.peer[p.rank] + p0.off_ret) + (size_t)t * nvec + v0;
-        float acc[4][8];
+    // the first item's row and the first round's pairs are requested before anything else: they need no routing
+    long long it = lo + warp;
+    int t = (int)(it / nchunk), c = (int)(it - (long long)t * nchunk);
+    uint4 q[U];
+    if (it < hi) load(t, c, q);
+    const int first_e = tid < min(kSoloRound, t1 - t0) * K ? ld_input(p.idx + (size_t)t0 * K + tid) : 0;
+    for (int e = tid; e < p.E; e += kThreads) s_cnt[e] = 0;
+    __syncthreads();
+    count_experts_before<kThreads>(p, t0, s_cnt);
+    for (int r0 = t0; r0 < t1; r0 += kSoloRound) {
+        const int nt = min(kSoloRound, t1 - r0), pairs = nt * K;
+        for (int i = tid; i < pairs; i += kThreads) s_idx[i] = r0 == t0 && i == tid ? first_e : ld_input(p.idx + (size_t)r0 * K + i);
+        __syncthreads();
+        resolve_round(p, s_idx, s_cnt, pairs, [&](int i, int tl, int k, int e, int j, bool ok) {
+            const unsigned place = ok ? pair_place(p, e, j) : kNoPair;
+            s_place[i] = place;
+            if ((long long)(r0 + tl) * nchunk < lo) return;  // the block that has the token's first chunk books its pairs
+            p.slot[(size_t)r0 * K + i] = j;
+            p.pairs[(size_t)r0 * K + i] = make_uint2(place, 0u);
+            if (ok) reinterpret_cast<int*>(p.peer[place >> 28] + p.off_meta)[place & kPairRow] = ((r0 + tl) << 8) | k;
+            else record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
+        });
+        __syncthreads();
+        for (int i = tid; i < pairs; i += kThreads)
+            if (s_place[i] != kNoPair) atomicAdd(s_cnt + s_idx[i], 1);
+        const long long end = min(hi, (long long)(r0 + nt) * nchunk);
+        while (it < end) {
+            const long long next = it + kSoloWarps;
+            int tn = t, cn = c + kSoloWarps;
+            while (cn >= nchunk) { cn -= nchunk; ++tn; }
+            uint4 qn[U];
+            if (next < hi) load(tn, cn, qn);
+            const int v0 = c * 32 * U + lane;
+            const unsigned place = lane < K ? s_place[(t - r0) * K + lane] : kNoPair;
+            if (PAYLOAD == A2A_PAYLOAD_DIRECT) {
+                unsigned long long my_row = 0;
+                if (place != kNoPair)
+                    my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p.peer[place >> 28] + p.off_rows) + (size_t)(place & kPairRow) * nvec);
+                for (unsigned left = __ballot_sync(0xffffffffu, place != kNoPair); left != 0u; left &= left - 1u) {
+                    uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, __ffs(left) - 1)) + v0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc[u][e] = 0.f;
-#pragma unroll
-        for (int d = 0; d < A2A_MAX_WORLD; d += 4) {  // sixteen loads in flight per lane
-            if (((mask >> d) & 0xfu) == 0u) continue;
-            uint4 q[4][4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if ((mask >> (d + j)) & 1u) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (v0 + u * 32 < nvec) q[j][u] = __ldcs(ret + (size_t)(d + j) * T_max * nvec + u * 32);
+                    for (int u = 0; u < U; ++u)
+                        if (v0 + u * 32 < nvec) st_stream(row + u * 32, q[u]);
                 }
+            } else {
+                float sc[U];
+                if (PAYLOAD == A2A_PAYLOAD_FP8) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if ((mask >> (d + j)) & 1u) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        float f[8];
-                        unpack8<T>(q[j][u], f);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) acc[u][e] += f[e];
+                    for (int u = 0; u < U; ++u) {  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
+                        const uint2 bytes = quantise8<T>(q[u], v0 + u * 32 < nvec, sc[u]);
+                        q[u].x = bytes.x;
+                        q[u].y = bytes.y;
                     }
                 }
-        }
-        uint4* y = reinterpret_cast<uint4*>(p.y) + (size_t)t * nvec + v0;
+                for (unsigned want = __reduce_or_sync(0xffffffffu, place != kNoPair ? 1u << (place >> 28) : 0u); want != 0u; want &= want - 1u) {
+                    uint8_t* wire = p.peer[__ffs(want) - 1] + p.off_stage + ((size_t)p.rank * p.T_max + t) * p.stage_row_bytes;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (v0 + u * 32 < nvec) __stcs(y + u * 32, pack8<T>(acc[u]));
-        a0 = a1;
+                    for (int u = 0; u < U; ++u) {
+                        const int v = v0 + u * 32;
+                        if (v >= nvec) continue;
+                        if (PAYLOAD == A2A_PAYLOAD_FP8) {
+                            st_stream(reinterpret_cast<uint2*>(wire) + v, make_uint2(q[u].x, q[u].y));
+                            if ((v & 15) == 0) reinterpret_cast<float*>(wire + p.H)[v >> 4] = sc[u];
+                        } else {
+                            st_stream(reinterpret_cast<uint4*>(wire) + v, q[u]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) q[u] = qn[u];
+            it = next;
+            t = tn;
+            c = cn;
+        }
+        __syncthreads();
     }
+    if (b == G - 1)  // this block's counts now cover every token
+        for (int e = tid; e < p.E; e += kThreads) {
+            const int d = e / p.L;
+            reinterpret_cast<int*>(p.peer[d] + p.off_counts)[(size_t)p.rank * kMaxChunks * p.L + (e - d * p.L)] = s_cnt[e];
+            p.send_counts[e] = s_cnt[e];
+        }
+    if (g.handed_on) return;
+    __syncthreads();
+    if (tid < p.ws) arrive_dest(p, tid, (uint32_t)G);
 }
 
-template <typename T>
-__device__ __forceinline__ void near_combine_pull(const NearGroup& g, int* s_pre) {
-    constexpr int U = 2;
-    const int lane = threadIdx.x & 31;
+// RECV and RECV_EXPERT of staged payloads (FANOUT: every slab row from its token's wire row, scaled by the expert op with SCALE),
+// EXPERT (SCALE: the slab rows in place) and RECV_EXPERT of DIRECT (both: in place).
+template <typename T, int PAYLOAD, bool FANOUT, bool SCALE>
+__global__ void __launch_bounds__(kThreads) near_expert_kernel(const __grid_constant__ NearGroup g) {
+    begin_after_previous();
+    __shared__ int s_missing;  // sources whose rows have not come
     const DevParams& p0 = g.p[0];
-    const int ws = p0.ws, K = p0.K, nvec = p0.H >> 3, T_max = p0.T_max;
-    NearTokens list;
-    // The launch before this one has raised the flags of the ranks whose expert phase ran.  Where one is missing, tokens
-    // wait for the ranks that have rows of theirs, and only for those: a rank without rows need not have run.
-    const bool all_up = near_tokens<false>(g, s_pre, (nvec + 32 * U - 1) / (32 * U), list);
-    struct Pair {  // lane k: expert, slot and weight of pair k
-        int e, j;
-        float w;
-    };
-    auto pair_of = [&](const NearTokens::At& a) {
-        Pair r = {-1, -1, 0.f};
-        if (a.row < list.total && lane < K) {
-            const DevParams& p = g.p[g.n - 1 - a.at];
-            const size_t i = (size_t)(a.row - s_pre[a.at]) * K + lane;
-            r.e = ld_input(p.idx + i);
-            r.j = ld_stream(p.slot + i);
-            r.w = ld_input(p.w + i);
+    const int tid = threadIdx.x, ws = p0.ws, nvec = p0.H >> 3;
+    if (FANOUT) {
+        if (g.handed_on) {
+            if (blockIdx.x == 0) raise_flags(g, 1u << kFlagDispatch);
+        } else {
+            if (tid == 0) s_missing = 0;
+            __syncthreads();
+            if (tid < g.n * ws) {
+                const DevParams& p = g.p[tid / ws];
+                if (!wait_flag_gpu(await_ptr(p, kFlagDispatch, tid % ws), flag_value(p, 0), p, kPhaseRecv, tid % ws)) atomicOr(&s_missing, 1 << tid % ws);
+            }
+            __syncthreads();
         }
-        return r;
-    };
-    NearTokens::At a0 = list.first(), a1 = list.after(a0);
-    Pair r0 = pair_of(a0), r1 = pair_of(a1);
-    auto go_on = [&](const NearTokens::At& a2, const Pair& r2) {
-        a0 = a1;
-        a1 = a2;
-        r0 = r1;
-        r1 = r2;
-    };
-    bool waited = false;
-    while (a0.row < list.total) {
-        const NearTokens::At a2 = list.after(a1);
-        const Pair r2 = pair_of(a2);
-        const DevParams& p = g.p[g.n - 1 - a0.at];
-        const int t = a0.row - s_pre[a0.at], v0 = a0.ch * 32 * U + lane;
-        const bool valid = r0.e >= 0 && r0.e < p0.E && r0.j >= 0;
-        const int d = valid ? r0.e / p0.L : 0;
-        if (!all_up) {
-            const uint32_t* flag = await_ptr(p, kFlagExpert, d);
-            const uint32_t want = flag_value(p, 0);
+    }
+    const NearItem<1> at(g);
+    if (at.there && (!FANOUT || g.handed_on || (s_missing >> at.s & 1) == 0)) {
+        int rank;
+        const unsigned long long my_row = near_row(g, at.s, at.t, at.v0, rank);
+        if (FANOUT && PAYLOAD != A2A_PAYLOAD_DIRECT) {
+            const unsigned want = __reduce_or_sync(0xffffffffu, rank >= 0 ? 1u << rank : 0u);
+            uint4 q[A2A_MAX_WORLD][1];  // every rank's wire row is requested before the first is written
+#pragma unroll
+            for (int d = 0; d < A2A_MAX_WORLD; ++d)
+                if (want >> d & 1u)
+                    load_wire_chunk<T, PAYLOAD, 1>(p0, false, p0.peer[d] + p0.off_stage + ((size_t)at.s * p0.T_max + at.t) * p0.stage_row_bytes,
+                                                   at.v0 - (tid & 31), nvec, q[d]);
+#pragma unroll
+            for (int d = 0; d < A2A_MAX_WORLD; ++d) {
+                if ((want >> d & 1u) == 0u) continue;
+                uint4 out = wire_vector<T, PAYLOAD>(false, q[d][0], at.v0 < nvec);
+                if (SCALE) out = scale8<T>(out, (float)(1 + d));
+                for (unsigned left = __ballot_sync(0xffffffffu, rank == d); left != 0u; left &= left - 1u) {
+                    uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, __ffs(left) - 1)) + at.v0;
+                    if (at.v0 < nvec) st_stream(row, out);
+                }
+            }
+        } else {
+            const unsigned there = __ballot_sync(0xffffffffu, rank >= 0);
+            for (int k0 = 0; k0 < p0.K; k0 += 8) {
+                uint4 q[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if ((there >> (k0 + i) & 1u) == 0u) continue;  // K <= 32: no bit beyond the last pair's
+                    const uint4* row = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
+                    if (at.v0 < nvec) q[i] = ld_stream(row);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if ((there >> (k0 + i) & 1u) == 0u) continue;
+                    uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
+                    const float scale = (float)(1 + __shfl_sync(0xffffffffu, rank, k0 + i));
+                    if (at.v0 < nvec) st_stream(row, scale8<T>(q[i], scale));
+                }
+            }
+        }
+    }
+    if (SCALE && !g.handed_on && grid_arrive_last(p0.ptickets + kPipeTicketSource * A2A_MAX_WORLD, (int)gridDim.x))
+        raise_flags(g, 1u << kFlagExpert);
+}
+
+// ---------------------------------------------------------------------------
+// Role 2 and the combine of the phases.
+//   PUSH: y[t] = T(sum over the ranks d holding experts of t, ascending, of float(partial[d][t])).
+//   PULL: y[t] = T(sum over k of w[t,k] * float(row k)), eight rows requested before the first is used.
+// ---------------------------------------------------------------------------
+template <typename T, bool PUSH, int U>
+__global__ void __launch_bounds__(kThreads) near_combine_kernel(const __grid_constant__ NearGroup g) {
+    begin_after_previous();
+    const DevParams& p0 = g.p[0];
+    const int tid = threadIdx.x, lane = tid & 31, ws = p0.ws, nvec = p0.H >> 3;
+    stamp(p0, kStampStart);
+    if (g.handed_on) {
+        if (blockIdx.x == 0) raise_flags(g, 1u << kFlagExpert);
+    } else if (PUSH) {
+        bool ok = true;
+        if (tid < g.n * ws) {
+            const DevParams& p = g.p[tid / ws];
+            ok = wait_flag_gpu(await_ptr(p, kFlagExpert, tid % ws), flag_value(p, 0), p, kPhaseCombine, tid % ws);
+        }
+        if (!__syncthreads_and(ok)) return;  // timeout recorded; y is left untouched
+    }
+    const NearItem<U> at(g);
+    bool go = at.there;
+    int rank = -1;
+    unsigned long long my_row = 0;
+    float my_w = 0.f;
+    const DevParams& p = g.p[g.n == ws && go ? at.s : 0];
+    if (go) {
+        // The launch before this one has raised the flags of the ranks whose expert phase ran.  Where one is missing, tokens
+        // wait for the ranks that have rows of theirs, and only for those: a rank without rows need not have run.
+        bool up = true;  // lane d: rank d's outputs are there
+        if (!PUSH && !g.handed_on) {
+            if (lane < ws) up = (int32_t)(ld_relaxed_gpu(await_ptr(p, kFlagExpert, lane)) - flag_value(p, 0)) >= 0;
+            fence_acq_rel_gpu();
+        }
+        my_row = near_row(g, at.s, at.t, at.v0, rank);
+        if (!PUSH && lane < p0.K) my_w = ld_input(p.w + (size_t)at.t * p0.K + lane);
+        const unsigned missing = ~__ballot_sync(0xffffffffu, up);
+        if (!PUSH && __any_sync(0xffffffffu, rank >= 0 && (missing >> rank & 1u))) {
             bool ok = true;
-            if (valid && !waited) {
-                ok = wait_flag_gpu(flag, want, p, kPhaseCombine, d);
-            } else if (valid) {  // one budget is spent: the other ranks' tokens are told at once
-                ok = (int32_t)(ld_relaxed_gpu(flag) - want) >= 0;
-                if (!ok) record_timeout(p, kPhaseCombine, d, want);
-                fence_acq_rel_gpu();
+            if (rank >= 0 && (missing >> rank & 1u)) {
+                bool spent = false;  // one rank's budget is enough: the other ranks' tokens are told at once
+                for (int i = 0; i < g.n; ++i) spent = spent || ld_volatile_i32(&g.p[i].status->code) == A2A_ERR_TIMEOUT;
+                if (spent) {
+                    ok = (int32_t)(ld_relaxed_gpu(await_ptr(p, kFlagExpert, rank)) - flag_value(p, 0)) >= 0;
+                    if (!ok) record_timeout(p, kPhaseCombine, rank, flag_value(p, 0));
+                    fence_acq_rel_gpu();
+                } else {
+                    ok = wait_flag_gpu(await_ptr(p, kFlagExpert, rank), flag_value(p, 0), p, kPhaseCombine, rank);
+                }
             }
-            if (!__all_sync(0xffffffffu, ok)) {  // timeout recorded; the token's output is left untouched
-                waited = true;
-                go_on(a2, r2);
-                continue;
-            }
+            go = __all_sync(0xffffffffu, ok);  // timeout recorded; the token's output is left untouched
         }
-        unsigned long long my_row = 0;
-        if (valid)
-            my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<const uint4*>(p0.peer[d] + p0.off_rows) +
-                                                          (((size_t)(r0.e - d * p0.L) * ws + p.rank) * T_max + r0.j) * nvec);
-        const unsigned there = __ballot_sync(0xffffffffu, valid);
+    }
+    if (go) {
         float acc[U][8];
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int e = 0; e < 8; ++e) acc[u][e] = 0.f;
-        for (int k0 = 0; k0 < K; k0 += 8) {
+        const unsigned mine = PUSH ? __reduce_or_sync(0xffffffffu, rank >= 0 ? 1u << rank : 0u) : __ballot_sync(0xffffffffu, rank >= 0);
+        const uint4* ret = reinterpret_cast<const uint4*>(p.peer[p.rank] + p0.off_ret) + (size_t)at.t * nvec + at.v0;
+        for (int k0 = 0; k0 < (PUSH ? A2A_MAX_WORLD : p0.K); k0 += 8) {
             uint4 q[8][U];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                if (((there >> (k0 + i)) & 1u) == 0u) continue;  // K <= 32: no bit beyond the last pair's
-                const uint4* row = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + v0;
+                if ((mine >> (k0 + i) & 1u) == 0u) continue;  // K <= 32: no bit beyond the last pair's
+                const uint4* row = PUSH ? ret + (size_t)i * p0.T_max * nvec : reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
 #pragma unroll
                 for (int u = 0; u < U; ++u)
-                    if (v0 + u * 32 < nvec) q[i][u] = __ldcs(row + u * 32);
+                    if (at.v0 + u * 32 < nvec) q[i][u] = __ldcs(row + u * 32);
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                if (((there >> (k0 + i)) & 1u) == 0u) continue;
-                const float w = __shfl_sync(0xffffffffu, r0.w, k0 + i);
+                if ((mine >> (k0 + i) & 1u) == 0u) continue;
+                const float w = PUSH ? 1.f : __shfl_sync(0xffffffffu, my_w, k0 + i);
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     float f[8];
                     unpack8<T>(q[i][u], f);
-                    fma8(f, w, acc[u]);
+                    if (PUSH) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) acc[u][e] += f[e];
+                    } else {
+                        fma8(f, w, acc[u]);
+                    }
                 }
             }
         }
-        uint4* y = reinterpret_cast<uint4*>(p.y) + (size_t)t * nvec + v0;
+        uint4* y = reinterpret_cast<uint4*>(p.y) + (size_t)at.t * nvec + at.v0;
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (v0 + u * 32 < nvec) __stcs(y + u * 32, pack8<T>(acc[u]));
-        go_on(a2, r2);
+            if (at.v0 + u * 32 < nvec) st_stream(y + u * 32, pack8<T>(acc[u]));
     }
-    if (!all_up && g.every_rank && blockIdx.x == 0 && threadIdx.x < g.n * ws) {
-        const DevParams& p = g.p[threadIdx.x / ws];
-        wait_flag_gpu(await_ptr(p, kFlagExpert, threadIdx.x % ws), flag_value(p, 0), p, kPhaseCombine, threadIdx.x % ws);
+    // role 2 is through when every rank is, also those whose outputs no token wants
+    if (!PUSH && g.every_rank && !g.handed_on && blockIdx.x == 0 && tid < g.n * ws) {
+        const DevParams& p = g.p[tid / ws];
+        wait_flag_gpu(await_ptr(p, kFlagExpert, tid % ws), flag_value(p, 0), p, kPhaseCombine, tid % ws);
     }
-}
-
-template <typename T, bool PUSH>
-__global__ void __launch_bounds__(kThreads, 2) near_combine_kernel(const __grid_constant__ NearGroup g) {
-    begin_after_previous();
-    __shared__ int s_pre[A2A_MAX_WORLD + 1];
-    stamp(g.p[0], kStampStart);
-    if (PUSH) near_combine_push<T>(g, s_pre);
-    else near_combine_pull<T>(g, s_pre);
-    stamp(g.p[0], kStampCombineDone);
+    stamp(p0, kStampCombineDone);
 }
 
 }  // namespace a2a

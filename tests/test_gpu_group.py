@@ -325,3 +325,45 @@ def test_a_whole_call_equals_its_roles(payload, combine, E, K, H, T, ws):
             assert all(torch.equal(a, b) for a, b in zip(state(world), tables))
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("payload", ["direct", "dedup", "fp8"])
+@pytest.mark.parametrize("E,K,H,T,ws", [
+    (12, 3, 640, 33, 3),      # ranks that do not divide the grid, rows that end inside a warp's piece
+    (48, 11, 1152, 70, 2),    # more pairs than are requested together
+    (8, 2, 7168, 300, 8),     # 1 KB a warp in every phase; 69 MB of rows: phases that begin with the last rows
+    (256, 32, 128, 20, 8),    # the most experts a token, a row of one scale block
+])
+def test_phases_of_a_group_equal_those_rank_by_rank(payload, E, K, H, T, ws):
+    """In one call, with receiving and expert op in one launch, phase by phase, and after sends rank by rank."""
+    rds = [pkg.generate_input(E, K, H, T, seed=9, rank=r, world_size=ws)[1].to(DEV) for r in range(ws)]
+    for name in ("x", "indices", "weights"):  # a rank without tokens
+        setattr(rds[1], name, getattr(rds[1], name)[:0].contiguous())
+    rds[1].num_tokens = 0
+    rds[0].indices[3, :] = rds[0].indices[3, 0]  # repeats, and a token without a valid expert: dropped, zero
+    rds[0].indices[T - 1, :] = E
+    world = LocalWorld(pkg.MoEConfig(E, K, H, T), ws, payload=payload)
+
+    def by_steps(together):
+        if together:
+            world._send(rds)
+        else:
+            for c, rd in zip(world.ctxs, rds):
+                c.route(rd.indices)
+                c.dispatch_send(rd.x)
+        world._step("recv")
+        world._step("expert")
+        return world._combine(rds)
+
+    try:
+        want = [bits(y) for y in rank_by_rank(world, rds)]
+        tables = state(world)
+        for run in (lambda: world.forward_phases(rds), lambda: world.forward(rds), lambda: by_steps(True), lambda: by_steps(False)):
+            for c in world.ctxs:
+                c.expert_buffers()[0].zero_()
+            assert all(torch.equal(bits(g), w) for g, w in zip(run(), want))
+            assert all(torch.equal(a, b) for a, b in zip(state(world), tables))
+        assert not want[0][T - 1].any()
+        assert [c.peek() for c in world.ctxs] == [_lib.A2A_ERR_ROUTING] + [0] * (ws - 1)
+    finally:
+        world.close()
