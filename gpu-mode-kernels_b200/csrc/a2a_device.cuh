@@ -572,6 +572,29 @@ __device__ __forceinline__ void unpack8_e4m3(const uint2& q, float (&f)[8]) {
     }
 }
 
+// f[i] / d, each rounded as the division rounds it, for a d that many values share: its reciprocal once, and for each value a product
+// and two corrections by the remainder.  The product is within two units in the last place of the quotient, so the first correction leaves
+// less than one, from which the second rounds correctly, r being the correctly rounded reciprocal (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  The remainder is exact where it does not underflow: the
+// caller sees to 2^-80 <= d <= 2^100, and rounds quotients below 2^-11 to zero whatever their last bits.  Zeros keep their sign.
+// Eight ranks, headline workload with FP8 rows, 66.3 -> 63.2 us a call; one rank 10.7 -> 10.3.
+__device__ __forceinline__ void divide8(float (&f)[8], float d) {
+    const float r = 1.f / d;
+    const float2 rr = make_float2(r, r), dd = make_float2(d, d);
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        const float2 v = make_float2(f[i], f[i + 1]), nv = make_float2(-f[i], -f[i + 1]);
+        float2 q = __fmul2_rn(v, rr);
+#pragma unroll
+        for (int step = 0; step < 2; ++step) {
+            const float2 e = __ffma2_rn(q, dd, nv);
+            q = __ffma2_rn(make_float2(-e.x, -e.y), rr, q);
+        }
+        f[i] = q.x;
+        f[i + 1] = q.y;
+    }
+}
+
 // A vector of a row as e4m3 bytes, and the scale of its 128-value block, which 16 lanes share.  All 32 lanes call
 // it; a lane without a vector (`valid` false) only takes part in the shuffles.
 template <typename T>
@@ -587,8 +610,12 @@ __device__ __forceinline__ uint2 quantise8(const uint4& q, bool valid, float& sc
     for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     sc = amax > 0.f ? amax / 448.f : 1.f;
     if (!valid) return make_uint2(0u, 0u);
+    if (sc >= 0x1p-80f && sc <= 0x1p100f) {
+        divide8(f, sc);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = f[i] / sc;
+        for (int i = 0; i < 8; ++i) f[i] = f[i] / sc;
+    }
     return pack8_e4m3(f);
 }
 

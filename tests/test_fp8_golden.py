@@ -138,3 +138,58 @@ def test_kernels_deliver_the_golden_rows(name):
         world.check()
     finally:
         world.close()
+
+
+def _blocks(dt, n, rng):
+    """`n` scale blocks of values of `dt`: amax over the type's whole range, values down to 2^-20 of it and signed zeros; and
+    scales of few bits with values on and beside the midpoints between e4m3 numbers."""
+    lo, hi = (-133, 127) if dt == torch.bfloat16 else (-24, 15)
+    bits = 8 if dt == torch.bfloat16 else 11
+    amax = np.ldexp(rng.integers(1 << (bits - 1), 1 << bits, n).astype(np.float64), rng.integers(lo, hi + 1, n) - bits + 1)
+    v = amax[:, None] * np.ldexp(rng.integers(128, 257, (n, 128)) / 256.0, -rng.integers(0, 21, (n, 128)))
+    few = rng.random(n) < 0.5
+    scale = np.ldexp(rng.integers(1, 32, n).astype(np.float64), rng.integers(lo + 20, hi - 14, n))
+    middle = np.ldexp(2.0 * rng.integers(8, 16, (n, 128)) + 1.0, rng.integers(-8, 5, (n, 128)))  # 17, 19 .. 31 times a power of two
+    v[few] = (middle * scale[:, None] * rng.choice([1.0, 1.0, 1 - 2.0 ** -bits, 1 + 2.0 ** -bits], (n, 128)))[few]
+    v[few, 0] = 448.0 * scale[few]
+    v = np.clip(v * rng.choice([-1.0, 1.0], (n, 128)), -3e38 if dt == torch.bfloat16 else -65504, 3e38 if dt == torch.bfloat16 else 65504)
+    v[rng.random((n, 128)) < 0.02] = 0.0
+    v[rng.random((n, 128)) < 0.02] = -0.0
+    v[: n // 50] = 0.0
+    return torch.from_numpy(v.astype(np.float32)).to(dt)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["bf16", "fp16"])
+def test_the_kernels_divide_as_the_checker_does(name):
+    """Rows quantised and dequantised by the kernels of one rank, of a group and of its phases, to the bit."""
+    from gpu_mode_kernels_b200 import MoEConfig, RankTestData
+    from gpu_mode_kernels_b200.all2all import A2AContext
+    from gpu_mode_kernels_b200.local_world import LocalWorld
+
+    dt, T, H = DTYPES[name], 256, 7168
+    x = _blocks(dt, 2 * T * H // 128, np.random.default_rng(17)).view(2, T, H)
+    want = torch.stack([O.fp8_dequantise(*O.fp8_quantise(part), dt) for part in x])
+    assert bool(want.isfinite().all())
+    rds = []
+    for r in range(2):
+        rd = object.__new__(RankTestData)
+        rd.num_tokens, rd.x = T, x[r].to("cuda:0")
+        rd.indices, rd.weights = torch.zeros(T, 1, dtype=torch.int32, device="cuda:0"), torch.ones(T, 1, device="cuda:0")
+        rds.append(rd)
+    cfg = MoEConfig(2, 1, H, T, dt, dt)
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="fp8", schedule="pipelined", combine="push")
+    worlds = [LocalWorld(cfg, 2, payload="fp8", schedule="pipelined", combine="push"), LocalWorld(cfg, 2, payload="fp8")]
+    try:
+        outs = [torch.stack([ctx.forward(rd.x, rd.indices, rd.weights) for rd in rds])]
+        outs += [torch.stack(worlds[0].forward_pipelined(rds)), torch.stack(worlds[1].forward_phases(rds))]
+        for y in outs:  # all rows at rank 0, whose expert multiplies by one; weights of one.  A sum makes no negative zero.
+            got, ref = y.cpu().view(torch.int16), want.view(torch.int16)
+            same = (got == ref) | ((got == 0) & (ref == -32768))
+            assert bool(same.all())
+        rows = worlds[1].ctxs[0].export_dispatch()[1][0].cpu()
+        assert torch.equal(rows.view(torch.int16), want.view(-1, H).view(torch.int16))
+    finally:
+        ctx.close()
+        for w in worlds:
+            w.close()
