@@ -91,6 +91,7 @@ struct a2a_ctx {
     bool near;              // ... by role 0 of a group on this GPU: rows stay where they are
     bool whole;             // ... and role 1 of the group has written the outputs too
     bool listed;            // every pair's place is in p.pairs
+    bool placed;            // ... and its row in its slab, whatever the payload
     bool backwards;         // the last launch that wrote the expert rows of the group began with the last tokens
     const void* near_x[A2A_MAX_WORLD];  // input rows of every rank in this call
     const uint2* near_pairs[A2A_MAX_WORLD];
@@ -335,20 +336,9 @@ template <typename T, int U>
 const void* near_combine_fn(bool push) {
     return push ? (const void*)near_combine_kernel<T, true, U> : (const void*)near_combine_kernel<T, false, U>;
 }
-template <typename T, int P>
-const void* near_wire_fn(bool scale) {
-    return scale ? (const void*)near_expert_kernel<T, P, true, true> : (const void*)near_expert_kernel<T, P, true, false>;
-}
-template <typename T>
-const void* near_expert_fn(int payload, bool fanout, bool scale) {
-    if (fanout && payload == A2A_PAYLOAD_FP8) return near_wire_fn<T, A2A_PAYLOAD_FP8>(scale);
-    if (fanout && payload == A2A_PAYLOAD_DEDUP) return near_wire_fn<T, A2A_PAYLOAD_DEDUP>(scale);
-    return fanout ? (const void*)near_expert_kernel<T, A2A_PAYLOAD_DIRECT, true, true> : (const void*)near_expert_kernel<T, A2A_PAYLOAD_DIRECT, false, true>;
-}
 template <typename T, int U>
-const void* near_dispatch_fn(int payload) {
-    if (payload == A2A_PAYLOAD_FP8) return (const void*)near_dispatch_kernel<T, A2A_PAYLOAD_FP8, U>;
-    return payload == A2A_PAYLOAD_DEDUP ? (const void*)near_dispatch_kernel<T, A2A_PAYLOAD_DEDUP, U> : (const void*)near_dispatch_kernel<T, A2A_PAYLOAD_DIRECT, U>;
+const void* near_dispatch_fn(bool fp8) {
+    return fp8 ? (const void*)near_dispatch_kernel<T, true, U> : (const void*)near_dispatch_kernel<T, false, U>;
 }
 
 PhaseFn combine_fn(const a2a_ctx* c) {
@@ -486,8 +476,7 @@ int near_blocks(const a2a_ctx* c, const NearParams<N>& g, int U) {
 constexpr int kBothFlags = 1 << kFlagDispatch | 1 << kFlagExpert;
 
 // Where the expert rows are more than the L2 keeps, a phase begins with those that the one before it wrote last: eight ranks of 200
-// tokens of 7168, top-8 of 256 experts, 183 MB, staged 171 -> 161 us a call, direct 132 -> 131; 128 tokens, 117 MB, 81.4 / 80.6.  Below 64 MB
-// no difference.
+// tokens of 7168, top-8 of 256 experts, 183 MB, 132 -> 131 us a call by phases; 128 tokens, 117 MB, 81.4 / 80.6.  Below 64 MB no difference.
 bool beyond_l2(const a2a_ctx* c, const NearGroup& g) {
     long long tokens = 0;
     for (int s = 0; s < c->cfg.world_size; ++s) tokens += g.T[s];
@@ -504,16 +493,16 @@ int launch_near_combine(a2a_ctx* const* cs, NearGroup& g, bool push, cudaStream_
     return launch_near(cs, g, fn, near_blocks(cs[0], g, wide ? 2 : 1), 0, st);
 }
 
-// RECV, EXPERT and RECV_EXPERT: 512 bytes a warp (1 KB: two ranks of 256 tokens of 7168 39.2 us a call by phases instead of 38.4).
-int launch_near_expert(a2a_ctx* const* cs, NearGroup& g, bool fanout, bool scale, cudaStream_t st) {
-    const int payload = cs[0]->cfg.payload;
-    if (fanout && !scale && payload == A2A_PAYLOAD_DIRECT)  // the rows are in place
-        return launch_near(cs, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, 1 << kFlagDispatch);
-    const bool bf = cs[0]->cfg.dtype == A2A_DTYPE_BF16;
-    g.backwards = !fanout && !cs[0]->backwards && beyond_l2(cs[0], g);
+// RECV, of rows that SEND has put into their slabs, EXPERT and RECV_EXPERT: 512 bytes a warp (1 KB: two ranks of 256 tokens of 7168 39.2 us
+// a call by phases instead of 38.4).
+int launch_near_expert(a2a_ctx* const* cs, NearGroup& g, bool wait, bool scale, cudaStream_t st) {
+    if (!scale) return launch_near(cs, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, 1 << kFlagDispatch);
+    g.backwards = beyond_l2(cs[0], g);
     for (int r = 0; r < g.n; ++r) cs[r]->backwards = g.backwards;
-    return launch_near(cs, g, bf ? near_expert_fn<__nv_bfloat16>(payload, fanout, scale) : near_expert_fn<__half>(payload, fanout, scale),
-                       near_blocks(cs[0], g, 1), 0, st);
+    const bool bf = cs[0]->cfg.dtype == A2A_DTYPE_BF16;
+    const void* fn = wait ? (bf ? (const void*)near_expert_kernel<__nv_bfloat16, true> : (const void*)near_expert_kernel<__half, true>)
+                          : (bf ? (const void*)near_expert_kernel<__nv_bfloat16, false> : (const void*)near_expert_kernel<__half, false>);
+    return launch_near(cs, g, fn, near_blocks(cs[0], g, 1), 0, st);
 }
 
 // SEND: as many blocks as are resident together, three per SM, each of which counts the experts of the tokens before its own; a second round
@@ -529,8 +518,9 @@ int launch_near_dispatch(a2a_ctx* const* cs, NearGroup& g, cudaStream_t st) {
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    const void* fn = wide ? (bf ? near_dispatch_fn<__nv_bfloat16, 2>(c->cfg.payload) : near_dispatch_fn<__half, 2>(c->cfg.payload))
-                          : (bf ? near_dispatch_fn<__nv_bfloat16, 1>(c->cfg.payload) : near_dispatch_fn<__half, 1>(c->cfg.payload));
+    const bool fp8 = c->cfg.payload == A2A_PAYLOAD_FP8;
+    const void* fn = wide ? (bf ? near_dispatch_fn<__nv_bfloat16, 2>(fp8) : near_dispatch_fn<__half, 2>(fp8))
+                          : (bf ? near_dispatch_fn<__nv_bfloat16, 1>(fp8) : near_dispatch_fn<__half, 1>(fp8));
     return launch_near(cs, g, fn, g.n * (int)blocks, 0, st);
 }
 
@@ -611,7 +601,7 @@ int begin_call(a2a_ctx* c, const int32_t* idx, int T) {
     c->cur_tokens = T;
     c->p.idx = idx;
     c->routed = true;
-    c->sent = c->recorded = c->near = c->whole = c->listed = c->backwards = false;
+    c->sent = c->recorded = c->near = c->whole = c->listed = c->placed = c->backwards = false;
     return A2A_OK;
 }
 
@@ -658,7 +648,7 @@ int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st, bo
         NearGroup g = near_params(cs, n, handed_on);
         const int rc = launch_near_dispatch(cs, g, st);
         if (rc == A2A_OK)
-            for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->listed = true;
+            for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->listed = cs[r]->placed = true;
         return rc;
     }
     // a warp per 2 KB of a pair's row (DIRECT) or 512 bytes of a token's, no more blocks than four per SM, each of which
@@ -681,16 +671,26 @@ int expert_grid(const a2a_ctx* c, int n, int per_sm) {
 }
 
 int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st, bool handed_on = false) {
-    bool listed = true;
+    bool placed = true;
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent) return A2A_ERR_STATE;
-        listed = listed && cs[r]->listed;
+        placed = placed && cs[r]->placed;
     }
-    if (listed && near_phases(cs, n)) {
+    if (placed && near_phases(cs, n)) {
         NearGroup g = near_params(cs, n, handed_on);
-        return launch_near_expert(cs, g, fanout, scale, st);
+        return launch_near_expert(cs, g, wait, scale, st);
     }
-    return launch_ranks(cs, n, select_tp<ExpertSel>(cs[0], wait, fanout, scale, publish), grid, cs[0]->smem_bytes, st);
+    if (!placed || cs[0]->cfg.payload == A2A_PAYLOAD_DIRECT)
+        return launch_ranks(cs, n, select_tp<ExpertSel>(cs[0], wait, fanout, scale, publish), grid, cs[0]->smem_bytes, st);
+    // Sent together, received rank by rank: there is nothing in the stages.
+    const PhaseFn fn = cs[0]->cfg.dtype == A2A_DTYPE_BF16 ? ExpertSel<__nv_bfloat16, A2A_PAYLOAD_DIRECT>::get(wait, fanout, scale, publish)
+                                                          : ExpertSel<__half, A2A_PAYLOAD_DIRECT>::get(wait, fanout, scale, publish);
+    CUDA_TRY(cudaFuncSetAttribute((const void*)fn.one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes));
+    for (int r = 0; r < n; ++r) {
+        const int rc = launch(cs[r], (const void*)fn.one, grid, cs[r]->smem_bytes, st);
+        if (rc != A2A_OK) return rc;
+    }
+    return A2A_OK;
 }
 
 int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st, bool handed_on = false) {

@@ -10,7 +10,7 @@
 //     keep its own blocks busy while the others' are through.
 //   * every flag of the role before is up when a launch starts (it is awaited all the same, bounded, at gpu
 //     scope, unless the launch before it in the same call is that role).
-// One rank with many tokens is a group of one, and the phases of a call (a2a_kernels.cuh) go by the same lists of pairs.
+// One rank with many tokens is a group of one, and the phases of a group's call (of one rank: a2a_kernels.cuh) go by the same lists of pairs.
 #pragma once
 
 #include "a2a_solo.cuh"
@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(A2A_MAX_WORLD * A2A_MAX_WORLD) near_flags_kern
 // The phases that a program with its own expert kernels calls, for all ranks of a group on one GPU: the same lists.  A token's place in
 // memory follows from its number and its pairs' places are looked up, so that no launch counts, scans or searches before its first row.
 // What bounds them: with tens of MB of rows the latencies (four ranks of 117 tokens of 4096, top-8, direct: SEND 9.7 us, RECV 3.0, EXPERT 8.8, COMBINE 7.1
-// by themselves, 25.8 together; 12.0, 2.9, 11.5, 8.6 and 33.3 by counts and bitmaps), with hundreds the memory (eight of 200 of 7168, staged:
-// 30, 48, 50 to 60, 31 to 37, 161 together; 33, 62, 68, 31 and 193).
+// by themselves, 25.7 together; 12.0, 2.9, 11.5, 8.6 and 33.3 by counts and bitmaps), with hundreds the memory (eight of 200 of 7168, 183 MB:
+// 40, 4, 54, 37 by themselves, 131 together; direct 141, and through the stages 33, 62, 68, 31 and 193).
 // ---------------------------------------------------------------------------
 // A warp's item in a launch whose blocks take no second one: U vectors a lane, from v0 on, of token t of rank s.
 template <int U>
@@ -290,9 +290,9 @@ __device__ __forceinline__ unsigned long long near_row(const NearGroup& g, int s
     return reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[rank] + p0.off_rows) + (size_t)(place & kPairRow) * (p0.H >> 3));
 }
 
-// SEND: routing and sending in one launch.  A block takes a contiguous range of a rank's (token, chunk) items, as solo_kernel does.
-//   DIRECT: the row, read once, goes into the slab of every pair.  DEDUP / FP8: to the stage of every rank that wants it, FP8 quantised.
-template <typename T, int PAYLOAD, int U>
+// SEND: routing and sending in one launch.  A block takes a contiguous range of a rank's (token, chunk) items, as solo_kernel does.  Whatever
+// the payload, a row, read once (and FP8, quantised and dequantised once), goes straight into the slabs: a stage is what a link needs.
+template <typename T, bool FP8, int U>
 __global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid_constant__ NearGroup g) {
     __shared__ int s_cnt[A2A_MAX_EXPERTS];                  // tokens before the current round that use expert e
     __shared__ int s_idx[kSoloRound * A2A_MAX_TOPK];        // the round's indices
@@ -345,40 +345,18 @@ __global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid
             if (next < hi) load(tn, cn, qn);
             const int v0 = c * 32 * U + lane;
             const unsigned place = lane < K ? s_place[(t - r0) * K + lane] : kNoPair;
-            if (PAYLOAD == A2A_PAYLOAD_DIRECT) {
-                unsigned long long my_row = 0;
-                if (place != kNoPair)
-                    my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p.peer[place >> 28] + p.off_rows) + (size_t)(place & kPairRow) * nvec);
-                for (unsigned left = __ballot_sync(0xffffffffu, place != kNoPair); left != 0u; left &= left - 1u) {
-                    uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, __ffs(left) - 1)) + v0;
+            unsigned long long my_row = 0;
+            if (place != kNoPair)
+                my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p.peer[place >> 28] + p.off_rows) + (size_t)(place & kPairRow) * nvec);
+            if (FP8) {
 #pragma unroll
-                    for (int u = 0; u < U; ++u)
-                        if (v0 + u * 32 < nvec) st_stream(row + u * 32, q[u]);
-                }
-            } else {
-                float sc[U];
-                if (PAYLOAD == A2A_PAYLOAD_FP8) {
+                for (int u = 0; u < U; ++u) q[u] = fp8_round_trip<T>(q[u], v0 + u * 32 < nvec);  // nvec % 16 == 0: a scale block's lanes are all in or all out
+            }
+            for (unsigned left = __ballot_sync(0xffffffffu, place != kNoPair); left != 0u; left &= left - 1u) {
+                uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, __ffs(left) - 1)) + v0;
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {  // nvec % 16 == 0: the 16 lanes of a scale block are all in or all out
-                        const uint2 bytes = quantise8<T>(q[u], v0 + u * 32 < nvec, sc[u]);
-                        q[u].x = bytes.x;
-                        q[u].y = bytes.y;
-                    }
-                }
-                for (unsigned want = __reduce_or_sync(0xffffffffu, place != kNoPair ? 1u << (place >> 28) : 0u); want != 0u; want &= want - 1u) {
-                    uint8_t* wire = p.peer[__ffs(want) - 1] + p.off_stage + ((size_t)p.rank * p.T_max + t) * p.stage_row_bytes;
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int v = v0 + u * 32;
-                        if (v >= nvec) continue;
-                        if (PAYLOAD == A2A_PAYLOAD_FP8) {
-                            st_stream(reinterpret_cast<uint2*>(wire) + v, make_uint2(q[u].x, q[u].y));
-                            if ((v & 15) == 0) reinterpret_cast<float*>(wire + p.H)[v >> 4] = sc[u];
-                        } else {
-                            st_stream(reinterpret_cast<uint4*>(wire) + v, q[u]);
-                        }
-                    }
-                }
+                for (int u = 0; u < U; ++u)
+                    if (v0 + u * 32 < nvec) st_stream(row + u * 32, q[u]);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) q[u] = qn[u];
@@ -399,70 +377,46 @@ __global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid
     if (tid < p.ws) arrive_dest(p, tid, (uint32_t)G);
 }
 
-// RECV and RECV_EXPERT of staged payloads (FANOUT: every slab row from its token's wire row, scaled by the expert op with SCALE),
-// EXPERT (SCALE: the slab rows in place) and RECV_EXPERT of DIRECT (both: in place).
-template <typename T, int PAYLOAD, bool FANOUT, bool SCALE>
+// EXPERT, and with WAIT RECV_EXPERT: the expert op on the slab rows, in place.
+template <typename T, bool WAIT>
 __global__ void __launch_bounds__(kThreads) near_expert_kernel(const __grid_constant__ NearGroup g) {
     begin_after_previous();
     __shared__ int s_missing;  // sources whose rows have not come
-    const DevParams& p0 = g.p[0];
-    const int tid = threadIdx.x, ws = p0.ws, nvec = p0.H >> 3;
-    if (FANOUT) {
-        if (g.handed_on) {
-            if (blockIdx.x == 0) raise_flags(g, 1u << kFlagDispatch);
-        } else {
-            if (tid == 0) s_missing = 0;
-            __syncthreads();
-            if (tid < g.n * ws) {
-                const DevParams& p = g.p[tid / ws];
-                if (!wait_flag_gpu(await_ptr(p, kFlagDispatch, tid % ws), flag_value(p, 0), p, kPhaseRecv, tid % ws)) atomicOr(&s_missing, 1 << tid % ws);
-            }
-            __syncthreads();
+    const int tid = threadIdx.x, ws = g.p[0].ws, K = g.p[0].K, nvec = g.p[0].H >> 3;
+    if (WAIT && g.handed_on) {
+        if (blockIdx.x == 0) raise_flags(g, 1u << kFlagDispatch);
+    } else if (WAIT) {
+        if (tid == 0) s_missing = 0;
+        __syncthreads();
+        if (tid < g.n * ws) {
+            const DevParams& p = g.p[tid / ws];
+            if (!wait_flag_gpu(await_ptr(p, kFlagDispatch, tid % ws), flag_value(p, 0), p, kPhaseRecv, tid % ws)) atomicOr(&s_missing, 1 << tid % ws);
         }
+        __syncthreads();
     }
     const NearItem<1> at(g);
-    if (at.there && (!FANOUT || g.handed_on || (s_missing >> at.s & 1) == 0)) {
+    if (at.there && (!WAIT || g.handed_on || (s_missing >> at.s & 1) == 0)) {
         int rank;
         const unsigned long long my_row = near_row(g, at.s, at.t, at.v0, rank);
-        if (FANOUT && PAYLOAD != A2A_PAYLOAD_DIRECT) {
-            const unsigned want = __reduce_or_sync(0xffffffffu, rank >= 0 ? 1u << rank : 0u);
-            uint4 q[A2A_MAX_WORLD][1];  // every rank's wire row is requested before the first is written
+        const unsigned there = __ballot_sync(0xffffffffu, rank >= 0);
+        for (int k0 = 0; k0 < K; k0 += 8) {  // eight rows are requested before the first is written
+            uint4 q[8];
 #pragma unroll
-            for (int d = 0; d < A2A_MAX_WORLD; ++d)
-                if (want >> d & 1u)
-                    load_wire_chunk<T, PAYLOAD, 1>(p0, false, p0.peer[d] + p0.off_stage + ((size_t)at.s * p0.T_max + at.t) * p0.stage_row_bytes,
-                                                   at.v0 - (tid & 31), nvec, q[d]);
-#pragma unroll
-            for (int d = 0; d < A2A_MAX_WORLD; ++d) {
-                if ((want >> d & 1u) == 0u) continue;
-                uint4 out = wire_vector<T, PAYLOAD>(false, q[d][0], at.v0 < nvec);
-                if (SCALE) out = scale8<T>(out, (float)(1 + d));
-                for (unsigned left = __ballot_sync(0xffffffffu, rank == d); left != 0u; left &= left - 1u) {
-                    uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, __ffs(left) - 1)) + at.v0;
-                    if (at.v0 < nvec) st_stream(row, out);
-                }
+            for (int i = 0; i < 8; ++i) {
+                if ((there >> (k0 + i) & 1u) == 0u) continue;  // K <= 32: no bit beyond the last pair's
+                const uint4* row = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
+                if (at.v0 < nvec) q[i] = ld_stream(row);
             }
-        } else {
-            const unsigned there = __ballot_sync(0xffffffffu, rank >= 0);
-            for (int k0 = 0; k0 < p0.K; k0 += 8) {
-                uint4 q[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if ((there >> (k0 + i) & 1u) == 0u) continue;  // K <= 32: no bit beyond the last pair's
-                    const uint4* row = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
-                    if (at.v0 < nvec) q[i] = ld_stream(row);
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if ((there >> (k0 + i) & 1u) == 0u) continue;
-                    uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
-                    const float scale = (float)(1 + __shfl_sync(0xffffffffu, rank, k0 + i));
-                    if (at.v0 < nvec) st_stream(row, scale8<T>(q[i], scale));
-                }
+            for (int i = 0; i < 8; ++i) {
+                if ((there >> (k0 + i) & 1u) == 0u) continue;
+                uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
+                const float scale = (float)(1 + __shfl_sync(0xffffffffu, rank, k0 + i));
+                if (at.v0 < nvec) st_stream(row, scale8<T>(q[i], scale));
             }
         }
     }
-    if (SCALE && !g.handed_on && grid_arrive_last(p0.ptickets + kPipeTicketSource * A2A_MAX_WORLD, (int)gridDim.x))
+    if (!g.handed_on && grid_arrive_last(g.p[0].ptickets + kPipeTicketSource * A2A_MAX_WORLD, (int)gridDim.x))
         raise_flags(g, 1u << kFlagExpert);
 }
 

@@ -335,7 +335,8 @@ def test_a_whole_call_equals_its_roles(payload, combine, E, K, H, T, ws):
     (256, 32, 128, 20, 8),    # the most experts a token, a row of one scale block
 ])
 def test_phases_of_a_group_equal_those_rank_by_rank(payload, E, K, H, T, ws):
-    """In one call, with receiving and expert op in one launch, phase by phase, and after sends rank by rank."""
+    """In one call, with receiving and expert op in one launch, phase by phase, sent rank by rank and received together, and
+    the other way round."""
     rds = [pkg.generate_input(E, K, H, T, seed=9, rank=r, world_size=ws)[1].to(DEV) for r in range(ws)]
     for name in ("x", "indices", "weights"):  # a rank without tokens
         setattr(rds[1], name, getattr(rds[1], name)[:0].contiguous())
@@ -344,21 +345,28 @@ def test_phases_of_a_group_equal_those_rank_by_rank(payload, E, K, H, T, ws):
     rds[0].indices[T - 1, :] = E
     world = LocalWorld(pkg.MoEConfig(E, K, H, T), ws, payload=payload)
 
-    def by_steps(together):
-        if together:
+    def by_steps(send, recv):
+        if send:
             world._send(rds)
         else:
             for c, rd in zip(world.ctxs, rds):
                 c.route(rd.indices)
                 c.dispatch_send(rd.x)
-        world._step("recv")
-        world._step("expert")
-        return world._combine(rds)
+        if recv:
+            world._step("recv")
+            world._step("expert")
+            return world._combine(rds)
+        for c in world.ctxs[:-1]:
+            c.dispatch_recv()
+            c.expert_placeholder()
+        world.ctxs[-1].dispatch_recv_expert()
+        return [c.combine(rd.weights) for c, rd in zip(world.ctxs, rds)]
 
     try:
         want = [bits(y) for y in rank_by_rank(world, rds)]
         tables = state(world)
-        for run in (lambda: world.forward_phases(rds), lambda: world.forward(rds), lambda: by_steps(True), lambda: by_steps(False)):
+        for run in (lambda: world.forward_phases(rds), lambda: world.forward(rds), lambda: by_steps(True, True), lambda: by_steps(False, True),
+                    lambda: by_steps(True, False)):
             for c in world.ctxs:
                 c.expert_buffers()[0].zero_()
             assert all(torch.equal(bits(g), w) for g, w in zip(run(), want))
