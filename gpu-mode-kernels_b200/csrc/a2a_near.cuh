@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kRouteThreads) near_route_kernel(const __grid_
         }
         for (int e = tid; e < (words + 1) * E; e += kRouteThreads) s_cnt[e] = 0;
         __syncthreads();
-        count_experts_before<kRouteThreads>(p, t0, s_cnt);
+        count_experts_before<kRouteThreads, 4>(p, t0, s_cnt);
         auto first_use = [&](int i) {  // pair i's expert is in range and of no earlier pair of its token
             const int e = s_idx[i];
             bool ok = e >= 0 && e < E;

@@ -136,6 +136,40 @@ def test_where_a_call_takes_two_launches(E, K, H, T, launches):
         world.close()
 
 
+@pytest.mark.parametrize("E,K,H,T", [(16, 4, 72, 100), (64, 12, 1024, 300), (16, 8, 4096, 900)])
+def test_indices_wherever_they_begin(E, K, H, T):
+    """Indices in whole 16-byte vectors and one to three words past them: one launch, two, a group and its phases."""
+    rds = [pkg.generate_input(E, K, H, T, seed=15, rank=r, world_size=2)[1].to(DEV) for r in range(2)]
+    for rd in rds:
+        rd.indices[T - 2, K - 1] = rd.indices[T - 2, 0]
+    cfg = pkg.MoEConfig(E, K, H, T)
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push")
+    worlds = [LocalWorld(cfg, 2, payload="dedup", schedule="pipelined", combine="push"), LocalWorld(cfg, 2)]
+    base = torch.empty(2, T * K + 4, dtype=torch.int32, device=DEV)
+    want = None
+    try:
+        for off in range(4):
+            for r, rd in enumerate(rds):
+                place = base[r, off:off + T * K].view(T, K)
+                place.copy_(rd.indices.clone())
+                rd.indices = place
+            got = [ctx.forward(rds[0].x, rds[0].indices, rds[0].weights)] + worlds[0].forward_pipelined(rds) + worlds[1].forward_phases(rds)
+            got = [bits(y) for y in got] + list(ctx.route_tables()) + [t for w in worlds for c in w.ctxs for t in c.route_tables()]
+            torch.cuda.synchronize()
+            want = want or got
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+        slots = torch.zeros_like(got[-2])
+        sent = torch.zeros(E, dtype=torch.int32, device=DEV)
+        lib = _lib.load()
+        assert lib.a2a_route_noalloc(rds[1].indices.data_ptr(), T, E, K, slots.data_ptr(), sent.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(got[-2], slots) and torch.equal(got[-1], sent)
+    finally:
+        ctx.close()
+        for w in worlds:
+            w.close()
+
+
 def test_dropped_pairs_match_the_stepped_roles_and_phases_can_follow():
     """Indices out of range and repeated, the repeats also across the eight indices the kernel loads
     together and in tokens before the reading block's own; then a combine called on its own, which
