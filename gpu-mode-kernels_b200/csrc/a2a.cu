@@ -431,16 +431,20 @@ int launch_near(a2a_ctx* const* cs, NearParams<N>& g, const void* fn, int blocks
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
-// Role 0 of ranks on one GPU: 32 tokens a block (64: headline workload of eight ranks 56.5 us a call instead of 56.4, two ranks of
-// 200 tokens 15.4 / 15.1), or more where there are so many that counting the tokens before the block's shows (2048 tokens of one
-// rank, 32 / 64: 56.2 / 55.4).
+// Role 0 of ranks on one GPU: 32 tokens a block (64: two ranks of 200 tokens of 7168 15.4 us a call instead of 15.1), or 256 where there are
+// so many that counting the tokens before the block's shows; up to 256 tokens one thread for each of them (1024 threads: four ranks of two tokens
+// 7.9 / 7.4, eight of 16 12.0 / 11.3, of 256 56.6 / 56.2), else 1024 (2048 tokens of one rank, 256 threads 56.9, 512 52.8, 1024 51.8).
 template <int N>
 int launch_near_route(a2a_ctx* const* cs, NearParams<N>& g, cudaStream_t st) {
     int most = 1;
     for (int r = 0; r < g.n; ++r) most = cs[r]->cur_tokens > most ? cs[r]->cur_tokens : most;
-    const int words = most > 8192 ? 8 : most > 1024 ? 2 : 1, nb = (most + 32 * words - 1) / (32 * words);
-    return launch_near(cs, g, (const void*)near_route_kernel<N>, g.n * nb, (int)near_route_smem(words, cs[0]->cfg.num_experts, cs[0]->cfg.experts_per_token),
-                       st, kRouteThreads, words);
+    const bool few = N > 1 && most <= kThreads;
+    const int words = most > 8192 ? 8 : 1, nb = (most + 32 * words - 1) / (32 * words);
+    const void* fn = (const void*)near_route_kernel<N, 1024>;
+    if constexpr (N > 1)
+        if (few) fn = (const void*)near_route_kernel<N, kThreads>;
+    return launch_near(cs, g, fn, g.n * nb, (int)near_route_smem(words, cs[0]->cfg.num_experts, cs[0]->cfg.experts_per_token), st,
+                       few ? kThreads : 1024, words);
 }
 
 // Role 1: a warp per 1 KB of a token's row, three blocks per SM, or per 512 bytes where that would be too few rounds of blocks:
@@ -1079,8 +1083,9 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
         c->pipe_smem = (int)align_up(a > b ? a : b, 128);
         opt_in_both(select_pipe<PipeForward>(c));
         opt_in((const void*)select_pipe<PipeRole>(c, 0).one);
-        opt_in((const void*)near_route_kernel<1>);
-        opt_in((const void*)near_route_kernel<A2A_MAX_WORLD>);
+        opt_in((const void*)near_route_kernel<1, 1024>);
+        opt_in((const void*)near_route_kernel<A2A_MAX_WORLD, 1024>);
+        opt_in((const void*)near_route_kernel<A2A_MAX_WORLD, kThreads>);
         if (e == cudaSuccess && cfg->world_size == 1) {
             c->forward_grid = c->num_sms;
             c->fused = true;  // the solo kernel: no block waits for another

@@ -40,11 +40,10 @@ enum NearOutput : int { kOutputNone = 0, kOutputWhole = 1, kOutputPartial = 2 };
 // more for itself (64 KB at 2048 x 8, out of the L2) instead of waiting for another block.  What bounds it: the chain
 // launch -> indices -> counts -> slots -> stores.
 // ---------------------------------------------------------------------------
-constexpr int kRouteThreads = 1024;
 __host__ __device__ inline size_t near_route_smem(int words, int E, int K) { return ((size_t)(words + 1) * E + (size_t)words * 64 * K) * 4; }
 
-template <int N>
-__global__ void __launch_bounds__(kRouteThreads) near_route_kernel(const __grid_constant__ NearParams<N> g, int words) {
+template <int N, int THREADS>
+__global__ void __launch_bounds__(THREADS) near_route_kernel(const __grid_constant__ NearParams<N> g, int words) {
     begin_after_previous();
     const int n = N == 1 ? 1 : g.n;
     const DevParams& p = g.p[blockIdx.x % n];
@@ -57,23 +56,23 @@ __global__ void __launch_bounds__(kRouteThreads) near_route_kernel(const __grid_
     stamp(p, kStampStart);
     const bool last = p.T > 0 ? pairs > 0 && t0 + tokens >= p.T : t0 == 0;
     if (pairs > 0 || last) {
-        for (int i = tid; i < pairs; i += kRouteThreads) {
+        for (int i = tid; i < pairs; i += THREADS) {
             s_idx[i] = ld_input(p.idx + (size_t)t0 * K + i);
             s_w[i] = ld_input(p.w + (size_t)t0 * K + i);
         }
-        for (int e = tid; e < (words + 1) * E; e += kRouteThreads) s_cnt[e] = 0;
+        for (int e = tid; e < (words + 1) * E; e += THREADS) s_cnt[e] = 0;
         __syncthreads();
-        count_experts_before<kRouteThreads, 4>(p, t0, s_cnt);
+        count_experts_before<THREADS, 4>(p, t0, s_cnt);
         auto first_use = [&](int i) {  // pair i's expert is in range and of no earlier pair of its token
             const int e = s_idx[i];
             bool ok = e >= 0 && e < E;
             for (int j = i / K * K; ok && j < i; ++j) ok = s_idx[j] != e;
             return ok;
         };
-        for (int i = tid; i < pairs; i += kRouteThreads)
+        for (int i = tid; i < pairs; i += THREADS)
             if (first_use(i)) atomicOr(s_bits + (i / K >> 5) * E + s_idx[i], 1u << (i / K & 31));
         __syncthreads();
-        for (int i = tid; i < pairs; i += kRouteThreads) {
+        for (int i = tid; i < pairs; i += THREADS) {
             const size_t at = (size_t)t0 * K + i;
             const int tl = i / K, e = s_idx[i];
             int j = -1;
@@ -91,7 +90,7 @@ __global__ void __launch_bounds__(kRouteThreads) near_route_kernel(const __grid_
             p.pairs[at] = make_uint2(place, __float_as_uint(s_w[i]));
         }
         if (last)
-            for (int e = tid; e < E; e += kRouteThreads) {
+            for (int e = tid; e < E; e += THREADS) {
                 int c = s_cnt[e];
                 for (int w = 0; w < words; ++w) c += __popc(s_bits[w * E + e]);
                 const int d = e / p.L;
