@@ -104,12 +104,18 @@ __global__ void __launch_bounds__(THREADS) near_route_kernel(const __grid_consta
     if (tid < p.ws) arrive_dest(p, tid, (uint32_t)nb);
 }
 
+// What has been recorded of the rank whose flags this thread raises.
+__device__ __forceinline__ int recorded_of_rank(const NearGroup& g) {
+    const int i = threadIdx.x / g.p[0].ws;
+    return ld_volatile_i32(&g.p[i < g.n ? i : 0].status->code);
+}
+
 // The flags of `kinds` of the ranks served go up, unless a wait of one of them gave up; called by a whole block, which has seen
 // what they stand for.
-__device__ __forceinline__ void raise_flags(const NearGroup& g, unsigned kinds) {
+__device__ __forceinline__ void raise_flags(const NearGroup& g, unsigned kinds, int recorded) {
     const int ws = g.p[0].ws, i = threadIdx.x / ws, s = threadIdx.x % ws;
-    const DevParams& p = g.p[i < g.n ? i : 0];
-    if (!__syncthreads_and(ld_volatile_i32(&p.status->code) != A2A_ERR_TIMEOUT) || i >= g.n) return;
+    if (!__syncthreads_and(recorded != A2A_ERR_TIMEOUT) || i >= g.n) return;
+    const DevParams& p = g.p[i];
     fence_acq_rel_gpu();
     if (kinds >> kFlagDispatch & 1u)  // rank s has sent to rank i
         st_relaxed_gpu(const_cast<uint32_t*>(await_ptr(p, kFlagDispatch, s)), flag_value(p, 0));
@@ -235,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
     } else if (grid_arrive_last(p0.ptickets + kPipeTicketSource * A2A_MAX_WORLD, (int)gridDim.x)) {
         // The block that arrives last tells every home rank that the expert outputs and partial rows are there, unless a
         // wait of one of the ranks gave up.  Every block arrives, whatever happened: the ticket is whole for the next call.
-        if constexpr (N > 1) raise_flags(g, 1u << kFlagExpert);
+        if constexpr (N > 1) raise_flags(g, 1u << kFlagExpert, recorded_of_rank(g));
     }
     stamp(p0, kStampExpertDone);
 }
@@ -245,10 +251,12 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
 // one another it raises the flags that nobody has needed until then; otherwise it ends when those of the last kind are up.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(A2A_MAX_WORLD * A2A_MAX_WORLD) near_flags_kernel(const __grid_constant__ NearGroup g, int kinds) {
+    // looked at while the launch before this one ends: no launch of a call that is handed on waits for anything, or records that it did
+    const int recorded = recorded_of_rank(g);
     begin_after_previous();
     const int ws = g.p[0].ws, i = threadIdx.x / ws, s = threadIdx.x % ws, kind = kinds >> kFlagExpert & 1 ? kFlagExpert : kFlagDispatch;
     stamp(g.p[0], kStampStart);
-    if (g.handed_on) raise_flags(g, (unsigned)kinds);
+    if (g.handed_on) raise_flags(g, (unsigned)kinds, recorded);
     else if (i < g.n) wait_flag_gpu(await_ptr(g.p[i], kind, s), flag_value(g.p[i], 0), g.p[i], kind == kFlagExpert ? kPhaseCombine : kPhaseRecv, s);
     stamp(g.p[0], kStampCombineDone);
 }
@@ -383,7 +391,7 @@ __global__ void __launch_bounds__(kThreads) near_expert_kernel(const __grid_cons
     __shared__ int s_missing;  // sources whose rows have not come
     const int tid = threadIdx.x, ws = g.p[0].ws, K = g.p[0].K, nvec = g.p[0].H >> 3;
     if (WAIT && g.handed_on) {
-        if (blockIdx.x == 0) raise_flags(g, 1u << kFlagDispatch);
+        if (blockIdx.x == 0) raise_flags(g, 1u << kFlagDispatch, recorded_of_rank(g));
     } else if (WAIT) {
         if (tid == 0) s_missing = 0;
         __syncthreads();
@@ -416,7 +424,7 @@ __global__ void __launch_bounds__(kThreads) near_expert_kernel(const __grid_cons
         }
     }
     if (!g.handed_on && grid_arrive_last(g.p[0].ptickets + kPipeTicketSource * A2A_MAX_WORLD, (int)gridDim.x))
-        raise_flags(g, 1u << kFlagExpert);
+        raise_flags(g, 1u << kFlagExpert, recorded_of_rank(g));
 }
 
 // ---------------------------------------------------------------------------
@@ -431,7 +439,7 @@ __global__ void __launch_bounds__(kThreads) near_combine_kernel(const __grid_con
     const int tid = threadIdx.x, lane = tid & 31, ws = p0.ws, nvec = p0.H >> 3;
     stamp(p0, kStampStart);
     if (g.handed_on) {
-        if (blockIdx.x == 0) raise_flags(g, 1u << kFlagExpert);
+        if (blockIdx.x == 0) raise_flags(g, 1u << kFlagExpert, recorded_of_rank(g));
     } else if (PUSH) {
         bool ok = true;
         if (tid < g.n * ws) {
