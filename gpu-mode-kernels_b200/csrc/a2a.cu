@@ -319,16 +319,13 @@ KernelFn solo_fn(const a2a_ctx* c) {
 }
 
 // role 1 of ranks on one GPU
-template <typename T, int P, bool PUSH, int N>
-const void* rows_fn(bool narrow) {
-    return narrow ? (const void*)near_rows_kernel<T, P, PUSH, 1, N> : (const void*)near_rows_kernel<T, P, PUSH, 2, N>;
-}
-template <bool PUSH, int N>
-const void* rows_fn(const a2a_ctx* c, bool narrow) {
-    const bool bf = c->cfg.dtype == A2A_DTYPE_BF16;
-    if (c->cfg.payload == A2A_PAYLOAD_FP8)
-        return bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_FP8, PUSH, N>(narrow) : rows_fn<__half, A2A_PAYLOAD_FP8, PUSH, N>(narrow);
-    return bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_DEDUP, PUSH, N>(narrow) : rows_fn<__half, A2A_PAYLOAD_DEDUP, PUSH, N>(narrow);
+template <typename T, int P, int N>
+const void* rows_fn(bool push, bool whole, bool narrow) {
+    if constexpr (N > 1) {
+        if (!whole) return push ? (const void*)near_rows_kernel<T, P, true, false, 1, N> : (const void*)near_rows_kernel<T, P, false, false, 1, N>;
+        if (push) return narrow ? (const void*)near_rows_kernel<T, P, true, true, 1, N> : (const void*)near_rows_kernel<T, P, true, true, 2, N>;
+    }
+    return narrow ? (const void*)near_rows_kernel<T, P, false, true, 1, N> : (const void*)near_rows_kernel<T, P, false, true, 2, N>;
 }
 
 // the kernels of the phases and the combine of ranks on one GPU: element type, U vectors a lane
@@ -453,16 +450,17 @@ int launch_near_route(a2a_ctx* const* cs, NearParams<N>& g, cudaStream_t st) {
 // 256 tokens, eight ranks 21.4 / 19.8 (2.3); top-2 of 6144, 110 tokens, eight 17.4 / 15.5 (2.9), four 11.8 / 11.3 (1.5), 256, two 11.5 / 10.8
 // (1.7); top-4 of 2880, 110, eight 14.6 / 14.1 (1.5).
 template <int N>
-int launch_near_rows(a2a_ctx* const* cs, NearParams<N>& g, bool push, cudaStream_t st) {
+int launch_near_rows(a2a_ctx* const* cs, NearParams<N>& g, bool push, bool whole, cudaStream_t st) {
     const a2a_ctx* c = cs[0];
     const long long nvec = c->cfg.hidden_dim / 8, wide = (nvec + 63) / 64, narrow = (nvec + 31) / 32, warps = kThreads / 32;
     long long tokens = 0;
     for (int s = 0; s < c->cfg.world_size; ++s) tokens += g.T[s];
-    const bool many = 2 * tokens * wide >= (c->cfg.experts_per_token >= 6 ? 13LL : 6LL) * c->num_sms * warps;
+    const bool many = whole && 2 * tokens * wide >= (c->cfg.experts_per_token >= 6 ? 13LL : 6LL) * c->num_sms * warps;
     const long long items = tokens * (many ? wide : narrow), blocks = items > 0 ? (items + warps - 1) / warps : 1;
-    const void* fn = rows_fn<false, N>(c, !many);
-    if constexpr (N > 1)
-        if (push) fn = rows_fn<true, N>(c, !many);
+    const bool bf = c->cfg.dtype == A2A_DTYPE_BF16;
+    const void* fn = c->cfg.payload == A2A_PAYLOAD_FP8
+        ? (bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_FP8, N>(push, whole, !many) : rows_fn<__half, A2A_PAYLOAD_FP8, N>(push, whole, !many))
+        : (bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_DEDUP, N>(push, whole, !many) : rows_fn<__half, A2A_PAYLOAD_DEDUP, N>(push, whole, !many));
     return launch_near(cs, g, fn, (int)blocks, 0, st);
 }
 
@@ -551,9 +549,9 @@ int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = host_rows ? c->num_sms / 2 : 2LL * c->num_sms;
     const long long two = c->cur_tokens * ((nvec + 63) / 64), one = c->cur_tokens * ((nvec + 31) / 32);
     if (!host_rows && c->p.trace == nullptr && solo_two_launches(c)) {
-        NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, /*backwards=*/0, kOutputWhole, /*handed_on=*/1};
+        NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, /*backwards=*/0, /*handed_on=*/1};
         const int rc = launch_near_route(&c, g, st);
-        return rc != A2A_OK ? rc : launch_near_rows(&c, g, /*push=*/false, st);
+        return rc != A2A_OK ? rc : launch_near_rows(&c, g, /*push=*/false, /*whole=*/true, st);
     }
     const bool wide = two >= cap * warps;
     long long blocks = ((wide ? two : one) + warps - 1) / warps;
@@ -800,11 +798,10 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool hand
             a2a_call calls[A2A_MAX_WORLD];
             for (int r = 0; r < n; ++r) calls[r] = {g.x[r], nullptr, nullptr, cs[r]->p.y, g.T[r]};
             // PULL: between these roles the expert rows are the caller's
-            if (handed_on || (push && !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2))) g.output = kOutputWhole;
-            else if (push) g.output = kOutputPartial;
-            const int rc = launch_near_rows(cs, g, push, st);
+            whole = handed_on || (push && !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2));
+            const int rc = launch_near_rows(cs, g, push, whole, st);
             if (rc == A2A_OK)
-                for (int r = 0; r < n; ++r) cs[r]->whole = g.output == kOutputWhole;
+                for (int r = 0; r < n; ++r) cs[r]->whole = whole;
             return rc;
         }
         // a role 2 is through when every rank is through with this call, whoever's rows its tokens want
@@ -818,9 +815,8 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool hand
             rc = launch_role(cs[r], role, 1 + blocks, push_smem, st);
         } else if (role == 1) {
             NearGroup g = near_params(cs + r, 1);
-            if (push) g.output = kOutputPartial;
-            else cs[r]->whole = false;  // the expert rows are written anew, and the caller's again
-            rc = launch_near_rows(cs + r, g, push, st);
+            if (!push) cs[r]->whole = false;  // the expert rows are written anew, and the caller's again
+            rc = launch_near_rows(cs + r, g, push, /*whole=*/false, st);
         } else if (cs[r]->whole) {
             NearGroup g = near_params(cs + r, 1);
             rc = launch_near(cs + r, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, kBothFlags);

@@ -29,11 +29,9 @@ struct NearParams {
     int n;
     int every_rank;  // a PULL combine ends only when every rank's outputs are there, also those no token wants
     int backwards;   // blocks take the items from the end
-    int output;      // role 1: kOutput...
     int handed_on;   // the launches of one call, one after the other on one stream: no flag is awaited or raised before the last
 };
 using NearGroup = NearParams<A2A_MAX_WORLD>;
-enum NearOutput : int { kOutputNone = 0, kOutputWhole = 1, kOutputPartial = 2 };
 
 // ---------------------------------------------------------------------------
 // Role 0: routing.  A block takes `words` * 32 tokens of a rank: it counts the experts of the tokens before them once
@@ -129,16 +127,17 @@ __device__ __forceinline__ void raise_flags(const NearGroup& g, unsigned kinds, 
 //   PUSH: y[t] = T(sum over the ranks d holding experts of t, ascending, of float(T(sum over k at d of w[t,k] * float(row k)))),
 //         the order and the roundings of a group with a GPU each.
 //   PULL: y[t] = T(sum over k of w[t,k] * float(row k)).
-// kOutputWhole writes that; kOutputPartial the partial rows to the home ranks' buffers, for near_combine_kernel: where
-// outputs lie over rows that are still to be read, and where a rank's experts run by themselves; kOutputNone neither.
+// WHOLE, for all ranks together, writes that.  Otherwise a combine follows: where outputs lie over rows that are still to be read, where a rank's
+// experts run by themselves, and where the expert rows are the caller's before a PULL combine; PUSH then writes the partial rows to the
+// home ranks' buffers.  (The two in one kernel: 80 registers and spills, headline 55.1 us a call against 54.0, FP8 62.3 / 58.4.)
 // What bounds it: the stores, K + 1 for each load; expert rows leave the L2 first, outputs, which the next layer reads, do not.
-// Eight ranks of 256 tokens of 7168, top-8 of 256 experts, a call: 56 us, 294 MB at 5.2 TB/s (134 with partial rows written
-// by one role, 87, and read by the next, 33; FP8 rows 66, 142; PULL, 200 tokens 44, 91); of 2048, top-6 of 64, skewed 19 (44).
+// Eight ranks of 256 tokens of 7168, top-8 of 256 experts, a call: 54 us, 294 MB at 5.4 TB/s (134 with partial rows written
+// by one role, 87, and read by the next, 33; FP8 rows 58, 142; PULL, 200 tokens 44, 91); of 2048, top-6 of 64, skewed 17 (44).
 // Slower: rows stored without evict-first (two ranks of 200 tokens 17.2 us against 16.2, skewed 21.6 / 20.4, headline 1 %), four
 // vectors a lane at two blocks per SM (13 %), two at four (64 registers, spills: 49 %), pairs' rows looked up one by one (7 %).  One rank
 // of 2048 tokens of 7168 54.6, inputs loaded with evict-first too 53.8, but 1500 of 2880 12.9 / 14.1.  FP8: the quantiser's arithmetic on top.
 // ---------------------------------------------------------------------------
-template <typename T, int PAYLOAD, bool PUSH, int U, int N>
+template <typename T, int PAYLOAD, bool PUSH, bool WHOLE, int U, int N>
 __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_constant__ NearParams<N> g) {
     begin_after_previous();
     __shared__ int s_here[A2A_MAX_WORLD];
@@ -165,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
         if (lane < K) pair = ld_stream(g.pairs[s] + (size_t)t * K + lane);
         // lane k: the rank of pair k, or -1 where it has no row or is not served, and this lane's place in its slab row
         int my_rank = pair.x == kNoPair ? -1 : (int)(pair.x >> 28);
-        if (N > 1 && g.n != ws && my_rank != p0.rank) my_rank = -1;
+        if (!WHOLE && g.n != ws && my_rank != p0.rank) my_rank = -1;
         unsigned long long my_row = 0;
         if (my_rank >= 0)
             my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[N == 1 ? 0 : my_rank] + p0.off_rows) + (size_t)(pair.x & kPairRow) * nvec);
@@ -206,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const uint4 r = pack8<T>(part[u]);
-                    if (g.output == kOutputPartial && v0 + u * 32 < nvec) st_stream(home + u * 32, r);
+                    if (!WHOLE && v0 + u * 32 < nvec) st_stream(home + u * 32, r);
                     float f[8];
                     unpack8<T>(r, f);
 #pragma unroll
@@ -228,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
                 expert_row(k, out, acc);
             }
         }
-        if (g.output == kOutputWhole) {
+        if (WHOLE) {
             uint4* y = reinterpret_cast<uint4*>(g.p[s].y) + (size_t)t * nvec + v0;
 #pragma unroll
             for (int u = 0; u < U; ++u)
