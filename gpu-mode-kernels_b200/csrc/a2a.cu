@@ -79,6 +79,7 @@ Layout make_layout(const a2a_config& c) {
 
 struct a2a_ctx {
     a2a_config cfg;
+    Fingerprint print;      // of cfg
     Layout lay;
     DevParams p;            // template of the kernel parameter block (per-call fields patched at launch)
     uint8_t* region;        // our symmetric region (cudaMalloc)
@@ -397,10 +398,11 @@ int launch_ranks(a2a_ctx* const* cs, int n, const PhaseFn& fn, int blocks, int s
 }
 
 // What a launch for a group on one GPU is told, or for one rank of it in a call that the group began together.
-NearGroup near_params(a2a_ctx* const* cs, int n, bool handed_on = false) {
-    NearGroup g{};
+void near_params(a2a_ctx* const* cs, int n, NearGroup& g) {
     for (int r = 0; r < n; ++r) {
-        g.p[r] = call_params(cs[r]);
+        g.p[r] = cs[r]->p;
+        g.p[r].T = cs[r]->cur_tokens;
+        g.p[r].epoch = cs[r]->epoch;
         g.p[r].local = 1;
         if (n > 1) g.p[r].trace = nullptr;  // a trace has a slot per block of one rank's grid
         g.x[r] = cs[r]->p.x;
@@ -413,8 +415,19 @@ NearGroup near_params(a2a_ctx* const* cs, int n, bool handed_on = false) {
         memcpy(g.T, cs[0]->near_T, sizeof(g.T));
     }
     g.n = n;
-    g.handed_on = handed_on;
-    return g;
+    g.every_rank = g.backwards = g.handed_on = 0;
+}
+
+// The same of the launches of one call, one after the other with nothing in between: `call` (n 0 before the first) keeps it from one to the
+// next.  Of a launch by itself (`call` null): in `own`.
+NearGroup& near_call(a2a_ctx* const* cs, int n, NearGroup* call, NearGroup& own) {
+    if (call == nullptr) {
+        near_params(cs, n, own);
+        return own;
+    }
+    if (call->n == 0) near_params(cs, n, *call);
+    call->handed_on = 1;
+    return *call;
 }
 
 template <int N>
@@ -638,7 +651,7 @@ bool any_traced(a2a_ctx* const* cs, int n) {
 // All ranks of a group on one GPU in a launch of a2a_near.cuh?
 bool near_phases(a2a_ctx* const* cs, int n) { return n > 1 && cs[0]->p.chunks == 1 && !any_traced(cs, n); }
 
-int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st, bool handed_on = false) {
+int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st, NearGroup* call = nullptr) {
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->routed || cs[r]->sent) return A2A_ERR_STATE;
         if (cs[r]->cur_tokens > 0 && x[r] == nullptr) return A2A_ERR_CONFIG;
@@ -647,7 +660,7 @@ int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st, bo
     for (int r = 0; r < n; ++r) cs[r]->p.x = x[r];
     const a2a_ctx* c = cs[0];
     if (near_phases(cs, n)) {
-        NearGroup g = near_params(cs, n, handed_on);
+        NearGroup own, &g = near_call(cs, n, call, own);
         const int rc = launch_near_dispatch(cs, g, st);
         if (rc == A2A_OK)
             for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->listed = cs[r]->placed = true;
@@ -672,14 +685,14 @@ int expert_grid(const a2a_ctx* c, int n, int per_sm) {
     return g < ws ? ws : g;
 }
 
-int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st, bool handed_on = false) {
+int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st, NearGroup* call = nullptr) {
     bool placed = true;
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent) return A2A_ERR_STATE;
         placed = placed && cs[r]->placed;
     }
     if (placed && near_phases(cs, n)) {
-        NearGroup g = near_params(cs, n, handed_on);
+        NearGroup own, &g = near_call(cs, n, call, own);
         return launch_near_expert(cs, g, wait, scale, st);
     }
     if (!placed || cs[0]->cfg.payload == A2A_PAYLOAD_DIRECT)
@@ -695,7 +708,7 @@ int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, boo
     return A2A_OK;
 }
 
-int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st, bool handed_on = false) {
+int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y, cudaStream_t st, NearGroup* call = nullptr) {
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent) return A2A_ERR_STATE;
         if (cs[r]->cur_tokens > 0 && (w[r] == nullptr || y[r] == nullptr)) return A2A_ERR_CONFIG;
@@ -709,7 +722,11 @@ int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y,
     bool listed = true;
     for (int r = 0; r < n; ++r) listed = listed && cs[r]->listed;
     if (listed && near_phases(cs, n)) {
-        NearGroup g = near_params(cs, n, handed_on);
+        NearGroup own, &g = near_call(cs, n, call, own);
+        for (int r = 0; r < n; ++r) {
+            g.p[r].w = w[r];
+            g.p[r].y = y[r];
+        }
         return launch_near_combine(cs, g, /*push=*/false, st);
     }
     const int nseg = (c->cfg.hidden_dim / 8 + 63) / 64;  // a warp per (token, 1 KB segment)
@@ -742,8 +759,8 @@ int launch_role(a2a_ctx* c, int role, int blocks, int smem, cudaStream_t st) {
 }
 
 // Role 0.  Contexts that are being traced are launched one by one, in the forms of a GPU per rank: a trace has a slot
-// per block of one rank's grid.  `handed_on`: roles 1 and 2 of the call follow on this stream, with nothing in between.
-int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st, bool handed_on = false) {
+// per block of one rank's grid.  `call`: roles 1 and 2 follow on this stream, with nothing in between.
+int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t st, NearGroup* call = nullptr) {
     const int begun = begin_pipe_call(cs, n, calls);
     if (begun != A2A_OK) return begun;
     const a2a_ctx* c = cs[0];
@@ -758,7 +775,7 @@ int do_pipe_send(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStream_t 
                 cs[r]->near_pairs[s] = cs[s]->p.pairs;
                 cs[r]->near_T[s] = calls[s].num_tokens;
             }
-        NearGroup g = near_params(cs, n, handed_on);
+        NearGroup own, &g = near_call(cs, n, call, own);
         rc = launch_near_route(cs, g, st);
         if (rc == A2A_OK)
             for (int r = 0; r < n; ++r) cs[r]->near = cs[r]->listed = true;
@@ -778,7 +795,7 @@ bool outputs_over_rows(const a2a_call* calls, int n, size_t row_bytes) {
 
 // Roles 1 and 2, of a call whose role 0 ran: the one launch of a single rank writes nothing for them, and what role 1 would
 // find there belongs to an earlier call.  A call begun for ranks on one GPU goes on in that form, whoever asks for it.
-int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool handed_on = false) {
+int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, NearGroup* call = nullptr) {
     bool near = true, whole = true;
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent || !cs[r]->recorded) return A2A_ERR_STATE;
@@ -793,12 +810,12 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool hand
             // Begun rank by rank: one launch, in which each rank has its share of two blocks per SM.  Role 0 of eight ranks one by
             // one and these two, 4 tokens of 2048 146 us (294 with a launch for each rank), 128 of 7168 222 (404).
             return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), blocks / n, push_smem, st);
-        NearGroup g = near_params(cs, n, handed_on);
+        NearGroup own, &g = near_call(cs, n, call, own);
         if (role == 1) {
             a2a_call calls[A2A_MAX_WORLD];
             for (int r = 0; r < n; ++r) calls[r] = {g.x[r], nullptr, nullptr, cs[r]->p.y, g.T[r]};
             // PULL: between these roles the expert rows are the caller's
-            whole = handed_on || (push && !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2));
+            whole = call != nullptr || (push && !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2));
             const int rc = launch_near_rows(cs, g, push, whole, st);
             if (rc == A2A_OK)
                 for (int r = 0; r < n; ++r) cs[r]->whole = whole;
@@ -814,14 +831,17 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, bool hand
         if (!cs[r]->near) {
             rc = launch_role(cs[r], role, 1 + blocks, push_smem, st);
         } else if (role == 1) {
-            NearGroup g = near_params(cs + r, 1);
+            NearGroup g;
+            near_params(cs + r, 1, g);
             if (!push) cs[r]->whole = false;  // the expert rows are written anew, and the caller's again
             rc = launch_near_rows(cs + r, g, push, /*whole=*/false, st);
         } else if (cs[r]->whole) {
-            NearGroup g = near_params(cs + r, 1);
+            NearGroup g;
+            near_params(cs + r, 1, g);
             rc = launch_near(cs + r, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, kBothFlags);
         } else {
-            NearGroup g = near_params(cs + r, 1);
+            NearGroup g;
+            near_params(cs + r, 1, g);
             g.every_rank = 1;
             rc = launch_near_combine(cs + r, g, push, st);
         }
@@ -868,12 +888,10 @@ int do_group_forward(a2a_ctx* const* cs, int n, const a2a_call* calls, cudaStrea
 // behind.
 int check_group(a2a_ctx* const* group) {
     if (group == nullptr || group[0] == nullptr) return A2A_ERR_CONFIG;
-    const Fingerprint mine = fingerprint_of(group[0]->cfg);
     for (int r = 0; r < group[0]->cfg.world_size; ++r) {
         const a2a_ctx* c = group[r];
         if (c == nullptr || c->cfg.rank != r || c->cfg.device != group[0]->cfg.device) return A2A_ERR_CONFIG;
-        const Fingerprint f = fingerprint_of(c->cfg);
-        if (memcmp(&f, &mine, sizeof(f)) != 0) return A2A_ERR_CONFIG;
+        if (memcmp(&c->print, &group[0]->print, sizeof(c->print)) != 0) return A2A_ERR_CONFIG;
         if (!c->peers_ready || c->epoch != group[0]->epoch) return A2A_ERR_STATE;
     }
     for (int r = 0; r < group[0]->cfg.world_size; ++r)
@@ -883,7 +901,7 @@ int check_group(a2a_ctx* const* group) {
 }
 
 // One phase of all ranks of a group that check_group has passed.
-int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStream_t st, bool handed_on = false) {
+int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStream_t st, NearGroup* call = nullptr) {
     const a2a_ctx* c = group[0];
     const int n = c->cfg.world_size;
     const bool pipe_phase = phase == A2A_GROUP_PIPE_SEND || phase == A2A_GROUP_PIPE_EXPERT || phase == A2A_GROUP_PIPE_COMBINE;
@@ -910,13 +928,13 @@ int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStr
                 if (!rows_aligned(x[r])) return A2A_ERR_CONFIG;
             }
             for (int r = 0; r < n; ++r) begin_call(group[r], calls[r].topk_idx, calls[r].num_tokens);
-            return do_send(group, n, x, st, handed_on);
+            return do_send(group, n, x, st, call);
         case A2A_GROUP_RECV:
             return do_expert(group, n, true, true, false, false,
-                             c->cfg.payload == A2A_PAYLOAD_DIRECT ? n : expert_grid(c, n, 4), st, handed_on);
-        case A2A_GROUP_EXPERT: return do_expert(group, n, false, false, true, true, expert_grid(c, n, 4), st, handed_on);
-        case A2A_GROUP_RECV_EXPERT: return do_expert(group, n, true, true, true, true, expert_grid(c, n, 4), st, handed_on);
-        case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st, handed_on);
+                             c->cfg.payload == A2A_PAYLOAD_DIRECT ? n : expert_grid(c, n, 4), st, call);
+        case A2A_GROUP_EXPERT: return do_expert(group, n, false, false, true, true, expert_grid(c, n, 4), st, call);
+        case A2A_GROUP_RECV_EXPERT: return do_expert(group, n, true, true, true, true, expert_grid(c, n, 4), st, call);
+        case A2A_GROUP_COMBINE: return do_combine(group, n, w, y, st, call);
         default: return A2A_ERR_CONFIG;
     }
 }
@@ -973,6 +991,7 @@ int a2a_create(a2a_ctx** out, const a2a_config* cfg) {
     memset(c, 0, sizeof(*c));
     c->cfg = *cfg;
     if (c->cfg.timeout_ms <= 0) c->cfg.timeout_ms = 2000;
+    c->print = fingerprint_of(c->cfg);
     c->lay = make_layout(c->cfg);
     const int E = cfg->num_experts, K = cfg->experts_per_token, T = cfg->max_num_tokens, H = cfg->hidden_dim;
     const int L = E / cfg->world_size;
@@ -1355,19 +1374,21 @@ int a2a_group_steps(a2a_ctx* const* group, const int32_t* phases, int num_phases
     const int n = c->cfg.world_size;
     DeviceGuard guard(c->cfg.device);
     cudaStream_t st = as_stream(stream);
+    NearGroup call;
+    call.n = 0;
     // The roles of a whole call: with nothing between them role 1 writes the outputs of a PULL combine too, and no launch
     // waits for flags of the one before it.
     const bool roles = num_phases == 3 && phases[0] == A2A_GROUP_PIPE_SEND && phases[1] == A2A_GROUP_PIPE_EXPERT && phases[2] == A2A_GROUP_PIPE_COMBINE;
     if (roles && n > 1 && calls != nullptr && c->cfg.schedule == A2A_SCHEDULE_PIPELINED && !any_traced(group, n) &&
         !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2)) {
-        rc = do_pipe_send(group, n, calls, st, /*handed_on=*/true);
-        for (; rc == A2A_OK && ++*done < 3;) rc = do_pipe_rest(group, n, *done, st, /*handed_on=*/true);
+        rc = do_pipe_send(group, n, calls, st, &call);
+        for (; rc == A2A_OK && ++*done < 3;) rc = do_pipe_rest(group, n, *done, st, &call);
         return rc;
     }
     static const int32_t four[] = {A2A_GROUP_SEND, A2A_GROUP_RECV, A2A_GROUP_EXPERT, A2A_GROUP_COMBINE}, three[] = {A2A_GROUP_SEND, A2A_GROUP_RECV_EXPERT, A2A_GROUP_COMBINE};
     const bool handed_on = near_phases(group, n) && ((num_phases == 4 && memcmp(phases, four, sizeof(four)) == 0) ||
                                                      (num_phases == 3 && memcmp(phases, three, sizeof(three)) == 0));
-    for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK) rc = group_phase(group, phases[*done], calls, st, handed_on);
+    for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK) rc = group_phase(group, phases[*done], calls, st, handed_on ? &call : nullptr);
     return rc;
 }
 

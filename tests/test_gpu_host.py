@@ -191,3 +191,33 @@ def test_calls_under_graph_capture(what):
         if world is not None:
             world.close()
         release_contexts(barrier=False)
+
+
+def test_a_dispatch_mode_still_hears_of_the_outputs():
+    """Outputs are allocated without the dispatcher only where no mode listens."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Listen(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.shapes = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            out = func(*args, **(kwargs or {}))
+            if "empty" in func.name():
+                self.shapes.append(tuple(out.shape))
+            return out
+
+    cfg = pkg.MoEConfig(8, 2, 64, 4)
+    rds = [pkg.generate_input(8, 2, 64, 4, seed=1, rank=r, world_size=2)[1].to(DEV) for r in range(2)]
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push")
+    world = LocalWorld(cfg, 2, payload="dedup", schedule="pipelined", combine="push")
+    try:
+        want = [ctx.forward(rds[0].x, rds[0].indices, rds[0].weights)] + world.forward_pipelined(rds)
+        with Listen() as heard:
+            got = [ctx.forward(rds[0].x, rds[0].indices, rds[0].weights)] + world.forward_pipelined(rds)
+        assert heard.shapes == [(4, 64)] * 3
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    finally:
+        ctx.close()
+        world.close()
