@@ -330,15 +330,28 @@ __global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid
         const int nt = min(kSoloRound, t1 - r0), pairs = nt * K;
         for (int i = tid; i < pairs; i += kThreads) s_idx[i] = r0 == t0 && i == tid ? first_e : ld_input(p.idx + (size_t)r0 * K + i);
         __syncthreads();
-        resolve_round(p, s_idx, s_cnt, pairs, [&](int i, int tl, int k, int e, int j, bool ok) {
+        for (int i = tid; i < pairs; i += kThreads) {
+            const int tl = i / K, k = i - tl * K, e = s_idx[i];
+            bool ok = e >= 0 && e < p.E;
+            for (int kk = 0; kk < k; ++kk) ok = ok && s_idx[tl * K + kk] != e;
+            int j = -1;
+            if (ok) {
+                j = s_cnt[e];
+                for (int u = 0; u < tl; ++u) {
+                    bool uses = false;
+                    for (int kk = 0; kk < K; ++kk) uses |= s_idx[u * K + kk] == e;
+                    j += uses ? 1 : 0;
+                }
+            }
             const unsigned place = ok ? pair_place(p, e, j) : kNoPair;
             s_place[i] = place;
-            if ((long long)(r0 + tl) * nchunk < lo) return;  // the block that has the token's first chunk books its pairs
-            p.slot[(size_t)r0 * K + i] = j;
-            p.pairs[(size_t)r0 * K + i] = make_uint2(place, 0u);
-            if (ok) reinterpret_cast<int*>(p.peer[place >> 28] + p.off_meta)[place & kPairRow] = ((r0 + tl) << 8) | k;
-            else record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
-        });
+            if ((long long)(r0 + tl) * nchunk >= lo) {  // the block that has the token's first chunk books its pairs
+                p.slot[(size_t)r0 * K + i] = j;
+                p.pairs[(size_t)r0 * K + i] = make_uint2(place, 0u);
+                if (ok) reinterpret_cast<int*>(p.peer[place >> 28] + p.off_meta)[place & kPairRow] = ((r0 + tl) << 8) | k;
+                else record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
+            }
+        }
         __syncthreads();
         for (int i = tid; i < pairs; i += kThreads)
             if (s_place[i] != kNoPair) atomicAdd(s_cnt + s_idx[i], 1);

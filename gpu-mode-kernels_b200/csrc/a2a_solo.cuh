@@ -61,28 +61,6 @@ __device__ __forceinline__ void count_experts_before(const DevParams& p, int t_e
     }
 }
 
-// The pairs of the `pairs / K` tokens of a round, whose indices lie in s_idx: each(i, token, k, expert, slot, valid), by a thread of the
-// block for every pair.  s_cnt: tokens before the round that use an expert.
-template <typename Each>
-__device__ __forceinline__ void resolve_round(const DevParams& p, const int* s_idx, const int* s_cnt, int pairs, Each each) {
-    const int K = p.K;
-    for (int i = threadIdx.x; i < pairs; i += kThreads) {
-        const int tl = i / K, k = i - tl * K, e = s_idx[i];
-        bool ok = e >= 0 && e < p.E;
-        for (int kk = 0; kk < k; ++kk) ok = ok && s_idx[tl * K + kk] != e;
-        int j = -1;
-        if (ok) {
-            j = s_cnt[e];
-            for (int u = 0; u < tl; ++u) {
-                bool uses = false;
-                for (int kk = 0; kk < K; ++kk) uses |= s_idx[u * K + kk] == e;
-                j += uses ? 1 : 0;
-            }
-        }
-        each(i, tl, k, e, j, ok);
-    }
-}
-
 // U 16-byte vectors per lane of one row of x as the expert's rank holds them after dispatch (FP8:
 // through the same quantise / dequantise arithmetic the wire applies).
 template <typename T, int PAYLOAD, int U>
@@ -158,14 +136,27 @@ __global__ void __launch_bounds__(kThreads) solo_kernel(const __grid_constant__ 
         }
         __syncthreads();
         if (r0 == t0) stamp(p, kStampSourceSeen);
-        resolve_round(p, s_idx, s_cnt, pairs, [&](int i, int tl, int k, int e, int j, bool ok) {
+        for (int i = tid; i < pairs; i += kThreads) {
+            const int tl = i / K, k = i - tl * K, e = s_idx[i];
+            const bool in_range = e >= 0 && e < p.E;
+            bool ok = in_range;
+            for (int kk = 0; kk < k; ++kk) ok = ok && s_idx[tl * K + kk] != e;
+            int j = -1;
+            if (ok) {
+                j = s_cnt[e];
+                for (int u = 0; u < tl; ++u) {
+                    bool uses = false;
+                    for (int kk = 0; kk < K; ++kk) uses |= s_idx[u * K + kk] == e;
+                    j += uses ? 1 : 0;
+                }
+            }
             s_row[i] = ok ? e * p.T_max + j : -1;
             if ((long long)(r0 + tl) * nchunk >= lo) {  // the block that has the token's first chunk books its pairs
                 p.slot[(size_t)r0 * K + i] = j;
                 if (ok) meta[(size_t)e * p.T_max + j] = ((r0 + tl) << 8) | k;
                 else record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
             }
-        });
+        }
         __syncthreads();
         for (int i = tid; i < pairs; i += kThreads)
             if (s_row[i] >= 0) atomicAdd(s_cnt + s_idx[i], 1);
