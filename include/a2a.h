@@ -227,7 +227,8 @@ int a2a_pipe_step(a2a_ctx* ctx, int role, const void* x, const int32_t* topk_idx
 /* One phase of EVERY rank of a group that lives on one GPU, as one launch: `group` holds the contexts of
  * all ranks in rank order (same configuration, same device, attached to one another, at the same call).  What runs together never waits for
  * itself, so the phases are called in order -- PIPE_SEND, PIPE_EXPERT, PIPE_COMBINE are the roles of
- * a2a_pipe_step (pipelined contexts; x of every rank is read until PIPE_EXPERT is through); SEND is a2a_route + a2a_dispatch_send, RECV, EXPERT, RECV_EXPERT and
+ * a2a_pipe_step (pipelined contexts; x of every rank is read until PIPE_EXPERT is through, which with the PUSH combine writes
+ * y already where no y lies over an x); SEND is a2a_route + a2a_dispatch_send, RECV, EXPERT, RECV_EXPERT and
  * COMBINE the entry points of those names.  `calls` (one per rank, rank order) is read by PIPE_SEND (all
  * fields), SEND (x, topk_idx, num_tokens) and COMBINE (topk_weights, y), and may be NULL otherwise.
  * Nothing is launched, and no call begun, unless the arguments of every rank are valid. */
