@@ -3,10 +3,10 @@
 Kernels that wait on a peer must never share a GPU with the kernel they wait
 for, so the ranks here are stepped in lock-step: one launch runs a phase of every
 rank, the sending phase before any waiting one, on one stream, and each wait finds its
-flag already set.  Routing, rows, records, flag values and epochs are those of a group
+flag already set.  Routing, rows, flag values and epochs are those of a group
 with a GPU per rank; what depends on where a peer is, is not: flags are awaited at gpu
-scope without watchers, and rows are read where they lie instead of being sent to a stage first
-(csrc/a2a_near.cuh).  The forms for distant peers run in ``forward_one_launch``, which puts every rank's blocks into one cooperative
+scope without watchers, rows are read where they lie and written where they belong instead of being sent to a
+stage, and a token's output is added up where its expert rows are written (csrc/a2a_near.cuh).  The forms for distant peers run in ``forward_one_launch``, which puts every rank's blocks into one cooperative
 launch, and in the phases called context by context.
 Validation tool: parity tests and the smoke check use it to cover world sizes
 2, 4 and 8 on a single device.
