@@ -441,15 +441,15 @@ int launch_near(a2a_ctx* const* cs, NearParams<N>& g, const void* fn, int blocks
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
-// Role 0 of ranks on one GPU: 32 tokens a block (64: two ranks of 200 tokens of 7168 15.4 us a call instead of 15.1), or 256 where there are
-// so many that counting the tokens before the block's shows; up to 256 tokens one thread for each of them (1024 threads: four ranks of two tokens
+// Role 0 of ranks on one GPU: 32 tokens a block (64: two ranks of 200 tokens of 7168 15.4 us a call instead of 15.1), or 64 and 256 where there are
+// so many that counting the tokens before the block's shows (one rank, 5000 tokens of 512 13.7 us with 32, 11.5 with 64; 2048 of 7168 53.0 / 53.1); up to 256 tokens one thread for each of them (1024 threads: four ranks of two tokens
 // 7.9 / 7.4, eight of 16 12.0 / 11.3, of 256 56.6 / 56.2), else 1024 (2048 tokens of one rank, 256 threads 56.9, 512 52.8, 1024 51.8).
 template <int N>
 int launch_near_route(a2a_ctx* const* cs, NearParams<N>& g, cudaStream_t st) {
     int most = 1;
     for (int r = 0; r < g.n; ++r) most = cs[r]->cur_tokens > most ? cs[r]->cur_tokens : most;
     const bool few = N > 1 && most <= kThreads;
-    const int words = most > 8192 ? 8 : 1, nb = (most + 32 * words - 1) / (32 * words);
+    const int words = most > 8192 ? 8 : most > 1024 ? 2 : 1, nb = (most + 32 * words - 1) / (32 * words);
     const void* fn = (const void*)near_route_kernel<N, 1024>;
     if constexpr (N > 1)
         if (few) fn = (const void*)near_route_kernel<N, kThreads>;
