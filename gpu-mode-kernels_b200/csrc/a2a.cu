@@ -939,6 +939,24 @@ int group_phase(a2a_ctx* const* group, int phase, const a2a_call* calls, cudaStr
     }
 }
 
+// The end of several phases of a group in one call, `last` the last that was launched.  Where they were handed on and a later one was
+// refused, or not launched, the flags that it would have raised go up now: the caller may go on phase by phase.
+int end_steps(a2a_ctx* const* group, NearGroup& call, int last, int rc, cudaStream_t st) {
+    if (rc == A2A_OK || call.n == 0) return rc;
+    int owed = 0;
+    switch (last) {
+        case A2A_GROUP_SEND:
+        case A2A_GROUP_PIPE_SEND: owed = 1 << kFlagDispatch; break;
+        case A2A_GROUP_EXPERT:
+        case A2A_GROUP_RECV_EXPERT: owed = 1 << kFlagExpert; break;
+        case A2A_GROUP_PIPE_EXPERT: owed = kBothFlags; break;
+        default: break;
+    }
+    if (owed != 0 && launch_near(group, call, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, owed) != A2A_OK)
+        for (int r = 0; r < call.n; ++r) group[r]->sent = false;  // nothing can follow: later phases are refused and wait for nothing
+    return rc;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1383,13 +1401,13 @@ int a2a_group_steps(a2a_ctx* const* group, const int32_t* phases, int num_phases
         !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2)) {
         rc = do_pipe_send(group, n, calls, st, &call);
         for (; rc == A2A_OK && ++*done < 3;) rc = do_pipe_rest(group, n, *done, st, &call);
-        return rc;
+        return *done == 0 ? rc : end_steps(group, call, phases[*done - 1], rc, st);
     }
     static const int32_t four[] = {A2A_GROUP_SEND, A2A_GROUP_RECV, A2A_GROUP_EXPERT, A2A_GROUP_COMBINE}, three[] = {A2A_GROUP_SEND, A2A_GROUP_RECV_EXPERT, A2A_GROUP_COMBINE};
     const bool handed_on = near_phases(group, n) && ((num_phases == 4 && memcmp(phases, four, sizeof(four)) == 0) ||
                                                      (num_phases == 3 && memcmp(phases, three, sizeof(three)) == 0));
     for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK) rc = group_phase(group, phases[*done], calls, st, handed_on ? &call : nullptr);
-    return rc;
+    return *done == 0 ? rc : end_steps(group, call, phases[*done - 1], rc, st);
 }
 
 int a2a_group_forward(a2a_ctx* const* group, const a2a_call* calls, void* stream) {

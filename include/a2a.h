@@ -244,8 +244,8 @@ typedef struct a2a_call {
 int a2a_group_step(a2a_ctx* const* group, int phase, const a2a_call* calls, void* stream);
 
 /* Several phases of such a group in order, on one stream, as a2a_group_step for each of them; `*done` receives how many
- * were launched before one was refused.  With nothing of the caller's between them, the three roles of a pipelined call
- * take less: see csrc/a2a_near.cuh. */
+ * were launched before one was refused, and the call can go on from there.  With nothing of the caller's between them, the roles
+ * of a pipelined call and the phases of a whole one take less: see csrc/a2a_near.cuh. */
 int a2a_group_steps(a2a_ctx* const* group, const int32_t* phases, int num_phases, const a2a_call* calls, void* stream, int32_t* done);
 
 /* a2a_forward of every rank of such a group (two ranks or more, pipelined contexts) as ONE cooperative launch

@@ -375,3 +375,42 @@ def test_phases_of_a_group_equal_those_rank_by_rank(payload, E, K, H, T, ws):
         assert [c.peek() for c in world.ctxs] == [_lib.A2A_ERR_ROUTING] + [0] * (ws - 1)
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("names", [("send", "recv", "expert", "combine"), ("send", "recv_expert", "combine")])
+@pytest.mark.parametrize("payload", ["direct", "fp8"])
+def test_phases_go_on_after_a_refused_combine(names, payload):
+    """What was launched before the refusal stands as if it had been called phase by phase: the combine follows, for all
+    ranks together or rank by rank, and waits for nothing that never comes."""
+    ws, E, K, H, T = 3, 12, 3, 640, 33
+    rds = [pkg.generate_input(E, K, H, T, seed=10, rank=r, world_size=ws)[1].to(DEV) for r in range(ws)]
+    world = LocalWorld(pkg.MoEConfig(E, K, H, T), ws, payload=payload, timeout_ms=300)
+    lib, handles = world.ctxs[0].lib, (C.c_void_p * ws)(*[c._h.value for c in world.ctxs])
+    phases = (C.c_int32 * len(names))(*[_lib.GROUP_PHASE[name] for name in names])
+    try:
+        want = [bits(y) for y in world.forward_phases(rds)]
+        tables = state(world)
+        for field, wrong in (("y", 0), ("y", 2), ("topk_weights", 0)):  # missing, off a 16-byte boundary, missing
+            for together in (True, False):
+                ys, calls, done = [torch.full_like(rd.x, 3) for rd in rds], (_lib.Call * ws)(), C.c_int32()
+                for c, call, rd, y in zip(world.ctxs, calls, rds, ys):
+                    call.x, call.topk_idx, call.topk_weights = rd.x.data_ptr(), rd.indices.data_ptr(), rd.weights.data_ptr()
+                    call.y, call.num_tokens = y.data_ptr(), rd.num_tokens
+                    c._num_tokens = rd.num_tokens
+                good = getattr(calls[ws - 1], field)
+                setattr(calls[ws - 1], field, good + wrong if wrong else None)
+                rc = lib.a2a_group_steps(handles, phases, len(names), calls, _lib.current_stream(), C.byref(done))
+                assert rc == _lib.A2A_ERR_CONFIG and done.value == len(names) - 1
+                setattr(calls[ws - 1], field, good)
+                if together:
+                    world._step("combine", calls)
+                else:
+                    ys = [c.combine(rd.weights) for c, rd in zip(world.ctxs, rds)]
+                torch.cuda.synchronize()
+                world.check()
+                assert all(torch.equal(bits(y), w) for y, w in zip(ys, want))
+                assert all(torch.equal(a, b) for a, b in zip(state(world), tables))
+        assert all(torch.equal(bits(y), w) for y, w in zip(world.forward_phases(rds), want))
+        world.check()
+    finally:
+        world.close()
