@@ -558,10 +558,19 @@ bool solo_two_launches(const a2a_ctx* c) {
     return mb >= 40 || (mb >= 16 && c->cur_tokens >= 800) || (mb >= 4 && c->cur_tokens >= 1280);
 }
 
+inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
+}
+
 int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     const long long nvec = c->cfg.hidden_dim / 8, warps = kThreads / 32, cap = host_rows ? c->num_sms / 2 : 2LL * c->num_sms;
     const long long two = c->cur_tokens * ((nvec + 63) / 64), one = c->cur_tokens * ((nvec + 31) / 32);
-    if (!host_rows && c->p.trace == nullptr && solo_two_launches(c)) {
+    // An output laid over the weights or the indices: the one launch reads them block by block while other blocks already write,
+    // the routing launch reads them all before the first row is written.
+    const size_t tk = (size_t)c->cur_tokens * c->cfg.experts_per_token * 4, rows = (size_t)c->cur_tokens * c->cfg.hidden_dim * 2;
+    const bool over = !host_rows && tk > 0 && (overlap(c->p.y, rows, c->p.w, tk) || overlap(c->p.y, rows, c->p.idx, tk));
+    if (over || (!host_rows && c->p.trace == nullptr && solo_two_launches(c))) {
         NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, /*backwards=*/0, /*handed_on=*/1};
         const int rc = launch_near_route(&c, g, st);
         return rc != A2A_OK ? rc : launch_near_rows(&c, g, /*push=*/false, /*whole=*/true, st);
@@ -595,11 +604,6 @@ void* mapped_address(const void* host, size_t bytes) {
     if (query(4, what, into, at) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || device == 0) return nullptr;
     if (at < start || at + bytes > start + size) return nullptr;
     return reinterpret_cast<void*>(device);
-}
-
-inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
-    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-    return x < y + nb && y < x + na;
 }
 
 int check_call(const a2a_ctx* c, const int32_t* idx, int T) {
@@ -1284,16 +1288,6 @@ int a2a_forward(a2a_ctx* c, const void* x, const int32_t* idx, const float* w, v
     if (c == nullptr) return A2A_ERR_CONFIG;
     DeviceGuard guard(c->cfg.device);
     cudaStream_t st = as_stream(stream);
-    const size_t tk = T > 0 ? (size_t)T * c->cfg.experts_per_token * 4 : 0, rows = T > 0 ? (size_t)T * c->cfg.hidden_dim * 2 : 0;
-    if (c->cfg.schedule == A2A_SCHEDULE_PIPELINED && c->cfg.world_size == 1 && T > 0 &&
-        (overlap(y, rows, w, tk) || overlap(y, rows, idx, tk))) {
-        // An output laid over the weights: the one launch of a single rank reads them block by block while other
-        // blocks already write.  The roles read them all before the first row is written.
-        const a2a_call call = {x, idx, w, y, T};
-        int rc = do_pipe_send(&c, 1, &call, st);
-        for (int role = 1; role <= 2 && rc == A2A_OK; ++role) rc = do_pipe_rest(&c, 1, role, st);
-        return rc;
-    }
     int r = begin_call(c, idx, T);
     if (r != A2A_OK) return r;
     if (T > 0 && (x == nullptr || w == nullptr || y == nullptr)) return A2A_ERR_CONFIG;

@@ -195,7 +195,7 @@ int a2a_combine(a2a_ctx* ctx, const float* topk_weights, void* y, void* stream);
 /* route + dispatch + expert placeholder + combine in one call; what
  * custom_kernel(data) runs.  Replaces torch.ops.p2p_module.custom_kernel
  * (submission_v9.py:734-831).  `y` may lie exactly over `x` with one rank; there it may also lie
- * over the weights (pipelined schedule). */
+ * over the weights or the indices (pipelined schedule). */
 int a2a_forward(a2a_ctx* ctx, const void* x, const int32_t* topk_idx, const float* topk_weights,
                 void* y, int num_tokens, void* stream);
 

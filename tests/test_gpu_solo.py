@@ -305,3 +305,35 @@ def test_output_laid_over_an_input(payload, H, over):
     finally:
         torch.cuda.synchronize()
         ctx.close()
+
+
+@pytest.mark.parametrize("over", ["weights", "indices"])
+@pytest.mark.parametrize("combine", ["push", "pull"])
+@pytest.mark.parametrize("payload,H,T,K", [("dedup", 72, 6000, 2), ("dedup", 2056, 37, 5), ("fp8", 256, 700, 8), ("dedup", 64, 1, 3)])
+def test_weights_and_indices_are_read_before_the_first_row_is_written(payload, H, T, K, combine, over):
+    """An output laid over them, with a repeat and a token without a valid expert, in every combine mode: slots and
+    outputs to the bit."""
+    cfg, rd, _, _ = pkg.generate_input(8, K, H, T, seed=42, rank=0, world_size=1, weights="rand")
+    rd.indices[T - 1, :] = 8
+    rd.indices[0, K - 1] = rd.indices[0, 0]
+    d = rd.to(DEV)
+    ctx = A2AContext(cfg, 0, 1, device=0, payload=payload, schedule="pipelined", combine=combine)
+    try:
+        want = bits(ctx.forward(d.x, d.indices, d.weights))
+        tables = [t.clone() for t in ctx.route_tables() + ctx.export_dispatch()]
+        for at in (0, 8, (T * H - 2 * T * K) // 8 * 8):
+            if at + 2 * T * K > T * H:
+                continue
+            y = torch.full_like(d.x, 7)
+            idx, w = d.indices, d.weights
+            place = y.view(-1)[at:at + 2 * T * K]
+            if over == "weights":
+                w = place.view(torch.float32).view(T, K).copy_(d.weights)
+            else:
+                idx = place.view(torch.int32).view(T, K).copy_(d.indices)
+            assert torch.equal(bits(ctx.forward(d.x, idx, w, y)), want)
+            assert all(torch.equal(a, b) for a, b in zip(ctx.route_tables() + ctx.export_dispatch(), tables))
+        assert ctx.peek() == _lib.A2A_ERR_ROUTING and not want[T - 1].any()
+    finally:
+        torch.cuda.synchronize()
+        ctx.close()
