@@ -91,8 +91,8 @@ struct a2a_ctx {
     bool recorded;          // roles 1 and 2 can follow: the call was begun by role 0, or by the one launch of several ranks
     bool near;              // ... by role 0 of a group on this GPU: rows stay where they are
     bool whole;             // ... and role 1 of the group has written the outputs too
-    bool listed;            // every pair's place is in p.pairs
-    bool placed;            // ... and its row in its slab, whatever the payload
+    bool listed;            // every pair's place is in p.pairs: role 0 or SEND of the group ran
+    bool placed;            // ... SEND: and its row in its slab, whatever the payload
     bool backwards;         // the last launch that wrote the expert rows of the group began with the last tokens
     const void* near_x[A2A_MAX_WORLD];  // input rows of every rank in this call
     const uint2* near_pairs[A2A_MAX_WORLD];
@@ -331,8 +331,9 @@ const void* rows_fn(bool push, bool whole, bool narrow) {
 
 // the kernels of the phases and the combine of ranks on one GPU: element type, U vectors a lane
 template <typename T, int U>
-const void* near_combine_fn(bool push) {
-    return push ? (const void*)near_combine_kernel<T, true, U> : (const void*)near_combine_kernel<T, false, U>;
+const void* near_combine_fn(bool push, bool listed) {
+    if (push) return (const void*)near_combine_kernel<T, true, true, U>;
+    return listed ? (const void*)near_combine_kernel<T, false, true, U> : (const void*)near_combine_kernel<T, false, false, U>;
 }
 template <typename T, int U>
 const void* near_dispatch_fn(bool fp8) {
@@ -500,11 +501,11 @@ bool beyond_l2(const a2a_ctx* c, const NearGroup& g) {
 
 // The combine: 512 bytes of a token's output a warp, 1 KB where fewer than six rows are added up (a call by
 // phases, us, 512 bytes / 1 KB: four ranks of 200 tokens of 6144, top-2, 26.2 / 25.6; two of 256 of 7168, top-8, 38.4 / 39.3).
-int launch_near_combine(a2a_ctx* const* cs, NearGroup& g, bool push, cudaStream_t st) {
+int launch_near_combine(a2a_ctx* const* cs, NearGroup& g, bool push, bool listed, cudaStream_t st) {
     g.backwards = !cs[0]->backwards && beyond_l2(cs[0], g);
     const bool bf = cs[0]->cfg.dtype == A2A_DTYPE_BF16, wide = cs[0]->cfg.experts_per_token < 6;
-    const void* fn = wide ? (bf ? near_combine_fn<__nv_bfloat16, 2>(push) : near_combine_fn<__half, 2>(push))
-                          : (bf ? near_combine_fn<__nv_bfloat16, 1>(push) : near_combine_fn<__half, 1>(push));
+    const void* fn = wide ? (bf ? near_combine_fn<__nv_bfloat16, 2>(push, listed) : near_combine_fn<__half, 2>(push, listed))
+                          : (bf ? near_combine_fn<__nv_bfloat16, 1>(push, listed) : near_combine_fn<__half, 1>(push, listed));
     return launch_near(cs, g, fn, near_blocks(cs[0], g, wide ? 2 : 1), 0, st);
 }
 
@@ -677,7 +678,7 @@ int do_send(a2a_ctx* const* cs, int n, const void* const* x, cudaStream_t st, Ne
     const long long items = direct ? T * c->cfg.experts_per_token * ((nvec + 127) / 128) : T * ((nvec + 31) / 32);
     const int rc = launch_ranks(cs, n, select_tp<SendSel>(c), grid_for_ranks(c, n, (items + warps - 1) / warps, 4), c->smem_bytes, st);
     if (rc == A2A_OK)
-        for (int r = 0; r < n; ++r) cs[r]->sent = cs[r]->listed = true;
+        for (int r = 0; r < n; ++r) cs[r]->sent = true;
     return rc;
 }
 
@@ -725,13 +726,13 @@ int do_combine(a2a_ctx* const* cs, int n, const float* const* w, void* const* y,
     const a2a_ctx* c = cs[0];
     bool listed = true;
     for (int r = 0; r < n; ++r) listed = listed && cs[r]->listed;
-    if (listed && near_phases(cs, n)) {
+    if (near_phases(cs, n)) {
         NearGroup own, &g = near_call(cs, n, call, own);
         for (int r = 0; r < n; ++r) {
             g.p[r].w = w[r];
             g.p[r].y = y[r];
         }
-        return launch_near_combine(cs, g, /*push=*/false, st);
+        return launch_near_combine(cs, g, /*push=*/false, listed, st);
     }
     const int nseg = (c->cfg.hidden_dim / 8 + 63) / 64;  // a warp per (token, 1 KB segment)
     const long long warps = (long long)most_tokens(cs, n) * nseg;
@@ -828,7 +829,7 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, NearGroup
         // a role 2 is through when every rank is through with this call, whoever's rows its tokens want
         if (whole) return launch_near(cs, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, kBothFlags);
         g.every_rank = 1;
-        return launch_near_combine(cs, g, push, st);
+        return launch_near_combine(cs, g, push, /*listed=*/true, st);
     }
     for (int r = 0; r < n; ++r) {
         int rc;
@@ -847,7 +848,7 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, NearGroup
             NearGroup g;
             near_params(cs + r, 1, g);
             g.every_rank = 1;
-            rc = launch_near_combine(cs + r, g, push, st);
+            rc = launch_near_combine(cs + r, g, push, /*listed=*/true, st);
         }
         if (rc != A2A_OK) return rc;
     }

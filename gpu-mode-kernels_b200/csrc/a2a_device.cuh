@@ -144,10 +144,10 @@ __device__ __forceinline__ void begin_after_previous() {
 constexpr unsigned kNoPair = 0xffffffffu, kPairRow = 0x0fffffffu;
 static_assert((long long)A2A_MAX_EXPERTS * 65535 < 1 << 28 && A2A_MAX_WORLD <= 8, "a slab row fits 28 bits, a rank three");
 
-// Pair (t, k) of rank p with slot j of expert e.
-__device__ __forceinline__ unsigned pair_place(const DevParams& p, int e, int j) {
+// Pair of rank `source` with slot j of expert e; p: of any rank of the group.
+__device__ __forceinline__ unsigned pair_place(const DevParams& p, int source, int e, int j) {
     const int d = e / p.L;
-    return (unsigned)d << 28 | (unsigned)(((e - d * p.L) * p.ws + p.rank) * p.T_max + j);
+    return (unsigned)d << 28 | (unsigned)(((e - d * p.L) * p.ws + source) * p.T_max + j);
 }
 
 __device__ __forceinline__ long long global_ns() {

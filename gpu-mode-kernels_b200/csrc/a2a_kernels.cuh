@@ -177,14 +177,12 @@ __device__ __forceinline__ void send_staged(const DevParams& p, const BlockSmem&
         if (lane < K) {
             const int e = s.idx[t * K + lane];
             const int j = pair_slot(p, s, t, lane, e);
-            const unsigned place = j >= 0 ? pair_place(p, e, j) : kNoPair;
-            if (v0 == 0) {
-                p.slot[(size_t)t * K + lane] = j;
-                p.pairs[(size_t)t * K + lane] = make_uint2(place, 0u);
-            }
+            if (v0 == 0) p.slot[(size_t)t * K + lane] = j;
             if (j >= 0) {
-                want = 1u << (place >> 28);
-                if (v0 == 0) reinterpret_cast<int*>(p.peer[place >> 28] + p.off_meta)[place & kPairRow] = (t << 8) | lane;
+                const int d = e / p.L;
+                want = 1u << d;
+                if (v0 == 0)
+                    reinterpret_cast<int*>(p.peer[d] + p.off_meta)[((size_t)(e - d * p.L) * p.ws + p.rank) * p.T_max + j] = (t << 8) | lane;
             }
         }
         want = __reduce_or_sync(0xffffffffu, want);
@@ -247,13 +245,9 @@ __device__ __forceinline__ void send_chunk(const DevParams& p, const BlockSmem& 
             }
             const int e = s.idx[pair];
             const int j = pair_slot(p, s, t, k, e);
-            const unsigned place = j >= 0 ? pair_place(p, e, j) : kNoPair;
-            if (lane == 0 && v0 == 0) {
-                p.slot[pair] = j;
-                p.pairs[pair] = make_uint2(place, 0u);
-            }
+            if (lane == 0 && v0 == 0) p.slot[pair] = j;
             if (j < 0) continue;
-            const unsigned d = place >> 28;
+            const unsigned place = pair_place(p, p.rank, e, j), d = place >> 28;
             const size_t row = place & kPairRow;
             uint4* dst = reinterpret_cast<uint4*>(p.peer[d] + p.off_rows) + row * nvec;
 #pragma unroll

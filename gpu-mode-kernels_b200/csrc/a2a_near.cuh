@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(THREADS) near_route_kernel(const __grid_consta
                 j = s_cnt[e];
                 for (int w = 0; w < tl >> 5; ++w) j += __popc(s_bits[w * E + e]);
                 j += __popc(s_bits[(tl >> 5) * E + e] & ((1u << (tl & 31)) - 1u));
-                place = pair_place(p, e, j);
+                place = pair_place(p, p.rank, e, j);
                 reinterpret_cast<int*>(p.peer[place >> 28] + p.off_meta)[place & kPairRow] = ((t0 + tl) << 8) | (i - tl * K);
             } else {
                 record_error(p.status, A2A_ERR_ROUTING, p.rank, -1, kPhaseRoute, p.epoch, e);
@@ -286,11 +286,21 @@ struct NearItem {
 };
 
 // Lane k: where the slab row of the item's pair k lies (this lane's first vector of it), and at which rank; -1: nowhere.
+// LISTED: role 0 or SEND of the group has left the places; else they follow from the slots and the caller's indices.
+template <bool LISTED>
 __device__ __forceinline__ unsigned long long near_row(const NearGroup& g, int s, int t, int v0, int& rank) {
     const DevParams& p0 = g.p[0];
     const int lane = threadIdx.x & 31;
     unsigned place = kNoPair;
-    if (lane < p0.K) place = ld_stream(g.pairs[s] + (size_t)t * p0.K + lane).x;
+    if (lane < p0.K) {
+        const size_t pair = (size_t)t * p0.K + lane;
+        if (LISTED) {
+            place = ld_stream(g.pairs[s] + pair).x;
+        } else {
+            const int e = ld_input(g.p[s].idx + pair), j = ld_stream(g.p[s].slot + pair);
+            if (j >= 0) place = pair_place(p0, s, e, j);
+        }
+    }
     rank = place == kNoPair ? -1 : (int)(place >> 28);
     if (rank < 0) return 0;
     return reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[rank] + p0.off_rows) + (size_t)(place & kPairRow) * (p0.H >> 3));
@@ -343,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid
                     j += uses ? 1 : 0;
                 }
             }
-            const unsigned place = ok ? pair_place(p, e, j) : kNoPair;
+            const unsigned place = ok ? pair_place(p, p.rank, e, j) : kNoPair;
             s_place[i] = place;
             if ((long long)(r0 + tl) * nchunk >= lo) {  // the block that has the token's first chunk books its pairs
                 p.slot[(size_t)r0 * K + i] = j;
@@ -416,7 +426,7 @@ __global__ void __launch_bounds__(kThreads) near_expert_kernel(const __grid_cons
     const NearItem<1> at(g);
     if (at.there && (!WAIT || g.handed_on || (s_missing >> at.s & 1) == 0)) {
         int rank;
-        const unsigned long long my_row = near_row(g, at.s, at.t, at.v0, rank);
+        const unsigned long long my_row = near_row<true>(g, at.s, at.t, at.v0, rank);
         const unsigned there = __ballot_sync(0xffffffffu, rank >= 0);
         for (int k0 = 0; k0 < K; k0 += 8) {  // eight rows are requested before the first is written
             uint4 q[8];
@@ -444,13 +454,13 @@ __global__ void __launch_bounds__(kThreads) near_expert_kernel(const __grid_cons
 //   PUSH: y[t] = T(sum over the ranks d holding experts of t, ascending, of float(partial[d][t])).
 //   PULL: y[t] = T(sum over k of w[t,k] * float(row k)), eight rows requested before the first is used.
 // ---------------------------------------------------------------------------
-template <typename T, bool PUSH, int U>
+template <typename T, bool PUSH, bool LISTED, int U>
 __global__ void __launch_bounds__(kThreads) near_combine_kernel(const __grid_constant__ NearGroup g) {
     begin_after_previous();
     const DevParams& p0 = g.p[0];
     const int tid = threadIdx.x, lane = tid & 31, ws = p0.ws, nvec = p0.H >> 3;
     stamp(p0, kStampStart);
-    if (g.handed_on) {
+    if (!PUSH && g.handed_on) {  // roles that are handed on have written the outputs
         if (blockIdx.x == 0) raise_flags(g, 1u << kFlagExpert, recorded_of_rank(g));
     } else if (PUSH) {
         bool ok = true;
@@ -474,7 +484,7 @@ __global__ void __launch_bounds__(kThreads) near_combine_kernel(const __grid_con
             if (lane < ws) up = (int32_t)(ld_relaxed_gpu(await_ptr(p, kFlagExpert, lane)) - flag_value(p, 0)) >= 0;
             fence_acq_rel_gpu();
         }
-        my_row = near_row(g, at.s, at.t, at.v0, rank);
+        my_row = near_row<LISTED>(g, at.s, at.t, at.v0, rank);
         if (!PUSH && lane < p0.K) my_w = ld_input(p.w + (size_t)at.t * p0.K + lane);
         const unsigned missing = ~__ballot_sync(0xffffffffu, up);
         if (!PUSH && __any_sync(0xffffffffu, rank >= 0 && (missing >> rank & 1u))) {
