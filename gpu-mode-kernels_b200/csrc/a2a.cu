@@ -100,6 +100,7 @@ struct a2a_ctx {
     uint32_t epoch, barrier_epoch;
     int cur_tokens;
     int64_t launches;
+    unsigned direct_opted_in;  // a bit for each receive-side kernel of the direct payload that may have this context's shared memory
     cudaStream_t side;      // private stream for status reads
     int* host_code;         // mapped host word mirroring the device status code
     // device staging for the host-buffer entry point
@@ -705,7 +706,11 @@ int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, boo
     // Sent together, received rank by rank: there is nothing in the stages.
     const PhaseFn fn = cs[0]->cfg.dtype == A2A_DTYPE_BF16 ? ExpertSel<__nv_bfloat16, A2A_PAYLOAD_DIRECT>::get(wait, fanout, scale, publish)
                                                           : ExpertSel<__half, A2A_PAYLOAD_DIRECT>::get(wait, fanout, scale, publish);
-    CUDA_TRY(cudaFuncSetAttribute((const void*)fn.one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes));
+    const unsigned kernel = 1u << ((wait ? 1 : 0) + (scale ? 2 : 0));
+    if ((cs[0]->direct_opted_in & kernel) == 0) {  // a2a_create has opted in for the context's own payload
+        CUDA_TRY(cudaFuncSetAttribute((const void*)fn.one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmemBytes));
+        cs[0]->direct_opted_in |= kernel;
+    }
     for (int r = 0; r < n; ++r) {
         const int rc = launch(cs[r], (const void*)fn.one, grid, cs[r]->smem_bytes, st);
         if (rc != A2A_OK) return rc;
