@@ -11,6 +11,7 @@
 
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_cuda_dispatch.h>
+#include <ATen/record_function.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -64,9 +65,9 @@ bool call_of(const Rank* r, PyObject* x, PyObject* idx, PyObject* w, a2a_call& c
 
 at::Tensor output_of(const Rank* r, a2a_call& c) {
     const at::TensorOptions options = at::TensorOptions().dtype(r->dtype).device(at::kCUDA, (c10::DeviceIndex)r->device);
-    // the allocation itself, unless a mode wants to hear of operators
-    at::Tensor y = c10::impl::dispatch_mode_enabled() ? at::empty({c.num_tokens, r->hidden}, options)
-                                                      : at::cuda::empty({c.num_tokens, r->hidden}, options);
+    // the allocation itself, unless a mode or an observer (a profiler) wants to hear of operators
+    const bool heard = c10::impl::dispatch_mode_enabled() || at::hasCallbacks();
+    at::Tensor y = heard ? at::empty({c.num_tokens, r->hidden}, options) : at::cuda::empty({c.num_tokens, r->hidden}, options);
     c.y = y.mutable_data_ptr();
     return y;
 }

@@ -221,3 +221,22 @@ def test_a_dispatch_mode_still_hears_of_the_outputs():
     finally:
         ctx.close()
         world.close()
+
+
+def test_a_profiler_still_sees_the_outputs():
+    """Observers of operators are no modes; they too hear of every output."""
+    from torch.profiler import ProfilerActivity, profile
+
+    cfg = pkg.MoEConfig(8, 2, 64, 4)
+    rds = [pkg.generate_input(8, 2, 64, 4, seed=1, rank=r, world_size=2)[1].to(DEV) for r in range(2)]
+    ctx = A2AContext(cfg, 0, 1, device=0, payload="dedup", schedule="pipelined", combine="push")
+    world = LocalWorld(cfg, 2, payload="dedup", schedule="pipelined", combine="push")
+    try:
+        want = [ctx.forward(rds[0].x, rds[0].indices, rds[0].weights)] + world.forward_pipelined(rds)
+        with profile(activities=[ProfilerActivity.CPU]) as seen:
+            got = [ctx.forward(rds[0].x, rds[0].indices, rds[0].weights)] + world.forward_pipelined(rds)
+        assert [e.name for e in seen.events()].count("aten::empty") == 3
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    finally:
+        ctx.close()
+        world.close()
