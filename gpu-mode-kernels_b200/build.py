@@ -64,7 +64,8 @@ def build_host(verbose: bool = False) -> None:
                sysconfig.get_paths()["include"]]
     run("g++", [
         os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
-        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + d for d in include), "-o", host_path(), HOST_SOURCE, "-L" + os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + d for d in include), "-o", host_path(), HOST_SOURCE,
+        "-L" + os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
         "-L" + PKG_DIR, "-la2a", "-Wl,-rpath,$ORIGIN",
     ], verbose)
 

@@ -324,8 +324,10 @@ KernelFn solo_fn(const a2a_ctx* c) {
 template <typename T, int P, int N>
 const void* rows_fn(bool push, bool whole, bool narrow) {
     if constexpr (N > 1) {
-        if (!whole) return push ? (const void*)near_rows_kernel<T, P, true, false, 1, N> : (const void*)near_rows_kernel<T, P, false, false, 1, N>;
-        if (push) return narrow ? (const void*)near_rows_kernel<T, P, true, true, 1, N> : (const void*)near_rows_kernel<T, P, true, true, 2, N>;
+        if (!whole)
+            return push ? (const void*)near_rows_kernel<T, P, true, false, 1, N> : (const void*)near_rows_kernel<T, P, false, false, 1, N>;
+        if (push)
+            return narrow ? (const void*)near_rows_kernel<T, P, true, true, 1, N> : (const void*)near_rows_kernel<T, P, true, true, 2, N>;
     }
     return narrow ? (const void*)near_rows_kernel<T, P, false, true, 1, N> : (const void*)near_rows_kernel<T, P, false, true, 2, N>;
 }
@@ -443,9 +445,10 @@ int launch_near(a2a_ctx* const* cs, NearParams<N>& g, const void* fn, int blocks
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }
 
-// Role 0 of ranks on one GPU: 32 tokens a block (64: two ranks of 200 tokens of 7168 15.4 us a call instead of 15.1), or 64 and 256 where there are
-// so many that counting the tokens before the block's shows (one rank, 5000 tokens of 512 13.7 us with 32, 11.5 with 64; 2048 of 7168 53.0 / 53.1); up to 256 tokens one thread for each of them (1024 threads: four ranks of two tokens
-// 7.9 / 7.4, eight of 16 12.0 / 11.3, of 256 56.6 / 56.2), else 1024 (2048 tokens of one rank, 256 threads 56.9, 512 52.8, 1024 51.8).
+// Role 0 of ranks on one GPU.  Tokens a block: 32 (64: eight ranks of 256 tokens of 7168 56.5 for 54.3, two of 200 15.8 / 14.4), or
+// 64 and 256 where there are so many that counting the tokens before the block's shows (32 at 5000 tokens of 512, one rank: 13.0 for
+// 10.9; 2048 of 7168: 52.0 / 52.3).  Threads: one for each token up to 256 (1024: four ranks of two tokens 6.7 for 6.4, eight of
+// 16 10.6 / 9.6, of 256 54.8 / 54.3), else 1024 (256 at two ranks of 1000 tokens of 2048: 18.7 for 17.6; four of 2000 of 512 15.5 / 13.4).
 template <int N>
 int launch_near_route(a2a_ctx* const* cs, NearParams<N>& g, cudaStream_t st) {
     int most = 1;
@@ -460,10 +463,10 @@ int launch_near_route(a2a_ctx* const* cs, NearParams<N>& g, cudaStream_t st) {
 }
 
 // Role 1: a warp per 1 KB of a token's row, three blocks per SM, or per 512 bytes where that would be too few rounds of blocks:
-// two where six or more stores follow each load, one where fewer do.  Calls of a group, 512 bytes / 1 KB (rounds of the
-// latter): top-8 of 7168, 256 tokens, eight ranks 64.6 / 56.4 us (8.1), two ranks 18.6 / 19.6 (2.0), 200 tokens 15.1 / 16.5 (1.6); top-6 of 2048,
-// 256 tokens, eight ranks 21.4 / 19.8 (2.3); top-2 of 6144, 110 tokens, eight 17.4 / 15.5 (2.9), four 11.8 / 11.3 (1.5), 256, two 11.5 / 10.8
-// (1.7); top-4 of 2880, 110, eight 14.6 / 14.1 (1.5).
+// 2.2 where six or more stores follow each load, one where fewer do.  512 bytes / 1 KB (rounds of the latter): top-8 of 7168,
+// 256 tokens, eight ranks 55.8 / 54.4 (8.1), two ranks 17.2 / 17.6 (2.0), 200 tokens 14.4 / 15.1 (1.6); top-6 of 2048, 256 tokens,
+// eight ranks 17.8 / 17.6 (2.3); top-2 of 6144, 110 tokens, eight 16.3 / 14.0 (2.9), four 10.6 / 9.8 (1.5), 256, two 10.3 / 9.7 (1.7);
+// top-4 of 2880, 110, eight 12.8 / 12.2 (1.5).
 template <int N>
 int launch_near_rows(a2a_ctx* const* cs, NearParams<N>& g, bool push, bool whole, cudaStream_t st) {
     const a2a_ctx* c = cs[0];
@@ -473,9 +476,11 @@ int launch_near_rows(a2a_ctx* const* cs, NearParams<N>& g, bool push, bool whole
     const bool many = whole && 2 * tokens * wide >= (c->cfg.experts_per_token >= 6 ? 13LL : 6LL) * c->num_sms * warps;
     const long long items = tokens * (many ? wide : narrow), blocks = items > 0 ? (items + warps - 1) / warps : 1;
     const bool bf = c->cfg.dtype == A2A_DTYPE_BF16;
-    const void* fn = c->cfg.payload == A2A_PAYLOAD_FP8
-        ? (bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_FP8, N>(push, whole, !many) : rows_fn<__half, A2A_PAYLOAD_FP8, N>(push, whole, !many))
-        : (bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_DEDUP, N>(push, whole, !many) : rows_fn<__half, A2A_PAYLOAD_DEDUP, N>(push, whole, !many));
+    const void* fn;
+    if (c->cfg.payload == A2A_PAYLOAD_FP8)
+        fn = bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_FP8, N>(push, whole, !many) : rows_fn<__half, A2A_PAYLOAD_FP8, N>(push, whole, !many);
+    else
+        fn = bf ? rows_fn<__nv_bfloat16, A2A_PAYLOAD_DEDUP, N>(push, whole, !many) : rows_fn<__half, A2A_PAYLOAD_DEDUP, N>(push, whole, !many);
     return launch_near(cs, g, fn, (int)blocks, 0, st);
 }
 
@@ -493,7 +498,8 @@ int near_blocks(const a2a_ctx* c, const NearParams<N>& g, int U) {
 constexpr int kBothFlags = 1 << kFlagDispatch | 1 << kFlagExpert;
 
 // Where the expert rows are more than the L2 keeps, a phase begins with those that the one before it wrote last: eight ranks of 200
-// tokens of 7168, top-8 of 256 experts, 183 MB, 132 -> 131 us a call by phases; 128 tokens, 117 MB, 81.4 / 80.6.  Below 64 MB no difference.
+// tokens of 7168, top-8 of 256 experts, 183 MB, 129.7 a call by phases, 131.9 without; 128 tokens, 117 MB, 79.8 / 80.9.  Below
+// 64 MB no difference.
 bool beyond_l2(const a2a_ctx* c, const NearGroup& g) {
     long long tokens = 0;
     for (int s = 0; s < c->cfg.world_size; ++s) tokens += g.T[s];
@@ -501,7 +507,7 @@ bool beyond_l2(const a2a_ctx* c, const NearGroup& g) {
 }
 
 // The combine: 512 bytes of a token's output a warp, 1 KB where fewer than six rows are added up (a call by
-// phases, us, 512 bytes / 1 KB: four ranks of 200 tokens of 6144, top-2, 26.2 / 25.6; two of 256 of 7168, top-8, 38.4 / 39.3).
+// phases, 512 bytes / 1 KB: four ranks of 200 tokens of 6144, top-2, 25.6 / 25.1; two of 256 of 7168, top-8, 37.7 / 38.7).
 int launch_near_combine(a2a_ctx* const* cs, NearGroup& g, bool push, bool listed, cudaStream_t st) {
     g.backwards = !cs[0]->backwards && beyond_l2(cs[0], g);
     const bool bf = cs[0]->cfg.dtype == A2A_DTYPE_BF16, wide = cs[0]->cfg.experts_per_token < 6;
@@ -510,10 +516,11 @@ int launch_near_combine(a2a_ctx* const* cs, NearGroup& g, bool push, bool listed
     return launch_near(cs, g, fn, near_blocks(cs[0], g, wide ? 2 : 1), 0, st);
 }
 
-// RECV, of rows that SEND has put into their slabs, EXPERT and RECV_EXPERT: 512 bytes a warp (1 KB: two ranks of 256 tokens of 7168 39.2 us
-// a call by phases instead of 38.4).
+// RECV, of rows that SEND has put into their slabs, EXPERT and RECV_EXPERT: 512 bytes a warp (1 KB: two ranks of 256 tokens of
+// 7168, by phases, 2 % slower when it was tried).
 int launch_near_expert(a2a_ctx* const* cs, NearGroup& g, bool wait, bool scale, cudaStream_t st) {
-    if (!scale) return launch_near(cs, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, 1 << kFlagDispatch);
+    if (!scale)
+        return launch_near(cs, g, (const void*)near_flags_kernel, 1, 0, st, A2A_MAX_WORLD * A2A_MAX_WORLD, 1 << kFlagDispatch);
     g.backwards = beyond_l2(cs[0], g);
     for (int r = 0; r < g.n; ++r) cs[r]->backwards = g.backwards;
     const bool bf = cs[0]->cfg.dtype == A2A_DTYPE_BF16;
@@ -522,9 +529,9 @@ int launch_near_expert(a2a_ctx* const* cs, NearGroup& g, bool wait, bool scale, 
     return launch_near(cs, g, fn, near_blocks(cs[0], g, 1), 0, st);
 }
 
-// SEND: as many blocks as are resident together, three per SM, each of which counts the experts of the tokens before its own; a second round
-// of them costs 3 us (phases of two ranks, 256 tokens of 2048, 15.9 us a call with three, 19.3 with six).  1 KB a warp where every warp
-// has that much, else 512 bytes.
+// SEND: as many blocks as are resident together, three per SM, each of which counts the experts of the tokens before its own; a
+// second round of them costs 3 us (by phases, two ranks of 256 tokens of 2048, 15.3 with three per SM, 18.8 with six).  1 KB a warp
+// where every warp has that much, else 512 bytes.
 int launch_near_dispatch(a2a_ctx* const* cs, NearGroup& g, cudaStream_t st) {
     const a2a_ctx* c = cs[0];
     int most = 0;
@@ -543,18 +550,19 @@ int launch_near_dispatch(a2a_ctx* const* cs, NearGroup& g, cudaStream_t st) {
 
 // The forward of one rank.  A warp's item is one or two 16-byte vectors per lane of a token's row: two
 // where that still gives every warp of two blocks per SM an item (headline workload, 256 tokens of 7168:
-// 9.4 us against 9.7 with one and 10.2 with four; 2048 tokens 61.0 / 62.1 / 61.5), one below that, where
-// more warps with less to do each finish sooner (one token of 2048: 4.1 against 4.2 and 4.6 us).  Two
-// blocks per SM: with a third or fourth that does not fit beside them a second, nearly empty wave of
-// blocks starts after the first (headline 13.2 us).
-// Rows in host memory: half an SM's worth of warps fills the link, and more only get in each other's way
-// (3.7 MB read and as much written by 74 / 148 / 296 blocks: 100 / 107 / 118 us).
-// Many tokens, or rows that outweigh a second launch: the routing of a group of one and then its rows (a2a_near.cuh).  Back to back,
-// us a call, the one launch and the two, by MB of expert rows: top-8 of 7168, 400 tokens 13.0 / 13.0 (46), 512 16.4 / 15.7 (59), 1000
-// 30.9 / 28.0; top-8 of 4096, 512 11.3 / 11.6 (34), 640 13.6 / 12.9 (42), 1279 23.0 / 21.7; top-2 of 6144, 640 8.9 / 8.9 (16), 800 10.2 / 9.8
-// (20), 1279 14.2 / 13.9; top-6 of 2048, 640 8.8 / 8.8 (16), 800 9.7 / 9.3 (20), 1279 13.5 / 12.0; top-4 of 2880, 640 8.2 / 9.0 (15), 800
-// 9.7 / 9.4 (18), 1279 12.7 / 12.1; below 16 MB the host's two launches, 6.5, are what a call waits for until the counting in
-// every block of the one launch does: top-2 of 512, 800 6.5 / 6.3, 2048 10.5 / 7.4, of 2048, 800 7.2 / 7.0, 2048 11.4 / 10.4.
+// 9.1 against 9.6 with one; with four 8 % slower when it was tried), one below that, where
+// more warps with less to do each finish sooner (93 tokens of 2880: 4.3 against 4.5; one token of 2048 3.8 either way).  Two
+// blocks per SM: with a third that does not fit beside them a second, nearly empty wave of
+// blocks starts after the first (headline 12.9).
+// Rows in host memory: 74 blocks fill the link, and more only get in each other's way (a call from pinned memory, 3.7 MB read and as
+// much written, by 37 / 74 / 148 / 296 blocks: 131.6 / 131 / 138.5 / 149 us).
+// Many tokens, or rows that outweigh a second launch: the routing of a group of one and then its rows (a2a_near.cuh).  Not captured,
+// us a call back to back, the one launch and the two (MB of expert rows): 40 MB: top-8 of 7168, 400 tokens 12.9 / 12.8 (46), 512
+// 15.7 / 15.3 (59), 1000 29.7 / 26.6, 2048 61.6 / 52.6; top-8 of 4096, 512 10.9 / 11.3 (34), 640 13.2 / 12.6 (42), 1279 22.2 / 20.7.
+// 800 tokens and 16 MB: top-2 of 6144, 640 9.0 / 8.9 (16), 800 10.3 / 10.0 (20); top-6 of 2048, 640 8.9 / 9.0 (16), 800 9.9 / 9.4 (20);
+// top-4 of 2880, 640 8.2 / 8.9 (15), 800 9.7 / 9.2 (18).  Below, the host's two launches, 6.5 to 7, are what a call waits for until the
+// counting in every block of the one launch does, 1280 tokens and 4 MB: top-2 of 512, 800 6.6 / 6.5 to 7.0 (2), 2048 10.5 / 7.5 (4);
+// of 2048, 800 7.3 / 7.0 (7), 2048 12.2 / 10.2 (17).
 bool solo_two_launches(const a2a_ctx* c) {
     const long long mb = (long long)c->cur_tokens * c->cfg.experts_per_token * c->cfg.hidden_dim * 2 >> 20;
     return mb >= 40 || (mb >= 16 && c->cur_tokens >= 800) || (mb >= 4 && c->cur_tokens >= 1280);
@@ -573,7 +581,8 @@ int launch_solo(a2a_ctx* c, cudaStream_t st, bool host_rows = false) {
     const size_t tk = (size_t)c->cur_tokens * c->cfg.experts_per_token * 4, rows = (size_t)c->cur_tokens * c->cfg.hidden_dim * 2;
     const bool over = !host_rows && tk > 0 && (overlap(c->p.y, rows, c->p.w, tk) || overlap(c->p.y, rows, c->p.idx, tk));
     if (over || (!host_rows && c->p.trace == nullptr && solo_two_launches(c))) {
-        NearParams<1> g = {{call_params(c)}, {c->p.x}, {c->p.pairs}, {c->cur_tokens}, /*n=*/1, /*every_rank=*/0, /*backwards=*/0, /*handed_on=*/1};
+        NearParams<1> g = {{call_params(c)}, {c->p.x},         {c->p.pairs},    {c->cur_tokens},
+                           /*n=*/1,          /*every_rank=*/0, /*backwards=*/0, /*handed_on=*/1};
         const int rc = launch_near_route(&c, g, st);
         return rc != A2A_OK ? rc : launch_near_rows(&c, g, /*push=*/false, /*whole=*/true, st);
     }
@@ -691,7 +700,8 @@ int expert_grid(const a2a_ctx* c, int n, int per_sm) {
     return g < ws ? ws : g;
 }
 
-int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st, NearGroup* call = nullptr) {
+int do_expert(a2a_ctx* const* cs, int n, bool wait, bool fanout, bool scale, bool publish, int grid, cudaStream_t st,
+              NearGroup* call = nullptr) {
     bool placed = true;
     for (int r = 0; r < n; ++r) {
         if (!cs[r]->sent) return A2A_ERR_STATE;
@@ -818,7 +828,7 @@ int do_pipe_rest(a2a_ctx* const* cs, int n, int role, cudaStream_t st, NearGroup
     if (n > 1 && !any_traced(cs, n)) {
         if (!near)
             // Begun rank by rank: one launch, in which each rank has its share of two blocks per SM.  Role 0 of eight ranks one by
-            // one and these two, 4 tokens of 2048 146 us (294 with a launch for each rank), 128 of 7168 222 (404).
+            // one and these two, 4 tokens of 2048 146 us a call (294 with a launch for each rank), 128 of 7168 222 (404).
             return launch_ranks(cs, n, select_pipe<PipeRole>(c, role), blocks / n, push_smem, st);
         NearGroup own, &g = near_call(cs, n, call, own);
         if (role == 1) {
@@ -1336,7 +1346,7 @@ int a2a_forward_host(a2a_ctx* c, const void* x, const int32_t* idx, const float*
     if (T > 0 && c->cfg.world_size == 1 && c->cfg.schedule == A2A_SCHEDULE_PIPELINED) {
         // One rank reads every row once and writes every output once: where the kernel can reach the caller's
         // memory it does so itself, and the link carries both directions at the same time instead of one copy
-        // after the other (256 tokens of 7168: 128 to 131 us a call, 192 with copies around the kernel).  The indices, which
+        // after the other (256 tokens of 7168: 128 to 131 us a call; 192 with copies around the kernel).  The indices, which
         // every block reads, are copied.
         void *dx, *dw, *dy;
         if (!overlap(y, row * T, x, row * T) && !overlap(y, row * T, w, tk) && !overlap(y, row * T, idx, tk) &&
@@ -1396,17 +1406,20 @@ int a2a_group_steps(a2a_ctx* const* group, const int32_t* phases, int num_phases
     call.n = 0;
     // The roles of a whole call: with nothing between them role 1 writes the outputs of a PULL combine too, and no launch
     // waits for flags of the one before it.
-    const bool roles = num_phases == 3 && phases[0] == A2A_GROUP_PIPE_SEND && phases[1] == A2A_GROUP_PIPE_EXPERT && phases[2] == A2A_GROUP_PIPE_COMBINE;
+    static const int32_t whole[] = {A2A_GROUP_PIPE_SEND, A2A_GROUP_PIPE_EXPERT, A2A_GROUP_PIPE_COMBINE};
+    const bool roles = num_phases == 3 && memcmp(phases, whole, sizeof(whole)) == 0;
     if (roles && n > 1 && calls != nullptr && c->cfg.schedule == A2A_SCHEDULE_PIPELINED && !any_traced(group, n) &&
         !outputs_over_rows(calls, n, (size_t)c->cfg.hidden_dim * 2)) {
         rc = do_pipe_send(group, n, calls, st, &call);
         for (; rc == A2A_OK && ++*done < 3;) rc = do_pipe_rest(group, n, *done, st, &call);
         return *done == 0 ? rc : end_steps(group, call, phases[*done - 1], rc, st);
     }
-    static const int32_t four[] = {A2A_GROUP_SEND, A2A_GROUP_RECV, A2A_GROUP_EXPERT, A2A_GROUP_COMBINE}, three[] = {A2A_GROUP_SEND, A2A_GROUP_RECV_EXPERT, A2A_GROUP_COMBINE};
+    static const int32_t four[] = {A2A_GROUP_SEND, A2A_GROUP_RECV, A2A_GROUP_EXPERT, A2A_GROUP_COMBINE};
+    static const int32_t three[] = {A2A_GROUP_SEND, A2A_GROUP_RECV_EXPERT, A2A_GROUP_COMBINE};
     const bool handed_on = near_phases(group, n) && ((num_phases == 4 && memcmp(phases, four, sizeof(four)) == 0) ||
                                                      (num_phases == 3 && memcmp(phases, three, sizeof(three)) == 0));
-    for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK) rc = group_phase(group, phases[*done], calls, st, handed_on ? &call : nullptr);
+    for (; rc == A2A_OK && *done < num_phases; *done += rc == A2A_OK)
+        rc = group_phase(group, phases[*done], calls, st, handed_on ? &call : nullptr);
     return *done == 0 ? rc : end_steps(group, call, phases[*done - 1], rc, st);
 }
 

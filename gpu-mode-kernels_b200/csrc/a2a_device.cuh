@@ -577,7 +577,7 @@ __device__ __forceinline__ void unpack8_e4m3(const uint2& q, float (&f)[8]) {
 // less than one, from which the second rounds correctly, r being the correctly rounded reciprocal (P. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  The remainder is exact where it does not underflow: the
 // caller sees to 2^-80 <= d <= 2^100, and rounds quotients below 2^-11 to zero whatever their last bits.  Zeros keep their sign.
-// Eight ranks, headline workload with FP8 rows, 66.3 -> 63.2 us a call; one rank 10.7 -> 10.3.
+// Captured, eight ranks, headline workload with FP8 rows, 58.0 us a call, 60.7 with a division each; one rank 10.2 / 10.5.
 __device__ __forceinline__ void divide8(float (&f)[8], float d) {
     const float r = 1.f / d;
     const float2 rr = make_float2(r, r), dd = make_float2(d, d);

@@ -10,7 +10,10 @@
 //     keep its own blocks busy while the others' are through.
 //   * every flag of the role before is up when a launch starts (it is awaited all the same, bounded, at gpu
 //     scope, unless the launch before it in the same call is that role).
-// One rank with many tokens is a group of one, and the phases of a group's call (of one rank: a2a_kernels.cuh) go by the same lists of pairs.
+// One rank with many tokens is a group of one, and the phases of a group's call (of one rank: a2a_kernels.cuh) go by the
+// same lists of pairs.
+// Times in this file and beside the launchers in a2a.cu are us a call, captured (calls one after the other in a graph, without
+// the host) unless something else is said.
 #pragma once
 
 #include "a2a_solo.cuh"
@@ -19,7 +22,7 @@ namespace a2a {
 
 // The ranks a launch serves (`n` of them, all of a group or one) and what role 0 knew or found of every rank.  N: the
 // most ranks a group may have; a type of its own for a single rank, whose launches are the cheaper for it (1500 tokens of 2880
-// in two launches 14.4 us with room for eight, 14.0 without).
+// 12.5 with room for eight, 11.9 without; 2048 of 7168 53.4 / 52.3).
 template <int N>
 struct NearParams {
     DevParams p[N];
@@ -38,7 +41,9 @@ using NearGroup = NearParams<A2A_MAX_WORLD>;
 // more for itself (64 KB at 2048 x 8, out of the L2) instead of waiting for another block.  What bounds it: the chain
 // launch -> indices -> counts -> slots -> stores.
 // ---------------------------------------------------------------------------
-__host__ __device__ inline size_t near_route_smem(int words, int E, int K) { return ((size_t)(words + 1) * E + (size_t)words * 64 * K) * 4; }
+__host__ __device__ inline size_t near_route_smem(int words, int E, int K) {
+    return ((size_t)(words + 1) * E + (size_t)words * 64 * K) * 4;
+}
 
 template <int N, int THREADS>
 __global__ void __launch_bounds__(THREADS) near_route_kernel(const __grid_constant__ NearParams<N> g, int words) {
@@ -127,22 +132,25 @@ __device__ __forceinline__ void raise_flags(const NearGroup& g, unsigned kinds, 
 //   PUSH: y[t] = T(sum over the ranks d holding experts of t, ascending, of float(T(sum over k at d of w[t,k] * float(row k)))),
 //         the order and the roundings of a group with a GPU each.
 //   PULL: y[t] = T(sum over k of w[t,k] * float(row k)).
-// WHOLE, for all ranks together, writes that.  Otherwise a combine follows: where outputs lie over rows that are still to be read, where a rank's
-// experts run by themselves, and where the expert rows are the caller's before a PULL combine; PUSH then writes the partial rows to the
-// home ranks' buffers.  (The two in one kernel: 80 registers and spills, headline 55.1 us a call against 54.0, FP8 62.3 / 58.4.)
+// WHOLE, for all ranks together, writes that.  Otherwise a combine follows: where outputs lie over rows that are still to be
+// read, where a rank's experts run by themselves, and where the expert rows are the caller's before a PULL combine; PUSH then
+// writes the partial rows to the home ranks' buffers.  (The two in one kernel: 2 % slower at the headline workload, 7 % with FP8 rows.)
 // What bounds it: the stores, K + 1 for each load; expert rows leave the L2 first, outputs, which the next layer reads, do not.
-// Eight ranks of 256 tokens of 7168, top-8 of 256 experts, a call: 54 us, 294 MB at 5.4 TB/s (134 with partial rows written
-// by one role, 87, and read by the next, 33; FP8 rows 58, 142; PULL, 200 tokens 44, 91); of 2048, top-6 of 64, skewed 17 (44).
-// Slower: rows stored without evict-first (two ranks of 200 tokens 17.2 us against 16.2, skewed 21.6 / 20.4, headline 1 %), four
-// vectors a lane at two blocks per SM (13 %), two at four (64 registers, spills: 49 %), pairs' rows looked up one by one (7 %).  One rank
-// of 2048 tokens of 7168 54.6, inputs loaded with evict-first too 53.8, but 1500 of 2880 12.9 / 14.1.  FP8: the quantiser's arithmetic on top.
+// Eight ranks of 256 tokens of 7168, top-8 of 256 experts: 54.3, 294 MB at 5.4 TB/s (with partial rows written by one role and
+// read by the next 134 a call, not captured); FP8 rows 58.0 (142), the quantiser's arithmetic on top; PULL, 200 tokens 44.0 (91);
+// of 2048, top-6 of 64, skewed 17.4 to 17.9 (44).
+// Rows stored without evict-first: skewed 18.8 for 17.9, two ranks of 200 tokens 15.2 / 14.4, one rank of 2048 53.0 / 52.3, headline
+// no difference.  Inputs loaded with it too: one rank of 2048 51.9, but 1500 of 2880 12.7 / 11.9, two ranks of 200 15.7 / 14.4.
+// Slower by more when they were tried: four vectors a lane at two blocks per SM (13 %), two at four (64 registers, spills: 49 %),
+// pairs' rows looked up one by one (7 %).
 // ---------------------------------------------------------------------------
 template <typename T, int PAYLOAD, bool PUSH, bool WHOLE, int U, int N>
 __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_constant__ NearParams<N> g) {
     begin_after_previous();
     __shared__ int s_here[A2A_MAX_WORLD];
     const DevParams& p0 = g.p[0];
-    const int tid = threadIdx.x, lane = tid & 31, ws = N == 1 ? 1 : p0.ws, K = p0.K, nvec = p0.H >> 3, nchunk = (nvec + 32 * U - 1) / (32 * U);
+    const int tid = threadIdx.x, lane = tid & 31, ws = N == 1 ? 1 : p0.ws, K = p0.K, nvec = p0.H >> 3;
+    const int nchunk = (nvec + 32 * U - 1) / (32 * U);
     const uint32_t want = flag_value(p0, 0);
     stamp(p0, kStampStart);
     if (!g.handed_on) {  // a rank's flag goes up when all its pairs are written, to whichever rank it is raised
@@ -166,11 +174,13 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
         int my_rank = pair.x == kNoPair ? -1 : (int)(pair.x >> 28);
         if (!WHOLE && g.n != ws && my_rank != p0.rank) my_rank = -1;
         unsigned long long my_row = 0;
-        if (my_rank >= 0)
-            my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[N == 1 ? 0 : my_rank] + p0.off_rows) + (size_t)(pair.x & kPairRow) * nvec);
-        if (PAYLOAD == A2A_PAYLOAD_FP8) {
+        if (my_rank >= 0) {
+            uint4* rows = reinterpret_cast<uint4*>(p0.peer[N == 1 ? 0 : my_rank] + p0.off_rows);
+            my_row = reinterpret_cast<unsigned long long>(rows + (size_t)(pair.x & kPairRow) * nvec);
+        }
+        if (PAYLOAD == A2A_PAYLOAD_FP8) {  // nvec % 16 == 0: a scale block's lanes are all in or all out
 #pragma unroll
-            for (int u = 0; u < U; ++u) q[u] = fp8_round_trip<T>(q[u], v0 + u * 32 < nvec);  // nvec % 16 == 0: a scale block's lanes are all in or all out
+            for (int u = 0; u < U; ++u) q[u] = fp8_round_trip<T>(q[u], v0 + u * 32 < nvec);
         }
         float acc[U][8];
 #pragma unroll
@@ -200,7 +210,8 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
 #pragma unroll
                     for (int e = 0; e < 8; ++e) part[u][e] = 0.f;
                 }
-                for (unsigned left = __ballot_sync(0xffffffffu, my_rank == d); left != 0u; left &= left - 1u) expert_row(__ffs(left) - 1, out, part);  // k ascending
+                for (unsigned left = __ballot_sync(0xffffffffu, my_rank == d); left != 0u; left &= left - 1u)  // k ascending
+                    expert_row(__ffs(left) - 1, out, part);
                 uint4* home = reinterpret_cast<uint4*>(p0.peer[s] + p0.off_ret) + ((size_t)d * p0.T_max + t) * nvec + v0;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
@@ -247,25 +258,31 @@ __global__ void __launch_bounds__(kThreads, 3) near_rows_kernel(const __grid_con
 
 // ---------------------------------------------------------------------------
 // Role 2 where role 1 has written the outputs, and RECV of rows that are in their slabs already.  In a call whose launches follow
-// one another it raises the flags that nobody has needed until then; otherwise it ends when those of the last kind are up.
+// one another it raises the flags that nobody has needed until then, also where such a call ends early; otherwise it ends when
+// those of the last kind are up.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(A2A_MAX_WORLD * A2A_MAX_WORLD) near_flags_kernel(const __grid_constant__ NearGroup g, int kinds) {
     // looked at while the launch before this one ends: no launch of a call that is handed on waits for anything, or records that it did
     const int recorded = recorded_of_rank(g);
     begin_after_previous();
-    const int ws = g.p[0].ws, i = threadIdx.x / ws, s = threadIdx.x % ws, kind = kinds >> kFlagExpert & 1 ? kFlagExpert : kFlagDispatch;
+    const int ws = g.p[0].ws, i = threadIdx.x / ws, s = threadIdx.x % ws;
+    const bool expert = kinds >> kFlagExpert & 1;
     stamp(g.p[0], kStampStart);
-    if (g.handed_on) raise_flags(g, (unsigned)kinds, recorded);
-    else if (i < g.n) wait_flag_gpu(await_ptr(g.p[i], kind, s), flag_value(g.p[i], 0), g.p[i], kind == kFlagExpert ? kPhaseCombine : kPhaseRecv, s);
+    if (g.handed_on)
+        raise_flags(g, (unsigned)kinds, recorded);
+    else if (i < g.n)
+        wait_flag_gpu(await_ptr(g.p[i], expert ? kFlagExpert : kFlagDispatch, s), flag_value(g.p[i], 0), g.p[i],
+                      expert ? kPhaseCombine : kPhaseRecv, s);
     stamp(g.p[0], kStampCombineDone);
 }
 
 // ---------------------------------------------------------------------------
-// The phases that a program with its own expert kernels calls, for all ranks of a group on one GPU: the same lists.  A token's place in
-// memory follows from its number and its pairs' places are looked up, so that no launch counts, scans or searches before its first row.
-// What bounds them: with tens of MB of rows the latencies (four ranks of 117 tokens of 4096, top-8, direct: SEND 9.7 us, RECV 3.0, EXPERT 8.8, COMBINE 7.1
-// by themselves, 25.7 together; 12.0, 2.9, 11.5, 8.6 and 33.3 by counts and bitmaps), with hundreds the memory (eight of 200 of 7168, 183 MB:
-// 40, 4, 54, 37 by themselves, 131 together; direct 141, and through the stages 33, 62, 68, 31 and 193).
+// The phases that a program with its own expert kernels calls, for all ranks of a group on one GPU: the same lists.  A token's
+// place in memory follows from its number and its pairs' places are looked up, so that no launch counts, scans or searches before
+// its first row.  What bounds them: with tens of MB of rows the latencies (four ranks of 117 tokens of 4096, top-8: SEND 9.7, RECV 3.0,
+// EXPERT 8.8, COMBINE 7.1 by themselves, 25.1 handed on from one to the next and 33.5 as four calls, in which tickets, flags and waits
+// are in every launch; by counts and bitmaps 33.3 handed on), with hundreds the memory (eight of 200 of 7168, 183 MB: 40, 4, 54, 37 by
+// themselves, 130 handed on, 151 as four calls; through the stages 193 handed on).
 // ---------------------------------------------------------------------------
 // A warp's item in a launch whose blocks take no second one: U vectors a lane, from v0 on, of token t of rank s.
 template <int U>
@@ -303,11 +320,14 @@ __device__ __forceinline__ unsigned long long near_row(const NearGroup& g, int s
     }
     rank = place == kNoPair ? -1 : (int)(place >> 28);
     if (rank < 0) return 0;
-    return reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p0.peer[rank] + p0.off_rows) + (size_t)(place & kPairRow) * (p0.H >> 3));
+    uint4* rows = reinterpret_cast<uint4*>(p0.peer[rank] + p0.off_rows);
+    return reinterpret_cast<unsigned long long>(rows + (size_t)(place & kPairRow) * (p0.H >> 3));
 }
 
-// SEND: routing and sending in one launch.  A block takes a contiguous range of a rank's (token, chunk) items, as solo_kernel does.  Whatever
-// the payload, a row, read once (and FP8, quantised and dequantised once), goes straight into the slabs: a stage is what a link needs.
+// SEND: routing and sending in one launch.  A block takes a contiguous range of a rank's (token, chunk) items, as solo_kernel does,
+// and resolves the pairs of a round by the same loop; it stands in both (a2a_solo.cuh), since as a function it cost solo_kernel
+// 0.17 us.  Whatever the payload, a row, read once (and FP8, quantised and dequantised once), goes straight into the slabs: a stage
+// is what a link needs.
 template <typename T, bool FP8, int U>
 __global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid_constant__ NearGroup g) {
     __shared__ int s_cnt[A2A_MAX_EXPERTS];                  // tokens before the current round that use expert e
@@ -375,11 +395,13 @@ __global__ void __launch_bounds__(kThreads, 3) near_dispatch_kernel(const __grid
             const int v0 = c * 32 * U + lane;
             const unsigned place = lane < K ? s_place[(t - r0) * K + lane] : kNoPair;
             unsigned long long my_row = 0;
-            if (place != kNoPair)
-                my_row = reinterpret_cast<unsigned long long>(reinterpret_cast<uint4*>(p.peer[place >> 28] + p.off_rows) + (size_t)(place & kPairRow) * nvec);
-            if (FP8) {
+            if (place != kNoPair) {
+                uint4* rows = reinterpret_cast<uint4*>(p.peer[place >> 28] + p.off_rows);
+                my_row = reinterpret_cast<unsigned long long>(rows + (size_t)(place & kPairRow) * nvec);
+            }
+            if (FP8) {  // nvec % 16 == 0: a scale block's lanes are all in or all out
 #pragma unroll
-                for (int u = 0; u < U; ++u) q[u] = fp8_round_trip<T>(q[u], v0 + u * 32 < nvec);  // nvec % 16 == 0: a scale block's lanes are all in or all out
+                for (int u = 0; u < U; ++u) q[u] = fp8_round_trip<T>(q[u], v0 + u * 32 < nvec);
             }
             for (unsigned left = __ballot_sync(0xffffffffu, place != kNoPair); left != 0u; left &= left - 1u) {
                 uint4* row = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, my_row, __ffs(left) - 1)) + v0;
@@ -419,7 +441,8 @@ __global__ void __launch_bounds__(kThreads) near_expert_kernel(const __grid_cons
         __syncthreads();
         if (tid < g.n * ws) {
             const DevParams& p = g.p[tid / ws];
-            if (!wait_flag_gpu(await_ptr(p, kFlagDispatch, tid % ws), flag_value(p, 0), p, kPhaseRecv, tid % ws)) atomicOr(&s_missing, 1 << tid % ws);
+            if (!wait_flag_gpu(await_ptr(p, kFlagDispatch, tid % ws), flag_value(p, 0), p, kPhaseRecv, tid % ws))
+                atomicOr(&s_missing, 1 << tid % ws);
         }
         __syncthreads();
     }
@@ -516,7 +539,8 @@ __global__ void __launch_bounds__(kThreads) near_combine_kernel(const __grid_con
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 if ((mine >> (k0 + i) & 1u) == 0u) continue;  // K <= 32: no bit beyond the last pair's
-                const uint4* row = PUSH ? ret + (size_t)i * p0.T_max * nvec : reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
+                const uint4* row = PUSH ? ret + (size_t)i * p0.T_max * nvec
+                                        : reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_row, k0 + i)) + at.v0;
 #pragma unroll
                 for (int u = 0; u < U; ++u)
                     if (at.v0 + u * 32 < nvec) q[i][u] = __ldcs(row + u * 32);

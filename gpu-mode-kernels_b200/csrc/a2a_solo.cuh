@@ -1,5 +1,7 @@
 // World size 1: the whole forward of a pipelined context as ONE ordinary launch whose blocks know
-// nothing of each other.  With a single rank nothing travels, so nothing has to be handed over: a
+// nothing of each other: calls of few tokens and few rows (solo_two_launches in a2a.cu), traced calls, and rows in host
+// memory.  Larger calls, and outputs over the weights or the indices, take the routing and the rows of a2a_near.cuh.
+// With a single rank nothing travels, so nothing has to be handed over: a
 // block that owns a contiguous range of (token, chunk) items works out the slots of its own tokens
 // from the caller's indices alone and then does everything for them -- the slab rows with the
 // placeholder expert op applied, the (token, k) words, the slot table and the weighted sum.
@@ -32,7 +34,8 @@ __device__ __forceinline__ void load_indices(const int* row, int k0, int K, bool
 
 // Counts of the experts used by tokens [0, t_end) into s_cnt (shared, cleared by the caller).  A
 // repeat inside a token counts once, an index out of range not at all.  N tokens' indices are requested together, in 16-byte vectors
-// where they lie so: one rank, 256 tokens of 7168, top-8 9.3 -> 9.0 us a call, 2048 53.8 -> 52.1 (one token at a time there 52.5).
+// where they lie so: captured, one rank, 256 tokens of 7168, top-8 9.1 us a call, index by index 9.3; 2048 52.3 / 53.7, and with one
+// token at a time 52.8.
 template <int THREADS, int N = 1>
 __device__ __forceinline__ void count_experts_before(const DevParams& p, int t_end, int* s_cnt) {
     const int K = p.K;
@@ -85,10 +88,10 @@ __device__ __forceinline__ void load_own_chunk(const DevParams& p, int t, int v0
 // launch -> indices -> slots -> stores.  Blocks take contiguous items so that each resolves the pairs
 // of the few tokens it touches once; the indices of the tokens before them (64 KB at 2048 x 8, out of
 // L2) are counted again by every block, 1 to 3 us that the first row's load hides in part and that no
-// exchange between blocks would undercut.  Measured back to back, this kernel against the role-split
-// kernel that handed slots, flags and rows from block to block: 4.1 / 11.9 us (one token of 2048, top-6),
-// 4.5 / 11.7 us (93 tokens of 2880, top-4), 9.4 / 18.7 us (256 tokens of 7168, top-8: 3.9 TB/s, in L2),
-// 61 / 270 us (2048 tokens of 7168, formerly the phase-by-phase kernel: 4.8 TB/s of 6.55 copied).
+// exchange between blocks would undercut.  Captured, and the role-split kernel that handed slots, flags and rows from block to
+// block (a call): 3.7 / 11.9 us (one token of 2048, top-6), 4.2 / 11.7 (93 tokens of 2880, top-4), 9.1 / 18.7 (256 tokens of
+// 7168, top-8: 4.0 TB/s into the L2, what a plain fill of the same 33 MB takes); 2048 tokens of 7168, traced, 60.7, in two launches 52.3.
+// The loop that resolves a round's pairs stands in near_dispatch_kernel (a2a_near.cuh) too: as a function it cost this kernel 0.17 us.
 template <typename T, int PAYLOAD, int U>
 __global__ void __launch_bounds__(kThreads) solo_kernel(const __grid_constant__ DevParams p) {
     __shared__ int s_cnt[A2A_MAX_EXPERTS];                 // tokens before the current round that use expert e

@@ -29,10 +29,13 @@ constexpr int kUnroll = 4;
 constexpr int kBins = 256;
 constexpr int kCluster = 8;
 // One cluster writes the counts itself: no zeroing in front, one launch, which gets ready while the launch before it ends.
-// Calls back to back, 30 KB 2.7 us (5.2 without the overlap, and with 32 KB a block one of eight at work), 256 KB 3.3 (6.2). Above, the
-// host needs 5 us for zero + count, 300 KB 5.2 to one cluster's 4.0, but the GPU 2.6 to 3.6, which is what a captured call takes.
+// Calls back to back, 30 KB 2.8 us, captured 2.3 (5.2 without the overlap, and with 32 KB a block one of eight at work), 256 KB 4.0,
+// captured 2.6.  Above, the host needs 5.2 us for zero + count where one cluster of 300 KB took 4.0, but the GPU 2.5 to 3.6, which is
+// what a captured call takes: the line favours captured calls, and plain ones from 256 to about 500 KB pay a quarter for it.
 constexpr size_t kClusterBytes = 256 * 1024;
-// Up to half a row of 8 KB for a block per SM, rows a grid apart: 300 KB 2.6 us on the GPU, 3.3 with 32 KB a block; 2 MB 3.6 / 3.1.
+// Up to here (592 KB with 148 SMs) every block has the one row of 8 KB that its grid of n / 8 KB blocks leaves it: captured, 300 KB
+// 2.5 us, 3.3 with 32 KB a block.  From here on 32 KB a block, on a grid of as many blocks as there are rows of 8 KB, one per SM at most:
+// up to 4.8 MB some find no data (56 of 75 just above, 84 of 148 at 2 MB) and add nothing.  2 MB 3.0 us, 3.6 with rows a grid apart.
 constexpr size_t kSpreadBytesPerSm = 4 * 1024;
 // Below this a block per SM: 256 sums per block meet at 256 global words, and with few bytes per block
 // that is what the call waits for.  10 MB 4.5 us on the GPU, 20 MB 6.2, 31 MB 7.9; with two blocks from 16 MB on 6.4 and 8.2.
@@ -63,7 +66,7 @@ __device__ __forceinline__ void load_vectors(const uint4* vec, size_t i, size_t 
 }
 
 // The grid is one cluster and stores the counts; or its blocks add theirs to `out`, which the launch before this one zeroes while
-// they already count: with no more than a round of data (kSpread) or with more.
+// they already count: with one row of data a block (kSpread) or with more (kRounds).
 enum Form { kCluster8, kSpread, kRounds };
 
 template <Form FORM>
@@ -80,7 +83,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) histogram256_kernel(co
     const size_t nvec = (n - head) / 16;
     const uint4* vec = reinterpret_cast<const uint4*>(data + head);
     // A block takes kUnroll rows of 8 KB at a time: one after the other, 32 KB of the memory's pages (512 MB 88 us, 97 with a row from
-    // each of four places), or, where there is no more than a round, rows a grid apart, so that every block has some.
+    // each of four places), or, in the smallest grids, rows a grid apart, so that every block has one.
     constexpr bool cluster = FORM == kCluster8, apart = FORM != kRounds;
     const size_t row = apart ? (size_t)gridDim.x * kThreads : kThreads, step = (size_t)gridDim.x * kThreads * kUnroll;
     size_t i = (size_t)blockIdx.x * kThreads * (apart ? 1 : kUnroll) + tid;
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) histogram256_kernel(co
 }
 
 // Gets ready while the launch before it ends, and starts the counting launch as soon as that has completed: the data is there then, and
-// only the adding to `out` waits for the zeros (10 MB 7.0 -> 5.2 us a call, 512 MB 87.6 -> 85.9).
+// only the adding to `out` waits for the zeros (10 MB 7.0 -> 5.2 us a call then, 512 MB in bursts 87.6 -> 85.9).
 __global__ void __launch_bounds__(kBins) zero_counts_kernel(unsigned long long* out) {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
@@ -181,6 +184,7 @@ extern "C" int a2a_histogram256(const uint8_t* data, size_t n, int64_t* out, voi
     const size_t want = (n / 16 + kThreads - 1) / kThreads;
     const size_t room = (size_t)sms * (n < kFullBytes ? 1 : kBlocksPerSm);
     launch.gridDim = dim3((unsigned)(want < room ? want : room));
-    e = cudaLaunchKernelEx(&launch, n <= (size_t)sms * kSpreadBytesPerSm ? histogram256_kernel<kSpread> : histogram256_kernel<kRounds>, data, n, counts);
+    const auto kernel = n <= (size_t)sms * kSpreadBytesPerSm ? histogram256_kernel<kSpread> : histogram256_kernel<kRounds>;
+    e = cudaLaunchKernelEx(&launch, kernel, data, n, counts);
     return e == cudaSuccess ? A2A_OK : -(int)e;
 }

@@ -24,7 +24,8 @@ def histogram256(data: torch.Tensor, output: torch.Tensor) -> torch.Tensor:
         return out if type(out) is not int else _lib.check(out)
     # something is wrong, or unusual: look again, one thing at a time
     if data.dtype is not torch.uint8 or not data.is_cuda or not data.is_contiguous() or data.dim() != 1:
-        raise _lib.A2AError(_lib.A2A_ERR_CONFIG, f"data must be a contiguous 1-D uint8 CUDA tensor, got {data.dtype} {tuple(data.shape)} on {data.device}")
+        raise _lib.A2AError(_lib.A2A_ERR_CONFIG, "data must be a contiguous 1-D uint8 CUDA tensor, got "
+                            f"{data.dtype} {tuple(data.shape)} on {data.device}")
     device = data.get_device()
     if (output.dtype is not torch.int64 or output.numel() != NUM_BINS or not output.is_contiguous()
             or not output.is_cuda or output.get_device() != device):

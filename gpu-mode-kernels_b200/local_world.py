@@ -6,10 +6,12 @@ rank, the sending phase before any waiting one, on one stream, and each wait fin
 flag already set.  Routing, rows, flag values and epochs are those of a group
 with a GPU per rank; what depends on where a peer is, is not: flags are awaited at gpu
 scope without watchers, rows are read where they lie and written where they belong instead of being sent to a
-stage, and a token's output is added up where its expert rows are written (csrc/a2a_near.cuh).  The forms for distant peers run in ``forward_one_launch``, which puts every rank's blocks into one cooperative
+stage, and a token's output is added up where its expert rows are written (csrc/a2a_near.cuh).  The forms for
+distant peers run in ``forward_one_launch``, which puts every rank's blocks into one cooperative
 launch, and in the phases called context by context.
 Validation tool: parity tests and the smoke check use it to cover world sizes
-2, 4 and 8 on a single device.
+2, 4 and 8 on a single device.  What it takes is the time of ranks that share a GPU, by kernels for near peers; it
+says nothing of a group with a GPU per rank, which runs the one-launch kernel (csrc/a2a_pipe.cuh) over links.
 """
 from __future__ import annotations
 
@@ -82,7 +84,8 @@ class LocalWorld:
         self._step("recv")
 
     def forward_phases(self, rank_datas: Sequence) -> List[torch.Tensor]:
-        """The four public phases, one after the other."""
+        """The four public phases, one after the other and handed on from one to the next: a program with expert kernels of its
+        own calls them one by one, in which each launch also raises and awaits flags."""
         ys = self._quick(rank_datas, _PHASES, False)
         if ys is not None:
             return ys
@@ -100,7 +103,7 @@ class LocalWorld:
         return self._combine(rank_datas)
 
     def forward_pipelined(self, rank_datas: Sequence) -> List[torch.Tensor]:
-        """The roles of the pipelined one-launch kernel as three launches, in lock-step:
+        """The roles of the pipelined one-launch kernel as three launches, in lock-step and in the forms of ranks on one GPU:
         every rank's routers, then every rank's expert blocks, then every rank's combine.  Nothing of the caller's
         runs in between, so the second writes the outputs too where they do not lie over inputs (csrc/a2a_near.cuh)."""
         ys = self._quick(rank_datas, _ROLES, True)

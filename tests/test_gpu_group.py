@@ -201,7 +201,7 @@ def test_a_call_goes_on_in_the_form_it_was_begun_in(payload, combine, together):
         world.close()
 
 
-@pytest.mark.parametrize("T", [8, 130])  # 1 MB of expert rows, and 18: the combine of many rows is another kernel
+@pytest.mark.parametrize("T", [8, 130])  # 1 MB of expert rows, and 18
 def test_a_rank_without_rows_need_not_run_its_expert_phase(T):
     """Phases called rank by rank by a program that steps only the ranks with rows; the combine for all ranks together."""
     ws, E, K, H = 4, 16, 4, 4096
