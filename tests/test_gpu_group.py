@@ -414,3 +414,23 @@ def test_phases_go_on_after_a_refused_combine(names, payload):
         world.check()
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("payload", ["dedup", "fp8"])
+@pytest.mark.parametrize("E,K,H,T,ws", [(12, 3, 640, 33, 3), (16, 8, 2944, 70, 2)])
+def test_a_combine_of_all_ranks_finds_rows_by_their_slots(payload, E, K, H, T, ws):
+    """After calls that leave no list of places, the one launch and the roles rank by rank: the bits of the PULL combine, dropped
+    pairs among them."""
+    rds = [pkg.generate_input(E, K, H, T, seed=11, rank=r, world_size=ws)[1].to(DEV) for r in range(ws)]
+    rds[0].indices[3, :] = rds[0].indices[3, 0]
+    rds[0].indices[T - 1, :] = E
+    world = LocalWorld(pkg.MoEConfig(E, K, H, T), ws, payload=payload, schedule="pipelined", combine="pull")
+    try:
+        for run in (lambda: world.forward_one_launch(rds), lambda: rank_by_rank(world, rds), lambda: world.forward_pipelined(rds)):
+            want = [bits(y) for y in run()]
+            for c, rd in zip(world.ctxs, rds):
+                c._num_tokens = T
+            assert all(torch.equal(bits(y), w) for y, w in zip(world._combine(rds), want))
+        assert [c.peek() for c in world.ctxs] == [_lib.A2A_ERR_ROUTING] + [0] * (ws - 1)
+    finally:
+        world.close()
